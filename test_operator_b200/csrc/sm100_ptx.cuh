@@ -33,6 +33,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in exactly one lane of a converged warp.  A branch on this (not on lane == 0) is how the compiler learns that a
+// single thread runs the block: the operands of tcgen05.mma / commit live in uniform registers, and behind a lane
+// comparison every one of those instructions is wrapped in a loop over the lanes (measured with a standalone probe: 94 -
+// 102 cycles per UMMA issued behind lane == 0 whatever its size, the tensor pipe's own 43 - 64 behind elect.sync).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---- mbarrier ----------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 }
 
 // =============================================================================================
-// recompute: persistent 2-CTA clusters, 19 warps per CTA; cluster c works on queries c, c + #clusters, ...
+// recompute: persistent 2-CTA clusters, 18 warps per CTA; cluster c works on queries c, c + #clusters, ...
 // The pair works on 256-key tiles with cta_group::2 UMMAs of shape M = 256 keys x N = 2*HP:
 //   A  each CTA gathers ITS 128 keys of the tile (every kv row is fetched once per query, not once
 //      per head group), chunk by chunk through a 5-slot ring of [128 keys x 64 col] chunks;
@@ -159,19 +159,18 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 //      ordered (head half 0: P, dP), (head half 1: P, dP); two buffers.
 //   warps 0-7   softmax-gradient on the CTA's own keys: warp w -> TMEM lane quarter w % 4, head half w / 4
 //   warps 8-15  gather producers (cp.async 16 B, swizzled); completion arrives on the slot's mbarrier
-//   warps 16,17 even CTA: the two UMMA issuers for the pair, taking alternate chunks.  A thread that issues a
-//               tcgen05.mma is held until the tensor pipe takes it, and whatever else it executes (barrier
-//               polls, commits) is time the pipe idles; with two threads handing over through a counter, one
-//               waits for its next chunk and commits while the other's UMMAs run.
-//               odd CTA: warp 16 forwards "my slot is full" to the even CTA (cp.async cannot signal remotely)
-//   warp 18     TMA of the CTA's Q / dO chunks, one barrier per column chunk
+//   warp 16     even CTA: the UMMA issuer for the pair, one elected thread (behind elect_one its UMMAs enter at the
+//               pipe's rate; two threads taking alternate chunks were needed only while a lane comparison guarded them:
+//               4096 queries x 128 heads x 2048 keys 2.02 -> 1.93 ms, 64 heads 1.40 -> 1.08 ms)
+//               odd CTA: forwards "my slot is full" to the even CTA (cp.async cannot signal remotely)
+//   warp 17     TMA of the CTA's Q / dO chunks, one barrier per column chunk
 // Slot-free, chunk-free and accumulator-ready signals are tcgen05.commit arrivals delivered to both CTAs.
 // Nothing is drained between queries: the ring, the two accumulator buffers and the counters behind their
 // barrier phases run on, the Q / dO chunk j of the next query is fetched as soon as the last tile's UMMAs
 // on chunk j have finished, and the softmax of a query's last tile overlaps the next query's first UMMAs.
 // =============================================================================================
 namespace rp {
-constexpr int kThreads = 608;
+constexpr int kThreads = 576;
 constexpr int kProducerThreads = 256;
 constexpr int kTileKeys = 256;             // per pair; 128 per CTA
 constexpr int kChunkA = 128 * 128;         // 16 KB gathered chunk
@@ -200,7 +199,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1;
     const int n_pairs = gridDim.x >> 1;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
 
     extern __shared__ uint8_t smem_raw[];
@@ -218,14 +217,12 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     const uint32_t bar_tempty = bar_tfull + 16;             // [2] (even CTA) both CTAs have read the buffer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 1024 + 8 * (2 * kStages + 2 * kQChunks + 4));
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const uint32_t tok = smem_u32(tmem_slot + 2);           // (even CTA) chunks issued so far, the issuers' hand-over
-    const uint32_t bar_drain = smem_u32(tmem_slot + 4);     // [2] one per issuer, used only while winding down after an abort
-    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 16 + 16 <= 512, "barrier area");
+    const uint32_t bar_drain = smem_u32(tmem_slot + 2);     // used only while winding down after an abort
+    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 16 <= 512, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
         *s_abort = 0;
-        tmem_slot[2] = 0;
         for (int i = 0; i < kStages; ++i) {
             // the even CTA's "full" also counts one arrival forwarded from the odd CTA
             mbar_init(bar_full + 8 * i, kProducerThreads + (rank == 0 ? 1 : 0));
@@ -238,8 +235,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         for (int i = 0; i < 2; ++i) {
             mbar_init(bar_tfull + 8 * i, 1);
             mbar_init(bar_tempty + 8 * i, 16);   // 8 softmax warps in each CTA
-            mbar_init(bar_drain + 8 * i, 1);
         }
+        mbar_init(bar_drain, 1);
         fence_mbar_init();
     }
     {   // zero block standing in for the dO half of column chunk 8 (never overwritten)
@@ -317,7 +314,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 }
             }
         }
-    } else if (warp == 18) {
+    } else if (warp == 17) {
         // ------------------------------------------------------------------ Q / dO chunks of this CTA's heads
         if (lane == 0) {
             tma_prefetch_desc(&tm_q);
@@ -337,10 +334,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 }
             }
         }
-    } else if (warp == 16 || warp == 17) {
-        if (lane == 0) {
+    } else if (warp == 16) {
+        if (elect_one()) {
             if (rank == 1) {
-                if (warp == 16) {
                 // -------------------------------------------------------------- forward slot-full to the even CTA
                 int s = 0;
                 uint32_t ph = 0, qpar = 0;
@@ -362,64 +358,44 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                         }
                     }
                 }
-                }
             } else {
-                // -------------------------------------------------------------- UMMA issuers for the pair
-                // Issuer x takes the chunks whose running number is x mod 2.  For a chunk it waits until the data is
-                // there, then until the other issuer has issued the chunk before (a counter in shared memory: the
-                // UMMAs enter the pipe in chunk order, so every accumulator is summed in one fixed order and the
-                // results are reproducible bit for bit), issues 4 UMMAs (512 cycles of math on both SMs), bumps the
-                // counter and commits.  The UMMAs of one accumulator form a dependency chain, so the commit behind a
-                // tile's last chunk covers the whole tile.
-                const int x = warp - 16;
+                // -------------------------------------------------------------- UMMA issuer for the pair
+                // One thread issues everything, so the UMMAs of an accumulator enter the pipe in chunk order and the
+                // results are reproducible bit for bit.
                 constexpr uint32_t idesc = make_idesc_bf16(256, C::kAccCols, 0, 0);
                 const uint64_t desc_hi = make_smem_desc(0, 16, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
                 const uint32_t desc_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
                 const uint32_t a_lo0 = desc_lo + ((s_base + C::kOffRing) >> 4);
                 const uint32_t b_lo0 = desc_lo + ((s_base + C::kOffB) >> 4);
-                const int n_queries = (nq - pair + n_pairs - 1) / n_pairs;
-                const int total = n_queries * n_tiles * kQChunks;
-                int j = x, tile = 0, gt = 0;    // running chunk `it` = column chunk j of tile `tile` of a query; gt counts tiles
-                uint32_t qpar = 0;
-                int s = x % kStages;
-                uint32_t ph = 0;
-                for (int it = x; it < total; it += 2) {
-                    const int b = gt & 1;
-                    if (j == 0) mbar_spin(bar_tempty + 8 * b, ((gt >> 1) & 1) ^ 1, wc, kErrRecompute + 13);
-                    if (tile == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 12);
-                    mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 14);
-                    flag_wait(tok, static_cast<uint32_t>(it), wc, kErrRecompute + 19);
-                    tc_fence_after_sync();
-                    const uint32_t d = tmem + b * C::kAccCols;
-                    const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
-                    const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
-                    umma_ss_2cta(d, desc_hi | a_lo, desc_hi | b_lo, idesc, j != 0);
+                int s = 0, gt = 0;              // ring slot; tiles so far
+                uint32_t ph = 0, qpar = 0;
+                for (int ql = pair; ql < nq; ql += n_pairs, qpar ^= 1) {
+                    for (int tile = 0; tile < n_tiles; ++tile, ++gt) {
+                        const int b = gt & 1;
+                        mbar_spin(bar_tempty + 8 * b, ((gt >> 1) & 1) ^ 1, wc, kErrRecompute + 13);
+                        const uint32_t d = tmem + b * C::kAccCols;
+                        for (int j = 0; j < kQChunks; ++j) {
+                            if (tile == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 12);
+                            mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 14);
+                            tc_fence_after_sync();
+                            const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
+                            const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
 #pragma unroll
-                    for (int kk = 1; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
-                        umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, 1);
-                    tc_fence_before_sync();
-                    flag_store(tok, static_cast<uint32_t>(it + 1));
-                    umma_commit_2cta_mask(bar_empty + 8 * s, 3);
-                    if (tile == n_tiles - 1) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);   // the next query's chunk may come in
-                    if (j == kQChunks - 1) umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
-                    j += 2;
-                    if (j >= kQChunks) {
-                        j -= kQChunks;
-                        ++gt;
-                        if (++tile == n_tiles) {
-                            tile = 0;
-                            qpar ^= 1;
+                            for (int kk = 0; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
+                                umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, (j | kk) != 0);
+                            umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                            if (tile == n_tiles - 1) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);   // the next query's chunk may come in
+                            if (++s == kStages) {
+                                s = 0;
+                                ph ^= 1;
+                            }
                         }
-                    }
-                    s += 2;
-                    if (s >= kStages) {
-                        s -= kStages;
-                        ph ^= 1;
+                        umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
                     }
                 }
                 if (*s_abort) {   // winding down: nothing of this thread's may still be in the tensor pipe at dealloc
-                    umma_commit_2cta_mask(bar_drain + 8 * x, 1);
-                    mbar_wait_drain(bar_drain + 8 * x, 0, p.wait_limit);
+                    umma_commit_2cta_mask(bar_drain, 1);
+                    mbar_wait_drain(bar_drain, 0, p.wait_limit);
                 }
             }
         }
@@ -540,10 +516,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // its own matter: a producer group that fills a slot has then itself seen the slot's previous use, so its wait on the
 // phase parity of "slot free" cannot be satisfied by the phase before last (with one ring shared by the two groups a
 // group that ran ahead of the other overwrote a slot in use and arrived twice on one barrier phase).
-// A thread that issues UMMAs executes everything slowly (cycle counters: ~450 cycles for the four UMMAs of a chunk,
-// ~270 for its commits, ~230 for advancing a handful of counters, against 256 cycles of tensor-pipe time), so a stream
-// is shared by two issuers that take alternate chunks and hand over through a counter in shared memory: the UMMAs of an
-// accumulator enter the pipe in chunk order and the result is reproducible bit for bit.
+// A stream is shared by two issuers that take alternate chunks (one polls and commits while the other's UMMAs run) and
+// hand over through a counter in shared memory: the UMMAs of an accumulator enter the pipe in chunk order and the result
+// is reproducible bit for bit.
 // Slot-free, chunk-free and accumulator-ready signals are tcgen05.commit arrivals delivered to both CTAs.
 // kMode 1: row maxima only (atomicMax per head at the end of a query); kMode 2: E = exp2(logit - max) as bf16 into the
 // scratch (the backward's S layout) and the row sums in 2^-22 fixed point.
@@ -585,7 +560,7 @@ smla_fwd_logits_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const KPar
     const uint32_t rank = cluster_ctarank();
     const int cta = blockIdx.x >> 1;         // the pair
     const int n_ctas = gridDim.x >> 1;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
 
     extern __shared__ uint8_t smem_raw[];
@@ -713,8 +688,8 @@ smla_fwd_logits_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const KPar
             }
         }
     } else if (warp >= kIssuerWarp && warp < kIssuerWarp + kIssuers) {
-        if (lane == 0 && rank == 1) {
-            if (warp == kIssuerWarp) {
+        if (rank == 1) {
+            if (warp == kIssuerWarp && elect_one()) {
                 // -------------------------------------------------------------- forward slot-full to the even CTA
                 int rs[2] = {0, 0};
                 uint32_t ph[2] = {0, 0}, qpar = 0;
@@ -741,7 +716,7 @@ smla_fwd_logits_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const KPar
                     }
                 }
             }
-        } else if (lane == 0) {
+        } else if (elect_one()) {
             // ------------------------------------------------------------------ UMMA issuers for the pair
             // Issuer i takes the ring positions i, i + kIssuers, ...: chunks y, y + kIssuersPerStream, ... (y = i / 2) of
             // stream x = i % 2, the tiles 2t + x, accumulated into buffer 2 * (pair parity) + x.
@@ -988,7 +963,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int pair = blockIdx.x >> 1;
     const int n_pairs = gridDim.x >> 1;
     const int nq = p.nq;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
 
     extern __shared__ uint8_t smem_raw[];
@@ -1071,7 +1046,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             if (rank == 1) {
                 // -------------------------------------------------------------- relay "landed" to the even CTA
                 // TMA wrote the data (async proxy) and the tensor core reads it (async proxy): no proxy fence; the
@@ -1356,7 +1331,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     const int part = blockIdx.x % kParts;
     const int ql = blockIdx.x / kParts;
     const int qg = p.q0 + ql;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
     // d-part i gathers kv column chunks [i kSplit, (i + 1) kSplit): 3 x 3 of 9 for dQ, 2 x 4 of 8 for o = S.V
     const int chunk0 = part * kSplit;
@@ -1456,7 +1431,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
             }
         }
     } else if (warp == 12) {
-        if (lane == 0) {
+        if (elect_one()) {
             // N = the part's column chunks (up to 256 d) in one UMMA
             const uint32_t idesc1 = make_idesc_bf16(128, n_ch * 64, 1, 1);
             // A = dS^T: [HP/8 head blocks][64 keys][8 heads], 8-key groups 128 B apart, head blocks 1 KB apart.
