@@ -67,6 +67,14 @@ typedef struct smla_bwd_params {
     const int32_t* query_meta;
 } smla_bwd_params;
 
+/* Fills the table `query_meta` points to for sequences packed along the query dimension: sequence i owns the query rows
+ * [q_start[i], q_start[i + 1]) (the last one ends at q_end) and the kv rows [kv_start[i], kv_start[i] + kv_len[i]); a
+ * query's position is q_start_index_s + its row inside the sequence; slots in use: topk, or topk_length[row] clamped to
+ * [0, topk] where that device array is given.  The sequence arrays are host memory and are read before the call
+ * returns; the table is written by a kernel on `stream`, so nothing is copied and nothing waits. */
+int smla_query_meta(int32_t* meta, int32_t n_seq, const int32_t* q_start, const int32_t* kv_start, const int32_t* kv_len,
+                    int32_t q_end, int32_t q_start_index_s, int32_t topk, const int32_t* topk_length, void* stream);
+
 /* Workspace (device memory) needed for `p`, never more than about `budget_bytes` when that is
  * non-zero (the query dimension is then processed in several passes).  0 on bad arguments. */
 size_t smla_bwd_workspace_size(const smla_bwd_params* p, size_t budget_bytes);

@@ -170,6 +170,13 @@ __device__ __forceinline__ void tc_fence_after_sync() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------------
+// A kernel launched with the programmatic-serialization attribute may start while its predecessor in the stream still
+// runs: pdl_wait() returns once every grid it depends on has completed and its writes are visible (at once when the
+// kernel was launched without the attribute); pdl_trigger() lets the stream's next such kernel start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- L2 eviction policies ------------------------------------------------------------------------
 // kv rows are re-read by every query and should stay in L2; scratch and per-query operands stream through.
 __device__ __forceinline__ uint64_t l2_policy_evict_last() {
@@ -252,6 +259,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
            (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46) |
            (static_cast<uint64_t>(swizzle) << 61);
 }
+// The address field alone, to be added to a descriptor made with address 0 (in a CTA of rank > 0 of a cluster the 32-bit
+// shared-memory address carries the rank above the 18 bits that belong in the descriptor).
+__device__ __forceinline__ uint32_t desc_addr(uint32_t saddr) { return (saddr & 0x3FFFFu) >> 4; }
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulation.
 // a_mn / b_mn: 0 = operand is K-major in shared memory, 1 = MN-major.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int a_mn, int b_mn) {
@@ -298,6 +308,20 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
+}
+__device__ __forceinline__ uint32_t cluster_nctas() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+// 16 bytes of another CTA's shared memory (address from map_to_cta)
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(cluster_addr)
+                 : "memory");
+    return v;
 }
 // All threads of both CTAs: arrive + wait on the hardware cluster barrier.
 __device__ __forceinline__ void cluster_sync_all() {

@@ -3,6 +3,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <climits>
 #include <cmath>
@@ -21,6 +22,7 @@ namespace {
 using smla::KParams;
 
 constexpr size_t kAlign = 256;
+constexpr int kTicketWord = 16;     // word of a workspace's first 256 bytes that the prep kernel's blocks count on
 constexpr size_t kDefaultBudget = size_t(6) << 30;  // scratch budget when the caller gives none
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -110,6 +112,17 @@ DevSched* dev_sched_locked() {
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// The descriptor encoder is a driver call and wants the device's context current in the calling thread, which a thread
+// that has made no runtime call yet (an autograd worker, say) does not have.
+bool bind_context() {
+    static thread_local int bound = -1;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (dev == bound) return true;
+    if (cudaSetDevice(dev) != cudaSuccess) return false;
+    bound = dev;
+    return true;
+}
 EncodeFn get_encode_fn() {
     static EncodeFn fn = nullptr;
     static std::once_flag once;
@@ -159,7 +172,7 @@ struct Plan {
     int h_pad;       // heads padded to 64 or 128
     int topk_pad;    // top-k padded to a multiple of 256
     int q_chunk;     // queries per pass
-    size_t err_off, delta_off, s_off, ds_off, total;
+    size_t err_off, delta_off, used_off, pre_off, s_off, ds_off, total;
 };
 
 bool check_params(const smla_bwd_params* p) {
@@ -179,7 +192,10 @@ bool make_plan(const smla_bwd_params* p, size_t budget, Plan* pl) {
     const size_t per_q = size_t(pl->topk_pad) * pl->h_pad * 2 /*bf16*/ * 2 /*S and dS*/;
     pl->err_off = 0;
     pl->delta_off = kAlign;
-    const size_t fixed = align_up(pl->delta_off + size_t(p->s_q) * p->h_q * 4, kAlign);
+    // Delta, slots in use per query, prefix sum of the queries' tiles
+    pl->used_off = align_up(pl->delta_off + size_t(p->s_q) * p->h_q * 4, 16);
+    pl->pre_off = pl->used_off + size_t(p->s_q) * 4;
+    const size_t fixed = align_up(pl->pre_off + (size_t(p->s_q) + 1) * 4, kAlign);
     if (budget == 0) budget = kDefaultBudget;
     size_t qc = budget > fixed ? (budget - fixed) / per_q : 0;
     if (qc < 1) qc = 1;
@@ -212,6 +228,54 @@ bool plan_for_workspace(const smla_bwd_params* p, size_t ws_bytes, Plan* pl) {
 template <typename K>
 bool set_smem(K kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
+// Function attributes belong to a device: set once on each, remembered in the caller's static `done`.
+constexpr int kMaxDevices = 64;
+template <typename F>
+bool once_per_device(std::atomic<bool> (&done)[kMaxDevices], F set) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return false;
+    if (dev < kMaxDevices && done[dev].load(std::memory_order_acquire)) return true;
+    if (!set()) return false;
+    if (dev < kMaxDevices) done[dev].store(true, std::memory_order_release);
+    return true;
+}
+
+// Launch with the optional attributes: `pdl`, the kernel may start under its predecessor's tail (it calls pdl_wait before
+// it touches anything another kernel of the stream uses); `cluster` > 1, CTAs per cluster.
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t st, bool pdl, int cluster, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);       // errors are read by the caller with cudaGetLastError
+    ++g_last_launches;
+}
+
+// CTAs that share one (query, d-part) of the dq kernel, splitting its keys: as many as keep the whole grid within one CTA
+// per SM.  From the call's query count, not a pass's, so that a query's dQ does not depend on how a call is cut into
+// passes; a query of one work tile (256 keys) is never split.
+int dq_key_split(int s_q, int topk_pad, int parts) {
+    int z = 1;
+    while (z < 8 && 2 * z <= topk_pad / smla::kWorkTileKeys && s_q <= 148 / (parts * 2 * z)) z *= 2;
+    return z;
 }
 
 // How many 2-CTA clusters of `kernel` the current device runs at once: the grid of a persistent kernel.  A
@@ -253,6 +317,7 @@ template <int HP>
 int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStream_t st, int stages, bool allow_overlap,
                  const smla_bwd_det_params* det = nullptr) {
     using namespace smla;
+    if (!bind_context()) return SMLA_ERR_LAUNCH;
     __nv_bfloat16* s_scr = reinterpret_cast<__nv_bfloat16*>(ws + pl.s_off);
     __nv_bfloat16* ds_scr = reinterpret_cast<__nv_bfloat16*>(ws + pl.ds_off);
     float* delta = reinterpret_cast<float*>(ws + pl.delta_off);
@@ -269,18 +334,25 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     ok &= make_map_scratch(&tm_ds, ds_scr, uint64_t(pl.q_chunk), pl.topk_pad, HP, 64);
     if (!ok) return SMLA_ERR_LAUNCH;
 
-    // per device, so set on every call (cheap) rather than once per process
-    bool attr_ok = set_smem(smla_recompute_pair_kernel<HP>, rp::Cfg<HP>::kSmemBytes);
-    attr_ok &= set_smem(smla_dkv_pair_kernel<HP>, dp::Cfg<HP>::kSmemBytes);
-    if (det) attr_ok &= set_smem(smla_dkv_pair_kernel<HP, true>, dp::Cfg<HP>::kSmemBytes);
-    attr_ok &= set_smem(smla_dq_kernel<HP, kDqChunks, kQChunks>, dq::Cfg<HP, kDqChunks>::kSmemBytes);
-    if (!attr_ok) return SMLA_ERR_LAUNCH;
+    constexpr int kDqParts = kQChunks / kDqChunks;
+    using DqCfg = dq::Cfg<HP, kDqChunks>;
+    static std::atomic<bool> attr_done[kMaxDevices];
+    if (!once_per_device(attr_done, [] {
+            bool done = set_smem(smla_recompute_pair_kernel<HP>, rp::Cfg<HP>::kSmemBytes);
+            done &= set_smem(smla_dkv_pair_kernel<HP>, dp::Cfg<HP>::kSmemBytes);
+            done &= set_smem(smla_dkv_pair_kernel<HP, true>, dp::Cfg<HP>::kSmemBytes);
+            done &= set_smem(smla_dq_kernel<HP, kDqChunks, kQChunks>, DqCfg::kSplitSmemBytes);
+            return done;
+        }))
+        return SMLA_ERR_LAUNCH;
 
     KParams kp{};
     kp.kv = reinterpret_cast<const __nv_bfloat16*>(p->kv);
     kp.indices = p->indices;
     kp.lse = p->lse;
     kp.delta = delta;
+    kp.n_used = reinterpret_cast<const int*>(ws + pl.used_off);
+    kp.tile_pre = reinterpret_cast<const int*>(ws + pl.pre_off);
     kp.s_scr = s_scr;
     kp.ds_scr = ds_scr;
     kp.dKV = p->dKV;
@@ -303,35 +375,47 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     kp.staging = det ? det->staging : nullptr;
 
     if (stages & SMLA_STAGE_DELTA) {
-        const int n_rows = p->s_q * p->h_q;
-        smla_delta_kernel<<<(n_rows + 7) / 8, 256, 0, st>>>(reinterpret_cast<const uint4*>(p->O),
-                                                          reinterpret_cast<const uint4*>(p->dO), delta, n_rows);
-        ++g_last_launches;
+        // one block per query, more where few queries come with a large dKV to clear
+        const size_t zero_n = (stages & SMLA_STAGE_ZERO) ? size_t(p->s_kv) * (kDQK / 4) : 0;     // 16-byte pieces
+        const size_t zero_blocks = (zero_n + kPrepThreads * 16 - 1) / (kPrepThreads * 16);
+        int grid = p->s_q;
+        if (size_t(grid) < zero_blocks) grid = int(zero_blocks < 8 * 148 ? zero_blocks : 8 * 148);
+        if (grid < p->s_q) grid = p->s_q;
+        launch(smla_prep_kernel, grid, kPrepThreads, 0, st, true, 1, reinterpret_cast<const uint4*>(p->O),
+               reinterpret_cast<const uint4*>(p->dO), delta, reinterpret_cast<int*>(ws + pl.used_off),
+               reinterpret_cast<int*>(ws + pl.pre_off), reinterpret_cast<int*>(ws + pl.err_off) + kTicketWord,
+               reinterpret_cast<uint4*>(p->dKV), zero_n, kp);
+    } else if (stages & SMLA_STAGE_ZERO) {
+        if (cudaMemsetAsync(p->dKV, 0, size_t(p->s_kv) * kDQK * sizeof(float), st) != cudaSuccess) return SMLA_ERR_LAUNCH;
     }
+    if (!(stages & (SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ)))
+        return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
     const int pairs_r = resident_pairs(smla_recompute_pair_kernel<HP>, rp::kThreads, rp::Cfg<HP>::kSmemBytes);
     const int pairs_d = resident_pairs(smla_dkv_pair_kernel<HP>, dp::kThreads, dp::Cfg<HP>::kSmemBytes);
     if (pairs_r <= 0 || pairs_d <= 0) return SMLA_ERR_LAUNCH;
-    auto launch_recompute = [&](cudaStream_t s_, int pairs) {
-        smla_recompute_pair_kernel<HP><<<2 * (kp.nq < pairs ? kp.nq : pairs), rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_>>>(tm_qnh, tm_donh, kp);
-        ++g_last_launches;
+    const int q_tiles = pl.topk_pad / kWorkTileKeys;          // at most; the kernels know how many are in use
+    auto grid_of = [&](int pairs) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * q_tiles)); };
+    // `pdl`: start under the previous kernel's tail (one-stream schedules only)
+    auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
+        launch(smla_recompute_pair_kernel<HP>, grid_of(pairs), rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
-    auto launch_dkv = [&](cudaStream_t s_, int pairs) {
-        const int grid = 2 * (kp.nq < pairs ? kp.nq : pairs);
+    auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl) {
         if (det) {
             // reproducible form: per-slot contributions to the staging rows, then one warp per kv row adds its slots
             // of this pass in CSR order
-            smla_dkv_pair_kernel<HP, true><<<grid, dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_>>>(tm_qhp, tm_dohp, tm_s, tm_ds, kp);
-            smla_dkv_segment_sum_kernel<<<(p->s_kv + 7) / 8, 256, 0, s_>>>(det->row_ptr, det->entries, det->staging, p->dKV, p->s_kv,
-                                                                           p->topk, pl.topk_pad, kp.q0, kp.q0 + kp.nq);
-            g_last_launches += 2;
+            launch(smla_dkv_pair_kernel<HP, true>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s,
+                   tm_ds, kp);
+            launch(smla_dkv_segment_sum_kernel, (p->s_kv + 7) / 8, 256, 0, s_, false, 1, det->row_ptr, det->entries, det->staging, p->dKV,
+                   p->s_kv, p->topk, pl.topk_pad, kp.q0, kp.q0 + kp.nq);
             return;
         }
-        smla_dkv_pair_kernel<HP><<<grid, dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_>>>(tm_qhp, tm_dohp, tm_s, tm_ds, kp);
-        ++g_last_launches;
+        launch(smla_dkv_pair_kernel<HP>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s, tm_ds, kp);
     };
-    auto launch_dq = [&](cudaStream_t s_) {
-        smla_dq_kernel<HP, kDqChunks, kQChunks><<<kp.nq * (kQChunks / kDqChunks), dq::kThreads, dq::Cfg<HP, kDqChunks>::kSmemBytes, s_>>>(tm_ds, kp);
-        ++g_last_launches;
+    const int dq_split = dq_key_split(p->s_q, pl.topk_pad, kDqParts);
+    auto launch_dq = [&](cudaStream_t s_, bool pdl, bool after_dkv) {
+        kp.dq_after_trigger = after_dkv;
+        launch(smla_dq_kernel<HP, kDqChunks, kQChunks>, kp.nq * kDqParts * dq_split, dq::kThreads,
+               dq_split > 1 ? DqCfg::kSplitSmemBytes : DqCfg::kSmemBytes, s_, pdl, dq_split, tm_ds, kp);
     };
 
     int chunks = 0, dkv_pairs = 0;
@@ -350,9 +434,9 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             kp.q0 = q0;
             kp.nq = nq;
             kp.scr0 = 0;
-            if (stages & SMLA_STAGE_RECOMPUTE) launch_recompute(st, pairs_r);
-            if (stages & SMLA_STAGE_DKV) launch_dkv(st, pairs_d);
-            if (stages & SMLA_STAGE_DQ) launch_dq(st);
+            if (stages & SMLA_STAGE_RECOMPUTE) launch_recompute(st, pairs_r, true);
+            if (stages & SMLA_STAGE_DKV) launch_dkv(st, pairs_d, true);
+            if (stages & SMLA_STAGE_DQ) launch_dq(st, true, (stages & SMLA_STAGE_DKV) && !det);
             continue;
         }
         std::lock_guard<std::mutex> lock(g_dev_sched_mutex);
@@ -368,12 +452,12 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             kp.q0 = q0 + a0;
             kp.nq = a1 - a0;
             kp.scr0 = a0;
-            launch_recompute(st, c == 0 ? pairs_r : pairs_r - dkv_pairs);
+            launch_recompute(st, c == 0 ? pairs_r : pairs_r - dkv_pairs, false);
             if (cudaEventRecord(ds->ev_part[c], st) != cudaSuccess ||
                 cudaStreamWaitEvent(ds->side, ds->ev_part[c], 0) != cudaSuccess)
                 return SMLA_ERR_LAUNCH;
-            launch_dkv(ds->side, c == parts - 1 ? pairs_d : dkv_pairs);
-            launch_dq(st);
+            launch_dkv(ds->side, c == parts - 1 ? pairs_d : dkv_pairs, false);
+            launch_dq(st, false, false);
         }
         if (cudaEventRecord(ds->ev_join, ds->side) != cudaSuccess || cudaStreamWaitEvent(st, ds->ev_join, 0) != cudaSuccess)
             return SMLA_ERR_LAUNCH;
@@ -443,6 +527,7 @@ bool fwd_plan_for_workspace(const smla_fwd_params* p, size_t ws_bytes, FwdPlan* 
 template <int HP>
 int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, cudaStream_t st) {
     using namespace smla;
+    if (!bind_context()) return SMLA_ERR_LAUNCH;
     __nv_bfloat16* s_scr = reinterpret_cast<__nv_bfloat16*>(ws + pl.s_off);
     CUtensorMap tm_qnh, tm_s;
     const uint64_t qrows = uint64_t(p->s_q) * p->h_q;
@@ -502,7 +587,6 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
 constexpr size_t kStaticWorkspaceBytes = size_t(32) << 20;
 static __device__ __align__(256) unsigned char g_static_workspace[kStaticWorkspaceBytes];
 
-constexpr int kMaxDevices = 64;
 std::mutex g_static_ws_mutex;
 void* g_static_ws_ptr[kMaxDevices] = {};   // device address of g_static_workspace, per device ordinal
 
@@ -568,10 +652,6 @@ int run_stages_impl(const smla_bwd_params* p, void* workspace, size_t workspace_
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-    if (stage_mask & SMLA_STAGE_ZERO) {
-        if (cudaMemsetAsync(p->dKV, 0, size_t(p->s_kv) * SMLA_D_QK * sizeof(float), st) != cudaSuccess)
-            return SMLA_ERR_LAUNCH;
-    }
     return pl.h_pad == 64 ? launch_chain<64>(p, pl, ws, st, stage_mask, allow_overlap, det)
                           : launch_chain<128>(p, pl, ws, st, stage_mask, allow_overlap, det);
 }
@@ -664,6 +744,29 @@ int smla_bwd_delta(const void* O, const void* dO, float* delta, int32_t s_q, int
     smla::smla_delta_kernel<<<(n_rows + 7) / 8, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const uint4*>(O), reinterpret_cast<const uint4*>(dO), delta, n_rows);
     g_last_launches = 1;
+    return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
+}
+
+int smla_query_meta(int32_t* meta, int32_t n_seq, const int32_t* q_start, const int32_t* kv_start, const int32_t* kv_len,
+                    int32_t q_end, int32_t q_start_index_s, int32_t topk, const int32_t* topk_length, void* stream) {
+    if (!meta || !q_start || !kv_start || !kv_len || n_seq <= 0 || topk < 0 || !aligned16(meta)) return SMLA_ERR_BAD_ARG;
+    for (int i = 0; i < n_seq; ++i)
+        if (q_start[i] < 0 || q_start[i] > (i + 1 < n_seq ? q_start[i + 1] : q_end)) return SMLA_ERR_BAD_ARG;
+    g_last_launches = 0;
+    for (int s0 = 0; s0 < n_seq; s0 += smla::kMetaSeqs) {
+        smla::MetaTable t;
+        const int n = std::min(smla::kMetaSeqs, n_seq - s0);
+        for (int i = 0; i < n; ++i) {
+            t.q0[i] = q_start[s0 + i];
+            t.kv0[i] = kv_start[s0 + i];
+            t.kv_len[i] = kv_len[s0 + i];
+        }
+        t.q0[n] = s0 + n < n_seq ? q_start[s0 + n] : q_end;
+        const int rows = t.q0[n] - t.q0[0];
+        if (rows > 0)
+            launch(smla::smla_query_meta_kernel, (rows + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream), false, 1,
+                   reinterpret_cast<int4*>(meta), t, n, q_start_index_s, topk, topk_length);
+    }
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 

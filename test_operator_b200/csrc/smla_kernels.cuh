@@ -39,6 +39,8 @@ struct KParams {
     const int32_t* indices;   // [s_q, topk]
     const float* lse;         // [s_q, h_q]
     const float* delta;       // [s_q, h_q]
+    const int* n_used;        // [s_q] slots up to and including the query's last valid one
+    const int* tile_pre;      // [s_q + 1] exclusive prefix sum of ceil(n_used / 256) over the queries
     __nv_bfloat16* s_scr;     // [q_chunk][HP/8 head blocks][topk_pad keys][8 heads], see scratch_offset
     __nv_bfloat16* ds_scr;    // likewise
     float* dKV;               // [s_kv, 576]
@@ -61,6 +63,7 @@ struct KParams {
     const int4* qmeta;        // optional per query {first kv row of its sequence, kv rows of its sequence,
                               // position for the causal rule, top-k slots in use}; null: one sequence
     long long wait_limit;     // cycles a bounded wait may take
+    int dq_after_trigger;     // dq: launched behind the dKV kernel's trigger (see smla_dq_kernel)
 };
 
 // What a query may attend to: rows [kv_base, kv_base + kv_len) of kv, index values relative to kv_base.
@@ -116,6 +119,29 @@ __device__ __forceinline__ float ordered_to_float(int o) {
 constexpr int kOrderedNegInf = static_cast<int>(0xff800000u ^ 0x7fffffffu);   // float_to_ordered(-inf)
 constexpr float kFixScale = 4194304.f;                                           // 2^22
 
+__device__ __forceinline__ float dot8_bf16(const uint4& a, const uint4& b, float acc) {
+    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
+    const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 x = __bfloat1622float2(pa[k]), y = __bfloat1622float2(pb[k]);
+        acc = fmaf(x.x, y.x, acc);
+        acc = fmaf(x.y, y.y, acc);
+    }
+    return acc;
+}
+// read once, so first out of the caches
+__device__ __forceinline__ uint4 ld_stream_v4(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
+    return v;
+}
+
 // =============================================================================================
 // Delta = rowsum(O * dO).  One warp per (query, head) row of 512 bf16; each lane reads 2 x 16 B
 // of each tensor, so a warp reads 2 x 1 KB fully coalesced.
@@ -129,26 +155,205 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
     const uint4* g = dO + static_cast<size_t>(row) * (kDV / 8);
     float acc = 0.f;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        uint4 a = __ldg(o + lane + 32 * i);
-        uint4 b = __ldg(g + lane + 32 * i);
-        const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-        const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float2 x = __bfloat1622float2(pa[k]);
-            float2 y = __bfloat1622float2(pb[k]);
-            acc = fmaf(x.x, y.x, acc);
-            acc = fmaf(x.y, y.y, acc);
-        }
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    for (int i = 0; i < 2; ++i) acc = dot8_bf16(__ldg(o + lane + 32 * i), __ldg(g + lane + 32 * i), acc);
+    acc = warp_sum(acc);
     if (lane == 0) delta[row] = acc;
 }
 
 // =============================================================================================
-// recompute: persistent 2-CTA clusters, 18 warps per CTA; cluster c works on queries c, c + #clusters, ...
+// prep: everything the three tensor-core kernels need that is not a contraction, in one launch.
+//   block b < s_q   Delta of query b's rows, and n_used[b]: the slots up to the query's last valid one (early tokens of a
+//                   causal sequence use a fraction of their top-k, the rest are out-of-range values at the end)
+//   every block     its share of dKV cleared (where the caller wants it cleared)
+//   last block      prefix sum of the queries' 256-key tiles, from which the persistent kernels take their ranges
+// Bound by HBM: O, dO and the indices read once, dKV written once.
+// =============================================================================================
+constexpr int kWorkTileKeys = 256;      // granularity of the work ranges: what the recompute kernel does per accumulator
+constexpr int kPrepThreads = 256;
+
+// Sum of one value per thread over the lower-numbered threads of the block; *total: over all.  warp_sums: 32 words.
+__device__ __forceinline__ int block_exclusive_sum(int v, int* warp_sums, int* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < n_warps; ++w) {
+        const int x = warp_sums[w];
+        if (w < warp) before += x;
+        all += x;
+    }
+    __syncthreads();
+    *total = all;
+    return before + incl - v;
+}
+
+__global__ void __launch_bounds__(kPrepThreads)
+smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, float* __restrict__ delta,
+                 int* __restrict__ n_used, int* __restrict__ tile_pre, int* ticket, uint4* __restrict__ zero_dst,
+                 size_t zero_n, const KParams p) {
+    __shared__ int red[32];
+    __shared__ int is_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kWarps = kPrepThreads / 32;
+    pdl_wait();                   // (nothing above touches memory another kernel of the stream may still use)
+    pdl_trigger();
+    const int q = blockIdx.x;
+    if (q < p.s_q) {
+        const QMeta qm = load_qmeta(p, q);
+        int last = -1;
+        for (int key = threadIdx.x; key < p.topk; key += kPrepThreads)
+            if (slot_valid(__ldg(p.indices + static_cast<size_t>(q) * p.topk + key), key, qm, p)) last = key;
+        last = __reduce_max_sync(0xffffffffu, last);
+        if (lane == 0) red[warp] = last;
+    }
+    __syncthreads();
+    // The block that takes the last ticket sees every query's count and sums up the tiles at the end.  The ticket is drawn
+    // here so that its round trip runs under the loads below.
+    if (threadIdx.x == 0) {
+        if (q < p.s_q) {
+            int m = red[0];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) m = max(m, red[w]);
+            n_used[q] = m + 1;
+        }
+        __threadfence();
+        is_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+        __threadfence();
+    }
+    if (q < p.s_q) {
+        const uint4* o = O + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
+        const uint4* g = dO + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
+        // two rows at a time: eight 16-byte loads of a lane in flight
+        for (int h = warp; h < p.h_q; h += 2 * kWarps) {
+            const int h2 = h + kWarps < p.h_q ? h + kWarps : h;
+            uint4 a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = (i < 2 ? h : h2) * (kDV / 8) + 32 * (i & 1);
+                a[i] = ld_stream_v4(o + at);
+                b[i] = ld_stream_v4(g + at);
+            }
+            const float s0 = warp_sum(dot8_bf16(a[1], b[1], dot8_bf16(a[0], b[0], 0.f)));
+            const float s1 = warp_sum(dot8_bf16(a[3], b[3], dot8_bf16(a[2], b[2], 0.f)));
+            if (lane == 0) {
+                delta[static_cast<size_t>(q) * p.h_q + h] = s0;
+                delta[static_cast<size_t>(q) * p.h_q + h2] = s1;
+            }
+        }
+    }
+    if (zero_n) {
+        const size_t z0 = zero_n * blockIdx.x / gridDim.x, z1 = zero_n * (blockIdx.x + 1) / gridDim.x;
+        for (size_t i = z0 + threadIdx.x; i < z1; i += kPrepThreads) zero_dst[i] = make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+    if (!is_last) return;
+    constexpr int kPer = 8;       // consecutive queries per thread and round
+    int carry = 0;
+    for (int base = 0; base < p.s_q; base += kPrepThreads * kPer) {
+        const int i0 = base + threadIdx.x * kPer;
+        int n[kPer], sum = 0;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            n[i] = i0 + i < p.s_q ? (__ldcg(n_used + i0 + i) + kWorkTileKeys - 1) / kWorkTileKeys : 0;
+            sum += n[i];
+        }
+        int total;
+        int at = carry + block_exclusive_sum(sum, red, &total);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            if (i0 + i < p.s_q) tile_pre[i0 + i] = at;
+            at += n[i];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        tile_pre[p.s_q] = carry;
+        *ticket = 0;
+    }
+}
+
+// Per-query table for packed sequences (KParams::qmeta) from a table of sequences that travels in the kernel's parameters:
+// no host-to-device copy, no synchronisation.  One launch covers kMetaSeqs sequences.
+constexpr int kMetaSeqs = 128;
+struct MetaTable {
+    int q0[kMetaSeqs + 1];        // first query row of each sequence, then the end of the last one
+    int kv0[kMetaSeqs], kv_len[kMetaSeqs];
+};
+__global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__ meta, const __grid_constant__ MetaTable t, int n_seq,
+                                                              int pos0, int topk, const int* __restrict__ topk_length) {
+    const int q = t.q0[0] + static_cast<int>(blockIdx.x) * 256 + static_cast<int>(threadIdx.x);
+    if (q >= t.q0[n_seq]) return;
+    int lo = 0, hi = n_seq - 1;                       // the last sequence that starts at or before q
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (t.q0[mid] <= q) lo = mid;
+        else hi = mid - 1;
+    }
+    const int used = topk_length ? min(max(__ldg(topk_length + q), 0), topk) : topk;
+    meta[q] = make_int4(t.kv0[lo], t.kv_len[lo], pos0 + q - t.q0[lo], used);
+}
+
+// ---- work ranges of the persistent kernels ---------------------------------------------------------------------------
+// The 256-key tiles of a launch's queries, one after the other (a query has ceil(n_used / 256) of them), are cut into as
+// many equal contiguous ranges as there are clusters: every cluster gets the same number of tiles (4096 queries of eight
+// tiles over 74 clusters as whole queries would be 56 queries for some and 55 for the others), a few long queries
+// spread over the whole chip, and tiles without a valid slot do not exist.  kMul: tiles of 256 / kMul keys.
+struct WorkRange {
+    int begin, end, q;            // positions in tile_pre's numbering; the query `begin` lies in
+};
+// One warp: which range is this cluster's.  32-way search over the prefix sums (two rounds up to 1024 queries).
+__device__ __forceinline__ WorkRange find_range(const KParams& p, int cluster, int n_clusters) {
+    const int lane = threadIdx.x & 31;
+    const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
+    WorkRange w;
+    w.begin = t0 + static_cast<int>(static_cast<long long>(t1 - t0) * cluster / n_clusters);
+    w.end = t0 + static_cast<int>(static_cast<long long>(t1 - t0) * (cluster + 1) / n_clusters);
+    int lo = p.q0, n = p.nq;      // the last query in [lo, lo + n) whose first tile is at or before `begin`
+    while (n > 1) {
+        const int step = (n + 31) >> 5;
+        const int at = lane * step;
+        const bool before = at < n && (at == 0 || __ldcg(p.tile_pre + lo + at) <= w.begin);
+        const int k = 31 - __clz(__ballot_sync(0xffffffffu, before));
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    w.q = lo;
+    return w;
+}
+template <int kMul> struct TileIter {
+    const int* pre;
+    int q, q_last, lo, hi, hi_next, pos, end;
+    __device__ __forceinline__ TileIter(const KParams& p, const WorkRange& w)
+        : pre(p.tile_pre), q(w.q), q_last(p.q0 + p.nq), pos(w.begin * kMul), end(w.end * kMul) {
+        lo = __ldcg(pre + q) * kMul;
+        hi = __ldcg(pre + q + 1) * kMul;
+        hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;      // one query ahead: the load is done when it is needed
+    }
+    __device__ __forceinline__ bool more() const { return pos < end; }
+    __device__ __forceinline__ int tile() const { return pos - lo; }
+    __device__ __forceinline__ bool last_of_query() const { return pos + 1 == hi || pos + 1 == end; }
+    // to the next tile; true if that is another query's (or the range is finished)
+    __device__ __forceinline__ bool advance() {
+        if (++pos < hi) return pos >= end;
+        while (pos < end) {
+            ++q;
+            lo = hi;
+            hi = hi_next;
+            hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;
+            if (hi > lo) break;
+        }
+        return true;
+    }
+};
+
+// =============================================================================================
+// recompute: persistent 2-CTA clusters, 18 warps per CTA
 // The pair works on 256-key tiles with cta_group::2 UMMAs of shape M = 256 keys x N = 2*HP:
 //   A  each CTA gathers ITS 128 keys of the tile (every kv row is fetched once per query, not once
 //      per head group), chunk by chunk through a 5-slot ring of [128 keys x 64 col] chunks;
@@ -165,7 +370,8 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 //               odd CTA: forwards "my slot is full" to the even CTA (cp.async cannot signal remotely)
 //   warp 17     TMA of the CTA's Q / dO chunks, one barrier per column chunk
 // Slot-free, chunk-free and accumulator-ready signals are tcgen05.commit arrivals delivered to both CTAs.
-// Nothing is drained between queries: the ring, the two accumulator buffers and the counters behind their
+// A cluster works through its range of (query, key tile) pairs (WorkRange); nothing is drained between queries: the ring,
+// the two accumulator buffers and the counters behind their
 // barrier phases run on, the Q / dO chunk j of the next query is fetched as soon as the last tile's UMMAs
 // on chunk j have finished, and the softmax of a query's last tile overlaps the next query's first UMMAs.
 // =============================================================================================
@@ -197,8 +403,6 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     constexpr int NH = C::NH;
     constexpr int kStages = C::kStages;
     const uint32_t rank = cluster_ctarank();
-    const int pair = blockIdx.x >> 1;
-    const int n_pairs = gridDim.x >> 1;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
 
@@ -218,7 +422,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 1024 + 8 * (2 * kStages + 2 * kQChunks + 4));
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t bar_drain = smem_u32(tmem_slot + 2);     // used only while winding down after an abort
-    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 16 <= 512, "barrier area");
+    WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 4);
+    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 16 + sizeof(WorkRange) <= 512, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
@@ -248,13 +453,19 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
         tmem_relinquish_2cta();
     }
+    pdl_wait();                  // tile counts and Delta of the prep kernel; the scratch's previous readers are done
+    pdl_trigger();
+    if (warp == 17) {
+        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
+        if (lane == 0) *range_s = w;
+    }
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const int n_tiles = p.topk_pad / kTileKeys;
-    const int nq = p.nq;
+    const WorkRange range = *range_s;
+    static_assert(kTileKeys == kWorkTileKeys, "one work tile per accumulator");
 
     if (warp >= 8 && warp < 16) {
         // ------------------------------------------------------------------ gather producers
@@ -264,53 +475,46 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         const uint32_t dst0 = s_base + C::kOffRing + r0 * 128 + ((u ^ (r0 & 7)) << 4);
         const char* kvb = reinterpret_cast<const char*>(p.kv) + u * 16;
         const uint64_t pol_keep = l2_policy_evict_last();
-        // index of slot (tile, row i) of query ql, -1 past the top-k; the loads for the next tile are issued
-        // before the current tile's copies so that their latency never stalls the ring
-        // (raw values: nothing may depend on a load here, or the wait for it would sit in front of the copies; they are
-        // turned into kv rows one tile later, when they are used)
-        QMeta qm_next = load_qmeta(p, p.q0 + (pair < nq ? pair : 0));
-        auto load_idx = [&](int ql, int tile, int (&idx)[4]) {
-            if (ql >= nq) {
-                idx[0] = idx[1] = idx[2] = idx[3] = -1;
-                return;
-            }
-            if (tile == 0) qm_next = load_qmeta(p, p.q0 + ql);
+        // Indices are loaded one tile ahead, so that their latency never stalls the ring (raw values: nothing may depend
+        // on a load here, or the wait for it would sit in front of the copies; they are turned into kv rows one tile
+        // later, when they are used).  -1 past the top-k.
+        TileIter<1> it(p, range);
+        QMeta qm_next = load_qmeta(p, range.q);
+        auto load_idx = [&](int (&idx)[4]) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int key = tile * kTileKeys + rank * 128 + r0 + 32 * i;
-                idx[i] = key < p.topk ? __ldg(p.indices + static_cast<size_t>(p.q0 + ql) * p.topk + key) : -1;
+                const int key = it.tile() * kTileKeys + static_cast<int>(rank) * 128 + r0 + 32 * i;
+                idx[i] = it.more() && key < p.topk ? __ldg(p.indices + static_cast<size_t>(it.q) * p.topk + key) : -1;
             }
         };
         int idx_next[4];
-        load_idx(pair, 0, idx_next);
+        load_idx(idx_next);
         int s = 0;
         uint32_t ph = 1;                    // parity that means "slot free" for the current pass over the ring
-        for (int ql = pair; ql < nq; ql += n_pairs) {
-            for (int tile = 0; tile < n_tiles; ++tile) {
-                // A slot whose index is out of range reads nothing and lands as zeros (its S, dS are forced to 0
-                // anyway).  Sending all of them to one stand-in row instead would make that row's cache lines a
-                // hot spot that every SM queues on.
-                const char* src[4];
-                uint32_t nb[4];
+        while (it.more()) {
+            // A slot whose index is out of range reads nothing and lands as zeros (its S, dS are forced to 0
+            // anyway).  Sending all of them to one stand-in row instead would make that row's cache lines a
+            // hot spot that every SM queues on.
+            const char* src[4];
+            uint32_t nb[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = gather_row(idx_next[i], qm_next, p);
-                    nb[i] = row >= 0 ? 16u : 0u;
-                    src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
-                }
-                if (tile + 1 < n_tiles) load_idx(ql, tile + 1, idx_next);
-                else load_idx(ql + n_pairs, 0, idx_next);
-                for (int j = 0; j < kQChunks; ++j) {
-                    mbar_wait(bar_empty + 8 * s, ph, wc, kErrRecompute + 11, kPollSleepNs);
-                    const uint32_t d = dst0 + s * kChunkA;
+            for (int i = 0; i < 4; ++i) {
+                const int row = gather_row(idx_next[i], qm_next, p);
+                nb[i] = row >= 0 ? 16u : 0u;
+                src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
+            }
+            if (it.advance() && it.more()) qm_next = load_qmeta(p, it.q);
+            load_idx(idx_next);
+            for (int j = 0; j < kQChunks; ++j) {
+                mbar_wait(bar_empty + 8 * s, ph, wc, kErrRecompute + 11, kPollSleepNs);
+                const uint32_t d = dst0 + s * kChunkA;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        cp_async16_zfill_hint(d + i * 32 * 128, src[i] + j * 128, nb[i], pol_keep);
-                    cp_async_mbar_arrive_noinc(bar_full + 8 * s);
-                    if (++s == kStages) {
-                        s = 0;
-                        ph ^= 1;
-                    }
+                for (int i = 0; i < 4; ++i)
+                    cp_async16_zfill_hint(d + i * 32 * 128, src[i] + j * 128, nb[i], pol_keep);
+                cp_async_mbar_arrive_noinc(bar_full + 8 * s);
+                if (++s == kStages) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -321,10 +525,11 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             tma_prefetch_desc(&tm_do);
             const uint64_t pol_stream = l2_policy_evict_first();
             uint32_t qpar = 1;              // parity of "chunk free" left by the previous query
-            for (int ql = pair; ql < nq; ql += n_pairs, qpar ^= 1) {
-                const int row0 = (p.q0 + ql) * p.h_q + NH * rank;
+            bool first = true;
+            for (TileIter<1> it(p, range); it.more(); first = false, qpar ^= 1) {
+                const int row0 = it.q * p.h_q + NH * static_cast<int>(rank);
                 for (int j = 0; j < kQChunks; ++j) {
-                    if (ql != pair) mbar_wait(bar_bfree + 8 * j, qpar, wc, kErrRecompute + 16, kPollSleepNs);
+                    if (!first) mbar_wait(bar_bfree + 8 * j, qpar, wc, kErrRecompute + 16, kPollSleepNs);
                     const bool with_do = j < kVChunks;
                     mbar_arrive_expect_tx(bar_bfull + 8 * j, (with_do ? 2 : 1) * C::kBHalf);
                     tma_load_2d_hint(s_base + C::kOffB + j * C::kBChunk, &tm_q, 64 * j, row0, bar_bfull + 8 * j, pol_stream);
@@ -332,6 +537,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                         tma_load_2d_hint(s_base + C::kOffB + j * C::kBChunk + C::kBHalf, &tm_do, 64 * j, row0,
                                          bar_bfull + 8 * j, pol_stream);
                 }
+                while (!it.advance()) {}
             }
         }
     } else if (warp == 16) {
@@ -340,23 +546,24 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 // -------------------------------------------------------------- forward slot-full to the even CTA
                 int s = 0;
                 uint32_t ph = 0, qpar = 0;
-                for (int ql = pair; ql < nq; ql += n_pairs, qpar ^= 1) {
-                    for (int tile = 0; tile < n_tiles; ++tile) {
-                        for (int j = 0; j < kQChunks; ++j) {
-                            // this CTA's half of Q / dO is part of what "full" promises
-                            if (tile == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 15);
-                            mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 17);
-                            // The copies have landed in this CTA's shared memory (the wait above saw them complete);
-                            // make them visible to the tensor core's proxy here, then signal without a cluster-scope
-                            // release, which would cost this thread about a thousand cycles per chunk.
-                            fence_proxy_async_smem();
-                            mbar_arrive_cluster_relaxed(map_to_cta(bar_full + 8 * s, 0));
-                            if (++s == kStages) {
-                                s = 0;
-                                ph ^= 1;
-                            }
+                bool new_query = true;
+                for (TileIter<1> it(p, range); it.more();) {
+                    for (int j = 0; j < kQChunks; ++j) {
+                        // this CTA's half of Q / dO is part of what "full" promises
+                        if (new_query) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 15);
+                        mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 17);
+                        // The copies have landed in this CTA's shared memory (the wait above saw them complete);
+                        // make them visible to the tensor core's proxy here, then signal without a cluster-scope
+                        // release, which would cost this thread about a thousand cycles per chunk.
+                        fence_proxy_async_smem();
+                        mbar_arrive_cluster_relaxed(map_to_cta(bar_full + 8 * s, 0));
+                        if (++s == kStages) {
+                            s = 0;
+                            ph ^= 1;
                         }
                     }
+                    new_query = it.advance();
+                    if (new_query) qpar ^= 1;
                 }
             } else {
                 // -------------------------------------------------------------- UMMA issuer for the pair
@@ -365,33 +572,35 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 constexpr uint32_t idesc = make_idesc_bf16(256, C::kAccCols, 0, 0);
                 const uint64_t desc_hi = make_smem_desc(0, 16, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
                 const uint32_t desc_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
-                const uint32_t a_lo0 = desc_lo + ((s_base + C::kOffRing) >> 4);
-                const uint32_t b_lo0 = desc_lo + ((s_base + C::kOffB) >> 4);
+                const uint32_t a_lo0 = desc_lo + desc_addr(s_base + C::kOffRing);
+                const uint32_t b_lo0 = desc_lo + desc_addr(s_base + C::kOffB);
                 int s = 0, gt = 0;              // ring slot; tiles so far
                 uint32_t ph = 0, qpar = 0;
-                for (int ql = pair; ql < nq; ql += n_pairs, qpar ^= 1) {
-                    for (int tile = 0; tile < n_tiles; ++tile, ++gt) {
-                        const int b = gt & 1;
-                        mbar_spin(bar_tempty + 8 * b, ((gt >> 1) & 1) ^ 1, wc, kErrRecompute + 13);
-                        const uint32_t d = tmem + b * C::kAccCols;
-                        for (int j = 0; j < kQChunks; ++j) {
-                            if (tile == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 12);
-                            mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 14);
-                            tc_fence_after_sync();
-                            const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
-                            const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
+                bool new_query = true;
+                for (TileIter<1> it(p, range); it.more(); ++gt) {
+                    const int b = gt & 1;
+                    const bool last = it.last_of_query();
+                    mbar_spin(bar_tempty + 8 * b, ((gt >> 1) & 1) ^ 1, wc, kErrRecompute + 13);
+                    const uint32_t d = tmem + b * C::kAccCols;
+                    for (int j = 0; j < kQChunks; ++j) {
+                        if (new_query) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 12);
+                        mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 14);
+                        tc_fence_after_sync();
+                        const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
+                        const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
-                                umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, (j | kk) != 0);
-                            umma_commit_2cta_mask(bar_empty + 8 * s, 3);
-                            if (tile == n_tiles - 1) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);   // the next query's chunk may come in
-                            if (++s == kStages) {
-                                s = 0;
-                                ph ^= 1;
-                            }
+                        for (int kk = 0; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
+                            umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, (j | kk) != 0);
+                        umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                        if (last) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);   // the next query's chunk may come in
+                        if (++s == kStages) {
+                            s = 0;
+                            ph ^= 1;
                         }
-                        umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
                     }
+                    umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
+                    new_query = it.advance();
+                    if (new_query) qpar ^= 1;
                 }
                 if (*s_abort) {   // winding down: nothing of this thread's may still be in the tensor pipe at dealloc
                     umma_commit_2cta_mask(bar_drain, 1);
@@ -409,25 +618,32 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         // lse (threads 0..HP-1) and Delta (threads HP..2HP-1) of a query go through shared memory; the value for
         // the next query is fetched one query ahead
         const int t = threadIdx.x;
-        auto load_stat = [&](int ql) -> float {
-            if (ql >= nq) return 0.f;
+        auto load_stat = [&](int qg) -> float {
+            if (qg >= p.q0 + p.nq) return 0.f;
             const int h = t < HP ? t : t - HP;
             if (t >= 2 * HP) return 0.f;
             if (h >= p.h_q) return t < HP ? __int_as_float(0x7f800000) : 0.f;
-            const size_t o = static_cast<size_t>(p.q0 + ql) * p.h_q + h;
+            const size_t o = static_cast<size_t>(qg) * p.h_q + h;
             return t < HP ? p.lse[o] * p.lse_mult : p.delta[o] * p.sm_scale;
         };
-        float stat_next = load_stat(pair);
+        int stat_q = range.q;               // the query stat_next belongs to
+        float stat_next = load_stat(stat_q);
         int gt = 0;
-        for (int ql = pair; ql < nq; ql += n_pairs) {
-            const int qg = p.q0 + ql;
-            const QMeta qm = load_qmeta(p, qg);
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // every softmax warp is done with the previous query
-            if (t < 2 * HP) lse_s[t] = stat_next;              // delta_s follows lse_s
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            stat_next = load_stat(ql + n_pairs);
-            for (int tile = 0; tile < n_tiles; ++tile, ++gt) {
-                const int key = tile * kTileKeys + rank * 128 + row;
+        QMeta qm{};
+        bool new_query = true;
+        for (TileIter<1> it(p, range); it.more(); new_query = it.advance(), ++gt) {
+            const int qg = it.q, tile = it.tile();
+            if (new_query) {
+                qm = load_qmeta(p, qg);
+                if (stat_q != qg) stat_next = load_stat(qg);       // queries without a valid slot lay in between
+                asm volatile("bar.sync 1, 256;" ::: "memory");      // every softmax warp is done with the previous query
+                if (t < 2 * HP) lse_s[t] = stat_next;              // delta_s follows lse_s
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                stat_q = qg + 1;
+                stat_next = load_stat(stat_q);
+            }
+            {
+                const int key = tile * kTileKeys + static_cast<int>(rank) * 128 + row;
                 const int idx = key < p.topk ? __ldg(p.indices + static_cast<size_t>(qg) * p.topk + key) : -1;
                 const bool valid = slot_valid(idx, key, qm, p);
                 const int b = gt & 1;
@@ -436,7 +652,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 {
                     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + b * C::kAccCols + g * 2 * NH;
                     // the 32 lanes hold consecutive keys: 32 x 16 bytes of consecutive addresses per store
-                    const size_t off = static_cast<size_t>(p.scr0 + ql) * p.topk_pad * HP + scratch_offset(key, g * NH, p.topk_pad);
+                    const size_t off = static_cast<size_t>(p.scr0 + qg - p.q0) * p.topk_pad * HP + scratch_offset(key, g * NH, p.topk_pad);
                     __nv_bfloat16* s_out = p.s_scr + off;
                     __nv_bfloat16* ds_out = p.ds_scr + off;
                     const uint32_t vmask = valid ? 0xFFFFFFFFu : 0u;
@@ -725,8 +941,8 @@ smla_fwd_logits_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const KPar
             constexpr uint32_t idesc = make_idesc_bf16(256, HP, 0, 0);
             const uint64_t desc_hi = make_smem_desc(0, 16, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
             const uint32_t desc_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
-            const uint32_t a_lo0 = desc_lo + ((s_base + C::kOffRing) >> 4);
-            const uint32_t b_lo0 = desc_lo + ((s_base + C::kOffB) >> 4);
+            const uint32_t a_lo0 = desc_lo + desc_addr(s_base + C::kOffRing);
+            const uint32_t b_lo0 = desc_lo + desc_addr(s_base + C::kOffB);
             const int n_queries = nq > cta ? (nq - cta + n_ctas - 1) / n_ctas : 0;
             const int total = n_queries * n_tp * kQChunks;      // chunks of a stream
             const uint32_t my_tok = tok + 4 * x;
@@ -915,7 +1131,7 @@ __global__ void smla_fwd_stats_init_kernel(int* m_ord, unsigned long long* l_fix
 }
 
 // =============================================================================================
-// dkv as persistent 2-CTA clusters: one pair per query, all 576 columns of d.
+// dkv as persistent 2-CTA clusters: a pair works through its range of (query, key tile) pairs, all 576 columns of d.
 //
 //   dKV^T[d, key] = dO^T . S + Q^T . dS with cta_group::2 UMMAs of M = 256 rows of d (128 per CTA) x N = 128 keys
 //   (64 supplied by each CTA): a CTA reads 4 KB of A and 2 KB of B per 64 cycles of math, where the single-CTA
@@ -960,9 +1176,6 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     using namespace dp;
     using C = Cfg<HP>;
     const uint32_t rank = cluster_ctarank();
-    const int pair = blockIdx.x >> 1;
-    const int n_pairs = gridDim.x >> 1;
-    const int nq = p.nq;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
 
@@ -978,8 +1191,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t bar_uempty = bar_ufull + 8 * kUnits;               // [kUnits] (even CTA) both CTAs have drained the unit
     const uint32_t bar_drain = bar_uempty + 8 * kUnits;               // 1  used only while winding down after an abort
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffMisc + 8 * (2 * kTileStages + 3 + 2 * kUnits));
-    static_assert(8 * (2 * kTileStages + 3 + 2 * kUnits) + 8 <= 256, "barrier area");
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 2);
+    static_assert(8 * (2 * kTileStages + 3 + 2 * kUnits) + 8 + sizeof(WorkRange) <= 256, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
@@ -1001,12 +1215,19 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_alloc_2cta(smem_u32(tmem_slot), 512);
         tmem_relinquish_2cta();
     }
+    pdl_wait();                  // the recompute kernel's S and dS, the prep kernel's tile counts and cleared dKV
+    pdl_trigger();
+    if (warp == 0) {
+        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
+        if (lane == 0) *range_s = w;
+    }
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const int n_tiles = p.topk_pad / kTileKeys;
+    const WorkRange range = *range_s;
+    using Iter = TileIter<kWorkTileKeys / kTileKeys>;    // two tiles per work tile: a range has an even number of them
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
@@ -1018,30 +1239,33 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint64_t pol_stream = l2_policy_evict_first();
             int s = 0;
             uint32_t ph = 1, k = 0;        // ph: parity that means "stage free" in the current pass over the ring
-            for (int ql = pair; ql < nq; ql += n_pairs, ++k) {
-                // the resident operands are replaced once the previous query's UMMAs are done; the drain warps
-                // meanwhile still work through the accumulator ring, so the reductions do not pause
-                if (k) mbar_wait(bar_resfree, (k - 1) & 1, wc, kErrDkv + 6, kPollSleepNs);
-                mbar_arrive_expect_tx(bar_res, 9 * C::kChunk);
-                const int row0 = (p.q0 + ql) * p.h_q;
-                for (int j = 0; j < 4; ++j) {          // slots 0..3: chunks {2r, 2r+1} of block 0 and block 1
-                    const int chunk = (j >> 1) * 4 + 2 * static_cast<int>(rank) + (j & 1);
-                    tma_load_2d_hint(s_base + C::kOffQ + j * C::kChunk, &tm_q, 64 * chunk, row0, bar_res, pol_stream);
-                    tma_load_2d_hint(s_base + C::kOffDO + j * C::kChunk, &tm_do, 64 * chunk, row0, bar_res, pol_stream);
-                }
-                tma_load_2d_hint(s_base + C::kOffQ + 4 * C::kChunk, &tm_q, 64 * 8, row0, bar_res, pol_stream);
-                for (int tile = 0; tile < n_tiles; ++tile) {
-                    mbar_wait(bar_tempty + 8 * s, ph, wc, kErrDkv + 1, kPollSleepNs);
-                    mbar_arrive_expect_tx(bar_tfull + 8 * s, C::kStage);
-                    const uint32_t dst = s_base + C::kOffStage + s * C::kStage;
-                    // box = this CTA's 64 keys of every head block -> [HP/8][64 keys][8 heads]
-                    const int kb = tile * (kTileKeys / 32) + 2 * static_cast<int>(rank);
-                    tma_load_4d_hint(dst, &tm_s, 0, kb, 0, p.scr0 + ql, bar_tfull + 8 * s, pol_stream);
-                    tma_load_4d_hint(dst + C::kHalfMat, &tm_ds, 0, kb, 0, p.scr0 + ql, bar_tfull + 8 * s, pol_stream);
-                    if (++s == kTileStages) {
-                        s = 0;
-                        ph ^= 1;
+            bool new_query = true;
+            for (Iter it(p, range); it.more(); new_query = it.advance()) {
+                if (new_query) {
+                    // the resident operands are replaced once the previous query's UMMAs are done; the drain warps
+                    // meanwhile still work through the accumulator ring, so the reductions do not pause
+                    if (k) mbar_wait(bar_resfree, (k - 1) & 1, wc, kErrDkv + 6, kPollSleepNs);
+                    ++k;
+                    mbar_arrive_expect_tx(bar_res, 9 * C::kChunk);
+                    const int row0 = it.q * p.h_q;
+                    for (int j = 0; j < 4; ++j) {          // slots 0..3: chunks {2r, 2r+1} of block 0 and block 1
+                        const int chunk = (j >> 1) * 4 + 2 * static_cast<int>(rank) + (j & 1);
+                        tma_load_2d_hint(s_base + C::kOffQ + j * C::kChunk, &tm_q, 64 * chunk, row0, bar_res, pol_stream);
+                        tma_load_2d_hint(s_base + C::kOffDO + j * C::kChunk, &tm_do, 64 * chunk, row0, bar_res, pol_stream);
                     }
+                    tma_load_2d_hint(s_base + C::kOffQ + 4 * C::kChunk, &tm_q, 64 * 8, row0, bar_res, pol_stream);
+                }
+                mbar_wait(bar_tempty + 8 * s, ph, wc, kErrDkv + 1, kPollSleepNs);
+                mbar_arrive_expect_tx(bar_tfull + 8 * s, C::kStage);
+                const uint32_t dst = s_base + C::kOffStage + s * C::kStage;
+                // box = this CTA's 64 keys of every head block -> [HP/8][64 keys][8 heads]
+                const int kb = it.tile() * (kTileKeys / 32) + 2 * static_cast<int>(rank);
+                const int sq = p.scr0 + it.q - p.q0;
+                tma_load_4d_hint(dst, &tm_s, 0, kb, 0, sq, bar_tfull + 8 * s, pol_stream);
+                tma_load_4d_hint(dst + C::kHalfMat, &tm_ds, 0, kb, 0, sq, bar_tfull + 8 * s, pol_stream);
+                if (++s == kTileStages) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -1053,16 +1277,18 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 // relaxed arrive costs a few cycles where a cluster-scope release costs hundreds.
                 int s = 0;
                 uint32_t ph = 0, k = 0;
-                for (int ql = pair; ql < nq; ql += n_pairs, ++k) {
-                    mbar_wait(bar_res, k & 1, wc, kErrDkv + 10);
-                    mbar_arrive_cluster_relaxed(map_to_cta(bar_res, 0));
-                    for (int tile = 0; tile < n_tiles; ++tile) {
-                        mbar_spin(bar_tfull + 8 * s, ph, wc, kErrDkv + 11);
-                        mbar_arrive_cluster_relaxed(map_to_cta(bar_tfull + 8 * s, 0));
-                        if (++s == kTileStages) {
-                            s = 0;
-                            ph ^= 1;
-                        }
+                bool new_query = true;
+                for (Iter it(p, range); it.more(); new_query = it.advance()) {
+                    if (new_query) {
+                        mbar_wait(bar_res, k & 1, wc, kErrDkv + 10);
+                        mbar_arrive_cluster_relaxed(map_to_cta(bar_res, 0));
+                        ++k;
+                    }
+                    mbar_spin(bar_tfull + 8 * s, ph, wc, kErrDkv + 11);
+                    mbar_arrive_cluster_relaxed(map_to_cta(bar_tfull + 8 * s, 0));
+                    if (++s == kTileStages) {
+                        s = 0;
+                        ph ^= 1;
                     }
                 }
             } else {
@@ -1070,41 +1296,42 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 constexpr uint32_t idesc = make_idesc_bf16(256, 128, 1, 0);   // A MN-major (d contiguous), B K-major
                 int s = 0;
                 uint32_t ph = 0, k = 0, unit = 0;
-                for (int ql = pair; ql < nq; ql += n_pairs, ++k) {
-                    mbar_wait(bar_res, k & 1, wc, kErrDkv + 2);
-                    for (int tile = 0; tile < n_tiles; ++tile) {
-                        mbar_wait(bar_tfull + 8 * s, ph, wc, kErrDkv + 4);
-                        const uint32_t st_s = s_base + C::kOffStage + s * C::kStage;
-                        const uint32_t st_ds = st_s + C::kHalfMat;
-                        for (int blk = 0; blk < 3; ++blk, ++unit) {
-                            const int us = unit % kUnits;
-                            mbar_wait(bar_uempty + 8 * us, ((unit / kUnits) & 1) ^ 1, wc, kErrDkv + 3);
-                            tc_fence_after_sync();
-                            const uint32_t d = tmem + us * 128;
-                            // each CTA's 128 rows: slot pair (0,1), (2,3) or, for block 2, (3,4)
-                            const int slot = blk == 2 ? 3 : 2 * blk;
-                            if (blk < 2) {
-                                const uint32_t a_do = s_base + C::kOffDO + slot * C::kChunk;
-#pragma unroll
-                                for (int ks = 0; ks < HP / 16; ++ks)
-                                    umma_ss_2cta(d, make_smem_desc(a_do + ks * 2048, C::kChunk, 1024, kSwizzle128),
-                                                 make_smem_desc(st_s + ks * 2048, 1024, 128, kSwizzleNone), idesc, ks != 0);
-                            }
-                            const uint32_t a_q = s_base + C::kOffQ + slot * C::kChunk;
+                bool new_query = true;
+                for (Iter it(p, range); it.more();) {
+                    if (new_query) mbar_wait(bar_res, k++ & 1, wc, kErrDkv + 2);
+                    const bool last = it.last_of_query();
+                    mbar_wait(bar_tfull + 8 * s, ph, wc, kErrDkv + 4);
+                    const uint32_t st_s = s_base + C::kOffStage + s * C::kStage;
+                    const uint32_t st_ds = st_s + C::kHalfMat;
+                    for (int blk = 0; blk < 3; ++blk, ++unit) {
+                        const int us = unit % kUnits;
+                        mbar_wait(bar_uempty + 8 * us, ((unit / kUnits) & 1) ^ 1, wc, kErrDkv + 3);
+                        tc_fence_after_sync();
+                        const uint32_t d = tmem + us * 128;
+                        // each CTA's 128 rows: slot pair (0,1), (2,3) or, for block 2, (3,4)
+                        const int slot = blk == 2 ? 3 : 2 * blk;
+                        if (blk < 2) {
+                            const uint32_t a_do = s_base + C::kOffDO + slot * C::kChunk;
 #pragma unroll
                             for (int ks = 0; ks < HP / 16; ++ks)
-                                umma_ss_2cta(d, make_smem_desc(a_q + ks * 2048, C::kChunk, 1024, kSwizzle128),
-                                             make_smem_desc(st_ds + ks * 2048, 1024, 128, kSwizzleNone), idesc,
-                                             blk < 2 || ks != 0);
-                            umma_commit_2cta_mask(bar_ufull + 8 * us, 3);
+                                umma_ss_2cta(d, make_smem_desc(a_do + ks * 2048, C::kChunk, 1024, kSwizzle128),
+                                             make_smem_desc(st_s + ks * 2048, 1024, 128, kSwizzleNone), idesc, ks != 0);
                         }
-                        umma_commit_2cta_mask(bar_tempty + 8 * s, 3);
-                        if (++s == kTileStages) {
-                            s = 0;
-                            ph ^= 1;
-                        }
+                        const uint32_t a_q = s_base + C::kOffQ + slot * C::kChunk;
+#pragma unroll
+                        for (int ks = 0; ks < HP / 16; ++ks)
+                            umma_ss_2cta(d, make_smem_desc(a_q + ks * 2048, C::kChunk, 1024, kSwizzle128),
+                                         make_smem_desc(st_ds + ks * 2048, 1024, 128, kSwizzleNone), idesc,
+                                         blk < 2 || ks != 0);
+                        umma_commit_2cta_mask(bar_ufull + 8 * us, 3);
                     }
-                    umma_commit_2cta_mask(bar_resfree, 3);
+                    umma_commit_2cta_mask(bar_tempty + 8 * s, 3);
+                    if (last) umma_commit_2cta_mask(bar_resfree, 3);
+                    if (++s == kTileStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                    new_query = it.advance();
                 }
                 if (*s_abort) {   // winding down: nothing of this thread's may still be in the tensor pipe at dealloc
                     umma_commit_2cta_mask(bar_drain, 1);
@@ -1121,7 +1348,6 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int quarter = warp & 3;           // the TMEM lane quarter a warp may read is warp % 4
         const int e = (dw >> 2) & 1;            // which 64 keys of the 128-key tile this warp scatters
         const int member = dw & 3;              // the four warps of a (group, key half) share one index buffer
-        const int upq = n_tiles * 3;            // units per query: even, because top-k is padded to 256 keys
         // index buffers [group][tile parity][key half][64]: filled by member 0 from registers it loaded one tile ahead,
         // published with a named barrier of the four warps.  Every tile shows up in both groups' unit sequences and
         // the barrier keeps the four within one tile of each other, so two buffers per (group, key half) suffice.
@@ -1133,12 +1359,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #endif
         int pf[2] = {-1, -1};
         // (the dKV row a valid slot adds to, -1 for an unused slot)
-        auto fetch_idx = [&](int ql, int tile) {
-            if (ql >= nq) {
-                pf[0] = pf[1] = -1;
-                return;
-            }
-            const int qg = p.q0 + ql;
+        auto fetch_idx = [&](int qg, int tile) {
             const QMeta qm = load_qmeta(p, qg);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -1147,39 +1368,33 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 pf[i] = slot_valid(idx, key, qm, p) ? qm.kv_base + idx : -1;
             }
         };
-        if (member == 0) fetch_idx(pair, 0);
-        uint32_t qn = 0;
-        for (int ql = pair; ql < nq; ql += n_pairs, ++qn) {
-            int last_tile = -1;
-            for (int ul = grp; ul < upq; ul += 2) {
-                const int tile = ul / 3, blk = ul - tile * 3;
-                const uint32_t unit = qn * upq + ul;
+        Iter it(p, range);
+        if (member == 0 && it.more()) fetch_idx(it.q, it.tile());
+        for (uint32_t n = 0; it.more(); ++n) {      // n: tiles so far; unit 3 n + blk of the range belongs to group (n + blk) % 2
+            const int tile = it.tile(), sq = p.scr0 + it.q - p.q0;
+            int* idx_s = idx_base + (n & 1) * 128;
+            if (member == 0) {
+                idx_s[lane] = pf[0];
+                idx_s[32 + lane] = pf[1];
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+            it.advance();
+            if (member == 0 && it.more()) fetch_idx(it.q, it.tile());
+            for (int blk = (n ^ grp) & 1; blk < 3; blk += 2) {
+                const uint32_t unit = 3 * n + blk;
                 const int us = unit % kUnits;
-                int* idx_s = idx_base + (tile & 1) * 128;
-                if (tile != last_tile) {
-                    last_tile = tile;
-                    if (member == 0) {
-                        idx_s[lane] = pf[0];
-                        idx_s[32 + lane] = pf[1];
-                    }
-                    asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-                    if (member == 0) {
-                        if (tile + 1 < n_tiles) fetch_idx(ql, tile + 1);
-                        else fetch_idx(ql + n_pairs, 0);
-                    }
-                }
                 mbar_wait(bar_ufull + 8 * us, (unit / kUnits) & 1, wc, kErrDkv + 5, kPollSleepNs);
                 tc_fence_after_sync();
                 // blocks 0, 1: every row is real (d = 256 blk + 128 rank + row).  Block 2: rows 64..127 are d 512..575
                 // in both CTAs; the CTA whose turn it is drains them.
-                const bool mine = blk < 2 || (quarter >= 2 && static_cast<uint32_t>(tile & 1) == rank);
+                const bool mine = blk < 2 || (quarter >= 2 && (n & 1) == rank);
                 if (mine) {
                     const int d0 = blk < 2 ? 256 * blk + 128 * static_cast<int>(rank) : 512 - 64;
                     float* out = p.dKV + d0 + quarter * 32 + lane;
                     // staged form: the row of slot (query, first key of this warp's 64) in the staging buffer
                     float* sout = nullptr;
                     if constexpr (kStaged)
-                        sout = p.staging + (static_cast<size_t>(p.scr0 + ql) * p.topk_pad + tile * kTileKeys + 64 * e) * kDQK +
+                        sout = p.staging + (static_cast<size_t>(sq) * p.topk_pad + tile * kTileKeys + 64 * e) * kDQK +
                                d0 + quarter * 32 + lane;
                     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + us * 128 + 64 * e;
 #pragma unroll
@@ -1316,6 +1531,12 @@ template <int HP, int kSplit> struct Cfg {
     static constexpr int kTmemCols = 256;                  // up to 256 columns of d; two CTAs share the SM's 512
     static constexpr int kRowBytes = kSplit * 128 + 16;    // epilogue staging of one head's row
     static_assert(128 * kRowBytes <= kOffMisc, "the epilogue stages its rows in the pipeline's memory");
+    // keys of a query split over a cluster: every CTA leaves its fp32 accumulator [heads][columns] behind the barriers for
+    // the others to read (rows 16 bytes apart modulo 128: conflict-free 16-byte accesses); one CTA per SM then
+    static constexpr int kPartPitch = kSplit * 64 + 4;
+    static constexpr int kOffPart = kOffMisc + 256;
+    static constexpr int kSplitSmemBytes = kOffPart + 128 * kPartPitch * 4 + 1024;
+    static_assert(kSplit > kDqChunks || kSplitSmemBytes <= 232448, "shared memory of one SM");   // (only dQ splits its keys)
 };
 }  // namespace dq
 
@@ -1328,8 +1549,11 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     using C = Cfg<HP, kSplit>;
     constexpr int kStages = C::kStages;
     constexpr int kParts = (kTotal + kSplit - 1) / kSplit;
-    const int part = blockIdx.x % kParts;
-    const int ql = blockIdx.x / kParts;
+    // the CTAs of a cluster (usually one) share a (query, d-part) and split its keys
+    const int nz = static_cast<int>(cluster_nctas()), z = static_cast<int>(cluster_ctarank());
+    const int unit = static_cast<int>(blockIdx.x) / nz;
+    const int part = unit % kParts;
+    const int ql = unit / kParts;
     const int qg = p.q0 + ql;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
@@ -1367,7 +1591,16 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const int n_tiles = p.topk_pad / kTileKeys;
+    // Behind the dKV kernel's trigger everything this kernel reads is in place already (that kernel triggers after it has
+    // waited for the recompute kernel), so its CTAs fill whatever SMs the dKV kernel leaves; the last CTA then holds the
+    // grid open until the dKV kernel is done, so that "dq done" still means "all done" to whatever follows.
+    if (!p.dq_after_trigger) pdl_wait();
+    int tile0 = 0, n_tiles = p.topk_pad / kTileKeys;
+    if constexpr (!kNorm) {
+        const int n = (__ldcg(p.n_used + qg) + kTileKeys - 1) / kTileKeys;
+        tile0 = n * z / nz;
+        n_tiles = n * (z + 1) / nz - tile0;
+    }
 
     if (warp >= 4 && warp < 12) {
         const int pt = threadIdx.x - 128;   // 0..255
@@ -1383,7 +1616,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         auto load_idx = [&](int tile) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int key = tile * kTileKeys + r0 + 32 * i;
+                const int key = (tile0 + tile) * kTileKeys + r0 + 32 * i;
                 idx_next[i] = (tile < n_tiles && key < p.topk) ? __ldg(p.indices + static_cast<size_t>(qg) * p.topk + key) : -1;
             }
         };
@@ -1423,7 +1656,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                 const uint32_t dst = s_base + s * C::kStage;
                 mbar_arrive_expect_tx(bar_full + 8 * s, C::kDsBytes);
                 // box = 64 keys of every head block -> [HP/8][64 keys][8 heads]
-                tma_load_4d_hint(dst + C::kKgBytes, &tm_ds, 0, tile * (kTileKeys / 32), 0, p.scr0 + ql, bar_full + 8 * s, pol_stream);
+                tma_load_4d_hint(dst + C::kKgBytes, &tm_ds, 0, (tile0 + tile) * (kTileKeys / 32), 0, p.scr0 + ql, bar_full + 8 * s, pol_stream);
                 if (++s == kStages) {
                     s = 0;
                     ph ^= 1;
@@ -1437,9 +1670,9 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
             // A = dS^T: [HP/8 head blocks][64 keys][8 heads], 8-key groups 128 B apart, head blocks 1 KB apart.
             // Descriptors: the fixed fields once, the address (16-byte units, the low 14 bits) added per UMMA.
             const uint64_t a_hi = make_smem_desc(0, 128, 1024, kSwizzleNone) & 0xFFFFFFFF00000000ull;
-            const uint32_t a_lo0 = static_cast<uint32_t>(make_smem_desc(0, 128, 1024, kSwizzleNone)) + ((s_base + C::kKgBytes) >> 4);
+            const uint32_t a_lo0 = static_cast<uint32_t>(make_smem_desc(0, 128, 1024, kSwizzleNone)) + desc_addr(s_base + C::kKgBytes);
             const uint64_t b_hi = make_smem_desc(0, 8192, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
-            const uint32_t b_lo0 = static_cast<uint32_t>(make_smem_desc(0, 8192, 1024, kSwizzle128)) + (s_base >> 4);
+            const uint32_t b_lo0 = static_cast<uint32_t>(make_smem_desc(0, 8192, 1024, kSwizzle128)) + desc_addr(s_base);
             int s = 0;
             uint32_t ph = 0;
             for (int tile = 0; tile < n_tiles; ++tile) {
@@ -1468,6 +1701,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         const int quarter = warp;
         mbar_wait(bar_acc, 0, wc, kErrDq + 3, kPollSleepNs);
         tc_fence_after_sync();
+        const uint32_t zero_mask = n_tiles > 0 ? 0xFFFFFFFFu : 0u;      // no tile at all: the accumulator was never written
         // lane = head, columns = d of the part.  Each thread converts its head's row to bf16 in shared memory (the
         // pipeline stages are idle by now; rows 16 bytes apart modulo 128 so that the 16-byte stores of a warp
         // spread over all banks) and sends it off as one bulk copy: whole cache lines instead of 32 scattered
@@ -1487,13 +1721,29 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                                             : __int_as_float(0x7f800000)) * p.lse_out_mult;
             }
         }
-        if (quarter * 32 < p.h_q) {               // warp-uniform: heads are padded to a multiple of 8 only
-            const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+        if (nz > 1) {
+            if (quarter * 32 < p.h_q) {
+                const uint32_t part_s = s_base + C::kOffPart + head * (C::kPartPitch * 4);
+#pragma unroll 1
+                for (int cg = 0; cg < n_ch * 4; ++cg) {
+                    uint32_t r[16];
+                    tmem_ld_32x16(taddr + cg * 16, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        st_shared_v4(part_s + cg * 64 + v * 16, r[4 * v] & zero_mask, r[4 * v + 1] & zero_mask, r[4 * v + 2] & zero_mask,
+                                     r[4 * v + 3] & zero_mask);
+                }
+            }
+        } else if (quarter * 32 < p.h_q) {        // warp-uniform: heads are padded to a multiple of 8 only
 #pragma unroll 1
             for (int cg = 0; cg < n_ch * 4; ++cg) {   // 16 columns at a time: two CTAs per SM leave 64 registers a thread
                 uint32_t r[16];
                 tmem_ld_32x16(taddr + cg * 16, r);
                 tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r[i] &= zero_mask;
                 if constexpr (kNorm) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * inv);
@@ -1515,8 +1765,31 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         }
     }
     abort_wind_down(s_abort);
+    if (p.dq_after_trigger && blockIdx.x == gridDim.x - 1) pdl_wait();
     tc_fence_before_sync();
     __syncthreads();
+    if (nz > 1) {
+        // every CTA adds up its share of the heads, always in rank order
+        cluster_sync_all();
+        constexpr int kGroups = kSplit * 8;      // 8 columns at a time
+        const int h0 = p.h_q * z / nz, h1 = p.h_q * (z + 1) / nz;
+        for (int i = threadIdx.x; i < (h1 - h0) * kGroups; i += kThreads) {
+            const int h = h0 + i / kGroups, c = (i % kGroups) * 8;
+            if (c >= n_ch * 64) continue;
+            const uint32_t at = s_base + C::kOffPart + (h * C::kPartPitch + c) * 4;
+            float acc[8] = {};
+            for (int r = 0; r < nz; ++r) {
+                const uint32_t a = map_to_cta(at, r);
+                const float4 lo = ld_cluster_v4(a), hi = ld_cluster_v4(a + 16);
+                acc[0] += lo.x; acc[1] += lo.y; acc[2] += lo.z; acc[3] += lo.w;
+                acc[4] += hi.x; acc[5] += hi.y; acc[6] += hi.z; acc[7] += hi.w;
+            }
+            *reinterpret_cast<uint4*>(p.gout + (static_cast<size_t>(qg) * p.h_q + h) * (kTotal * 64) + chunk0 * 64 + c) =
+                make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
+                           pack_bf16x2(acc[6], acc[7]));
+        }
+        cluster_sync_all();                      // nobody leaves while another still reads its part
+    }
     if (warp == 12) tmem_dealloc(tmem, C::kTmemCols);
 }
 
