@@ -10,6 +10,7 @@ There is no CPU or eager fallback: if the library is missing and cannot be built
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 import threading
@@ -81,6 +82,8 @@ _lib_lock = threading.Lock()
 def load_library() -> ctypes.CDLL:
     """Load (building first if the sources are newer) the C-ABI shared library."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lib_lock:
         if _lib is not None:
             return _lib
@@ -99,6 +102,9 @@ def load_library() -> ctypes.CDLL:
         lib.smla_bwd_run_stages.restype = ctypes.c_int
         lib.smla_bwd_run_stages.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p,
                                             ctypes.c_int]
+        lib.smla_query_meta.restype = ctypes.c_int
+        lib.smla_query_meta.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
+                                        ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
         lib.smla_bwd_delta.restype = ctypes.c_int
         lib.smla_bwd_delta.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
                                        ctypes.c_int32, ctypes.c_void_p]
@@ -158,6 +164,39 @@ def load_library() -> ctypes.CDLL:
         return lib
 
 
+# Host path of a call.  The smallest calls take the GPU some tens of microseconds, so what Python does per call counts:
+# the current device is only switched when it has to be, the stream is taken as the raw handle, workspace sizes are
+# remembered per shape, and a call that passes one quick look at its tensors skips the itemised checks.
+class _NoSwitch:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_SWITCH = _NoSwitch()
+
+
+def _on_device(index: int):
+    return _NO_SWITCH if torch.cuda.current_device() == index else torch.cuda.device(index)
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+@functools.lru_cache(maxsize=4096)
+def _bwd_workspace_bytes(s_q: int, s_kv: int, h_q: int, topk: int, budget: int) -> int:
+    p = _Params(0, 0, 0, 0, 0, 0, 0, 0, s_q, s_kv, h_q, topk, 0.0, 0, 1, None)
+    return load_library().smla_bwd_workspace_size(ctypes.byref(p), budget)
+
+
+@functools.lru_cache(maxsize=4096)
+def _fwd_workspace_bytes(s_q: int, s_kv: int, h_q: int, topk: int, budget: int) -> int:
+    p = _FwdParams(0, 0, 0, 0, 0, s_q, s_kv, h_q, topk, 0.0, 0, 1, None)
+    return load_library().smla_fwd_workspace_size(ctypes.byref(p), budget)
+
+
 def _check(cond: bool, msg: str) -> None:
     if not cond:
         raise RuntimeError(msg)
@@ -178,10 +217,7 @@ class Workspace:
         self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
         self.buf[:256].zero_()
         self.nbytes = nbytes
-
-    @property
-    def ptr(self) -> int:
-        return self.buf.data_ptr()
+        self.ptr = self.buf.data_ptr()
 
 
 # Workspaces handed out when the caller passes none, one per (device, stream) so that calls queued on different
@@ -191,8 +227,8 @@ _ws_cache_lock = threading.Lock()
 
 
 def _cached_workspace(need: int, device: torch.device) -> Workspace:
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (index, _raw_stream(index))
     with _ws_cache_lock:
         ws = _ws_cache.get(key)
         if ws is None or ws.nbytes < need:
@@ -208,8 +244,8 @@ _buf_cache = {}
 
 def _cached_buffer(kind: str, need: int, device: torch.device) -> torch.Tensor:
     """A byte buffer kept per (kind, device, stream) and grown on demand, like the workspaces."""
-    key = (kind, device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (kind, index, _raw_stream(index))
     with _ws_cache_lock:
         buf = _buf_cache.get(key)
         if buf is None or buf.numel() < need:
@@ -252,6 +288,26 @@ def _check_query_meta(query_meta, q) -> None:
 def _check_out(t, like_shape_numel, dtype, device, name) -> None:
     _check(isinstance(t, torch.Tensor) and t.is_cuda and t.device == device and t.dtype == dtype and t.is_contiguous()
            and t.numel() == like_shape_numel, f"{name} must be a contiguous {dtype} CUDA tensor of {like_shape_numel} elements on {device}")
+
+
+def _plainly_valid(q, kv, dO, lse, O, indices) -> bool:
+    """True for what nearly every call passes: accepts only what `_validate` accepts, which has the error messages."""
+    try:
+        s_q, h_q, d = q.shape
+        s_kv, d_kv = kv.shape
+        n, topk = indices.shape
+        index = q.get_device()
+        want = (s_q, h_q, D_V)
+        return (d == D_QK and d_kv == D_QK and n == s_q and topk > 0 and 0 < h_q <= 128 and h_q % 8 == 0 and index >= 0
+                and dO.shape == want and O.shape == want and lse.shape == (s_q, h_q)
+                and q.dtype is torch.bfloat16 and kv.dtype is torch.bfloat16 and dO.dtype is torch.bfloat16
+                and O.dtype is torch.bfloat16 and lse.dtype is torch.float32 and indices.dtype is torch.int32
+                and kv.get_device() == index and dO.get_device() == index and lse.get_device() == index
+                and O.get_device() == index and indices.get_device() == index and q.is_cuda
+                and q.is_contiguous() and kv.is_contiguous() and dO.is_contiguous() and lse.is_contiguous()
+                and O.is_contiguous() and indices.is_contiguous())
+    except (AttributeError, TypeError, ValueError):
+        return False
 
 
 def _validate(q, kv, dO, lse, O, indices):
@@ -316,30 +372,32 @@ def mla_bwd(
     bytes per slot), for runs that must repeat exactly.  The call enqueues on the current stream and does not
     synchronise unless `check_device_status=True`, which also raises if a kernel reported a timed-out wait.
     """
-    _validate(q, kv, dO, lse, O, indices)
+    if not _plainly_valid(q, kv, dO, lse, O, indices):
+        _validate(q, kv, dO, lse, O, indices)
     _check_query_meta(query_meta, q)
     lib = load_library()
-    kv2 = kv.reshape(kv.shape[0], D_QK)
-    idx2 = indices.reshape(indices.shape[0], indices.shape[-1])
-    with torch.cuda.device(q.device):
+    kv2 = kv if kv.dim() == 2 else kv.reshape(kv.shape[0], D_QK)
+    idx2 = indices if indices.dim() == 2 else indices.reshape(indices.shape[0], indices.shape[-1])
+    index = q.get_device()
+    with _on_device(index):
         if out_dq is None:
             dQ = torch.empty_like(q)
         else:
             _check_out(out_dq, q.numel(), torch.bfloat16, q.device, "out_dq")
             dQ = out_dq
         if out_dkv is None:
-            dKV = torch.empty(kv.shape, dtype=torch.float32, device=q.device)
+            dKV = torch.empty_like(kv, dtype=torch.float32)
             _check(not accumulate, "accumulate=True needs out_dkv")
         else:
             _check_out(out_dkv, kv.numel(), torch.float32, q.device, "out_dkv")
             dKV = out_dkv
         params = _make_params(q, kv2, dO, lse, O, idx2, dQ, dKV, sm_scale, q_start_index_s, lse_is_base2, query_meta)
         if workspace is None:
-            need = lib.smla_bwd_workspace_size(ctypes.byref(params), workspace_budget)
+            need = _bwd_workspace_bytes(params.s_q, params.s_kv, params.h_q, params.topk, workspace_budget)
             _check(need > 0, "unsupported shapes for the sparse MLA backward")
             # a budget asks for a particular size: do not serve it from a (possibly larger) cached one
             workspace = Workspace(need, q.device) if workspace_budget else _cached_workspace(need, q.device)
-        stream = torch.cuda.current_stream().cuda_stream
+        stream = _raw_stream(index)
         stages = STAGE_ALL & ~STAGE_ZERO if accumulate else STAGE_ALL
         if deterministic:
             _check(query_meta is None, "deterministic=True handles one sequence per call (no query_meta)")
@@ -369,6 +427,25 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
     `topk_length` ([T_q], optional) limits the slots in use per query, the per-query field of the reference's
     richer parameter block (`dq_test/dq_phase_capture.cuh:107-109`)."""
     n_seq = len(seq_q_len)
+    device = torch.device(device)
+    if device.type == "cuda" and n_seq and all(
+            b == a + n for a, n, b in zip(seq_q_start, seq_q_len, seq_q_start[1:])):
+        t_q = sum(seq_q_len)
+        if topk_length is not None:
+            _check_topk_length(topk_length, t_q)
+            topk_length = topk_length.reshape(-1).to(device=device, dtype=torch.int32).contiguous()
+        _check(seq_q_start[0] == 0, "the query rows of the sequences start at row 0")
+        meta = torch.empty(t_q, 4, dtype=torch.int32, device=device)
+        if t_q == 0:
+            return meta
+        table = [(ctypes.c_int32 * n_seq)(*v) for v in (seq_q_start, seq_kv_start, seq_kv_len)]
+        lib = load_library()
+        index = meta.get_device()
+        with _on_device(index):
+            st = lib.smla_query_meta(meta.data_ptr(), n_seq, *table, t_q, q_start_index_s or 0, topk,
+                                     topk_length.data_ptr() if topk_length is not None else None, _raw_stream(index))
+        _raise_status(lib, st, "smla_query_meta")
+        return meta
     lens = torch.tensor(list(seq_q_len), dtype=torch.int64)
     seq_of_q = torch.repeat_interleave(torch.arange(n_seq), lens)
     t_q = int(lens.sum().item())
@@ -380,9 +457,13 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
     meta[:, 3] = topk
     meta = meta.to(device)
     if topk_length is not None:
-        _check(not topk_length.is_floating_point() and topk_length.numel() == t_q, "topk_length must be an integer tensor with one entry per query")
+        _check_topk_length(topk_length, t_q)
         meta[:, 3] = topk_length.reshape(-1).to(device=device, dtype=torch.int32).clamp(0, topk)
     return meta.contiguous()
+
+
+def _check_topk_length(topk_length: torch.Tensor, t_q: int) -> None:
+    _check(not topk_length.is_floating_point() and topk_length.numel() == t_q, "topk_length must be an integer tensor with one entry per query")
 
 
 def mla_bwd_batched(q, kv, dO, lse, O, indices, topk_length: Optional[torch.Tensor] = None,
@@ -447,30 +528,35 @@ def mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor, sm_scale: 
     lse) so that `mla_bwd(q, kv, dO, lse, o, indices)` can consume the outputs directly.
     """
     for name, t in (("q", q), ("kv", kv), ("indices", indices)):
-        _check(isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous(), f"{name} must be a contiguous CUDA tensor")
-    _check(q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and indices.dtype == torch.int32, "dtypes: bf16, bf16, int32")
-    _check(q.dim() == 3 and q.shape[2] == D_QK and kv.shape[-1] == D_QK, f"q [s_q,h_q,{D_QK}], kv [s_kv,{D_QK}]")
-    _check(kv.dim() == 2 or (kv.dim() == 3 and kv.shape[1] == 1), "kv must be [s_kv,576] or [s_kv,1,576]")
-    _check(indices.shape[0] == q.shape[0] and (indices.dim() == 2 or (indices.dim() == 3 and indices.shape[1] == 1)),
-           "indices must be [s_q,topk] or [s_q,1,topk]")
-    s_q, h_q, _ = q.shape
-    _check(0 < h_q <= 128 and h_q % 8 == 0, f"h_q must be a multiple of 8 in [8, 128], got {h_q}")
+        if not (isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous()):
+            raise RuntimeError(f"{name} must be a contiguous CUDA tensor")
+    _check(q.dtype is torch.bfloat16 and kv.dtype is torch.bfloat16 and indices.dtype is torch.int32, "dtypes: bf16, bf16, int32")
+    qs, ks, ids = q.shape, kv.shape, indices.shape
+    _check(len(qs) == 3 and qs[2] == D_QK and ks[-1] == D_QK, "q [s_q,h_q,576], kv [s_kv,576]")
+    _check(len(ks) == 2 or (len(ks) == 3 and ks[1] == 1), "kv must be [s_kv,576] or [s_kv,1,576]")
+    _check(ids[0] == qs[0] and (len(ids) == 2 or (len(ids) == 3 and ids[1] == 1)), "indices must be [s_q,topk] or [s_q,1,topk]")
+    s_q, h_q, _ = qs
+    if not (0 < h_q <= 128 and h_q % 8 == 0):
+        raise RuntimeError(f"h_q must be a multiple of 8 in [8, 128], got {h_q}")
     _check_query_meta(query_meta, q)
     lib = load_library()
-    with torch.cuda.device(q.device):
-        o = torch.empty(s_q, h_q, D_V, dtype=torch.bfloat16, device=q.device)
-        lse = torch.empty(s_q, h_q, dtype=torch.float32, device=q.device)
+    index = q.get_device()
+    with _on_device(index):
+        o = torch.empty((s_q, h_q, D_V), dtype=torch.bfloat16, device=q.device)
+        lse = torch.empty((s_q, h_q), dtype=torch.float32, device=q.device)
         params = _FwdParams(q.data_ptr(), kv.data_ptr(), indices.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                            s_q, kv.shape[0], h_q, indices.shape[-1],
+                            s_q, ks[0], h_q, ids[-1],
                             float(sm_scale) if sm_scale is not None else 0.0,
                             NO_CAUSAL if q_start_index_s is None else int(q_start_index_s), 1 if lse_is_base2 else 0,
                             query_meta.data_ptr() if query_meta is not None else None)
         if workspace is None:
-            need = lib.smla_fwd_workspace_size(ctypes.byref(params), workspace_budget)
+            need = _fwd_workspace_bytes(s_q, ks[0], h_q, ids[-1], workspace_budget)
             _check(need > 0, "unsupported shapes for the sparse MLA forward")
-            workspace = Workspace(need, q.device)
-        stream = torch.cuda.current_stream().cuda_stream
-        _raise_status(lib, lib.smla_fwd_run(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream), "smla_fwd_run")
+            workspace = Workspace(need, q.device) if workspace_budget else _cached_workspace(need, q.device)
+        stream = _raw_stream(index)
+        st = lib.smla_fwd_run(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream)
+        if st:
+            _raise_status(lib, st, "smla_fwd_run")
         if check_device_status:
             _raise_status(lib, lib.smla_bwd_status(workspace.ptr, stream), "smla_fwd device status")
     return o, lse
@@ -511,14 +597,14 @@ def index_inverse(indices: torch.Tensor, s_kv: int, q_start_index_s: Optional[in
     lib = load_library()
     need = lib.smla_index_inverse_workspace_size(s_q, topk, s_kv)
     _check(need > 0, "unsupported shape (s_kv and topk positive, s_q * topk below 2^31)")
-    with torch.cuda.device(indices.device):
-        ws = torch.empty(need, dtype=torch.uint8, device=indices.device)
+    index = indices.get_device()
+    with _on_device(index):
+        ws = _cached_buffer("inverse", need, indices.device)
         row_ptr = torch.empty(s_kv + 1, dtype=torch.int32, device=indices.device)
         entries = torch.empty(s_q * topk, dtype=torch.int32, device=indices.device)
         st = lib.smla_index_inverse(indices.data_ptr(), s_q, topk, s_kv,
                                     NO_CAUSAL if q_start_index_s is None else int(q_start_index_s),
-                                    row_ptr.data_ptr(), entries.data_ptr(), ws.data_ptr(), need,
-                                    torch.cuda.current_stream().cuda_stream)
+                                    row_ptr.data_ptr(), entries.data_ptr(), ws.data_ptr(), need, _raw_stream(index))
     _raise_status(lib, st, "smla_index_inverse")
     return row_ptr, entries
 
