@@ -96,6 +96,27 @@ __device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, const W
     if (mbar_test_wait(bar, parity)) return true;
     return mbar_spin_slow(bar, parity, ctx, code);
 }
+// The consumer's place in a ring of slots, with the barrier of the NEXT slot polled while the current one is worked on: a
+// poll takes a few hundred cycles behind a busy load/store pipe, which a thread that issues UMMAs (or forwards signals)
+// one slot at a time cannot afford per slot (standalone probe, idle SM, slots of four 64-cycle UMMAs: 300 cycles per slot
+// polling when the slot is due, 259 polling ahead).
+template <int kSlots> struct RingReader {
+    uint32_t full0;               // barrier of slot 0
+    uint32_t slot = 0, phase = 0;
+    bool ready = false;           // the current slot has been seen full
+    __device__ __forceinline__ explicit RingReader(uint32_t full0_) : full0(full0_) {}
+    __device__ __forceinline__ void wait(const WaitCtx& ctx, int code) {
+        if (!ready) mbar_spin(full0 + 8 * slot, phase, ctx, code);
+    }
+    // to the next slot, polling it; call before the work on `slot`'s data is issued, with the old slot number kept
+    __device__ __forceinline__ void next() {
+        if (++slot == kSlots) {
+            slot = 0;
+            phase ^= 1;
+        }
+        ready = mbar_test_wait(full0 + 8 * slot, phase);
+    }
+};
 // Bounded wait.  Returns false if it gave up (error `code` recorded) or the CTA is aborting.
 // `sleep_ns` > 0 makes the waiter yield its issue slots between polls: many warps spinning on barriers
 // otherwise starve the single thread that issues the UMMAs of the scheduler they share.
@@ -347,6 +368,10 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_bar
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 #endif
 }
+// The same with the release: for data written by this warp's own stores.
+__device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_2cta(uint32_t dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
                  : "memory");
@@ -384,6 +409,15 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_global_v4_hint(void* addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d,
                                                   uint64_t policy) {
     asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(addr), "r"(a), "r"(b), "r"(c), "r"(d),
@@ -397,17 +431,6 @@ __device__ __forceinline__ void st_global_v8(void* addr, const uint32_t (&v)[8])
 }
 
 // ---- small helpers -----------------------------------------------------------------------------
-// Reductions over the 32 lanes of a warp in one instruction (every lane receives the result).
-__device__ __forceinline__ float redux_max_f32(float v) {
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ unsigned redux_add_u32(unsigned v) {
-    unsigned r;
-    asm volatile("redux.sync.add.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
-    return r;
-}
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -334,14 +334,13 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     ok &= make_map_scratch(&tm_ds, ds_scr, uint64_t(pl.q_chunk), pl.topk_pad, HP, 64);
     if (!ok) return SMLA_ERR_LAUNCH;
 
-    constexpr int kDqParts = kQChunks / kDqChunks;
-    using DqCfg = dq::Cfg<HP, kDqChunks>;
+    using DqCfg = dq::Cfg<HP>;
     static std::atomic<bool> attr_done[kMaxDevices];
     if (!once_per_device(attr_done, [] {
             bool done = set_smem(smla_recompute_pair_kernel<HP>, rp::Cfg<HP>::kSmemBytes);
             done &= set_smem(smla_dkv_pair_kernel<HP>, dp::Cfg<HP>::kSmemBytes);
             done &= set_smem(smla_dkv_pair_kernel<HP, true>, dp::Cfg<HP>::kSmemBytes);
-            done &= set_smem(smla_dq_kernel<HP, kDqChunks, kQChunks>, DqCfg::kSplitSmemBytes);
+            done &= set_smem(smla_dq_kernel<HP>, DqCfg::kSplitSmemBytes);
             return done;
         }))
         return SMLA_ERR_LAUNCH;
@@ -357,7 +356,6 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     kp.ds_scr = ds_scr;
     kp.dKV = p->dKV;
     kp.dQ = reinterpret_cast<__nv_bfloat16*>(p->dQ);
-    kp.gout = kp.dQ;
     kp.g_err = reinterpret_cast<int*>(ws + pl.err_off);
     kp.s_q = p->s_q;
     kp.s_kv = p->s_kv;
@@ -411,10 +409,10 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
         }
         launch(smla_dkv_pair_kernel<HP>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s, tm_ds, kp);
     };
-    const int dq_split = dq_key_split(p->s_q, pl.topk_pad, kDqParts);
+    const int dq_split = dq_key_split(p->s_q, pl.topk_pad, dq::kParts);
     auto launch_dq = [&](cudaStream_t s_, bool pdl, bool after_dkv) {
         kp.dq_after_trigger = after_dkv;
-        launch(smla_dq_kernel<HP, kDqChunks, kQChunks>, kp.nq * kDqParts * dq_split, dq::kThreads,
+        launch(smla_dq_kernel<HP>, kp.nq * dq::kParts * dq_split, dq::kThreads,
                dq_split > 1 ? DqCfg::kSplitSmemBytes : DqCfg::kSmemBytes, s_, pdl, dq_split, tm_ds, kp);
     };
 
@@ -468,10 +466,12 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---- forward ---------------------------------------------------------------------------------------------
-// Workspace: error word | row maxima [s_q, h_q] i32 | row sums [s_q, h_q] u64 | E scratch (bf16, one matrix per query).
+// Workspace: error word | slots in use per query | prefix sum of the queries' tiles | partial results of the queries whose
+// tiles are spread over several clusters, two per cluster.
+constexpr int kMaxFwdClusters = 80;
 struct FwdPlan {
-    int h_pad, topk_pad, q_chunk;
-    size_t err_off, m_off, l_off, s_off, total;
+    int h_pad, topk_pad, clusters;      // clusters: at most this many have room for their partial results
+    size_t err_off, used_off, pre_off, ml_off, o_off, total;
 };
 
 bool check_fwd_params(const smla_fwd_params* p) {
@@ -483,70 +483,46 @@ bool check_fwd_params(const smla_fwd_params* p) {
     return true;
 }
 
-void fwd_layout(const smla_fwd_params* p, FwdPlan* pl, size_t qc) {
-    const size_t unit = size_t(pl->topk_pad) * pl->h_pad * 2;   // one bf16 matrix per query
-    const size_t rows = size_t(p->s_q) * p->h_q;
-    pl->q_chunk = int(qc);
-    pl->err_off = 0;
-    pl->m_off = kAlign;
-    pl->l_off = align_up(pl->m_off + rows * 4, kAlign);
-    pl->s_off = align_up(pl->l_off + rows * 8, kAlign);
-    pl->total = align_up(pl->s_off + qc * unit, kAlign);
-}
-
-bool make_fwd_plan(const smla_fwd_params* p, size_t budget, FwdPlan* pl) {
+// `bytes`: the workspace at hand, or the budget a size is asked for (0: as much as can be used).
+bool make_fwd_plan(const smla_fwd_params* p, size_t bytes, FwdPlan* pl) {
     if (!check_fwd_params(p)) return false;
     pl->h_pad = p->h_q <= 64 ? 64 : 128;
-    pl->topk_pad = (p->topk + 511) / 512 * 512;   // the logits kernel walks pairs of 256-key tiles
-    const size_t unit = size_t(pl->topk_pad) * pl->h_pad * 2;
-    if (budget == 0) budget = kDefaultBudget;
-    fwd_layout(p, pl, 1);
-    const size_t fixed = pl->s_off;
-    size_t qc = budget > fixed ? (budget - fixed) / unit : 0;
-    if (qc < 1) qc = 1;
-    if (qc > size_t(p->s_q)) qc = p->s_q;
-    while (qc > 1 && qc * size_t(pl->topk_pad) > size_t(INT_MAX)) qc /= 2;
-    fwd_layout(p, pl, qc);
+    pl->topk_pad = (p->topk + smla::kWorkTileKeys - 1) / smla::kWorkTileKeys * smla::kWorkTileKeys;
+    pl->err_off = 0;
+    pl->used_off = kAlign;
+    pl->pre_off = pl->used_off + size_t(p->s_q) * 4;
+    pl->ml_off = align_up(pl->pre_off + (size_t(p->s_q) + 1) * 4, kAlign);
+    const size_t per_cluster = 2 * size_t(pl->h_pad) * (SMLA_D_V + 2) * 4;
+    const long long tiles = static_cast<long long>(p->s_q) * (pl->topk_pad / smla::kWorkTileKeys);
+    long long c = std::min<long long>(kMaxFwdClusters, tiles);
+    if (bytes) c = std::min<long long>(c, bytes > pl->ml_off + kAlign ? (bytes - pl->ml_off - kAlign) / per_cluster : 0);
+    if (c < 2) c = 0;                   // one cluster has every query whole
+    pl->clusters = int(c);
+    pl->o_off = align_up(pl->ml_off + 2 * size_t(c) * pl->h_pad * 8, kAlign);
+    pl->total = pl->o_off + 2 * size_t(c) * pl->h_pad * SMLA_D_V * 4;
     return true;
 }
 
 bool fwd_plan_for_workspace(const smla_fwd_params* p, size_t ws_bytes, FwdPlan* pl) {
-    if (!make_fwd_plan(p, ws_bytes, pl)) return false;
-    const size_t unit = size_t(pl->topk_pad) * pl->h_pad * 2;
-    while (pl->total > ws_bytes && pl->q_chunk > 1) {
-        const size_t over = pl->total - ws_bytes;
-        const int dec = int(over / unit) + 1;
-        fwd_layout(p, pl, pl->q_chunk - dec < 1 ? 1 : pl->q_chunk - dec);
-    }
-    return pl->total <= ws_bytes;
+    return make_fwd_plan(p, ws_bytes, pl) && pl->total <= ws_bytes;
 }
 
-// Three passes over the queries: row maxima of the logits (nothing but 4 bytes per row is written); E = exp2(logit -
-// max) as bf16 into the scratch plus its row sums; o = E.V divided by the sum on the way out, and lse.  The logits are
-// computed twice (576 of the forward's 1088 multiply-adds per slot) in exchange for never existing in memory.
 template <int HP>
 int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, cudaStream_t st) {
     using namespace smla;
     if (!bind_context()) return SMLA_ERR_LAUNCH;
-    __nv_bfloat16* s_scr = reinterpret_cast<__nv_bfloat16*>(ws + pl.s_off);
-    CUtensorMap tm_qnh, tm_s;
-    const uint64_t qrows = uint64_t(p->s_q) * p->h_q;
-    bool ok = true;
-    ok &= make_map_2d(&tm_qnh, p->q, kDQK, qrows, kDQK * 2, 64, HP / 2);
-    ok &= make_map_scratch(&tm_s, s_scr, uint64_t(pl.q_chunk), pl.topk_pad, HP, 64);
-    if (!ok) return SMLA_ERR_LAUNCH;
-    bool attr_ok = set_smem(smla_fwd_logits_pair_kernel<HP, 1>, fp::Cfg<HP>::kSmemBytes);
-    attr_ok &= set_smem(smla_fwd_logits_pair_kernel<HP, 2>, fp::Cfg<HP>::kSmemBytes);
-    // o = E.V: the two d-parts gather V column chunks [0,4) and [4,8)
-    attr_ok &= set_smem(smla_dq_kernel<HP, kVChunks / 2, kVChunks, true>, dq::Cfg<HP, kVChunks / 2>::kSmemBytes);
-    if (!attr_ok) return SMLA_ERR_LAUNCH;
+    CUtensorMap tm_q;
+    if (!make_map_2d(&tm_q, p->q, kDQK, uint64_t(p->s_q) * p->h_q, kDQK * 2, 64, HP / 2)) return SMLA_ERR_LAUNCH;
+    static std::atomic<bool> attr_done[kMaxDevices];
+    if (!once_per_device(attr_done, [] { return set_smem(smla_fwd_kernel<HP>, ff::kSmemBytes); })) return SMLA_ERR_LAUNCH;
 
     KParams kp{};
     kp.kv = reinterpret_cast<const __nv_bfloat16*>(p->kv);
     kp.indices = p->indices;
-    kp.s_scr = s_scr;
-    kp.m_ord = reinterpret_cast<int*>(ws + pl.m_off);
-    kp.l_fix = reinterpret_cast<unsigned long long*>(ws + pl.l_off);
+    kp.n_used = reinterpret_cast<const int*>(ws + pl.used_off);
+    kp.tile_pre = reinterpret_cast<const int*>(ws + pl.pre_off);
+    kp.part_ml = reinterpret_cast<float2*>(ws + pl.ml_off);
+    kp.part_o = reinterpret_cast<float*>(ws + pl.o_off);
     kp.lse_out = p->lse;
     kp.lse_out_mult = p->lse_is_base2 ? 1.0f : 0.6931471805599453f;
     kp.g_err = reinterpret_cast<int*>(ws + pl.err_off);
@@ -562,23 +538,17 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     kp.gout = reinterpret_cast<__nv_bfloat16*>(p->o);
     kp.qmeta = reinterpret_cast<const int4*>(p->query_meta);
     kp.wait_limit = g_wait_limit.load();
-    kp.scr0 = 0;
-    const int n_rows = p->s_q * p->h_q;
-    smla_fwd_stats_init_kernel<<<(n_rows + 255) / 256, 256, 0, st>>>(kp.m_ord, kp.l_fix, n_rows);
-    ++g_last_launches;
-    const int pairs_1 = resident_pairs(smla_fwd_logits_pair_kernel<HP, 1>, fp::kThreads, fp::Cfg<HP>::kSmemBytes);
-    const int pairs_2 = resident_pairs(smla_fwd_logits_pair_kernel<HP, 2>, fp::kThreads, fp::Cfg<HP>::kSmemBytes);
-    if (pairs_1 <= 0 || pairs_2 <= 0) return SMLA_ERR_LAUNCH;
-    for (int q0 = 0; q0 < p->s_q; q0 += pl.q_chunk) {
-        const int nq = (p->s_q - q0 < pl.q_chunk) ? p->s_q - q0 : pl.q_chunk;
-        kp.q0 = q0;
-        kp.nq = nq;
-        // persistent 2-CTA clusters, one per SM pair (each CTA takes the whole shared memory of its SM)
-        smla_fwd_logits_pair_kernel<HP, 1><<<2 * (nq < pairs_1 ? nq : pairs_1), fp::kThreads, fp::Cfg<HP>::kSmemBytes, st>>>(tm_qnh, kp);
-        smla_fwd_logits_pair_kernel<HP, 2><<<2 * (nq < pairs_2 ? nq : pairs_2), fp::kThreads, fp::Cfg<HP>::kSmemBytes, st>>>(tm_qnh, kp);
-        smla_dq_kernel<HP, kVChunks / 2, kVChunks, true><<<nq * 2, dq::kThreads, dq::Cfg<HP, kVChunks / 2>::kSmemBytes, st>>>(tm_s, kp);
-        g_last_launches += 3;
-    }
+    kp.q0 = 0;
+    kp.nq = p->s_q;
+    launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, static_cast<const uint4*>(nullptr), static_cast<const uint4*>(nullptr),
+           static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), reinterpret_cast<int*>(ws + pl.pre_off),
+           reinterpret_cast<int*>(ws + pl.err_off) + kTicketWord, static_cast<uint4*>(nullptr), size_t(0), kp);
+    const int pairs = resident_pairs(smla_fwd_kernel<HP>, ff::kThreads, ff::kSmemBytes);
+    if (pairs <= 0) return SMLA_ERR_LAUNCH;
+    const int clusters = std::max(1, std::min(pairs, pl.clusters));
+    launch(smla_fwd_kernel<HP>, 2 * clusters, ff::kThreads, ff::kSmemBytes, st, true, 1, tm_q, kp);
+    if (clusters > 1)
+        launch(smla_fwd_combine_kernel, (clusters - 1) * ((p->h_q + 7) / 8), 256, 0, st, true, 1, kp, clusters, HP);
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 

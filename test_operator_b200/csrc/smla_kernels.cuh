@@ -10,9 +10,8 @@
 //              fp32 reduction per (key, 32 consecutive d) straight from TMEM registers
 //   dq         dQ[head, d] = dS^T K_g (tcgen05, heads on the M axis, d on N) accumulated over all keys
 //
-// The forward (o, lse for the same indices) has a logits kernel of its own (2-CTA pairs with Q resident and two tiles
-// in flight), run once to find every row's maximum logit and once to write E = exp2(logit - max) and the row sums, and
-// reuses the dq kernel on the V columns, dividing by the sums on the way out.
+// The forward (o, lse for the same indices) is one kernel of its own, smla_fwd_kernel: heads on the M axis, an online
+// softmax between the two contractions, nothing but o and lse written.
 //
 // Heads are padded to HP = 64 or 128, so h_q = 16 / 64 / 128 use the same code.  Gathered kv rows and
 // Q / dO are held as 128-byte-swizzled [rows x 64 bf16] chunks (kv rows by 16-byte cp.async, Q / dO by
@@ -47,12 +46,11 @@ struct KParams {
     float* staging;           // reproducible mode: [q_chunk][topk_pad slots][576] fp32, one row per slot
     __nv_bfloat16* dQ;        // [s_q, h_q, 576]
     // forward only
-    int* m_ord;               // [s_q, h_q] row maximum of the raw logits Q.K, as order-preserving integers
-    unsigned long long* l_fix;// [s_q, h_q] row sum of exp2(logit - max) in 2^-22 fixed point
     float* lse_out;           // [s_q, h_q]
     float lse_out_mult;       // 1 (base 2) or ln 2 (natural log)
-    // dq-style kernel: where the result goes (dQ with pitch 576, or o with pitch 512)
-    __nv_bfloat16* gout;      // [s_q, h_q, 576] (dQ) or [s_q, h_q, 512] (o)
+    float* part_o;            // partial results of queries spread over several clusters: [slot][HP][512]
+    float2* part_ml;          // [slot][HP] {reference of the exponentials (log2), sum}
+    __nv_bfloat16* gout;      // [s_q, h_q, 512] o (forward only)
     int* g_err;
     int q0;                   // first query (global row) of this launch
     int nq;                   // queries in this launch
@@ -107,18 +105,6 @@ __device__ __forceinline__ bool slot_valid(int idx, int key, const QMeta& m, con
     return key < m.topk_len && idx >= 0 && idx < m.kv_len && m.kv_base + idx < p.s_kv && (!p.causal || idx <= m.q_pos);
 }
 
-// fp32 <-> integers that compare like the floats they came from (so that integer max instructions and atomics work
-// on them); -inf maps to the smallest value used
-__device__ __forceinline__ int float_to_ordered(float x) {
-    const int i = __float_as_int(x);
-    return i ^ ((i >> 31) & 0x7fffffff);
-}
-__device__ __forceinline__ float ordered_to_float(int o) {
-    return __int_as_float(o ^ ((o >> 31) & 0x7fffffff));
-}
-constexpr int kOrderedNegInf = static_cast<int>(0xff800000u ^ 0x7fffffffu);   // float_to_ordered(-inf)
-constexpr float kFixScale = 4194304.f;                                           // 2^22
-
 __device__ __forceinline__ float dot8_bf16(const uint4& a, const uint4& b, float acc) {
     const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
     const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
@@ -162,7 +148,7 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 
 // =============================================================================================
 // prep: everything the three tensor-core kernels need that is not a contraction, in one launch.
-//   block b < s_q   Delta of query b's rows, and n_used[b]: the slots up to the query's last valid one (early tokens of a
+//   block b < s_q   Delta of query b's rows (backward), and n_used[b]: the slots up to the query's last valid one (early tokens of a
 //                   causal sequence use a fraction of their top-k, the rest are out-of-range values at the end)
 //   every block     its share of dKV cleared (where the caller wants it cleared)
 //   last block      prefix sum of the queries' 256-key tiles, from which the persistent kernels take their ranges
@@ -226,7 +212,17 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
         is_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
         __threadfence();
     }
-    if (q < p.s_q) {
+    if (q < p.s_q && O == nullptr) {             // forward: a query without a valid slot is in nobody's range
+        int m = -1;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) m = max(m, red[w]);
+        if (m < 0) {
+            uint4* o = reinterpret_cast<uint4*>(p.gout) + static_cast<size_t>(q) * p.h_q * (kDV / 8);
+            for (int i = threadIdx.x; i < p.h_q * (kDV / 8); i += kPrepThreads) o[i] = make_uint4(0, 0, 0, 0);
+            for (int h = threadIdx.x; h < p.h_q; h += kPrepThreads)
+                p.lse_out[static_cast<size_t>(q) * p.h_q + h] = __int_as_float(0x7f800000) * p.lse_out_mult;
+        }
+    } else if (q < p.s_q) {
         const uint4* o = O + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
         const uint4* g = dO + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
         // two rows at a time: eight 16-byte loads of a lane in flight
@@ -307,13 +303,16 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 struct WorkRange {
     int begin, end, q;            // positions in tile_pre's numbering; the query `begin` lies in
 };
+__device__ __forceinline__ int range_start(int t0, int t1, int cluster, int n_clusters) {
+    return t0 + static_cast<int>(static_cast<long long>(t1 - t0) * cluster / n_clusters);
+}
 // One warp: which range is this cluster's.  32-way search over the prefix sums (two rounds up to 1024 queries).
 __device__ __forceinline__ WorkRange find_range(const KParams& p, int cluster, int n_clusters) {
     const int lane = threadIdx.x & 31;
     const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
     WorkRange w;
-    w.begin = t0 + static_cast<int>(static_cast<long long>(t1 - t0) * cluster / n_clusters);
-    w.end = t0 + static_cast<int>(static_cast<long long>(t1 - t0) * (cluster + 1) / n_clusters);
+    w.begin = range_start(t0, t1, cluster, n_clusters);
+    w.end = range_start(t0, t1, cluster + 1, n_clusters);
     int lo = p.q0, n = p.nq;      // the last query in [lo, lo + n) whose first tile is at or before `begin`
     while (n > 1) {
         const int step = (n + 31) >> 5;
@@ -325,6 +324,12 @@ __device__ __forceinline__ WorkRange find_range(const KParams& p, int cluster, i
     }
     w.q = lo;
     return w;
+}
+// Broadcast, so that the compiler knows the bounds of the loops below to be the same in all lanes: it then keeps what the
+// UMMAs of an issuing thread need (descriptors, addresses) in uniform registers, where tcgen05.mma takes its operands from.
+// With a loop bound or a ring position it takes for lane-dependent it moves every operand over first.
+__device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
+    return WorkRange{__shfl_sync(0xffffffffu, w.begin, 0), __shfl_sync(0xffffffffu, w.end, 0), __shfl_sync(0xffffffffu, w.q, 0)};
 }
 template <int kMul> struct TileIter {
     const int* pre;
@@ -463,8 +468,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const WorkRange range = *range_s;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const WorkRange range = uniform_range(*range_s);
     static_assert(kTileKeys == kWorkTileKeys, "one work tile per accumulator");
 
     if (warp >= 8 && warp < 16) {
@@ -544,23 +549,22 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         if (elect_one()) {
             if (rank == 1) {
                 // -------------------------------------------------------------- forward slot-full to the even CTA
-                int s = 0;
-                uint32_t ph = 0, qpar = 0;
+                RingReader<kStages> ring(bar_full);
+                const uint32_t full_even = map_to_cta(bar_full, 0);
+                uint32_t qpar = 0;
                 bool new_query = true;
                 for (TileIter<1> it(p, range); it.more();) {
                     for (int j = 0; j < kQChunks; ++j) {
                         // this CTA's half of Q / dO is part of what "full" promises
                         if (new_query) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 15);
-                        mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 17);
+                        ring.wait(wc, kErrRecompute + 17);
+                        const uint32_t s = ring.slot;
+                        ring.next();
                         // The copies have landed in this CTA's shared memory (the wait above saw them complete);
                         // make them visible to the tensor core's proxy here, then signal without a cluster-scope
                         // release, which would cost this thread about a thousand cycles per chunk.
                         fence_proxy_async_smem();
-                        mbar_arrive_cluster_relaxed(map_to_cta(bar_full + 8 * s, 0));
-                        if (++s == kStages) {
-                            s = 0;
-                            ph ^= 1;
-                        }
+                        mbar_arrive_cluster_relaxed(full_even + 8 * s);
                     }
                     new_query = it.advance();
                     if (new_query) qpar ^= 1;
@@ -574,17 +578,23 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 const uint32_t desc_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
                 const uint32_t a_lo0 = desc_lo + desc_addr(s_base + C::kOffRing);
                 const uint32_t b_lo0 = desc_lo + desc_addr(s_base + C::kOffB);
-                int s = 0, gt = 0;              // ring slot; tiles so far
-                uint32_t ph = 0, qpar = 0;
+                RingReader<kStages> ring(bar_full);
+                int gt = 0;                     // tiles so far
+                uint32_t qpar = 0;
                 bool new_query = true;
-                for (TileIter<1> it(p, range); it.more(); ++gt) {
+                TileIter<1> it(p, range);
+                const int n_tiles = range.end - range.begin;
+                for (; gt < n_tiles; ++gt) {
                     const int b = gt & 1;
                     const bool last = it.last_of_query();
                     mbar_spin(bar_tempty + 8 * b, ((gt >> 1) & 1) ^ 1, wc, kErrRecompute + 13);
                     const uint32_t d = tmem + b * C::kAccCols;
+#pragma unroll
                     for (int j = 0; j < kQChunks; ++j) {
                         if (new_query) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrRecompute + 12);
-                        mbar_spin(bar_full + 8 * s, ph, wc, kErrRecompute + 14);
+                        ring.wait(wc, kErrRecompute + 14);
+                        const uint32_t s = ring.slot;
+                        ring.next();
                         tc_fence_after_sync();
                         const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
                         const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
@@ -593,10 +603,6 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                             umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, (j | kk) != 0);
                         umma_commit_2cta_mask(bar_empty + 8 * s, 3);
                         if (last) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);   // the next query's chunk may come in
-                        if (++s == kStages) {
-                            s = 0;
-                            ph ^= 1;
-                        }
                     }
                     umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
                     new_query = it.advance();
@@ -716,418 +722,545 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 }
 
 // =============================================================================================
-// forward logits as persistent 2-CTA clusters: one pair per query (queries round-robin).
+// forward: o = softmax(scale q K_g^T) V_g and lse in one pass over the keys, as persistent 2-CTA clusters.
 //
-// With B = Q only there is no dO to share the shared memory with: a CTA holds Q of HALF the heads (9 chunks of
-// [HP/2 heads x 64 col], 72 KB at 128 heads), which leaves nine ring slots for the gathered keys.
-//   cta_group::2 UMMAs of M = 256 keys (128 gathered by each CTA) x N = HP heads (HP/2 supplied by each CTA) x K = 16;
-//   D  this CTA's [128 keys] x [HP heads] in TMEM, four buffers of HP columns
-//   warps 0-7   row statistics / exponentials on the CTA's own keys: warp w -> TMEM lane quarter w % 4, head half w / 4
-//   warps 8-15  gather producers (cp.async 16 B, swizzled), one group of four warps per tile stream
-//   warps 16-19 even CTA: the four UMMA issuers for the pair; odd CTA: warp 16 forwards "my slot is full"
-//   warp 20     TMA of the CTA's Q chunks
-// Two 256-key tiles are in flight at a time, as two independent streams (the even tiles and the odd tiles): each stream
-// has its own producer group, its own ring slots (five and four), its own pair of accumulator buffers (one is read by
-// the statistics warps while the other fills) and two issuers; the streams share only the tensor pipe.  Ring slots of
-// its own matter: a producer group that fills a slot has then itself seen the slot's previous use, so its wait on the
-// phase parity of "slot free" cannot be satisfied by the phase before last (with one ring shared by the two groups a
-// group that ran ahead of the other overwrote a slot in use and arrived twice on one barrier phase).
-// A stream is shared by two issuers that take alternate chunks (one polls and commits while the other's UMMAs run) and
-// hand over through a counter in shared memory: the UMMAs of an accumulator enter the pipe in chunk order and the result
-// is reproducible bit for bit.
-// Slot-free, chunk-free and accumulator-ready signals are tcgen05.commit arrivals delivered to both CTAs.
-// kMode 1: row maxima only (atomicMax per head at the end of a query); kMode 2: E = exp2(logit - max) as bf16 into the
-// scratch (the backward's S layout) and the row sums in 2^-22 fixed point.
+// Heads are the M side of both contractions (cta_group::2 UMMAs of M = 128: 64 head rows per CTA, which run at the full
+// rate of the pair: a 128 x 256 x 16 UMMA takes 64 cycles), so a head's logits, probabilities and outputs all sit in the
+// same tensor-memory lanes of the same CTA: no exchange of probabilities between the CTAs and row statistics that are
+// local to four threads.
+//   S  [64 heads per CTA x 256 keys] = Q . K_g^T    A = this CTA's Q rows (resident, 72 KB), B = this CTA's 128 gathered
+//      keys; lanes 0-63 hold keys 0-127 of the tile, lanes 64-127 the same heads with keys 128-255; two buffers
+//   O  [64 heads per CTA x 512 d] += P . V_g        A = P (bf16, written to shared memory by the softmax warps), B = for two
+//      d-blocks of 256 this CTA's 128 columns of all 256 keys, gathered a second time in that form
+//   tensor memory: O 2 x 128 columns, S 2 x 128 columns
+// Both gathers go through one ring of 16 KB slots in the order the UMMAs consume them: K of tile n + 1 (nine slots of
+// [128 keys x 64 columns]), then V of tile n (eight slots of [64 keys x 128 columns]); a slot feeds four UMMAs of 64
+// cycles either way, and the softmax of tile n runs under the UMMAs of S n + 1.
+//   warps 0-7   softmax: warp w reads lane quarter w % 4, columns [64 (w / 4), + 64) of S: one head, 64 keys per thread
+//   warps 8-15  gather producers (cp.async 16 B, swizzled)
+//   warp 16     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full"
+//   warp 17     TMA of the CTA's Q chunks
+// Row maxima are used lazily: the exponentials are taken against a reference that is only moved (and O rescaled) when a
+// tile's maximum exceeds it by more than 2^8, so O is rescaled once in a while instead of once per tile; nothing
+// depends on timing, o and lse repeat bit for bit.
+// What bounds it: per tile and CTA 17 slots x 4 UMMAs x 64 cycles = 4352 cycles of tensor pipe; 275 KB of gathered rows
+// written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Measured (4096 queries x 128 heads x
+// top-k 2048): 8100 cycles a tile, 2.25 ms at the 1.65 GHz the power cap leaves, against 3.27 ms for two logit passes and
+// an E.V pass; without the gathers 7000 cycles, without the softmax 6300, without both 6100.  The ring's depth does not
+// matter (five, six or seven slots: 2.32 / 2.32 / 2.31 ms).  Row gathers by TMA (tile::gather4 from eight warps) in place
+// of cp.async: 3.0 ms; two producer groups on alternate slots: 2.36 ms; one arrival per producer warp: 2.34 ms.
+// With 64 heads half of the UMMAs' rows are zeros: 2.4 ms.
+// A query whose tiles lie in several clusters' ranges leaves unnormalised partial results, which
+// smla_fwd_combine_kernel adds up.
 // =============================================================================================
-namespace fp {
-constexpr int kProducerWarps = 8;
-constexpr int kProducerThreads = 32 * kProducerWarps;
-constexpr int kRowStep = 2 * kProducerWarps;              // a producer thread copies rows r0 + kRowStep * i of its tile
-constexpr int kRowsPerThread = 128 / kRowStep;
-constexpr int kIssuerWarp = 8 + kProducerWarps;           // the first issuer warp
-constexpr int kIssuersPerStream = 2;
-constexpr int kIssuers = 2 * kIssuersPerStream;
-constexpr int kThreads = 256 + kProducerThreads + 32 * kIssuers + 32;   // statistics, producers, issuers, Q loader
+namespace ff {
+constexpr int kThreads = 576;
+constexpr int kProducerThreads = 256;
 constexpr int kTileKeys = 256;             // per pair; 128 per CTA
-constexpr int kChunkA = 128 * 128;
-template <int HP> struct Cfg {
-    static constexpr int kBChunk = (HP / 2) * 128;                 // Q_j of this CTA's heads
-    static constexpr int kStages = HP == 128 ? 9 : 11;
-    // every tile stream has ring slots of its own (a slot is then always filled by the same producer group, which has
-    // seen its previous use: waits on a barrier's phase parity cannot be taken for the phase before last)
-    static constexpr int kStages0 = (kStages + 1) / 2;             // stream 0: slots [0, kStages0)
-    static constexpr int kStages1 = kStages / 2;                   // stream 1: slots [kStages0, kStages)
-    static constexpr int kOffB = 0;
-    static constexpr int kOffRing = kQChunks * kBChunk;
-    static constexpr int kOffMisc = kOffRing + kStages * kChunkA;
-    static constexpr int kSmemBytes = kOffMisc + 1024 + 512 + 1024;   // row maxima + barriers + alignment slack
-    static constexpr int kTmemCols = 4 * HP;                       // two pairs of accumulator buffers
-    static_assert(kSmemBytes <= 232448, "shared memory of one SM");
-};
-}  // namespace fp
+constexpr int kSlotBytes = 16384;
+constexpr int kStages = 7;
+constexpr int kQChunk = 64 * 128;          // [64 head rows x 64 columns]
+constexpr int kPChunk = 64 * 128;          // [64 head rows x 64 keys]
+constexpr int kVSlots = 8;                 // per tile: four groups of 64 keys x two d-blocks
+constexpr int kOffQ = 0;
+constexpr int kOffP = kQChunks * kQChunk;
+constexpr int kOffRing = kOffP + 4 * kPChunk;
+constexpr int kOffRows = kOffRing + kStages * kSlotBytes;     // [3 tiles][256] kv rows
+constexpr int kOffStat = kOffRows + 3 * kTileKeys * 4;        // [2 tile parities][4 key quarters][64 heads] row maxima / sums
+constexpr int kOffMisc = kOffStat + 2 * 4 * 64 * 4;
+constexpr int kSmemBytes = kOffMisc + 512 + 1024;             // barriers + alignment slack
+constexpr int kTmemO = 0, kTmemS = 256;
+constexpr float kMaxLag = 8.f;             // how far (log2) a row's logits may exceed the reference of its exponentials
+constexpr int kPartFloats = kDV;           // a partial result: [HP heads][512] fp32 and [HP heads]{reference, sum}
+static_assert(kSmemBytes <= 232448, "shared memory of one SM");
+}  // namespace ff
 
-template <int HP, int kMode>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(fp::kThreads, 1)
-smla_fwd_logits_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
-    using namespace fp;
-    using C = Cfg<HP>;
-    constexpr int NH = HP / 2;
-    constexpr int kStages = C::kStages;
+template <int HP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ff::kThreads, 1)
+smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
+    using namespace ff;
+    constexpr int NH = HP / 2;               // heads of this CTA (of the 64 rows the UMMAs compute)
+    constexpr int kSoftmaxWarps = NH / 8;    // with 64 heads a CTA's rows 32-63 do not exist: the warps of that lane quarter idle
     const uint32_t rank = cluster_ctarank();
-    const int cta = blockIdx.x >> 1;         // the pair
-    const int n_ctas = gridDim.x >> 1;
-    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t s_base = smem_u32(smem);
-    uint8_t* misc = smem + C::kOffMisc;
-    float* m2_s = reinterpret_cast<float*>(misc);             // [HP] row maximum in base-2 units, +inf for padded heads
-    uint64_t* bars = reinterpret_cast<uint64_t*>(misc + 1024);
-    const uint32_t bar_full = smem_u32(bars);               // [kStages] gathered chunk landed
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffMisc);
+    const uint32_t bar_full = smem_u32(bars);               // [kStages] slot landed (even CTA: in both CTAs)
     const uint32_t bar_empty = bar_full + 8 * kStages;      // [kStages] the UMMAs reading the slot finished
-    const uint32_t bar_bfull = bar_empty + 8 * kStages;     // [9] Q column chunk of the current query landed
-    const uint32_t bar_bfree = bar_bfull + 8 * kQChunks;    // [9] the query's last UMMAs on the chunk finished
-    const uint32_t bar_tfull = bar_bfree + 8 * kQChunks;    // [4] accumulator buffer complete
-    const uint32_t bar_tempty = bar_tfull + 32;             // [4] the softmax warps have read the buffer
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 1024 + 8 * (2 * kStages + 2 * kQChunks + 8));
+    const uint32_t bar_qfull = bar_empty + 8 * kStages;     // [9] Q column chunk of the current query landed
+    const uint32_t bar_qfree = bar_qfull + 8 * kQChunks;    // [9] the query's last UMMAs on the chunk finished
+    const uint32_t bar_tfull = bar_qfree + 8 * kQChunks;    // [2] S buffer complete
+    const uint32_t bar_tempty = bar_tfull + 16;             // [2] (even CTA) both CTAs have read the S buffer
+    const uint32_t bar_pfull = bar_tempty + 16;             // (even CTA) P of the tile written in both CTAs
+    const uint32_t bar_pv = bar_pfull + 8;                  // O += P V of the tile finished
+    const uint32_t bar_drain = bar_pv + 8;                  // used only while winding down after an abort
+    constexpr int kBars = 2 * kStages + 2 * kQChunks + 7;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc + 8 * kBars);
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const uint32_t tok = smem_u32(tmem_slot + 2);           // [2] chunks issued so far in each stream: the issuers' hand-over
-    const uint32_t bar_drain = smem_u32(tmem_slot + 4);     // [kIssuers] used only while winding down after an abort
-    static_assert(8 * (2 * kStages + 2 * kQChunks + 8) + 16 + 8 * kIssuers <= 512, "barrier area");
+    WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 2);
+    static_assert(8 * kBars + 8 + sizeof(WorkRange) <= 512, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
         *s_abort = 0;
-        tmem_slot[2] = tmem_slot[3] = 0;
         for (int i = 0; i < kStages; ++i) {
-            // the even CTA's "full" also counts one arrival forwarded from the odd CTA
-            mbar_init(bar_full + 8 * i, kProducerThreads / 2 + (rank == 0 ? 1 : 0));   // one producer group per slot
+            mbar_init(bar_full + 8 * i, kProducerThreads + (rank == 0 ? 1 : 0));   // + the odd CTA's forwarded arrival
             mbar_init(bar_empty + 8 * i, 1);
         }
         for (int i = 0; i < kQChunks; ++i) {
-            mbar_init(bar_bfull + 8 * i, 1);
-            mbar_init(bar_bfree + 8 * i, 2);     // both issuers' last UMMAs on the chunk
+            mbar_init(bar_qfull + 8 * i, 1);
+            mbar_init(bar_qfree + 8 * i, 1);
         }
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 2; ++i) {
             mbar_init(bar_tfull + 8 * i, 1);
-            mbar_init(bar_tempty + 8 * i, 16);   // eight statistics warps in each CTA
+            mbar_init(bar_tempty + 8 * i, 2 * kSoftmaxWarps);
         }
-        for (int i = 0; i < kIssuers; ++i) mbar_init(bar_drain + 8 * i, 1);
+        mbar_init(bar_pfull, 2 * kSoftmaxWarps);
+        mbar_init(bar_pv, 1);
+        mbar_init(bar_drain, 1);
         fence_mbar_init();
     }
-    if (warp == kIssuerWarp) {
-        tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
+    if constexpr (NH < 64) {     // head rows that do not exist: computed from zeros, never read
+        for (int i = threadIdx.x; i < kQChunks * (64 - NH) * 8; i += kThreads) {
+            const int j = i / ((64 - NH) * 8), r = i % ((64 - NH) * 8);
+            *reinterpret_cast<uint4*>(smem + kOffQ + j * kQChunk + NH * 128 + r * 16) = make_uint4(0, 0, 0, 0);
+        }
+        fence_proxy_async_smem();
+    }
+    if (warp == 16) {
+        tmem_alloc_2cta(smem_u32(tmem_slot), 512);
         tmem_relinquish_2cta();
+    }
+    if (warp == 17 && lane == 0) tma_prefetch_desc(&tm_q);
+    pdl_wait();                  // the prep kernel's tile counts
+    pdl_trigger();
+    if (warp == 17) {
+        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
+        if (lane == 0) *range_s = w;
     }
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const int n_tp = p.topk_pad / (2 * kTileKeys);      // tile pairs; the forward pads the top-k to a multiple of 512
-    const int nq = p.nq;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const WorkRange range = uniform_range(*range_s);
+    const int n_tiles = range.end - range.begin;
 
-    if (warp >= 8 && warp < kIssuerWarp) {
+    if (warp >= 8 && warp < 16) {
         // ------------------------------------------------------------------ gather producers
-        // Two groups of kProducerWarps / 2 warps, one per tile stream: group x fills every second ring position, the
-        // chunks of tile 2t + x, so a warp waits and arrives once per two positions and the streams do not hold each
-        // other up.
-        const int grp = (warp - 8) / (kProducerWarps / 2);
-        const int pt = threadIdx.x - 256 - grp * (kProducerThreads / 2);
-        const int u = pt & 7;               // 16-byte unit inside a 128-byte chunk row
-        const int r0 = pt >> 3;             // rows r0 + kRowStep * i of the CTA's 128 keys
-        const uint32_t dst0 = s_base + C::kOffRing + r0 * 128 + ((u ^ (r0 & 7)) << 4);
-        const char* kvb = reinterpret_cast<const char*>(p.kv) + u * 16;
+        const int pt = threadIdx.x - 256;   // 0..255
+        const char* kvb = reinterpret_cast<const char*>(p.kv);
         const uint64_t pol_keep = l2_policy_evict_last();
-        // raw index values, loaded one tile ahead and turned into kv rows when they are used
-        QMeta qm_next = load_qmeta(p, p.q0 + (cta < nq ? cta : 0));
-        int idx_next[kRowsPerThread];
-        auto load_idx = [&](int ql, int tp) {
-            if (ql >= nq) {
-#pragma unroll
-                for (int i = 0; i < kRowsPerThread; ++i) idx_next[i] = -1;
-                return;
-            }
-            if (tp == 0) qm_next = load_qmeta(p, p.q0 + ql);
-#pragma unroll
-            for (int i = 0; i < kRowsPerThread; ++i) {
-                const int key = (2 * tp + grp) * kTileKeys + static_cast<int>(rank) * 128 + r0 + kRowStep * i;
-                idx_next[i] = key < p.topk ? __ldg(p.indices + static_cast<size_t>(p.q0 + ql) * p.topk + key) : -1;
+        int* rows = reinterpret_cast<int*>(smem + kOffRows);
+        // K: thread copies 16-byte unit uk of rows rk + 32 i of this CTA's 128 keys
+        const int uk = pt & 7, rk = pt >> 3;
+        const uint32_t dst_k = s_base + kOffRing + rk * 128 + ((uk ^ (rk & 7)) << 4);
+        // V: unit uv of the 256 bytes (two swizzled 64-column halves of 8 KB) of rows rv + 16 i of 64 keys
+        const int uv = pt & 15, rv = pt >> 4;
+        const uint32_t dst_v = s_base + kOffRing + (uv >> 3) * 8192 + rv * 128 + (((uv & 7) ^ (rv & 7)) << 4);
+        const char* src_v = kvb + rank * 256 + uv * 16;      // columns [256 block + 128 rank, + 128)
+        int s = 0;
+        uint32_t ph = 1;                    // parity that means "slot free" for the current pass over the ring
+        // key pt of every tile: raw index loaded one tile ahead, turned into a kv row when it is published
+        TileIter<1> it(p, range);
+        QMeta qm = load_qmeta(p, range.q);
+        auto load_idx = [&]() {
+            const int key = it.tile() * kTileKeys + pt;
+            return it.more() && key < p.topk ? __ldg(p.indices + static_cast<size_t>(it.q) * p.topk + key) : -1;
+        };
+        int idx_next = load_idx();
+        auto next_slot = [&]() {
+            cp_async_mbar_arrive_noinc(bar_full + 8 * s);
+            if (++s == kStages) {
+                s = 0;
+                ph ^= 1;
             }
         };
-        load_idx(cta, 0);
-        const int ring0 = grp ? C::kStages0 : 0, ring_n = grp ? C::kStages1 : C::kStages0;
-        int rs = 0;                         // slot of the group's ring
-        uint32_t ph = 1;                    // parity that means "slot free" for the current pass over the ring
-        for (int ql = cta; ql < nq; ql += n_ctas) {
-            for (int tp = 0; tp < n_tp; ++tp) {
-                const char* src[kRowsPerThread];
-                uint32_t nb[kRowsPerThread];    // 0: slot out of range, read nothing and land zeros
+        for (int n = -1; n < n_tiles; ++n) {            // K of tile n + 1, then V of tile n
+            if (n + 1 < n_tiles) {
+                // three buffers: the one written now was last read two steps ago, before the previous step's barrier
+                int* mine = rows + (n + 1) % 3 * kTileKeys;
+                mine[pt] = gather_row(idx_next, qm, p);
+                if (it.advance() && it.more()) qm = load_qmeta(p, it.q);
+                idx_next = load_idx();
+                asm volatile("bar.sync 3, 256;" ::: "memory");
+                const char* src[4];
+                uint32_t nb[4];             // 0: slot out of range, read nothing and land zeros
 #pragma unroll
-                for (int i = 0; i < kRowsPerThread; ++i) {
-                    const int row = gather_row(idx_next[i], qm_next, p);
+                for (int i = 0; i < 4; ++i) {
+                    const int row = mine[rank * 128 + rk + 32 * i];
                     nb[i] = row >= 0 ? 16u : 0u;
-                    src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
+                    src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2) + uk * 16;
                 }
-                if (tp + 1 < n_tp) load_idx(ql, tp + 1);
-                else load_idx(ql + n_ctas, 0);
                 for (int j = 0; j < kQChunks; ++j) {
-                    const int s = ring0 + rs;
                     mbar_wait(bar_empty + 8 * s, ph, wc, kErrFwd + 11, kPollSleepNs);
-                    const uint32_t d = dst0 + s * kChunkA;
+                    const uint32_t d = dst_k + s * kSlotBytes;
 #pragma unroll
-                    for (int i = 0; i < kRowsPerThread; ++i)
-                        cp_async16_zfill_hint(d + i * kRowStep * 128, src[i] + j * 128, nb[i], pol_keep);
-                    cp_async_mbar_arrive_noinc(bar_full + 8 * s);
-                    if (++rs == ring_n) {
-                        rs = 0;
-                        ph ^= 1;
+                    for (int i = 0; i < 4; ++i) cp_async16_zfill_hint(d + i * 32 * 128, src[i] + j * 128, nb[i], pol_keep);
+                    next_slot();
+                }
+            }
+            if (n >= 0) {
+                const int* mine = rows + n % 3 * kTileKeys;
+                for (int g = 0; g < 4; ++g) {
+                    const char* src[4];
+                    uint32_t nb[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = mine[g * 64 + rv + 16 * i];
+                        nb[i] = row >= 0 ? 16u : 0u;
+                        src[i] = src_v + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
+                    }
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        mbar_wait(bar_empty + 8 * s, ph, wc, kErrFwd + 11, kPollSleepNs);
+                        const uint32_t d = dst_v + s * kSlotBytes;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) cp_async16_zfill_hint(d + i * 16 * 128, src[i] + b * 512, nb[i], pol_keep);
+                        next_slot();
                     }
                 }
             }
         }
-    } else if (warp == kIssuerWarp + kIssuers) {
-        // ------------------------------------------------------------------ Q chunks of the query (all heads)
+    } else if (warp == 17) {
+        // ------------------------------------------------------------------ Q chunks of this CTA's heads
         if (lane == 0) {
-            tma_prefetch_desc(&tm_q);
             const uint64_t pol_stream = l2_policy_evict_first();
             uint32_t qpar = 1;              // parity of "chunk free" left by the previous query
-            for (int ql = cta; ql < nq; ql += n_ctas, qpar ^= 1) {
-                const int row0 = (p.q0 + ql) * p.h_q + NH * static_cast<int>(rank);
+            bool first = true;
+            for (TileIter<1> it(p, range); it.more(); first = false, qpar ^= 1) {
+                const int row0 = it.q * p.h_q + NH * static_cast<int>(rank);
                 for (int j = 0; j < kQChunks; ++j) {
-                    if (ql != cta) mbar_wait(bar_bfree + 8 * j, qpar, wc, kErrFwd + 16, kPollSleepNs);
-                    mbar_arrive_expect_tx(bar_bfull + 8 * j, C::kBChunk);
-                    tma_load_2d_hint(s_base + C::kOffB + j * C::kBChunk, &tm_q, 64 * j, row0, bar_bfull + 8 * j, pol_stream);
+                    if (!first) mbar_wait(bar_qfree + 8 * j, qpar, wc, kErrFwd + 16, kPollSleepNs);
+                    mbar_arrive_expect_tx(bar_qfull + 8 * j, NH * 128);
+                    tma_load_2d_hint(s_base + kOffQ + j * kQChunk, &tm_q, 64 * j, row0, bar_qfull + 8 * j, pol_stream);
                 }
+                while (!it.advance()) {}
             }
         }
-    } else if (warp >= kIssuerWarp && warp < kIssuerWarp + kIssuers) {
-        if (rank == 1) {
-            if (warp == kIssuerWarp && elect_one()) {
+    } else if (warp == 16) {
+        if (elect_one()) {
+            if (rank == 1) {
                 // -------------------------------------------------------------- forward slot-full to the even CTA
-                int rs[2] = {0, 0};
-                uint32_t ph[2] = {0, 0}, qpar = 0;
-                for (int ql = cta; ql < nq; ql += n_ctas, qpar ^= 1) {
-                    for (int tp = 0; tp < n_tp; ++tp) {
+                RingReader<kStages> ring(bar_full);
+                const uint32_t full_even = map_to_cta(bar_full, 0);
+                uint32_t qpar = 0;
+                TileIter<1> it(p, range);
+                bool new_query = true;
+                for (int n = -1; n < n_tiles; ++n) {
+                    const int k_slots = n + 1 < n_tiles ? kQChunks : 0;
+                    const int slots = k_slots + (n >= 0 ? kVSlots : 0);
+                    for (int j = 0; j < slots; ++j) {
+                        // this CTA's half of Q is part of what "full" promises
+                        if (j < k_slots && new_query) mbar_wait(bar_qfull + 8 * j, qpar, wc, kErrFwd + 15);
+                        ring.wait(wc, kErrFwd + 17);
+                        const uint32_t s = ring.slot;
+                        ring.next();
+                        // The copies have landed in this CTA's shared memory (the wait above saw them complete); make them
+                        // visible to the tensor core's proxy here, then signal without a cluster-scope release
+                        // (hundreds of cycles per call).
+                        fence_proxy_async_smem();
+                        mbar_arrive_cluster_relaxed(full_even + 8 * s);
+                    }
+                    if (k_slots) {
+                        new_query = it.advance();
+                        if (new_query) qpar ^= 1;
+                    }
+                }
+            } else {
+                // -------------------------------------------------------------- UMMA issuer for the pair
+                constexpr uint32_t idesc_s = make_idesc_bf16(128, 256, 0, 0);
+                constexpr uint32_t idesc_o = make_idesc_bf16(128, 256, 0, 1);      // V: d contiguous (MN-major)
+                const uint64_t k_hi = make_smem_desc(0, 16, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
+                const uint32_t k_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
+                const uint64_t v_hi = make_smem_desc(0, 8192, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
+                const uint32_t v_lo = static_cast<uint32_t>(make_smem_desc(0, 8192, 1024, kSwizzle128)) + desc_addr(s_base + kOffRing);
+                const uint32_t q_lo = k_lo + desc_addr(s_base + kOffQ), p_lo = k_lo + desc_addr(s_base + kOffP);
+                const uint32_t kr_lo = k_lo + desc_addr(s_base + kOffRing);
+                RingReader<kStages> ring(bar_full);
+                uint32_t qpar = 0;
+                TileIter<1> it(p, range);
+                bool new_query = true;
+                uint32_t first_bits = 0;      // bit n & 1: tile n is its query's first in this range
+                for (int n = -1; n < n_tiles; ++n) {
+                    if (n + 1 < n_tiles) {
+                        // S of tile n + 1
+                        const int t = n + 1, b = t & 1;
+                        const bool last = it.last_of_query();
+                        mbar_wait(bar_tempty + 8 * b, ((t >> 1) & 1) ^ 1, wc, kErrFwd + 13);
+                        const uint32_t d = tmem + kTmemS + b * 128;
+#pragma unroll
                         for (int j = 0; j < kQChunks; ++j) {
-                            // this CTA's half of Q is part of what "full" promises
-                            if (tp == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrFwd + 15);
+                            if (new_query) mbar_wait(bar_qfull + 8 * j, qpar, wc, kErrFwd + 12);
+                            ring.wait(wc, kErrFwd + 14);
+                            const uint32_t s = ring.slot;
+                            ring.next();
+                            fence_proxy_async_smem();        // the slot was written by cp.async, the tensor core reads it
+                            tc_fence_after_sync();
+                            const uint32_t a = q_lo + j * (kQChunk >> 4), bb = kr_lo + s * (kSlotBytes >> 4);
 #pragma unroll
-                            for (int sub = 0; sub < 2; ++sub) {
-                                const int s = (sub ? C::kStages0 : 0) + rs[sub];
-                                mbar_spin(bar_full + 8 * s, ph[sub], wc, kErrFwd + 17);
-                                // The copies have landed in this CTA's shared memory (the wait above saw them
-                                // complete); make them visible to the tensor core's proxy here, then signal without
-                                // a cluster-scope release (hundreds of cycles per call).
-                                fence_proxy_async_smem();
-                                mbar_arrive_cluster_relaxed(map_to_cta(bar_full + 8 * s, 0));
-                                if (++rs[sub] == (sub ? C::kStages1 : C::kStages0)) {
-                                    rs[sub] = 0;
-                                    ph[sub] ^= 1;
-                                }
-                            }
+                            for (int kk = 0; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
+                                umma_ss_2cta(d, k_hi | (a + 2 * kk), k_hi | (bb + 2 * kk), idesc_s, (j | kk) != 0);
+                            umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                            if (last) umma_commit_2cta_mask(bar_qfree + 8 * j, 3);   // the next query's chunk may come in
                         }
+                        umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
+                        first_bits = (first_bits & ~(1u << b)) | (static_cast<uint32_t>(new_query) << b);
+                        new_query = it.advance();
+                        if (new_query) qpar ^= 1;
                     }
-                }
-            }
-        } else if (elect_one()) {
-            // ------------------------------------------------------------------ UMMA issuers for the pair
-            // Issuer i takes the ring positions i, i + kIssuers, ...: chunks y, y + kIssuersPerStream, ... (y = i / 2) of
-            // stream x = i % 2, the tiles 2t + x, accumulated into buffer 2 * (pair parity) + x.
-            const int i = warp - kIssuerWarp;
-            const int x = i & 1, y = i >> 1;
-            constexpr uint32_t idesc = make_idesc_bf16(256, HP, 0, 0);
-            const uint64_t desc_hi = make_smem_desc(0, 16, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
-            const uint32_t desc_lo = static_cast<uint32_t>(make_smem_desc(0, 16, 1024, kSwizzle128));
-            const uint32_t a_lo0 = desc_lo + desc_addr(s_base + C::kOffRing);
-            const uint32_t b_lo0 = desc_lo + desc_addr(s_base + C::kOffB);
-            const int n_queries = nq > cta ? (nq - cta + n_ctas - 1) / n_ctas : 0;
-            const int total = n_queries * n_tp * kQChunks;      // chunks of a stream
-            const uint32_t my_tok = tok + 4 * x;
-            int j = y, tp = 0, gtp = 0;
-            uint32_t qpar = 0;
-            const int ring0 = x ? C::kStages0 : 0, ring_n = x ? C::kStages1 : C::kStages0;
-            static_assert(kIssuersPerStream < C::kStages1, "an issuer meets a slot again only after the stream's other issuers");
-            int rs = y;                     // chunk c of the stream sits in slot c mod ring_n of the stream's ring
-            uint32_t ph = 0;
-            for (int c = y; c < total; c += kIssuersPerStream) {
-                const int s = ring0 + rs;
-                const int b = 2 * (gtp & 1) + x;
-                if (j == 0) mbar_spin(bar_tempty + 8 * b, ((gtp >> 1) & 1) ^ 1, wc, kErrFwd + 13);
-                if (tp == 0) mbar_wait(bar_bfull + 8 * j, qpar, wc, kErrFwd + 12);
-                mbar_spin(bar_full + 8 * s, ph, wc, kErrFwd + 14);
-                fence_proxy_async_smem();        // the chunk was written by cp.async, the tensor core reads it
-                flag_wait(my_tok, static_cast<uint32_t>(c), wc, kErrFwd + 19);
-                tc_fence_after_sync();
-                const uint32_t d = tmem + b * HP;
-                const uint32_t a_lo = a_lo0 + s * (kChunkA >> 4);
-                const uint32_t b_lo = b_lo0 + j * (C::kBChunk >> 4);
-                umma_ss_2cta(d, desc_hi | a_lo, desc_hi | b_lo, idesc, j != 0);
+                    if (n >= 0) {
+                        // O += P V of tile n
+                        const uint32_t acc0 = ((first_bits >> (n & 1)) & 1u) ^ 1u;
+                        mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 19);
 #pragma unroll
-                for (int kk = 1; kk < 4; ++kk)   // 32 bytes further along K = +2 in the address field
-                    umma_ss_2cta(d, desc_hi | (a_lo + 2 * kk), desc_hi | (b_lo + 2 * kk), idesc, 1);
-                tc_fence_before_sync();
-                flag_store(my_tok, static_cast<uint32_t>(c + 1));
-                // The UMMAs on one accumulator complete in the order they were issued, so the commit behind a tile's
-                // last chunk covers the chunks the stream's other issuer put in before it.
-                umma_commit_2cta_mask(bar_empty + 8 * s, 3);
-                if (tp == n_tp - 1) umma_commit_2cta_mask(bar_bfree + 8 * j, 3);
-                if (j == kQChunks - 1) umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
-                j += kIssuersPerStream;
-                if (j >= kQChunks) {
-                    j -= kQChunks;
-                    ++gtp;
-                    if (++tp == n_tp) {
-                        tp = 0;
-                        qpar ^= 1;
+                        for (int v = 0; v < kVSlots; ++v) {
+                            const int g = v >> 1, b = v & 1;
+                            ring.wait(wc, kErrFwd + 14);
+                            const uint32_t s = ring.slot;
+                            ring.next();
+                            fence_proxy_async_smem();        // the slot was written by cp.async, the tensor core reads it
+                            tc_fence_after_sync();
+                            const uint32_t a = p_lo + g * (kPChunk >> 4), bb = v_lo + s * (kSlotBytes >> 4);
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)   // 16 keys: 32 bytes along P's rows, 16 rows (2 KB) of V
+                                umma_ss_2cta(tmem + kTmemO + b * 128, k_hi | (a + 2 * kk), v_hi | (bb + kk * (2048 >> 4)), idesc_o,
+                                             (g | kk) != 0 ? 1u : acc0);
+                            umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                        }
+                        umma_commit_2cta_mask(bar_pv, 3);
                     }
                 }
-                rs += kIssuersPerStream;
-                if (rs >= ring_n) {
-                    rs -= ring_n;
-                    ph ^= 1;
+                if (*s_abort) {   // winding down: nothing of this thread's may still be in the tensor pipe at dealloc
+                    umma_commit_2cta_mask(bar_drain, 1);
+                    mbar_wait_drain(bar_drain, 0, p.wait_limit);
                 }
-            }
-            if (*s_abort) {
-                umma_commit_2cta_mask(bar_drain + 8 * i, 1);
-                mbar_wait_drain(bar_drain + 8 * i, 0, p.wait_limit);
             }
         }
-    } else {
-        // ------------------------------------------------------------------ row statistics / exponentials
-        const int quarter = warp & 3;
-        const int g = warp >> 2;            // head half
-        const int row = quarter * 32 + lane;
-        const uint32_t tempty0 = map_to_cta(bar_tempty, 0);
-        const uint64_t pol_stream = l2_policy_evict_first();
-        const int t = threadIdx.x;
-        // second pass: the row maximum found by the first pass, in base-2 units, fetched one query ahead
-        auto load_stat = [&](int ql) -> float {
-            if (kMode == 1 || ql >= nq || t >= HP) return 0.f;
-            if (t >= p.h_q) return __int_as_float(0x7f800000);
-            return ordered_to_float(p.m_ord[static_cast<size_t>(p.q0 + ql) * p.h_q + t]) * p.scale_log2e;
+    } else if ((warp & 1) * 32 < NH) {
+        // ------------------------------------------------------------------ softmax (one head, 64 keys of the tile per thread)
+        const int quarter = warp & 3, ch = warp >> 2;
+        const int part = (quarter >> 1) * 2 + ch;                // which 64 keys of the tile: its 64-key chunk of P
+        const int row = (quarter & 1) * 32 + lane;               // head row of this CTA
+        const int head = static_cast<int>(rank) * NH + row;
+        const bool real = head < p.h_q;
+        const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
+        const uint32_t tempty0 = map_to_cta(bar_tempty, 0), pfull0 = map_to_cta(bar_pfull, 0);
+        const uint32_t p_row = s_base + kOffP + part * kPChunk + row * 128;
+        const int bar_id = 1 + (quarter & 1);                    // the four warps that share 32 rows
+        float* stat = reinterpret_cast<float*>(smem + kOffStat);
+        const float ninf = __int_as_float(0xff800000);
+        TileIter<1> it(p, range);
+        QMeta qm = load_qmeta(p, range.q);
+        // which of the warp's 64 keys are valid: one bit per key, loaded a tile ahead
+        int idx0 = -1, idx1 = -1;
+        auto load_idx = [&]() {
+            const int key = it.tile() * kTileKeys + part * 64 + lane;
+            const int32_t* src = p.indices + static_cast<size_t>(it.q) * p.topk + key;
+            idx0 = it.more() && key < p.topk ? __ldg(src) : -1;
+            idx1 = it.more() && key + 32 < p.topk ? __ldg(src + 32) : -1;
         };
-        float stat_next = load_stat(cta);
-        int gt = 0;                         // tiles so far: pair gt >> 1, tile gt & 1 of the pair
-        const int n_tiles = 2 * n_tp;
-        for (int ql = cta; ql < nq; ql += n_ctas) {
-            const int qg = p.q0 + ql;
-            const QMeta qm = load_qmeta(p, qg);
-            if constexpr (kMode == 2) {
-                asm volatile("bar.sync 1, 256;" ::: "memory");      // every softmax warp is done with the previous query
-                if (t < HP) m2_s[t] = stat_next;
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                stat_next = load_stat(ql + n_ctas);
+        load_idx();
+        bool new_query = true;
+        float ref = ninf, sum = 0.f;         // reference of the row's exponentials (log2 units), sum over this thread's keys
+        int seg_begin = 0;
+        for (int n = 0; n < n_tiles; ++n) {
+            const int key = it.tile() * kTileKeys + part * 64 + lane;
+            const uint32_t mask0 = __ballot_sync(0xffffffffu, slot_valid(idx0, key, qm, p));
+            const uint32_t mask1 = __ballot_sync(0xffffffffu, slot_valid(idx1, key + 32, qm, p));
+            if (new_query) {
+                ref = ninf;
+                sum = 0.f;
+                seg_begin = it.pos;
             }
-            // what this lane keeps for heads g * NH + lane and g * NH + 32 + lane over the query's tiles
-            float keep_max[2] = {__int_as_float(0xff800000), __int_as_float(0xff800000)};
-            unsigned long long keep_sum[2] = {0ull, 0ull};
-            for (int tile = 0; tile < n_tiles; ++tile, ++gt) {
-                const int key = tile * kTileKeys + static_cast<int>(rank) * 128 + row;
-                const int idx = key < p.topk ? __ldg(p.indices + static_cast<size_t>(qg) * p.topk + key) : -1;
-                const bool valid = slot_valid(idx, key, qm, p);
-                const int b = gt & 3;               // 2 * (pair parity) + tile of the pair
-                mbar_wait(bar_tfull + 8 * b, (gt >> 2) & 1, wc, kErrFwd + 18, kPollSleepNs);
+            const int qg = it.q, q_lo = it.lo, q_hi = it.hi;
+            const bool last = it.last_of_query();
+            const int seg_end = it.pos + 1;
+            const bool next_query = it.advance();
+            if (next_query && it.more()) qm = load_qmeta(p, it.q);
+            load_idx();
+
+            const int b = n & 1;
+            mbar_wait(bar_tfull + 8 * b, (n >> 1) & 1, wc, kErrFwd + 18, kPollSleepNs);
+            tc_fence_after_sync();
+            uint32_t sv[64];
+            tmem_ld_32x32(tmem + lanes + kTmemS + b * 128 + ch * 64, *reinterpret_cast<uint32_t(*)[32]>(sv));
+            tmem_ld_32x32(tmem + lanes + kTmemS + b * 128 + ch * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(sv + 32));
+            tmem_ld_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            // the S buffer has been read (tcgen05.wait::ld), which is all the issuer needs to know
+            if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * b);
+            if ((mask0 & mask1) != 0xffffffffu) {            // warp-uniform
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    if (!((mask0 >> i) & 1u)) sv[i] = 0xff800000u;
+                    if (!((mask1 >> i) & 1u)) sv[32 + i] = 0xff800000u;
+                }
+            }
+            float m[4] = {ninf, ninf, ninf, ninf};
+#pragma unroll
+            for (int i = 0; i < 64; i += 4) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) m[k] = fmaxf(m[k], __uint_as_float(sv[i + k]));
+            }
+            stat[(b * 4 + part) * 64 + row] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+            float scale_o = 1.f;
+            bool rescale = false;
+            uint32_t pk[32];
+            const float* st = stat + b * 4 * 64 + row;
+            const float top = fmaxf(fmaxf(st[0], st[64]), fmaxf(st[128], st[192])) * p.scale_log2e;
+            if (top > ref + kMaxLag || ref == ninf) {
+                // first valid tile: O and the sum are still empty; later the row moves to a new reference
+                scale_o = ref == ninf ? 1.f : ex2_approx(ref - top);
+                rescale = ref != ninf && top > ninf;
+                if (top > ninf) ref = top;
+            }
+            const float neg = ref == ninf ? 0.f : -ref;
+            sum *= scale_o;
+            float add[2] = {0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const float x = ex2_approx(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2e, neg));
+                const float y = ex2_approx(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2e, neg));
+                add[0] += x;
+                add[1] += y;
+                pk[i] = pack_bf16x2(x, y);
+            }
+            sum += add[0] + add[1];
+            // P of the previous tile has been consumed and O is at rest
+            if (n > 0) mbar_wait(bar_pv, (n - 1) & 1, wc, kErrFwd + 20, kPollSleepNs);
+            tc_fence_after_sync();
+            if (__any_sync(0xffffffffu, rescale)) {          // this warp's half of the columns of both d-blocks
+#pragma unroll 1
+                for (int c = 0; c < 256; c += 128) {
+#pragma unroll 1
+                    for (int e = 0; e < 64; e += 16) {
+                        const uint32_t at = tmem + lanes + kTmemO + c + ch * 64 + e;
+                        uint32_t o[16];
+                        tmem_ld_32x16(at, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale_o);
+                        tmem_st_32x16(at, o);
+                    }
+                }
+                tmem_st_wait();
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                st_shared_v4(p_row + ((u ^ (row & 7)) << 4), pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
+            fence_proxy_async_smem();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_release(pfull0);
+
+            if (last) {
+                // ---- the query's (or the range's) last tile: o, lse - or an unnormalised part of them
+                const bool whole = seg_begin == q_lo && seg_end == q_hi;
+                stat[(4 * ((n + 1) & 1) + part) * 64 + row] = sum;
+                asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+                const float* sums = stat + 4 * ((n + 1) & 1) * 64 + row;
+                const float total = (sums[0] + sums[64]) + (sums[128] + sums[192]);
+                asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // the next tile's maxima go to the same place
+                const float inv = total > 0.f ? 1.f / total : 0.f;
+                const size_t orow = static_cast<size_t>(qg) * p.h_q + head;
+                // partial results: slot 2 c for a range that starts inside the query, 2 c + 1 for one that starts at or before it
+                const int slot = static_cast<int>(blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0);
+                if (real && part == 0) {
+                    if (whole)
+                        p.lse_out[orow] = (total > 0.f ? ref + __log2f(total) : __int_as_float(0x7f800000)) * p.lse_out_mult;
+                    else
+                        p.part_ml[static_cast<size_t>(slot) * HP + head] = make_float2(ref, total);
+                }
+                mbar_wait(bar_pv, n & 1, wc, kErrFwd + 21, kPollSleepNs);
                 tc_fence_after_sync();
-                const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + b * HP + g * NH;
-                if constexpr (kMode == 1) {
-                    // the maximum over the warp's 32 keys of every head: one warp reduction per head
-                    const float ninf = __int_as_float(0xff800000);
+                // lanes 0-63: columns [256 block, + 128), lanes 64-127: [256 block + 128, + 128)
 #pragma unroll 1
-                    for (int c0 = 0; c0 < NH; c0 += 32) {
-                        uint32_t pv[32];
-                        tmem_ld_32x32(taddr + c0, pv);
-                        tmem_ld_wait();
-                        float mine = ninf;
+                for (int c = 0; c < 4; ++c) {
+                    const int blk = c >> 1, e = (c & 1) * 32;
+                    uint32_t o[32];
+                    tmem_ld_32x32(tmem + lanes + kTmemO + blk * 128 + ch * 64 + e, o);
+                    tmem_ld_wait();
+                    const int col = blk * 256 + (quarter >> 1) * 128 + ch * 64 + e;
+                    if (real && whole) {
+                        __nv_bfloat16* out = p.gout + orow * kDV + col;
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const float r = redux_max_f32(valid ? __uint_as_float(pv[c]) : ninf);
-                            if (lane == c) mine = r;
-                        }
-                        if (c0 == 0) keep_max[0] = fmaxf(keep_max[0], mine);
-                        else keep_max[1] = fmaxf(keep_max[1], mine);
-                    }
-                } else {
-                    const size_t off = static_cast<size_t>(p.scr0 + ql) * p.topk_pad * HP + scratch_offset(key, g * NH, p.topk_pad);
-                    __nv_bfloat16* s_out = p.s_scr + off;
-                    const uint32_t vmask = valid ? 0xFFFFFFFFu : 0u;
-                    const uint32_t fxmask = valid ? 0x007FFFFFu : 0u;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < NH; c0 += 16) {
-                        uint32_t pv[16];
-                        tmem_ld_32x16(taddr + c0, pv);
-                        tmem_ld_wait();
-                        uint32_t so[8];
-                        const float4* l4 = reinterpret_cast<const float4*>(m2_s + g * NH + c0);
-                        unsigned mine = 0;
+                        for (int v = 0; v < 2; ++v) {
+                            uint32_t w[8];
 #pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            const float4 l = l4[v];
-                            const float lv[4] = {l.x, l.y, l.z, l.w};
-                            float sv[4];
+                            for (int i = 0; i < 8; ++i)
+                                w[i] = pack_bf16x2(__uint_as_float(o[16 * v + 2 * i]) * inv, __uint_as_float(o[16 * v + 2 * i + 1]) * inv);
+                            st_global_v8(out + 16 * v, w);
+                        }
+                    } else if (real) {
+                        float* out = p.part_o + (static_cast<size_t>(slot) * HP + head) * kDV + col;
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int c = 4 * v + e;
-                                // E <= 1 (+ one rounding): the same logits produced the maximum in the first pass
-                                const float ex = ex2_approx(fmaf(__uint_as_float(pv[c]), p.scale_log2e, -lv[e]));
-                                sv[e] = ex;
-                                // Row sums in 2^-22 fixed point: integer warp reductions and integer atomics add in
-                                // any order to the same result.  E + 2.0f lies in [2, 4), where one unit of the mantissa
-                                // is 2^-22: the low 23 bits of the sum's bit pattern are E in fixed point, rounded to
-                                // nearest, without a conversion instruction (conversions, exponentials and warp
-                                // reductions share one quarter-rate pipe).  2048 terms lose at most 2^-12 of a sum >= 1.
-                                const unsigned fx = __float_as_uint(ex + 2.0f) & fxmask;
-                                const unsigned r = redux_add_u32(fx);
-                                if (lane == ((c0 + c) & 31)) mine = r;
-                            }
-                            so[2 * v] = pack_bf16x2(sv[0], sv[1]) & vmask;
-                            so[2 * v + 1] = pack_bf16x2(sv[2], sv[3]) & vmask;
-                        }
-                        // columns c0 .. c0 + 15 went to lanes (c0 & 31) .. (c0 & 31) + 15
-                        if (static_cast<unsigned>(lane - (c0 & 31)) < 16u) {
-                            if (c0 < 32) keep_sum[0] += mine;
-                            else keep_sum[1] += mine;
-                        }
-                        __nv_bfloat16* s0 = s_out + static_cast<size_t>(c0) * p.topk_pad;
-                        const size_t blk = static_cast<size_t>(p.topk_pad) * 8;
-                        st_global_v4_hint(s0, so[0], so[1], so[2], so[3], pol_stream);
-                        st_global_v4_hint(s0 + blk, so[4], so[5], so[6], so[7], pol_stream);
+                        for (int v = 0; v < 4; ++v)
+                            st_global_v8(out + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
                     }
                 }
-                tc_fence_before_sync();
-                __syncwarp();
-                // the accumulator reads have completed (tcgen05.wait::ld), which is all the issuers need to know
-                if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * b);
+                tc_fence_before_sync();      // O may be overwritten once this warp arrives for the next tile's P
             }
-            // this warp's share of the query's row statistics: integer atomics, so the order in which the warps
-            // arrive does not change the result
-#pragma unroll
-            for (int k = 0; k < NH / 32; ++k) {
-                const int head = g * NH + 32 * k + lane;
-                if (head < p.h_q) {
-                    const size_t o = static_cast<size_t>(qg) * p.h_q + head;
-                    if constexpr (kMode == 1) atomicMax(p.m_ord + o, float_to_ordered(keep_max[k]));
-                    else atomicAdd(p.l_fix + o, keep_sum[k]);
-                }
-            }
+            new_query = next_query;
         }
     }
     abort_wind_down(s_abort);
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // neither CTA leaves while the other may still signal it or read its operands
-    if (warp == kIssuerWarp) tmem_dealloc_2cta(tmem, C::kTmemCols);
+    if (warp == 16) tmem_dealloc_2cta(tmem, 512);
 }
 
-// Row statistics of the forward start at -inf (maximum) and 0 (sum).
-__global__ void smla_fwd_stats_init_kernel(int* m_ord, unsigned long long* l_fix, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        m_ord[i] = kOrderedNegInf;
-        l_fix[i] = 0ull;
+// Queries whose tiles were spread over several clusters: o = sum of 2^(ref_i - ref) O_i over the parts, divided by the sum
+// of their weighted row sums.  One warp per (boundary between two ranges, head); the boundary that is the query's first
+// does the work, in the order of the parts.  Bound by the latency of a few dependent loads (256 KB per part, in L2).
+__global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int per_boundary = (p.h_q + 7) / 8;
+    const int c = static_cast<int>(blockIdx.x) / per_boundary + 1;
+    const int head = static_cast<int>(blockIdx.x) % per_boundary * 8 + (threadIdx.x >> 5);
+    const WorkRange w = find_range(p, c, n_clusters);
+    const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
+    const int q_begin = __ldcg(p.tile_pre + w.q), q_end = __ldcg(p.tile_pre + w.q + 1);
+    if (w.begin <= q_begin || w.begin >= q_end || range_start(t0, t1, c - 1, n_clusters) > q_begin || head >= p.h_q) return;
+    float ref = __int_as_float(0xff800000), sum = 0.f, acc[16] = {};
+    for (int k = c - 1; k < n_clusters; ++k) {
+        const int begin = range_start(t0, t1, k, n_clusters);
+        if (begin >= q_end) break;
+        if (begin == range_start(t0, t1, k + 1, n_clusters)) continue;
+        const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head;
+        const float2 ml = __ldcg(p.part_ml + row);
+        const float4* o = reinterpret_cast<const float4*>(p.part_o + row * kDV) + lane;
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __ldcg(o + 32 * i);
+        if (!(ml.y > 0.f)) continue;             // no valid slot in this part
+        const float top = fmaxf(ref, ml.x);
+        const float keep = ex2_approx(ref - top), add = ex2_approx(ml.x - top);
+        sum = sum * keep + ml.y * add;
+        ref = top;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            acc[4 * i] = acc[4 * i] * keep + v[i].x * add;
+            acc[4 * i + 1] = acc[4 * i + 1] * keep + v[i].y * add;
+            acc[4 * i + 2] = acc[4 * i + 2] * keep + v[i].z * add;
+            acc[4 * i + 3] = acc[4 * i + 3] * keep + v[i].w * add;
+        }
     }
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    const size_t orow = static_cast<size_t>(w.q) * p.h_q + head;
+    if (lane == 0) p.lse_out[orow] = (sum > 0.f ? ref + __log2f(sum) : __int_as_float(0x7f800000)) * p.lse_out_mult;
+    uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV) + lane;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        out[32 * i] = make_uint2(pack_bf16x2(acc[4 * i] * inv, acc[4 * i + 1] * inv), pack_bf16x2(acc[4 * i + 2] * inv, acc[4 * i + 3] * inv));
 }
 
 // =============================================================================================
@@ -1225,8 +1358,8 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const WorkRange range = *range_s;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const WorkRange range = uniform_range(*range_s);
     using Iter = TileIter<kWorkTileKeys / kTileKeys>;    // two tiles per work tile: a range has an even number of them
 
     if (warp == 0) {
@@ -1297,7 +1430,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 int s = 0;
                 uint32_t ph = 0, k = 0, unit = 0;
                 bool new_query = true;
-                for (Iter it(p, range); it.more();) {
+                Iter it(p, range);
+                const int n_tiles = (range.end - range.begin) * (kWorkTileKeys / kTileKeys);
+                for (int n = 0; n < n_tiles; ++n) {
                     if (new_query) mbar_wait(bar_res, k++ & 1, wc, kErrDkv + 2);
                     const bool last = it.last_of_query();
                     mbar_wait(bar_tfull + 8 * s, ph, wc, kErrDkv + 4);
@@ -1498,7 +1633,7 @@ __global__ void __launch_bounds__(256) smla_dkv_segment_sum_kernel(const int* __
 }
 
 // =============================================================================================
-// dq: one CTA per (query, d-part of kSplit column chunks); 14 warps; two CTAs per SM, so that one's start-up (TMEM,
+// dq: one CTA per (query, d-part of three column chunks); 14 warps; two CTAs per SM, so that one's start-up (TMEM,
 // first gathers) and epilogue run under the other's tiles.
 //   warps 0-3   epilogue: TMEM -> bf16 -> dQ[q, head, d]; lane = head, so a thread stores whole 64-byte pieces of
 //               its head's row
@@ -1506,22 +1641,19 @@ __global__ void __launch_bounds__(256) smla_dkv_segment_sum_kernel(const int* __
 //               cp.async into the swizzled layout)
 //   warp 13     TMA: the dS scratch tile
 //   warp 12     UMMA issuer: acc[128 heads, d of the part] += dS^T . Kg  (both operands MN-major: the key index is
-//               the contraction and runs along shared-memory rows).  Heads are the M side so that N can be 256
-//               columns of d: a 128x256x16 UMMA reads 12 KB of shared memory per 128 cycles of math, whereas the
-//               transposed 128x128x16 form reads 8 KB per 64 cycles, which is all the bandwidth there is (measured
-//               ~100 cycles per UMMA instead of 64).  With HP = 64 the upper 64 accumulator rows are computed from
-//               whatever follows the dS tile in shared memory and never read.
-//               (Two issuers taking alternate tiles, handing over through a counter, changed nothing at one CTA
-//               per SM: the kernel waits for its gathers, not for the issuer.)
+//               the contraction and runs along shared-memory rows).  Heads are the M side so that N can be the 192
+//               columns of the part.  With HP = 64 the upper 64 accumulator rows are computed from whatever follows the
+//               dS tile in shared memory and never read.
+// With few queries a cluster of up to eight CTAs splits the keys of one (query, d-part) and adds up in rank order.
 // =============================================================================================
 namespace dq {
 constexpr int kThreads = 448;
 constexpr int kProducerWarps = 8;
 constexpr int kTileKeys = 64;
-template <int HP, int kSplit> struct Cfg {
-    static constexpr int kStages = (HP == 64 && kSplit <= 3) ? 3 : 2;   // what fits twice into an SM's shared memory
-    static_assert(kSplit >= 1 && kSplit <= 4, "one UMMA covers the part: N = 64 kSplit <= 256");
-    static constexpr int kKgBytes = kSplit * 8192;
+constexpr int kParts = kQChunks / kDqChunks;
+template <int HP> struct Cfg {
+    static constexpr int kStages = HP == 64 ? 3 : 2;        // what fits twice into an SM's shared memory
+    static constexpr int kKgBytes = kDqChunks * 8192;
     static constexpr int kDsBytes = (HP / 64) * 8192;
     static constexpr int kStage = kKgBytes + kDsBytes;     // dS right after Kg
     static constexpr int kOffMisc = kStages * kStage;
@@ -1529,26 +1661,23 @@ template <int HP, int kSplit> struct Cfg {
     static constexpr int kSmemBytes = kOffMisc + 256 + 1024 + (HP == 64 ? 8192 : 0);
     static_assert(2 * (kSmemBytes + 1024) <= 233472, "two CTAs per SM");
     static constexpr int kTmemCols = 256;                  // up to 256 columns of d; two CTAs share the SM's 512
-    static constexpr int kRowBytes = kSplit * 128 + 16;    // epilogue staging of one head's row
+    static constexpr int kRowBytes = kDqChunks * 128 + 16;    // epilogue staging of one head's row
     static_assert(128 * kRowBytes <= kOffMisc, "the epilogue stages its rows in the pipeline's memory");
     // keys of a query split over a cluster: every CTA leaves its fp32 accumulator [heads][columns] behind the barriers for
     // the others to read (rows 16 bytes apart modulo 128: conflict-free 16-byte accesses); one CTA per SM then
-    static constexpr int kPartPitch = kSplit * 64 + 4;
+    static constexpr int kPartPitch = kDqChunks * 64 + 4;
     static constexpr int kOffPart = kOffMisc + 256;
     static constexpr int kSplitSmemBytes = kOffPart + 128 * kPartPitch * 4 + 1024;
-    static_assert(kSplit > kDqChunks || kSplitSmemBytes <= 232448, "shared memory of one SM");   // (only dQ splits its keys)
+    static_assert(kSplitSmemBytes <= 232448, "shared memory of one SM");
 };
 }  // namespace dq
 
-// kNorm (forward, o = S.V): the scratch holds unnormalised E = exp2(logit - max); every head's row is divided by its
-// row sum on the way out, and the CTA of d-part 0 writes lse = max + log2(sum).
-template <int HP, int kSplit, int kTotal, bool kNorm = false>
+template <int HP>
 __global__ void __launch_bounds__(dq::kThreads, 2)
 smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     using namespace dq;
-    using C = Cfg<HP, kSplit>;
+    using C = Cfg<HP>;
     constexpr int kStages = C::kStages;
-    constexpr int kParts = (kTotal + kSplit - 1) / kSplit;
     // the CTAs of a cluster (usually one) share a (query, d-part) and split its keys
     const int nz = static_cast<int>(cluster_nctas()), z = static_cast<int>(cluster_ctarank());
     const int unit = static_cast<int>(blockIdx.x) / nz;
@@ -1557,9 +1686,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     const int qg = p.q0 + ql;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
-    // d-part i gathers kv column chunks [i kSplit, (i + 1) kSplit): 3 x 3 of 9 for dQ, 2 x 4 of 8 for o = S.V
-    const int chunk0 = part * kSplit;
-    const int n_ch = kTotal - chunk0 < kSplit ? kTotal - chunk0 : kSplit;
+    const int chunk0 = part * kDqChunks;      // first kv column chunk of the d-part
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1590,17 +1717,13 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // Behind the dKV kernel's trigger everything this kernel reads is in place already (that kernel triggers after it has
     // waited for the recompute kernel), so its CTAs fill whatever SMs the dKV kernel leaves; the last CTA then holds the
     // grid open until the dKV kernel is done, so that "dq done" still means "all done" to whatever follows.
     if (!p.dq_after_trigger) pdl_wait();
-    int tile0 = 0, n_tiles = p.topk_pad / kTileKeys;
-    if constexpr (!kNorm) {
-        const int n = (__ldcg(p.n_used + qg) + kTileKeys - 1) / kTileKeys;
-        tile0 = n * z / nz;
-        n_tiles = n * (z + 1) / nz - tile0;
-    }
+    const int n_all = __shfl_sync(0xffffffffu, (__ldcg(p.n_used + qg) + kTileKeys - 1) / kTileKeys, 0);
+    const int tile0 = n_all * z / nz, n_tiles = n_all * (z + 1) / nz - tile0;
 
     if (warp >= 4 && warp < 12) {
         const int pt = threadIdx.x - 128;   // 0..255
@@ -1635,7 +1758,8 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
             load_idx(tile + 1);
             mbar_wait(bar_empty + 8 * s, ph, wc, kErrDq + 1, kPollSleepNs);
             const uint32_t d = dst0 + s * C::kStage;
-            for (int c = 0; c < n_ch; ++c) {
+#pragma unroll
+            for (int c = 0; c < kDqChunks; ++c) {
                 cp_async16_zfill_hint(d + c * 8192, src[0] + c * 128, nb[0], pol_keep);
                 cp_async16_zfill_hint(d + c * 8192 + 32 * 128, src[1] + c * 128, nb[1], pol_keep);
             }
@@ -1665,18 +1789,18 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         }
     } else if (warp == 12) {
         if (elect_one()) {
-            // N = the part's column chunks (up to 256 d) in one UMMA
-            const uint32_t idesc1 = make_idesc_bf16(128, n_ch * 64, 1, 1);
+            constexpr uint32_t idesc1 = make_idesc_bf16(128, kDqChunks * 64, 1, 1);     // N = the part's columns in one UMMA
             // A = dS^T: [HP/8 head blocks][64 keys][8 heads], 8-key groups 128 B apart, head blocks 1 KB apart.
             // Descriptors: the fixed fields once, the address (16-byte units, the low 14 bits) added per UMMA.
             const uint64_t a_hi = make_smem_desc(0, 128, 1024, kSwizzleNone) & 0xFFFFFFFF00000000ull;
             const uint32_t a_lo0 = static_cast<uint32_t>(make_smem_desc(0, 128, 1024, kSwizzleNone)) + desc_addr(s_base + C::kKgBytes);
             const uint64_t b_hi = make_smem_desc(0, 8192, 1024, kSwizzle128) & 0xFFFFFFFF00000000ull;
             const uint32_t b_lo0 = static_cast<uint32_t>(make_smem_desc(0, 8192, 1024, kSwizzle128)) + desc_addr(s_base);
-            int s = 0;
-            uint32_t ph = 0;
+            RingReader<kStages> ring(bar_full);
             for (int tile = 0; tile < n_tiles; ++tile) {
-                mbar_spin(bar_full + 8 * s, ph, wc, kErrDq + 2);
+                ring.wait(wc, kErrDq + 2);
+                const uint32_t s = ring.slot;
+                ring.next();
                 fence_proxy_async_smem();
                 tc_fence_after_sync();
                 const uint32_t a_lo = a_lo0 + s * (C::kStage >> 4), b_lo = b_lo0 + s * (C::kStage >> 4);
@@ -1686,10 +1810,6 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                     umma_ss(tmem, a, b_hi | (b_lo + ks * (2048 >> 4)), idesc1, (tile | ks) != 0);
                 }
                 umma_commit(bar_empty + 8 * s);
-                if (++s == kStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
             }
             umma_commit(bar_acc);
             if (*s_abort) {   // winding down: nothing of this thread's may still be in the tensor pipe at dealloc
@@ -1706,27 +1826,15 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         // pipeline stages are idle by now; rows 16 bytes apart modulo 128 so that the 16-byte stores of a warp
         // spread over all banks) and sends it off as one bulk copy: whole cache lines instead of 32 scattered
         // 16-byte pieces per store instruction.
-        constexpr int kPitch = kTotal * 64;      // 576 for dQ, 512 for o
         constexpr int kRowBytes = C::kRowBytes;
         const int head = quarter * 32 + lane;
         const uint32_t row_s = s_base + head * kRowBytes;
-        float inv = 1.f;
-        if constexpr (kNorm) {
-            if (head < p.h_q) {
-                const size_t o = static_cast<size_t>(qg) * p.h_q + head;
-                const float l = static_cast<float>(p.l_fix[o]) * (1.f / kFixScale);
-                inv = l > 0.f ? 1.f / l : 0.f;               // no valid slot: o = 0, lse = +inf
-                if (part == 0)
-                    p.lse_out[o] = (l > 0.f ? fmaf(ordered_to_float(p.m_ord[o]), p.scale_log2e, __log2f(l))
-                                            : __int_as_float(0x7f800000)) * p.lse_out_mult;
-            }
-        }
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
         if (nz > 1) {
             if (quarter * 32 < p.h_q) {
                 const uint32_t part_s = s_base + C::kOffPart + head * (C::kPartPitch * 4);
 #pragma unroll 1
-                for (int cg = 0; cg < n_ch * 4; ++cg) {
+                for (int cg = 0; cg < kDqChunks * 4; ++cg) {
                     uint32_t r[16];
                     tmem_ld_32x16(taddr + cg * 16, r);
                     tmem_ld_wait();
@@ -1738,16 +1846,12 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
             }
         } else if (quarter * 32 < p.h_q) {        // warp-uniform: heads are padded to a multiple of 8 only
 #pragma unroll 1
-            for (int cg = 0; cg < n_ch * 4; ++cg) {   // 16 columns at a time: two CTAs per SM leave 64 registers a thread
+            for (int cg = 0; cg < kDqChunks * 4; ++cg) {   // 16 columns at a time: two CTAs per SM leave 64 registers a thread
                 uint32_t r[16];
                 tmem_ld_32x16(taddr + cg * 16, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 16; ++i) r[i] &= zero_mask;
-                if constexpr (kNorm) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * inv);
-                }
 #pragma unroll
                 for (int v = 0; v < 2; ++v)
                     st_shared_v4(row_s + cg * 32 + v * 16,
@@ -1758,7 +1862,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
             }
             if (head < p.h_q) {
                 fence_proxy_async_smem();         // this thread's row only: no one else touches it
-                bulk_store(p.gout + (static_cast<size_t>(qg) * p.h_q + head) * kPitch + chunk0 * 64, row_s, n_ch * 128);
+                bulk_store(p.dQ + (static_cast<size_t>(qg) * p.h_q + head) * kDQK + chunk0 * 64, row_s, kDqChunks * 128);
                 bulk_commit();
                 bulk_wait_read();
             }
@@ -1771,11 +1875,10 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     if (nz > 1) {
         // every CTA adds up its share of the heads, always in rank order
         cluster_sync_all();
-        constexpr int kGroups = kSplit * 8;      // 8 columns at a time
+        constexpr int kGroups = kDqChunks * 8;   // 8 columns at a time
         const int h0 = p.h_q * z / nz, h1 = p.h_q * (z + 1) / nz;
         for (int i = threadIdx.x; i < (h1 - h0) * kGroups; i += kThreads) {
             const int h = h0 + i / kGroups, c = (i % kGroups) * 8;
-            if (c >= n_ch * 64) continue;
             const uint32_t at = s_base + C::kOffPart + (h * C::kPartPitch + c) * 4;
             float acc[8] = {};
             for (int r = 0; r < nz; ++r) {
@@ -1784,7 +1887,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                 acc[0] += lo.x; acc[1] += lo.y; acc[2] += lo.z; acc[3] += lo.w;
                 acc[4] += hi.x; acc[5] += hi.y; acc[6] += hi.z; acc[7] += hi.w;
             }
-            *reinterpret_cast<uint4*>(p.gout + (static_cast<size_t>(qg) * p.h_q + h) * (kTotal * 64) + chunk0 * 64 + c) =
+            *reinterpret_cast<uint4*>(p.dQ + (static_cast<size_t>(qg) * p.h_q + h) * kDQK + chunk0 * 64 + c) =
                 make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
                            pack_bf16x2(acc[6], acc[7]));
         }
