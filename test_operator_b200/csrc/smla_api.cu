@@ -575,6 +575,75 @@ int static_workspace_ptr(void** out) {
     return SMLA_OK;
 }
 
+// ---- index inverse (CSR by kv row): layout and launches ------------------------------------------------------------
+inline size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+struct InvLayout { size_t keys_a, keys_b, vals_a, vals_b, hist, totals, heads, total; };
+inline InvLayout inv_layout(int64_t n, int32_t s_kv, const inv::Plan& pl) {
+    InvLayout l;
+    const size_t key_bytes = static_cast<size_t>(n) * (pl.key16 ? 2 : 4);
+    size_t off = 0;
+    l.keys_a = off; off += up256(key_bytes);
+    l.keys_b = off; off += pl.passes > 2 ? up256(key_bytes) : 0;
+    l.vals_a = off; off += pl.passes > 1 ? up256(static_cast<size_t>(n) * 4) : 0;
+    l.vals_b = off; off += pl.passes > 2 ? up256(static_cast<size_t>(n) * 4) : 0;
+    l.hist = off; off += up256(static_cast<size_t>(inv::kMaxRadix) * pl.n_blocks * 4);
+    l.totals = off; off += up256(inv::kMaxRadix * 4);
+    l.heads = off; off += up256((static_cast<size_t>(s_kv) + 1) * 4);
+    l.total = off;
+    return l;
+}
+
+// Two passes (up to 65535 rows) on 8.4 M slots and 32768 rows: 214 us with keys formed by a kernel of their own, read twice by
+// every scatter, carried as 32 bits and written by the last pass for a binary search per row; 139 us in this form.
+template <typename KeyT, int kItems>
+int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvLayout& l, uint8_t* ws, int64_t n64, int32_t* row_ptr,
+                         int32_t* entries, cudaStream_t st) {
+    const uint32_t n = static_cast<uint32_t>(n64);
+    constexpr int kSmem = inv::scatter_smem<KeyT, kItems>();
+    static std::atomic<bool> attr_done[kMaxDevices];
+    if (!once_per_device(attr_done, [] {
+            bool ok = set_smem(inv::scatter_kernel<KeyT, true, true, kItems>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, true, false, kItems>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, false, true, kItems>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, false, false, kItems>, kSmem);
+            if (kItems == inv::kItemsLarge) ok &= set_smem(inv::small_sort_kernel<KeyT>, kSmem);
+            return ok;
+        }))
+        return SMLA_ERR_LAUNCH;
+    KeyT* keys[2] = {reinterpret_cast<KeyT*>(ws + l.keys_a), reinterpret_cast<KeyT*>(ws + l.keys_b)};
+    int32_t* vals[2] = {reinterpret_cast<int32_t*>(ws + l.vals_a), reinterpret_cast<int32_t*>(ws + l.vals_b)};
+    uint32_t* hist = reinterpret_cast<uint32_t*>(ws + l.hist);
+    uint32_t* totals = reinterpret_cast<uint32_t*>(ws + l.totals);
+    int32_t* heads = reinterpret_cast<int32_t*>(ws + l.heads);
+    if (n64 <= inv::kSmallInput) {
+        launch(inv::small_sort_kernel<KeyT>, 1, inv::kThreads, kSmem, st, true, 1, src, keys[0], entries, n, pl.passes, pl.digit_bits);
+        launch(inv::small_row_ptr_kernel<KeyT>, src.s_kv / 256 + 1, 256, 0, st, true, 1, keys[0], row_ptr, static_cast<int32_t>(n), src.s_kv);
+        return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
+    }
+    const uint32_t mask = (1u << pl.digit_bits) - 1u;
+    for (int pass = 0; pass < pl.passes; ++pass) {
+        const int shift = pass * pl.digit_bits;
+        const bool first = pass == 0, last = pass == pl.passes - 1;
+        const KeyT* kin = keys[(pass + 1) & 1];
+        const int32_t* vin = vals[(pass + 1) & 1];
+        KeyT* kout = keys[pass & 1];
+        int32_t* vout = last ? entries : vals[pass & 1];
+        launch(first ? inv::histogram_kernel<KeyT, true, kItems> : inv::histogram_kernel<KeyT, false, kItems>, pl.n_blocks, inv::kThreads, 0, st, true, 1, kin,
+               src, hist, n, shift, mask, pl.n_blocks, heads);
+        launch(inv::scan_rows_kernel, static_cast<int>(mask) + 1, 1024, 0, st, true, 1, hist, totals, pl.n_blocks);
+        launch(first ? (last ? inv::scatter_kernel<KeyT, true, true, kItems> : inv::scatter_kernel<KeyT, true, false, kItems>)
+                     : (last ? inv::scatter_kernel<KeyT, false, true, kItems> : inv::scatter_kernel<KeyT, false, false, kItems>),
+               pl.n_blocks, inv::kThreads, kSmem, st, true, 1, kin, vin, src, kout, vout, hist, totals, n, shift, mask, pl.n_blocks, heads);
+    }
+    launch(inv::row_ptr_kernel, src.s_kv / inv::kRowTile + 1, inv::kRowTile, 0, st, true, 1, heads, row_ptr, static_cast<int32_t>(n), src.s_kv);
+    return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
+}
+
+inline bool inv_shape_ok(int32_t s_q, int32_t topk, int32_t s_kv) {
+    return s_q >= 0 && topk > 0 && s_kv > 0 && s_kv < INT32_MAX &&
+           static_cast<int64_t>(s_q) * topk <= static_cast<int64_t>(INT32_MAX);
+}
+
 }  // namespace
 
 extern "C" {
@@ -769,30 +838,11 @@ int smla_selftest_wait_timeout(void* workspace, int which, long long limit_cycle
 }
 
 // ---- index inverse (CSR by kv row) -------------------------------------------------------------
-namespace {
-inline size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
-struct InvLayout { size_t keys_a, keys_b, vals_tmp, hist, totals, total; };
-inline InvLayout inv_layout(int64_t n, const inv::Plan& pl) {
-    InvLayout l;
-    size_t off = 0;
-    l.keys_a = off; off += up256(static_cast<size_t>(n) * 4);
-    l.keys_b = off; off += up256(static_cast<size_t>(n) * 4);
-    l.vals_tmp = off; off += up256(static_cast<size_t>(n) * 4);
-    l.hist = off; off += up256(static_cast<size_t>(inv::kMaxRadix) * pl.n_blocks * 4);
-    l.totals = off; off += up256(inv::kMaxRadix * 4);
-    l.total = off;
-    return l;
-}
-inline bool inv_shape_ok(int32_t s_q, int32_t topk, int32_t s_kv) {
-    return s_q >= 0 && topk > 0 && s_kv > 0 && s_kv < INT32_MAX &&
-           static_cast<int64_t>(s_q) * topk <= static_cast<int64_t>(INT32_MAX);
-}
-}  // namespace
-
 size_t smla_index_inverse_workspace_size(int32_t s_q, int32_t topk, int32_t s_kv) {
     if (!inv_shape_ok(s_q, topk, s_kv)) return 0;
     const int64_t n = static_cast<int64_t>(s_q) * topk;
-    return inv_layout(n, inv::make_plan(n, s_kv)).total + 256;
+    // (never less than twelve bytes a slot, what the documentation promises to be about the size)
+    return std::max(inv_layout(n, s_kv, inv::make_plan(n, s_kv)).total, static_cast<size_t>(n) * 12) + 256;
 }
 
 int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_t s_kv, int32_t q_start_index_s,
@@ -808,40 +858,20 @@ int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_
     if (!indices || !entries || !workspace) return SMLA_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return SMLA_ERR_BAD_ARG;
     const inv::Plan pl = inv::make_plan(n, s_kv);
-    const InvLayout l = inv_layout(n, pl);
+    const InvLayout l = inv_layout(n, s_kv, pl);
     if (workspace_bytes < l.total) return SMLA_ERR_WORKSPACE;
-    if (cudaFuncSetAttribute(inv::scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, inv::kScatterDynSmem) !=
-        cudaSuccess)
-        return SMLA_ERR_LAUNCH;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    uint32_t* kbuf[2] = {reinterpret_cast<uint32_t*>(ws + l.keys_a), reinterpret_cast<uint32_t*>(ws + l.keys_b)};
-    int32_t* vtmp = reinterpret_cast<int32_t*>(ws + l.vals_tmp);
-    uint32_t* hist = reinterpret_cast<uint32_t*>(ws + l.hist);
-    uint32_t* totals = reinterpret_cast<uint32_t*>(ws + l.totals);
-    const uint32_t mask = (1u << pl.digit_bits) - 1u;
-    const int radix = 1 << pl.digit_bits;
-    const int causal = q_start_index_s != SMLA_NO_CAUSAL;
-    int launches = 0;
-    const int32_t* vin = nullptr;
-    for (int pass = 0; pass < pl.passes; ++pass) {
-        const int shift = pass * pl.digit_bits;
-        if (pass == 0)
-            inv::make_keys_kernel<<<pl.n_blocks, inv::kThreads, 0, st>>>(indices, kbuf[0], hist, n, topk, s_kv, causal,
-                                                                         causal ? q_start_index_s : 0, mask, pl.n_blocks);
-        else
-            inv::histogram_kernel<<<pl.n_blocks, inv::kThreads, 0, st>>>(kbuf[pass & 1], hist, n, shift, mask, pl.n_blocks);
-        inv::scan_rows_kernel<<<radix, 1024, 0, st>>>(hist, totals, pl.n_blocks);
-        // the last pass must land in `entries`: passes alternate between the temporary and the output
-        int32_t* vout = ((pl.passes - 1 - pass) & 1) ? vtmp : entries;
-        inv::scatter_kernel<<<pl.n_blocks, inv::kThreads, inv::kScatterDynSmem, st>>>(kbuf[pass & 1], vin, kbuf[(pass + 1) & 1], vout, hist,
-                                                                   totals, n, shift, mask, pl.n_blocks);
-        vin = vout;
-        launches += 3;
-    }
-    const int rows = s_kv + 1;
-    inv::row_ptr_kernel<<<(rows + 255) / 256, 256, 0, st>>>(kbuf[pl.passes & 1], row_ptr, n, s_kv);
-    g_last_launches = launches + 1;
-    return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
+    inv::Source src;
+    src.indices = indices;
+    src.topk = static_cast<uint32_t>(topk);
+    src.s_kv = s_kv;
+    src.causal = q_start_index_s != SMLA_NO_CAUSAL;
+    src.q_start = src.causal ? q_start_index_s : 0;
+    if (pl.items == inv::kItemsMid)
+        return pl.key16 ? launch_index_inverse<uint16_t, inv::kItemsMid>(src, pl, l, ws, n, row_ptr, entries, st)
+                        : launch_index_inverse<uint32_t, inv::kItemsMid>(src, pl, l, ws, n, row_ptr, entries, st);
+    return pl.key16 ? launch_index_inverse<uint16_t, inv::kItemsLarge>(src, pl, l, ws, n, row_ptr, entries, st)
+                    : launch_index_inverse<uint32_t, inv::kItemsLarge>(src, pl, l, ws, n, row_ptr, entries, st);
 }
 
 // ---- sum of the ranks' partial dKV over NVLink (query-sharded runs) ---------------------------------------------

@@ -6,26 +6,40 @@
 // Method: a stable least-significant-digit radix sort of (key = kv row, value = flat slot id).  The values start in
 // ascending order, so a stable sort by key alone yields (row, flat id) order.  Unused slots get the key s_kv and end
 // up behind row_ptr[s_kv] in flat order.  Per pass three kernels: digit histogram per block, exclusive scan of the
-// [digit][block] matrix, stable scatter.  All of it is integer work bound by HBM: 4 B read + 4 B written per slot
-// to form the keys, then 8 B read + 8 B written per slot and pass.
+// [digit][block] matrix, stable scatter; keys are formed from the indices on the fly in the first pass, travel as 16 bits
+// where s_kv fits, and are not written by the last pass.  row_ptr: the last pass takes, for every row, the smallest
+// position at which a run of its key begins (integer minimum: order does not matter), and a last kernel gives rows without
+// a slot the next row's position.  Inputs of at most one block (8192 slots) are sorted by that block in shared memory.
+// All kernels are launched behind their predecessor's start (programmatic dependent launch).
 //
 // The reference has no such operator; the validity rule is the one of its kernel (mla_bwd/mla_bwd.cu:765-789).
 #pragma once
 #include <cstdint>
+#include <climits>
 #include <cuda_runtime.h>
+
+#include "sm100_ptx.cuh"
 
 namespace inv {
 
 constexpr int kThreads = 512;
-constexpr int kItems = 16;                       // entries per thread
-constexpr int kBlockItems = kThreads * kItems;   // entries per block, contiguous
+// Entries per thread; a block's entries are contiguous, a warp's are (32 kItems of them): (warp, step, lane) order is flat
+// order.  Large inputs take sixteen (long runs on the way out; 8.4 M slots: 139 us with sixteen, 144 with twelve, 159 with
+// eight).  Below kLargeInput they take four, so that there are blocks for all SMs (270,000 slots: 46 us with sixteen, 29 with
+// eight).
+constexpr int kItemsLarge = 16, kItemsMid = 4;
+constexpr int64_t kLargeInput = 1 << 20;
+constexpr int kSmallInput = kThreads * kItemsLarge;     // one block sorts this many alone
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxRadix = 256;
+constexpr int kRowTile = 1024;                   // rows per block of the row_ptr kernel
 
 struct Plan {
     int passes;      // 1..4
     int digit_bits;  // <= 8
+    int items;       // entries per thread
     int n_blocks;
+    bool key16;      // keys fit 16 bits
 };
 
 inline Plan make_plan(int64_t n, int32_t s_kv) {
@@ -34,50 +48,55 @@ inline Plan make_plan(int64_t n, int32_t s_kv) {
     Plan pl;
     pl.passes = (bits + 7) / 8;
     pl.digit_bits = (bits + pl.passes - 1) / pl.passes;
-    pl.n_blocks = static_cast<int>((n + kBlockItems - 1) / kBlockItems);
+    pl.items = n > kSmallInput && n < kLargeInput ? kItemsMid : kItemsLarge;
+    pl.n_blocks = static_cast<int>((n + kThreads * pl.items - 1) / (kThreads * pl.items));
+    pl.key16 = s_kv < 65536;
     return pl;
 }
 
+// What turns a flat slot into its key.
+struct Source {
+    const int32_t* indices;
+    uint32_t topk;
+    int32_t s_kv, causal, q_start;
+    __device__ __forceinline__ uint32_t key(uint32_t i, int idx) const {
+        bool valid = idx >= 0 && idx < s_kv;
+        if (causal) valid = valid && idx <= q_start + static_cast<int>(i / topk);
+        return static_cast<uint32_t>(valid ? idx : s_kv);
+    }
+};
+
 __device__ __forceinline__ uint32_t digit_of(uint32_t key, int shift, uint32_t mask) { return (key >> shift) & mask; }
 
-// keys[i] = kv row of flat slot i, or s_kv for an unused slot; also the first pass's digit histogram.
+// Digit histogram of every block's entries -> hist[digit][block].  kFirst: keys come from the indices, and row_ptr is
+// set to "no run yet".  Bound by reading the keys once.
+template <typename KeyT, bool kFirst, int kItems>
 __global__ void __launch_bounds__(kThreads)
-make_keys_kernel(const int32_t* __restrict__ indices, uint32_t* __restrict__ keys, uint32_t* __restrict__ hist,
-                 int64_t n, int32_t topk, int32_t s_kv, int32_t causal, int32_t q_start, uint32_t mask, int n_blocks) {
+histogram_kernel(const KeyT* __restrict__ keys, const Source src, uint32_t* __restrict__ hist, uint32_t n, int shift, uint32_t mask,
+                 int n_blocks, int32_t* __restrict__ row_ptr) {
     __shared__ uint32_t h[kMaxRadix];
-    for (int i = threadIdx.x; i <= static_cast<int>(mask); i += kThreads) h[i] = 0;
+    if (threadIdx.x <= mask) h[threadIdx.x] = 0;
+    smla::pdl_wait();
+    smla::pdl_trigger();
     __syncthreads();
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kBlockItems;
-#pragma unroll 4
+    const uint32_t first = blockIdx.x * (kThreads * kItems) + threadIdx.x;
+    uint32_t k[kItems];
+#pragma unroll
     for (int t = 0; t < kItems; ++t) {
-        const int64_t i = base + static_cast<int64_t>(t) * kThreads + threadIdx.x;
-        if (i < n) {
-            const int idx = indices[i];
-            const int q = static_cast<int>(i / topk);
-            const bool valid = idx >= 0 && idx < s_kv && (!causal || idx <= q_start + q);
-            const uint32_t key = valid ? static_cast<uint32_t>(idx) : static_cast<uint32_t>(s_kv);
-            keys[i] = key;
-            atomicAdd(&h[key & mask], 1u);
-        }
+        const uint32_t i = first + t * kThreads;
+        if (kFirst) k[t] = i < n ? static_cast<uint32_t>(__ldg(src.indices + i)) : 0u;
+        else k[t] = i < n ? keys[i] : 0u;
+    }
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+        const uint32_t i = first + t * kThreads;
+        if (i < n) atomicAdd(&h[digit_of(kFirst ? src.key(i, static_cast<int>(k[t])) : k[t], shift, mask)], 1u);
+    }
+    if (kFirst) {
+        for (uint32_t r = blockIdx.x * kThreads + threadIdx.x; r <= static_cast<uint32_t>(src.s_kv); r += gridDim.x * kThreads) row_ptr[r] = INT_MAX;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= static_cast<int>(mask); i += kThreads) hist[static_cast<size_t>(i) * n_blocks + blockIdx.x] = h[i];
-}
-
-__global__ void __launch_bounds__(kThreads)
-histogram_kernel(const uint32_t* __restrict__ keys, uint32_t* __restrict__ hist, int64_t n, int shift, uint32_t mask,
-                 int n_blocks) {
-    __shared__ uint32_t h[kMaxRadix];
-    for (int i = threadIdx.x; i <= static_cast<int>(mask); i += kThreads) h[i] = 0;
-    __syncthreads();
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kBlockItems;
-#pragma unroll 4
-    for (int t = 0; t < kItems; ++t) {
-        const int64_t i = base + static_cast<int64_t>(t) * kThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[digit_of(keys[i], shift, mask)], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= static_cast<int>(mask); i += kThreads) hist[static_cast<size_t>(i) * n_blocks + blockIdx.x] = h[i];
+    if (threadIdx.x <= mask) hist[static_cast<size_t>(threadIdx.x) * n_blocks + blockIdx.x] = h[threadIdx.x];
 }
 
 // Block-wide exclusive scan of one value per thread (blockDim.x a multiple of 32, at most 1024); returns the
@@ -115,6 +134,8 @@ __global__ void __launch_bounds__(1024)
 scan_rows_kernel(uint32_t* __restrict__ hist, uint32_t* __restrict__ totals, int n_blocks) {
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t tile_total;
+    smla::pdl_wait();
+    smla::pdl_trigger();
     uint32_t* row = hist + static_cast<size_t>(blockIdx.x) * n_blocks;
     uint32_t carry = 0;
     for (int base = 0; base < n_blocks; base += 1024) {
@@ -127,18 +148,6 @@ scan_rows_kernel(uint32_t* __restrict__ hist, uint32_t* __restrict__ totals, int
     }
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
-
-// Stable scatter of one pass.  Warp w of a block owns the contiguous entries [w * kWarpItems, (w + 1) * kWarpItems)
-// of the block's range, so (warp, step, lane) order is flat order.
-//   1. every warp counts the digits of its entries (private shared-memory counters);
-//   2. the counts are prefixed over the warps and over the digits: block-local position of every (digit, warp) run;
-//   3. every warp places its entries, step by step, into a shared-memory copy of the block's output in digit order
-//      (position = running base of (warp, digit) + rank among the lanes of the step with the same digit);
-//   4. the staged entries go out in that order: entry j of digit d lands at global base of (d, block) + j - local
-//      base of d, so consecutive threads write consecutive addresses inside a digit's run (about kBlockItems / radix
-//      entries) instead of 32 different lines per warp instruction.
-// vals_in == nullptr means the values are the flat positions themselves (first pass).
-constexpr int kScatterDynSmem = kBlockItems * 8;   // staged keys + values
 
 // Lanes of the warp whose digit (below 256) equals this lane's, among the active lanes.  Eight ballots: the
 // `match.any` instruction gives the same mask but runs on a pipe that takes a warp every ~64 cycles per SM, which
@@ -154,110 +163,235 @@ __device__ __forceinline__ uint32_t same_digit_lanes(uint32_t d, bool active) {
     return peers;
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
-scatter_kernel(const uint32_t* __restrict__ keys_in, const int32_t* __restrict__ vals_in,
-               uint32_t* __restrict__ keys_out, int32_t* __restrict__ vals_out, const uint32_t* __restrict__ hist,
-               const uint32_t* __restrict__ totals, int64_t n, int shift, uint32_t mask, int n_blocks) {
-    constexpr int kWarpItems = kBlockItems / kWarps;   // 512
-    constexpr int kSteps = kWarpItems / 32;            // 16
-    extern __shared__ __align__(16) uint32_t staged[];
-    uint32_t* skeys = staged;
-    int32_t* svals = reinterpret_cast<int32_t*>(staged + kBlockItems);
-    __shared__ uint32_t global_base[kMaxRadix];   // first output position of (digit, this block)
-    __shared__ uint32_t local_base[kMaxRadix];    // first staged position of the digit
-    __shared__ uint32_t warp_count[kWarps][kMaxRadix];
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t total;
-    const int radix = static_cast<int>(mask) + 1;
-    for (int i = threadIdx.x; i < kWarps * kMaxRadix; i += kThreads) (&warp_count[0][0])[i] = 0;
-    {
-        // exclusive prefix of the digit totals (radix <= 256 <= kThreads: one value per thread)
-        const uint32_t t = threadIdx.x < radix ? totals[threadIdx.x] : 0u;
-        const uint32_t ex = block_exclusive_scan(t, warp_sums, &total);
-        if (threadIdx.x < radix) global_base[threadIdx.x] = ex + hist[static_cast<size_t>(threadIdx.x) * n_blocks + blockIdx.x];
-    }
+constexpr int kChains = 2;                       // independent ranking chains per warp, half of its entries each
+constexpr int kRuns = kWarps * kChains;
+struct RankShared {
+    uint16_t count[kRuns][kMaxRadix];           // entries so far of (run, digit); then the position of the first of them
+    uint32_t half[kMaxRadix];                   // entries of the digit in the lower half of the runs
+    uint32_t local_base[kMaxRadix];             // first staged position of the digit
+    uint32_t warp_sums[32];
+    uint32_t total;
+};
+
+// Position of every entry of the block in digit order (stable): pos[t] of entry (warp, t, lane).  A warp ranks its
+// entries 32 at a time against its own running counts, with no counting round before, as two chains with counts of their
+// own (a step's read of a count waits for the step before it; two chains hide that); the counts then are
+// prefixed over the runs and the digits.  Ends with all threads past a barrier.
+template <int kItems>
+__device__ __forceinline__ void block_rank(const uint32_t (&keys)[kItems], int shift, uint32_t mask, uint32_t first, uint32_t n,
+                                           RankShared& sh, uint32_t (&pos)[kItems]) {
+    static_assert(kChains == 2 && kThreads == 2 * kMaxRadix, "two threads per digit below");
+    constexpr int kSteps = kItems / kChains;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lanes_below = (1u << lane) - 1u;
-    const int64_t block0 = static_cast<int64_t>(blockIdx.x) * kBlockItems;
-    const int64_t first = block0 + static_cast<int64_t>(warp) * kWarpItems + lane;
-    uint32_t* mine = warp_count[warp];
+    uint16_t* mine = sh.count[warp * kChains];
+    for (int d = lane; d < kChains * kMaxRadix / 2; d += 32) reinterpret_cast<uint32_t*>(mine)[d] = 0;
+    __syncwarp();
 #pragma unroll
     for (int t = 0; t < kSteps; ++t) {
-        const int64_t i = first + t * 32;
-        const bool active = i < n;
-        if (active) atomicAdd(&mine[digit_of(keys_in[i], shift, mask)], 1u);   // counts only: order does not matter
-    }
-    __syncthreads();
-    {
-        // per digit: counts of the warps -> offsets inside the digit's run; the run lengths -> local bases
-        uint32_t run = 0;
-        if (threadIdx.x < radix) {
+        uint32_t d[kChains], peers[kChains], before[kChains];
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = warp_count[w][threadIdx.x];
-                warp_count[w][threadIdx.x] = run;
-                run += c;
-            }
+        for (int c = 0; c < kChains; ++c) {
+            const int e = c * kSteps + t;
+            d[c] = digit_of(keys[e], shift, mask);
+            peers[c] = same_digit_lanes(d[c], first + e * 32 < n);
+            before[c] = mine[c * kMaxRadix + d[c]];
+            pos[e] = before[c] + __popc(peers[c] & lanes_below);
         }
-        const uint32_t lb = block_exclusive_scan(run, warp_sums, &total);
-        if (threadIdx.x < radix) {
-            local_base[threadIdx.x] = lb;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) warp_count[w][threadIdx.x] += lb;
-        }
-    }
-    __syncthreads();
-    // second read of the warp's 2 KB of keys (L1 / L2), all of it in flight before the dependent ranking starts
-    uint32_t keys[kSteps];
-    int32_t vals[kSteps];
-#pragma unroll
-    for (int t = 0; t < kSteps; ++t) {
-        const int64_t i = first + t * 32;
-        keys[t] = i < n ? keys_in[i] : 0u;
-        vals[t] = (vals_in && i < n) ? vals_in[i] : static_cast<int32_t>(i);
-    }
-#pragma unroll
-    for (int t = 0; t < kSteps; ++t) {
-        const int64_t i = first + t * 32;
-        const bool active = i < n;
-        const uint32_t key = keys[t];
-        const uint32_t d = active ? digit_of(key, shift, mask) : 0u;
-        const uint32_t peers = same_digit_lanes(d, active);
-        const uint32_t rank = __popc(peers & lanes_below);
-        uint32_t pos = 0;
-        if (active) pos = mine[d] + rank;
         __syncwarp();
-        if (active && rank == 0) mine[d] += __popc(peers);
+#pragma unroll
+        for (int c = 0; c < kChains; ++c)
+            if (first + (c * kSteps + t) * 32 < n && (peers[c] & lanes_below) == 0)
+                mine[c * kMaxRadix + d[c]] = static_cast<uint16_t>(before[c] + __popc(peers[c]));
         __syncwarp();
-        if (active) {
-            skeys[pos] = key;
-            svals[pos] = vals[t];
+    }
+    __syncthreads();
+    // thread (h, digit): the runs [16 h, 16 h + 16)
+    const int digit = threadIdx.x & (kMaxRadix - 1), h = threadIdx.x / kMaxRadix;
+    uint32_t c[kRuns / 2], run = 0;
+#pragma unroll
+    for (int w = 0; w < kRuns / 2; ++w) {
+        c[w] = sh.count[h * (kRuns / 2) + w][digit];
+        run += c[w];
+    }
+    if (h == 0) sh.half[digit] = run;
+    __syncthreads();
+    const uint32_t upper = block_exclusive_scan(h == 0 ? 0u : sh.half[digit] + run, sh.warp_sums, &sh.total);   // totals sit in the upper threads
+    if (h == 1) sh.local_base[digit] = upper;
+    __syncthreads();
+    uint32_t at = sh.local_base[digit] + (h == 0 ? 0u : sh.half[digit]);
+#pragma unroll
+    for (int w = 0; w < kRuns / 2; ++w) {
+        sh.count[h * (kRuns / 2) + w][digit] = static_cast<uint16_t>(at);
+        at += c[w];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < kItems; ++e) pos[e] += mine[(e / kSteps) * kMaxRadix + digit_of(keys[e], shift, mask)];
+}
+
+// Stable scatter of one pass: rank, put the entries into a shared-memory copy of the block's output in digit order, send
+// that out (entry j of digit d lands at the global base of (d, block) + j - local base of d, so consecutive threads write
+// consecutive addresses inside a digit's run instead of 32 different lines per warp instruction).
+// kFirst: keys from the indices, values are the flat positions themselves.  kLast: keys are not written; the head of every
+// run of equal keys lowers its row's row_ptr to its position.
+// What bounds it: instruction issue, shared-memory bank conflicts of the ranked accesses and latency, about a third each;
+// occupancy and block size change little.  8.4 M slots, 32768 rows: 76 -> 55 us per pass.
+template <typename KeyT, int kItems> constexpr int scatter_smem() { return kThreads * kItems * static_cast<int>(4 + sizeof(KeyT)); }
+
+template <typename KeyT, bool kFirst, bool kLast, int kItems>
+__global__ void __launch_bounds__(kThreads, 2)
+scatter_kernel(const KeyT* __restrict__ keys_in, const int32_t* __restrict__ vals_in, const Source src, KeyT* __restrict__ keys_out,
+               int32_t* __restrict__ vals_out, const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, uint32_t n,
+               int shift, uint32_t mask, int n_blocks, int32_t* __restrict__ row_ptr) {
+    constexpr int kBlockItems = kThreads * kItems, kWarpItems = 32 * kItems;
+    extern __shared__ __align__(16) uint32_t staged[];
+    int32_t* svals = reinterpret_cast<int32_t*>(staged);
+    KeyT* skeys = reinterpret_cast<KeyT*>(staged + kBlockItems);
+    __shared__ RankShared sh;
+    __shared__ uint32_t out_base[kMaxRadix];      // global position of staged position 0 of the digit's run
+    const int radix = static_cast<int>(mask) + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t block0 = blockIdx.x * kBlockItems;
+    const uint32_t first = block0 + warp * kWarpItems + lane;
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    uint32_t keys[kItems], pos[kItems];
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+        const uint32_t i = first + t * 32;
+        if (kFirst) keys[t] = i < n ? static_cast<uint32_t>(__ldg(src.indices + i)) : 0u;
+        else keys[t] = i < n ? keys_in[i] : 0u;
+    }
+    const uint32_t tot = threadIdx.x < radix ? totals[threadIdx.x] : 0u;
+    const uint32_t blk = threadIdx.x < radix ? hist[static_cast<size_t>(threadIdx.x) * n_blocks + blockIdx.x] : 0u;
+    if (kFirst) {
+#pragma unroll
+        for (int t = 0; t < kItems; ++t) keys[t] = src.key(first + t * 32, static_cast<int>(keys[t]));
+    }
+    const uint32_t digit0 = block_exclusive_scan(tot, sh.warp_sums, &sh.total);
+    block_rank(keys, shift, mask, first, n, sh, pos);
+    if (threadIdx.x < radix) out_base[threadIdx.x] = digit0 + blk - sh.local_base[threadIdx.x];
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+        const uint32_t i = first + t * 32;
+        if (i < n) {
+            skeys[pos[t]] = static_cast<KeyT>(keys[t]);
+            svals[pos[t]] = kFirst ? static_cast<int32_t>(i) : __ldg(vals_in + i);
         }
     }
     __syncthreads();
-    const int64_t left = n - block0;
-    const int count = left < kBlockItems ? static_cast<int>(left) : kBlockItems;
-#pragma unroll 4
-    for (int j = threadIdx.x; j < count; j += kThreads) {
+    const uint32_t count = min(n - block0, static_cast<uint32_t>(kBlockItems));
+#pragma unroll 8
+    for (uint32_t j = threadIdx.x; j < count; j += kThreads) {
         const uint32_t key = skeys[j];
-        const uint32_t d = digit_of(key, shift, mask);
-        const uint32_t pos = global_base[d] + (static_cast<uint32_t>(j) - local_base[d]);
-        keys_out[pos] = key;
-        vals_out[pos] = svals[j];
+        const uint32_t at = out_base[digit_of(key, shift, mask)] + j;
+        vals_out[at] = svals[j];
+        if (!kLast) keys_out[at] = static_cast<KeyT>(key);
+        else if (j == 0 || skeys[j - 1] != key) atomicMin(row_ptr + key, static_cast<int32_t>(at));
     }
 }
 
-// row_ptr[r] = number of sorted keys below r = first position whose key is >= r, for r in [0, s_kv].
-__global__ void row_ptr_kernel(const uint32_t* __restrict__ sorted_keys, int32_t* __restrict__ row_ptr, int64_t n,
-                               int32_t s_kv) {
+// Rows without a slot take the next row's position: suffix minimum of the run heads (they ascend with the row).  In place
+// and out of place: heads are read, row_ptr written.
+__global__ void __launch_bounds__(kRowTile)
+row_ptr_kernel(const int32_t* __restrict__ heads, int32_t* __restrict__ row_ptr, int32_t n, int32_t s_kv) {
+    __shared__ int warp_min[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    const int r = blockIdx.x * kRowTile + threadIdx.x;
+    int v = r <= s_kv ? heads[r] : INT_MAX;
+    // the first run behind this block's rows, a block's width at a time (nearly always within the first)
+    int later = INT_MAX;
+    for (int64_t base = static_cast<int64_t>(blockIdx.x + 1) * kRowTile; base <= s_kv; base += kRowTile) {
+        const int64_t i = base + threadIdx.x;
+        const int h = i <= s_kv ? heads[i] : INT_MAX;
+        if (__syncthreads_or(h != INT_MAX)) {
+            later = h;
+            break;
+        }
+    }
+    later = __reduce_min_sync(0xffffffffu, later);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int down = __shfl_down_sync(0xffffffffu, v, o);
+        if (lane + o < 32) v = min(v, down);
+    }
+    __shared__ int later_min[32];
+    if (lane == 0) {
+        warp_min[warp] = v;
+        later_min[warp] = later;
+    }
+    __syncthreads();
+    int m = min(later_min[lane], n);
+    if (lane > warp) m = min(m, warp_min[lane]);
+    m = __reduce_min_sync(0xffffffffu, m);
+    if (r <= s_kv) row_ptr[r] = min(v, m);
+}
+
+// ---- at most one block's worth of slots: every pass in shared memory -----------------------------------------------------
+template <typename KeyT>
+__global__ void __launch_bounds__(kThreads, 1)
+small_sort_kernel(const Source src, KeyT* __restrict__ keys_out, int32_t* __restrict__ vals_out, uint32_t n, int passes, int digit_bits) {
+    constexpr int kItems = kItemsLarge, kBlockItems = kSmallInput, kWarpItems = 32 * kItems;
+    extern __shared__ __align__(16) uint32_t staged[];
+    int32_t* svals = reinterpret_cast<int32_t*>(staged);
+    KeyT* skeys = reinterpret_cast<KeyT*>(staged + kBlockItems);
+    __shared__ RankShared sh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = warp * kWarpItems + lane;
+    const uint32_t mask = (1u << digit_bits) - 1u;
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    uint32_t keys[kItems], vals[kItems], pos[kItems];
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+        const uint32_t i = first + t * 32;
+        keys[t] = i < n ? src.key(i, __ldg(src.indices + i)) : 0u;
+        vals[t] = i;
+    }
+    for (int pass = 0; pass < passes; ++pass) {
+        block_rank(keys, pass * digit_bits, mask, first, n, sh, pos);
+#pragma unroll
+        for (int t = 0; t < kItems; ++t)
+            if (first + t * 32 < n) {
+                skeys[pos[t]] = static_cast<KeyT>(keys[t]);
+                svals[pos[t]] = static_cast<int32_t>(vals[t]);
+            }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kItems; ++t) {
+            const uint32_t i = first + t * 32;
+            keys[t] = i < n ? skeys[i] : 0u;
+            vals[t] = i < n ? static_cast<uint32_t>(svals[i]) : 0u;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+        const uint32_t i = first + t * 32;
+        if (i < n) {
+            keys_out[i] = static_cast<KeyT>(keys[t]);
+            vals_out[i] = static_cast<int32_t>(vals[t]);
+        }
+    }
+}
+// row_ptr[r] = first position in the sorted keys whose key is >= r, for r in [0, s_kv] (a few thousand keys: they sit in L1).
+template <typename KeyT>
+__global__ void __launch_bounds__(256)
+small_row_ptr_kernel(const KeyT* __restrict__ sorted_keys, int32_t* __restrict__ row_ptr, int32_t n, int32_t s_kv) {
+    smla::pdl_wait();
+    smla::pdl_trigger();
     const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r > s_kv) return;
-    int64_t lo = 0, hi = n;
+    int lo = 0, hi = n;
     while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (sorted_keys[mid] < static_cast<uint32_t>(r)) lo = mid + 1; else hi = mid;
+        const int mid = (lo + hi) >> 1;
+        if (sorted_keys[mid] < static_cast<uint32_t>(r)) lo = mid + 1;
+        else hi = mid;
     }
-    row_ptr[r] = static_cast<int32_t>(lo);
+    row_ptr[r] = lo;
 }
 
 }  // namespace inv
