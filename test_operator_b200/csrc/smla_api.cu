@@ -397,7 +397,8 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
         launch(smla_recompute_pair_kernel<HP>, grid_of(pairs), rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
-    auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl) {
+    auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl, bool after_recompute) {
+        kp.early_start = after_recompute;
         if (det) {
             // reproducible form: per-slot contributions to the staging rows, then one warp per kv row adds its slots
             // of this pass in CSR order
@@ -411,7 +412,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     };
     const int dq_split = dq_key_split(p->s_q, pl.topk_pad, dq::kParts);
     auto launch_dq = [&](cudaStream_t s_, bool pdl, bool after_dkv) {
-        kp.dq_after_trigger = after_dkv;
+        kp.early_start = after_dkv;
         launch(smla_dq_kernel<HP>, kp.nq * dq::kParts * dq_split, dq::kThreads,
                dq_split > 1 ? DqCfg::kSplitSmemBytes : DqCfg::kSmemBytes, s_, pdl, dq_split, tm_ds, kp);
     };
@@ -433,7 +434,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             kp.nq = nq;
             kp.scr0 = 0;
             if (stages & SMLA_STAGE_RECOMPUTE) launch_recompute(st, pairs_r, true);
-            if (stages & SMLA_STAGE_DKV) launch_dkv(st, pairs_d, true);
+            if (stages & SMLA_STAGE_DKV) launch_dkv(st, pairs_d, true, stages & SMLA_STAGE_RECOMPUTE);
             if (stages & SMLA_STAGE_DQ) launch_dq(st, true, (stages & SMLA_STAGE_DKV) && !det);
             continue;
         }
@@ -454,7 +455,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             if (cudaEventRecord(ds->ev_part[c], st) != cudaSuccess ||
                 cudaStreamWaitEvent(ds->side, ds->ev_part[c], 0) != cudaSuccess)
                 return SMLA_ERR_LAUNCH;
-            launch_dkv(ds->side, c == parts - 1 ? pairs_d : dkv_pairs, false);
+            launch_dkv(ds->side, c == parts - 1 ? pairs_d : dkv_pairs, false, false);
             launch_dq(st, false, false);
         }
         if (cudaEventRecord(ds->ev_join, ds->side) != cudaSuccess || cudaStreamWaitEvent(st, ds->ev_join, 0) != cudaSuccess)
@@ -548,7 +549,7 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     const int clusters = std::max(1, std::min(pairs, pl.clusters));
     launch(smla_fwd_kernel<HP>, 2 * clusters, ff::kThreads, ff::kSmemBytes, st, true, 1, tm_q, kp);
     if (clusters > 1)
-        launch(smla_fwd_combine_kernel, (clusters - 1) * ((p->h_q + 7) / 8), 256, 0, st, true, 1, kp, clusters, HP);
+        launch(smla_fwd_combine_kernel, std::min(p->s_q, clusters - 1) * ((p->h_q + 3) / 4), 256, 0, st, true, 1, kp, clusters, HP);
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 

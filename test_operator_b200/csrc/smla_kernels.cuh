@@ -61,7 +61,7 @@ struct KParams {
     const int4* qmeta;        // optional per query {first kv row of its sequence, kv rows of its sequence,
                               // position for the causal rule, top-k slots in use}; null: one sequence
     long long wait_limit;     // cycles a bounded wait may take
-    int dq_after_trigger;     // dq: launched behind the dKV kernel's trigger (see smla_dq_kernel)
+    int early_start;          // dkv, dq: launched behind the trigger of the kernel before in the same call (see there)
 };
 
 // What a query may attend to: rows [kv_base, kv_base + kv_len) of kv, index values relative to kv_base.
@@ -333,24 +333,38 @@ __device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
 }
 template <int kMul> struct TileIter {
     const int* pre;
+    const int* used;
     int q, q_last, lo, hi, hi_next, pos, end;
+    int stop;                     // behind the query's last tile with a slot in use (kMul 2: hi or hi - 1)
+    int n_next;                   // kMul 2: slots in use of query q + 1
     __device__ __forceinline__ TileIter(const KParams& p, const WorkRange& w)
-        : pre(p.tile_pre), q(w.q), q_last(p.q0 + p.nq), pos(w.begin * kMul), end(w.end * kMul) {
+        : pre(p.tile_pre), used(p.n_used), q(w.q), q_last(p.q0 + p.nq), pos(w.begin * kMul), end(w.end * kMul) {
         lo = __ldcg(pre + q) * kMul;
         hi = __ldcg(pre + q + 1) * kMul;
         hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;      // one query ahead: the load is done when it is needed
+        if constexpr (kMul > 1) n_next = __ldcg(used + q);
+        set_stop();
+    }
+    __device__ __forceinline__ void set_stop() {
+        stop = hi;
+        if constexpr (kMul > 1) {
+            stop = lo + (n_next + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul);
+            n_next = __ldcg(used + min(q + 1, q_last - 1));
+        }
     }
     __device__ __forceinline__ bool more() const { return pos < end; }
     __device__ __forceinline__ int tile() const { return pos - lo; }
-    __device__ __forceinline__ bool last_of_query() const { return pos + 1 == hi || pos + 1 == end; }
+    __device__ __forceinline__ bool last_of_query() const { return pos + 1 == stop || pos + 1 == end; }
     // to the next tile; true if that is another query's (or the range is finished)
     __device__ __forceinline__ bool advance() {
-        if (++pos < hi) return pos >= end;
+        if (++pos < stop) return pos >= end;
+        pos = hi;
         while (pos < end) {
             ++q;
             lo = hi;
             hi = hi_next;
             hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;
+            set_stop();
             if (hi > lo) break;
         }
         return true;
@@ -1218,48 +1232,80 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 }
 
 // Queries whose tiles were spread over several clusters: o = sum of 2^(ref_i - ref) O_i over the parts, divided by the sum
-// of their weighted row sums.  One warp per (boundary between two ranges, head); the boundary that is the query's first
-// does the work, in the order of the parts.  Bound by the latency of a few dependent loads (256 KB per part, in L2).
-__global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
+// of their weighted row sums.  One warp per (item, head, half of the columns); the items are the queries where there are at most as many as
+// boundaries between ranges, else the boundaries (the one that is its query's first does the work).  Lane i takes the
+// reference and the sum of part i, all weights are known before the first row of O is loaded, and the rows are added in
+// the order of the parts with four in flight.  Bound by the latency of its dependent rounds of loads (eight tokens, eight
+// parts each: 20 us with a block per boundary and a round per part, 7.6 us so).
+__global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int per_boundary = (p.h_q + 7) / 8;
-    const int c = static_cast<int>(blockIdx.x) / per_boundary + 1;
-    const int head = static_cast<int>(blockIdx.x) % per_boundary * 8 + (threadIdx.x >> 5);
-    const WorkRange w = find_range(p, c, n_clusters);
+    const int per_item = (p.h_q + 3) / 4;
+    const int item = static_cast<int>(blockIdx.x) / per_item;
+    const int head = static_cast<int>(blockIdx.x) % per_item * 4 + (threadIdx.x >> 6);
+    const int half = (threadIdx.x >> 5) & 1;
+    if (head >= p.h_q) return;
+    const bool by_query = p.nq < n_clusters;
+    const int q = by_query ? p.q0 + item : find_range(p, item + 1, n_clusters).q;
     const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
-    const int q_begin = __ldcg(p.tile_pre + w.q), q_end = __ldcg(p.tile_pre + w.q + 1);
-    if (w.begin <= q_begin || w.begin >= q_end || range_start(t0, t1, c - 1, n_clusters) > q_begin || head >= p.h_q) return;
-    float ref = __int_as_float(0xff800000), sum = 0.f, acc[16] = {};
-    for (int k = c - 1; k < n_clusters; ++k) {
-        const int begin = range_start(t0, t1, k, n_clusters);
-        if (begin >= q_end) break;
-        if (begin == range_start(t0, t1, k + 1, n_clusters)) continue;
+    const int q_begin = __ldcg(p.tile_pre + q), q_end = __ldcg(p.tile_pre + q + 1);
+    if (q_begin >= q_end) return;                // no valid slot: the prep kernel has written o and lse
+    // the cluster whose range holds the query's first tile: the largest k with range_start(k) <= q_begin
+    const int first = static_cast<int>((static_cast<long long>(q_begin - t0 + 1) * n_clusters - 1) / (t1 - t0));
+    if (range_start(t0, t1, first + 1, n_clusters) >= q_end || (!by_query && first != item)) return;
+    const float ninf = __int_as_float(0xff800000);
+    float ref = ninf, sum = 0.f, acc[8] = {};
+    for (int k0 = first; k0 < n_clusters; k0 += 32) {          // 32 parts at a time
+        const int k = k0 + lane;
+        const int begin = k < n_clusters ? range_start(t0, t1, k, n_clusters) : t1;
+        const bool part = k < n_clusters && begin < q_end && begin < range_start(t0, t1, k + 1, n_clusters);
         const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head;
-        const float2 ml = __ldcg(p.part_ml + row);
-        const float4* o = reinterpret_cast<const float4*>(p.part_o + row * kDV) + lane;
-        float4 v[4];
+        float2 ml = make_float2(ninf, 0.f);
+        if (part) ml = __ldcg(p.part_ml + row);
+        if (!(ml.y > 0.f)) ml.x = ninf;                         // no valid slot in this part
+        float top = ml.x;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = __ldcg(o + 32 * i);
-        if (!(ml.y > 0.f)) continue;             // no valid slot in this part
-        const float top = fmaxf(ref, ml.x);
-        const float keep = ex2_approx(ref - top), add = ex2_approx(ml.x - top);
-        sum = sum * keep + ml.y * add;
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        top = fmaxf(top, ref);
+        const float weight = ml.x > ninf ? ex2_approx(ml.x - top) : 0.f;
+        const float keep = ref > ninf ? ex2_approx(ref - top) : 0.f;
+        sum = sum * keep + warp_sum(weight * ml.y);
         ref = top;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            acc[4 * i] = acc[4 * i] * keep + v[i].x * add;
-            acc[4 * i + 1] = acc[4 * i + 1] * keep + v[i].y * add;
-            acc[4 * i + 2] = acc[4 * i + 2] * keep + v[i].z * add;
-            acc[4 * i + 3] = acc[4 * i + 3] * keep + v[i].w * add;
+        for (int i = 0; i < 8; ++i) acc[i] *= keep;
+        uint32_t todo = __ballot_sync(0xffffffffu, weight > 0.f);
+        const float* mine = p.part_o + row * kDV + half * (kDV / 2);
+        while (todo) {
+            float4 v[4][2];
+            float wt[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int src = todo ? __ffs(todo) - 1 : 0;
+                wt[u] = todo ? __shfl_sync(0xffffffffu, weight, src) : 0.f;
+                const float4* o = reinterpret_cast<const float4*>(
+                    reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), src))) + lane;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) v[u][i] = wt[u] > 0.f ? __ldcg(o + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                todo &= todo - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    acc[4 * i] = fmaf(v[u][i].x, wt[u], acc[4 * i]);
+                    acc[4 * i + 1] = fmaf(v[u][i].y, wt[u], acc[4 * i + 1]);
+                    acc[4 * i + 2] = fmaf(v[u][i].z, wt[u], acc[4 * i + 2]);
+                    acc[4 * i + 3] = fmaf(v[u][i].w, wt[u], acc[4 * i + 3]);
+                }
         }
+        if (__shfl_sync(0xffffffffu, begin, 31) >= q_end) break;
     }
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
-    const size_t orow = static_cast<size_t>(w.q) * p.h_q + head;
-    if (lane == 0) p.lse_out[orow] = (sum > 0.f ? ref + __log2f(sum) : __int_as_float(0x7f800000)) * p.lse_out_mult;
-    uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV) + lane;
+    const size_t orow = static_cast<size_t>(q) * p.h_q + head;
+    if (lane == 0 && half == 0) p.lse_out[orow] = (sum > 0.f ? ref + __log2f(sum) : __int_as_float(0x7f800000)) * p.lse_out_mult;
+    uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV + half * (kDV / 2)) + lane;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
         out[32 * i] = make_uint2(pack_bf16x2(acc[4 * i] * inv, acc[4 * i + 1] * inv), pack_bf16x2(acc[4 * i + 2] * inv, acc[4 * i + 3] * inv));
 }
 
@@ -1348,8 +1394,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_alloc_2cta(smem_u32(tmem_slot), 512);
         tmem_relinquish_2cta();
     }
-    pdl_wait();                  // the recompute kernel's S and dS, the prep kernel's tile counts and cleared dKV
-    pdl_trigger();
+    // Behind the recompute kernel's trigger (it triggers after it has waited for the prep kernel) everything but S and dS is in
+    // place already: tile counts, indices, Q, dO, a cleared dKV.  Then only the first S / dS load waits.
+    if (!p.early_start) pdl_wait();
     if (warp == 0) {
         const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
         if (lane == 0) *range_s = w;
@@ -1360,7 +1407,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
-    using Iter = TileIter<kWorkTileKeys / kTileKeys>;    // two tiles per work tile: a range has an even number of them
+    using Iter = TileIter<kWorkTileKeys / kTileKeys>;    // up to two tiles per work tile
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
@@ -1370,6 +1417,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             tma_prefetch_desc(&tm_s);
             tma_prefetch_desc(&tm_ds);
             const uint64_t pol_stream = l2_policy_evict_first();
+            bool waited = false;
             int s = 0;
             uint32_t ph = 1, k = 0;        // ph: parity that means "stage free" in the current pass over the ring
             bool new_query = true;
@@ -1388,6 +1436,11 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     }
                     tma_load_2d_hint(s_base + C::kOffQ + 4 * C::kChunk, &tm_q, 64 * 8, row0, bar_res, pol_stream);
                 }
+                if (!waited) {
+                    waited = true;
+                    pdl_wait();
+                    pdl_trigger();
+                }
                 mbar_wait(bar_tempty + 8 * s, ph, wc, kErrDkv + 1, kPollSleepNs);
                 mbar_arrive_expect_tx(bar_tfull + 8 * s, C::kStage);
                 const uint32_t dst = s_base + C::kOffStage + s * C::kStage;
@@ -1400,6 +1453,10 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     s = 0;
                     ph ^= 1;
                 }
+            }
+            if (!waited) {                 // nothing to do: the kernel behind this one still relies on the wait
+                pdl_wait();
+                pdl_trigger();
             }
         }
     } else if (warp == 1) {
@@ -1430,9 +1487,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 int s = 0;
                 uint32_t ph = 0, k = 0, unit = 0;
                 bool new_query = true;
-                Iter it(p, range);
-                const int n_tiles = (range.end - range.begin) * (kWorkTileKeys / kTileKeys);
-                for (int n = 0; n < n_tiles; ++n) {
+                for (Iter it(p, range); it.more();) {
                     if (new_query) mbar_wait(bar_res, k++ & 1, wc, kErrDkv + 2);
                     const bool last = it.last_of_query();
                     mbar_wait(bar_tfull + 8 * s, ph, wc, kErrDkv + 4);
@@ -1721,7 +1776,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     // Behind the dKV kernel's trigger everything this kernel reads is in place already (that kernel triggers after it has
     // waited for the recompute kernel), so its CTAs fill whatever SMs the dKV kernel leaves; the last CTA then holds the
     // grid open until the dKV kernel is done, so that "dq done" still means "all done" to whatever follows.
-    if (!p.dq_after_trigger) pdl_wait();
+    if (!p.early_start) pdl_wait();
     const int n_all = __shfl_sync(0xffffffffu, (__ldcg(p.n_used + qg) + kTileKeys - 1) / kTileKeys, 0);
     const int tile0 = n_all * z / nz, n_tiles = n_all * (z + 1) / nz - tile0;
 
@@ -1869,7 +1924,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         }
     }
     abort_wind_down(s_abort);
-    if (p.dq_after_trigger && blockIdx.x == gridDim.x - 1) pdl_wait();
+    if (p.early_start && blockIdx.x == gridDim.x - 1) pdl_wait();
     tc_fence_before_sync();
     __syncthreads();
     if (nz > 1) {
