@@ -66,11 +66,11 @@ void schedule(int* chunks, int* dkv_pairs) {
 // Clusters for the dkv kernel when the caller leaves the choice to the library: its share of the three kernels'
 // time, measured with each kernel alone on a whole B200 (top-k 2048; dkv 3.8 ms at either head count, recompute +
 // dq 3.4 ms at 128 heads and 2.65 ms at 64).  The step time is flat within +-3 clusters of these.
-// Measured on B200, alternating the schedules on one GPU: with 64 heads two overlapped parts beat one kernel after the
-// other by 4 % (5.89 against 6.16 ms; three parts and more lose to two, each launch has its own tail); with 128 heads the
-// kernels one after the other are 2.5 % faster than any overlapped form (7.39 against 7.60 ms, 8.64 against 8.85 ms over
-// a second of steps): there the recompute and dQ kernels want all of the SMs more than the dKV kernel minds having them.
-int auto_chunks(int h_pad) { return h_pad > 64 ? 0 : 2; }
+// Measured on B200, alternating the schedules on one GPU over a second of calls: one kernel after the other is the faster
+// form with 128 heads (8.04 against 8.40 ms on 4096 queries x top-k 2048) and with 64 (6.23 against 6.32 ms at top-k 2048,
+// 1.84 / 1.85 at 512, 0.436 / 0.448 on 777 queries x 600): the dKV kernel's reductions and the other kernels' gathers share
+// the L2, so running them side by side gives the sum of their times.  The overlapped form stays for queries of one tile.
+int auto_chunks(int h_pad, int topk_pad) { return h_pad > 64 || topk_pad > smla::kWorkTileKeys ? 0 : 2; }
 
 int auto_dkv_pairs(int h_pad, int resident) {
     const double share = h_pad > 64 ? 0.50 : 0.60;
@@ -419,7 +419,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
 
     int chunks = 0, dkv_pairs = 0;
     schedule(&chunks, &dkv_pairs);
-    if (chunks < 0) chunks = auto_chunks(HP);
+    if (chunks < 0) chunks = auto_chunks(HP, pl.topk_pad);
     const int all = SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ;
     if (dkv_pairs <= 0) dkv_pairs = auto_dkv_pairs(HP, pairs_d < pairs_r ? pairs_d : pairs_r);
     if (!allow_overlap || det || (stages & all) != all || dkv_pairs >= pairs_d || dkv_pairs >= pairs_r) chunks = 0;
