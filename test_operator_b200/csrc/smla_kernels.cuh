@@ -50,6 +50,7 @@ struct KParams {
     float lse_out_mult;       // 1 (base 2) or ln 2 (natural log)
     float* part_o;            // partial results of queries spread over several clusters: [slot][HP][512]
     float2* part_ml;          // [slot][HP] {reference of the exponentials (log2), sum}
+    int* range_q;             // [clusters] first query of each cluster's range
     __nv_bfloat16* gout;      // [s_q, h_q, 512] o (forward only)
     int* g_err;
     int q0;                   // first query (global row) of this launch
@@ -182,15 +183,16 @@ __device__ __forceinline__ int block_exclusive_sum(int v, int* warp_sums, int* t
 __global__ void __launch_bounds__(kPrepThreads)
 smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, float* __restrict__ delta,
                  int* __restrict__ n_used, int* __restrict__ tile_pre, int* ticket, uint4* __restrict__ zero_dst,
-                 size_t zero_n, const KParams p) {
+                 size_t zero_n, int head_parts, const KParams p) {
     __shared__ int red[32];
     __shared__ int is_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kWarps = kPrepThreads / 32;
     pdl_wait();                   // (nothing above touches memory another kernel of the stream may still use)
     pdl_trigger();
-    const int q = blockIdx.x;
-    if (q < p.s_q) {
+    // with few queries several blocks share one query's heads; the first of them also looks at its indices
+    const int q = blockIdx.x / head_parts, hp = blockIdx.x % head_parts;
+    if (q < p.s_q && hp == 0) {
         const QMeta qm = load_qmeta(p, q);
         int last = -1;
         for (int key = threadIdx.x; key < p.topk; key += kPrepThreads)
@@ -202,7 +204,7 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
     // The block that takes the last ticket sees every query's count and sums up the tiles at the end.  The ticket is drawn
     // here so that its round trip runs under the loads below.
     if (threadIdx.x == 0) {
-        if (q < p.s_q) {
+        if (q < p.s_q && hp == 0) {
             int m = red[0];
 #pragma unroll
             for (int w = 1; w < kWarps; ++w) m = max(m, red[w]);
@@ -226,8 +228,9 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
         const uint4* o = O + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
         const uint4* g = dO + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
         // two rows at a time: eight 16-byte loads of a lane in flight
-        for (int h = warp; h < p.h_q; h += 2 * kWarps) {
-            const int h2 = h + kWarps < p.h_q ? h + kWarps : h;
+        const int h_end = p.h_q * (hp + 1) / head_parts;
+        for (int h = p.h_q * hp / head_parts + warp; h < h_end; h += 2 * kWarps) {
+            const int h2 = h + kWarps < h_end ? h + kWarps : h;
             uint4 a[4], b[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -854,7 +857,10 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     pdl_trigger();
     if (warp == 17) {
         const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
-        if (lane == 0) *range_s = w;
+        if (lane == 0) {
+            *range_s = w;
+            if (rank == 0) p.range_q[blockIdx.x >> 1] = w.q;
+        }
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -1081,6 +1087,33 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         load_idx();
         bool new_query = true;
         float ref = ninf, sum = 0.f;         // reference of the row's exponentials (log2 units), sum over this thread's keys
+        // A query's O leaves when the next tile's exponentials are done: waiting for the last P V right behind its P held
+        // up the next query's softmax, and the tensor pipe with it, by about 4000 cycles a query.
+        bool pending = false, pend_whole = false;
+        float pend_inv = 0.f;
+        size_t pend_row = 0;
+        auto write_out = [&]() {
+            pending = false;
+            // lanes 0-63: columns [256 block, + 128), lanes 64-127: [256 block + 128, + 128)
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) {
+                const int blk = c >> 2, e = (c & 3) * 16;
+                uint32_t o[16];
+                tmem_ld_32x16(tmem + lanes + kTmemO + blk * 128 + ch * 64 + e, o);
+                tmem_ld_wait();
+                const size_t at = pend_row * kDV + blk * 256 + (quarter >> 1) * 128 + ch * 64 + e;
+                if (real && pend_whole) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        w[i] = pack_bf16x2(__uint_as_float(o[2 * i]) * pend_inv, __uint_as_float(o[2 * i + 1]) * pend_inv);
+                    st_global_v8(p.gout + at, w);
+                } else if (real) {
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) st_global_v8(p.part_o + at + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
+                }
+            }
+        };
         int seg_begin = 0;
         for (int n = 0; n < n_tiles; ++n) {
             const int key = it.tile() * kTileKeys + part * 64 + lane;
@@ -1150,6 +1183,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             // P of the previous tile has been consumed and O is at rest
             if (n > 0) mbar_wait(bar_pv, (n - 1) & 1, wc, kErrFwd + 20, kPollSleepNs);
             tc_fence_after_sync();
+            if (pending) write_out();
             if (__any_sync(0xffffffffu, rescale)) {          // this warp's half of the columns of both d-blocks
 #pragma unroll 1
                 for (int c = 0; c < 256; c += 128) {
@@ -1175,53 +1209,33 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             if (lane == 0) mbar_arrive_cluster_release(pfull0);
 
             if (last) {
-                // ---- the query's (or the range's) last tile: o, lse - or an unnormalised part of them
+                // ---- the query's (or the range's) last tile: lse now, o once its P V is done - or an unnormalised part of them
                 const bool whole = seg_begin == q_lo && seg_end == q_hi;
                 stat[(4 * ((n + 1) & 1) + part) * 64 + row] = sum;
                 asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
                 const float* sums = stat + 4 * ((n + 1) & 1) * 64 + row;
                 const float total = (sums[0] + sums[64]) + (sums[128] + sums[192]);
                 asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // the next tile's maxima go to the same place
-                const float inv = total > 0.f ? 1.f / total : 0.f;
                 const size_t orow = static_cast<size_t>(qg) * p.h_q + head;
                 // partial results: slot 2 c for a range that starts inside the query, 2 c + 1 for one that starts at or before it
-                const int slot = static_cast<int>(blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0);
+                const size_t prow = static_cast<size_t>((blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0)) * HP + head;
                 if (real && part == 0) {
                     if (whole)
                         p.lse_out[orow] = (total > 0.f ? ref + __log2f(total) : __int_as_float(0x7f800000)) * p.lse_out_mult;
                     else
-                        p.part_ml[static_cast<size_t>(slot) * HP + head] = make_float2(ref, total);
+                        p.part_ml[prow] = make_float2(ref, total);
                 }
-                mbar_wait(bar_pv, n & 1, wc, kErrFwd + 21, kPollSleepNs);
-                tc_fence_after_sync();
-                // lanes 0-63: columns [256 block, + 128), lanes 64-127: [256 block + 128, + 128)
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    const int blk = c >> 1, e = (c & 1) * 32;
-                    uint32_t o[32];
-                    tmem_ld_32x32(tmem + lanes + kTmemO + blk * 128 + ch * 64 + e, o);
-                    tmem_ld_wait();
-                    const int col = blk * 256 + (quarter >> 1) * 128 + ch * 64 + e;
-                    if (real && whole) {
-                        __nv_bfloat16* out = p.gout + orow * kDV + col;
-#pragma unroll
-                        for (int v = 0; v < 2; ++v) {
-                            uint32_t w[8];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                w[i] = pack_bf16x2(__uint_as_float(o[16 * v + 2 * i]) * inv, __uint_as_float(o[16 * v + 2 * i + 1]) * inv);
-                            st_global_v8(out + 16 * v, w);
-                        }
-                    } else if (real) {
-                        float* out = p.part_o + (static_cast<size_t>(slot) * HP + head) * kDV + col;
-#pragma unroll
-                        for (int v = 0; v < 4; ++v)
-                            st_global_v8(out + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
-                    }
-                }
-                tc_fence_before_sync();      // O may be overwritten once this warp arrives for the next tile's P
+                pending = true;
+                pend_whole = whole;
+                pend_inv = total > 0.f ? 1.f / total : 0.f;
+                pend_row = whole ? orow : prow;
             }
             new_query = next_query;
+        }
+        if (pending) {
+            mbar_wait(bar_pv, (n_tiles - 1) & 1, wc, kErrFwd + 21, kPollSleepNs);
+            tc_fence_after_sync();
+            write_out();
         }
     }
     abort_wind_down(s_abort);
@@ -1232,21 +1246,24 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 }
 
 // Queries whose tiles were spread over several clusters: o = sum of 2^(ref_i - ref) O_i over the parts, divided by the sum
-// of their weighted row sums.  One warp per (item, head, half of the columns); the items are the queries where there are at most as many as
-// boundaries between ranges, else the boundaries (the one that is its query's first does the work).  Lane i takes the
-// reference and the sum of part i, all weights are known before the first row of O is loaded, and the rows are added in
-// the order of the parts with four in flight.  Bound by the latency of its dependent rounds of loads (eight tokens, eight
-// parts each: 20 us with a block per boundary and a round per part, 7.6 us so).
+// of their weighted row sums.  The items are the queries where there are at most as many as boundaries between ranges, else
+// the boundaries (the one that is its query's first does the work; the forward kernel has noted each range's first
+// query).  One warp per (item, kHeads heads, half of the columns): lane i takes the references and sums of part i, all
+// weights are known before the first row of O is loaded, and the rows are added in the order of the parts.  Bound by the
+// latency of its dependent rounds of loads: eight tokens of eight parts each 20 us with a block per boundary and a round
+// per part, 7.6 us so (kHeads 1); 94 queries over 73 boundaries 35 us with a search of the query in every block and a
+// warp per head, 15 us so (kHeads 4).
+template <int kHeads>
 __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int per_item = (p.h_q + 3) / 4;
+    const int per_item = (p.h_q + 4 * kHeads - 1) / (4 * kHeads);
     const int item = static_cast<int>(blockIdx.x) / per_item;
-    const int head = static_cast<int>(blockIdx.x) % per_item * 4 + (threadIdx.x >> 6);
+    const int head0 = (static_cast<int>(blockIdx.x) % per_item * 4 + (threadIdx.x >> 6)) * kHeads;
     const int half = (threadIdx.x >> 5) & 1;
-    if (head >= p.h_q) return;
+    if (head0 >= p.h_q) return;
     const bool by_query = p.nq < n_clusters;
-    const int q = by_query ? p.q0 + item : find_range(p, item + 1, n_clusters).q;
+    const int q = by_query ? p.q0 + item : __ldcg(p.range_q + item + 1);
     const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
     const int q_begin = __ldcg(p.tile_pre + q), q_end = __ldcg(p.tile_pre + q + 1);
     if (q_begin >= q_end) return;                // no valid slot: the prep kernel has written o and lse
@@ -1254,59 +1271,86 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
     const int first = static_cast<int>((static_cast<long long>(q_begin - t0 + 1) * n_clusters - 1) / (t1 - t0));
     if (range_start(t0, t1, first + 1, n_clusters) >= q_end || (!by_query && first != item)) return;
     const float ninf = __int_as_float(0xff800000);
-    float ref = ninf, sum = 0.f, acc[8] = {};
+    float ref[kHeads], sum[kHeads], acc[kHeads][8];
+#pragma unroll
+    for (int h = 0; h < kHeads; ++h) {
+        ref[h] = ninf;
+        sum[h] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[h][i] = 0.f;
+    }
     for (int k0 = first; k0 < n_clusters; k0 += 32) {          // 32 parts at a time
         const int k = k0 + lane;
         const int begin = k < n_clusters ? range_start(t0, t1, k, n_clusters) : t1;
         const bool part = k < n_clusters && begin < q_end && begin < range_start(t0, t1, k + 1, n_clusters);
-        const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head;
-        float2 ml = make_float2(ninf, 0.f);
-        if (part) ml = __ldcg(p.part_ml + row);
-        if (!(ml.y > 0.f)) ml.x = ninf;                         // no valid slot in this part
-        float top = ml.x;
+        const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head0;
+        float2 ml[kHeads];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        top = fmaxf(top, ref);
-        const float weight = ml.x > ninf ? ex2_approx(ml.x - top) : 0.f;
-        const float keep = ref > ninf ? ex2_approx(ref - top) : 0.f;
-        sum = sum * keep + warp_sum(weight * ml.y);
-        ref = top;
+        for (int h = 0; h < kHeads; ++h)
+            ml[h] = part && head0 + h < p.h_q ? __ldcg(p.part_ml + row + h) : make_float2(ninf, 0.f);
+        float weight[kHeads];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] *= keep;
-        uint32_t todo = __ballot_sync(0xffffffffu, weight > 0.f);
+        for (int h = 0; h < kHeads; ++h) {
+            const float m = ml[h].y > 0.f ? ml[h].x : ninf;     // no valid slot in this part
+            float top = m;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            top = fmaxf(top, ref[h]);
+            weight[h] = m > ninf ? ex2_approx(m - top) : 0.f;
+            const float keep = ref[h] > ninf ? ex2_approx(ref[h] - top) : 0.f;
+            sum[h] = sum[h] * keep + warp_sum(weight[h] * ml[h].y);
+            ref[h] = top;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[h][i] *= keep;
+        }
+        uint32_t todo = __ballot_sync(0xffffffffu, part);
         const float* mine = p.part_o + row * kDV + half * (kDV / 2);
+        constexpr int kFly = 4 / kHeads;                       // parts in flight (times kHeads rows of 1 KB)
         while (todo) {
-            float4 v[4][2];
-            float wt[4];
+            float4 v[kFly][kHeads][2];
+            float wt[kFly][kHeads];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kFly; ++u) {
                 const int src = todo ? __ffs(todo) - 1 : 0;
-                wt[u] = todo ? __shfl_sync(0xffffffffu, weight, src) : 0.f;
                 const float4* o = reinterpret_cast<const float4*>(
                     reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), src))) + lane;
 #pragma unroll
-                for (int i = 0; i < 2; ++i) v[u][i] = wt[u] > 0.f ? __ldcg(o + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int h = 0; h < kHeads; ++h) {
+                    wt[u][h] = __shfl_sync(0xffffffffu, weight[h], src);
+                    if (!todo) wt[u][h] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        v[u][h][i] = wt[u][h] > 0.f ? __ldcg(o + h * (kDV / 4) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
                 todo &= todo - 1;
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < kFly; ++u)
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    acc[4 * i] = fmaf(v[u][i].x, wt[u], acc[4 * i]);
-                    acc[4 * i + 1] = fmaf(v[u][i].y, wt[u], acc[4 * i + 1]);
-                    acc[4 * i + 2] = fmaf(v[u][i].z, wt[u], acc[4 * i + 2]);
-                    acc[4 * i + 3] = fmaf(v[u][i].w, wt[u], acc[4 * i + 3]);
-                }
+                for (int h = 0; h < kHeads; ++h)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        acc[h][4 * i] = fmaf(v[u][h][i].x, wt[u][h], acc[h][4 * i]);
+                        acc[h][4 * i + 1] = fmaf(v[u][h][i].y, wt[u][h], acc[h][4 * i + 1]);
+                        acc[h][4 * i + 2] = fmaf(v[u][h][i].z, wt[u][h], acc[h][4 * i + 2]);
+                        acc[h][4 * i + 3] = fmaf(v[u][h][i].w, wt[u][h], acc[h][4 * i + 3]);
+                    }
         }
         if (__shfl_sync(0xffffffffu, begin, 31) >= q_end) break;
     }
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
-    const size_t orow = static_cast<size_t>(q) * p.h_q + head;
-    if (lane == 0 && half == 0) p.lse_out[orow] = (sum > 0.f ? ref + __log2f(sum) : __int_as_float(0x7f800000)) * p.lse_out_mult;
-    uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV + half * (kDV / 2)) + lane;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-        out[32 * i] = make_uint2(pack_bf16x2(acc[4 * i] * inv, acc[4 * i + 1] * inv), pack_bf16x2(acc[4 * i + 2] * inv, acc[4 * i + 3] * inv));
+    for (int h = 0; h < kHeads; ++h) {
+        if (head0 + h >= p.h_q) break;
+        const float inv = sum[h] > 0.f ? 1.f / sum[h] : 0.f;
+        const size_t orow = static_cast<size_t>(q) * p.h_q + head0 + h;
+        if (lane == 0 && half == 0)
+            p.lse_out[orow] = (sum[h] > 0.f ? ref[h] + __log2f(sum[h]) : __int_as_float(0x7f800000)) * p.lse_out_mult;
+        uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV + half * (kDV / 2)) + lane;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            out[32 * i] = make_uint2(pack_bf16x2(acc[h][4 * i] * inv, acc[h][4 * i + 1] * inv),
+                                     pack_bf16x2(acc[h][4 * i + 2] * inv, acc[h][4 * i + 3] * inv));
+    }
 }
 
 // =============================================================================================
