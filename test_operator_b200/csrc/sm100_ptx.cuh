@@ -150,11 +150,8 @@ __device__ __noinline__ void mbar_wait_drain(uint32_t bar, uint32_t parity, long
     }
 }
 
-// ---- plain shared-memory counter as a hand-over between two threads of a CTA ------------------------------
-// An mbarrier arrival takes ~180 cycles to become visible to a poller; a volatile word takes a few tens.
-__device__ __forceinline__ void flag_store(uint32_t saddr, uint32_t v) {
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory");
-}
+// ---- plain shared-memory counter -----------------------------------------------------------------------
+// Only the bounded-wait self-test polls one: every kernel issues its UMMAs from a single thread, so none is handed over.
 __device__ __forceinline__ uint32_t flag_load(uint32_t saddr) {
     uint32_t v;
     asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
@@ -460,16 +457,6 @@ __device__ __forceinline__ void st_global_f32_if_row(float* addr, float v, int r
         "setp.ge.s32 p, %2, 0;\n\t"
         "@p st.global.f32 [%0], %1;\n\t}"
         ::"l"(addr), "f"(v), "r"(row)
-        : "memory");
-}
-// The same with an L2 eviction policy: the accumulator rows are touched again by later queries and should
-// outlive the operands that only stream through.
-__device__ __forceinline__ void red_add_f32_if_row_hint(float* addr, float v, int row, uint64_t policy) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ge.s32 p, %2, 0;\n\t"
-        "@p red.global.add.L2::cache_hint.f32 [%0], %1, %3;\n\t}"
-        ::"l"(addr), "f"(v), "r"(row), "l"(policy)
         : "memory");
 }
 

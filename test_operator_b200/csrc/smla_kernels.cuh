@@ -1588,9 +1588,6 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         int* idx_base = reinterpret_cast<int*>(smem + C::kOffIdx) + (grp * 4 + e) * 64;
         const int bar_id = 1 + grp * 2 + e;
         const uint32_t uempty0 = map_to_cta(bar_uempty, 0);
-#ifdef SMLA_RED_EVICT_LAST
-        const uint64_t pol_keep = l2_policy_evict_last();
-#endif
         int pf[2] = {-1, -1};
         // (the dKV row a valid slot adds to, -1 for an unused slot)
         auto fetch_idx = [&](int qg, int tile) {
@@ -1648,14 +1645,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                 st_global_f32_if_row(sout + static_cast<size_t>(32 * i + j) * kDQK, __uint_as_float(r[j]), ix[j]);
                         } else {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-#ifdef SMLA_RED_EVICT_LAST
-                            red_add_f32_if_row_hint(out + static_cast<size_t>(static_cast<unsigned>(ix[j])) * kDQK,
-                                                    __uint_as_float(r[j]), ix[j], pol_keep);
-#else
-                            red_add_f32_if_row(out + static_cast<size_t>(static_cast<unsigned>(ix[j])) * kDQK,
-                                               __uint_as_float(r[j]), ix[j]);
-#endif
+                            for (int j = 0; j < 32; ++j)
+                                red_add_f32_if_row(out + static_cast<size_t>(static_cast<unsigned>(ix[j])) * kDQK,
+                                                   __uint_as_float(r[j]), ix[j]);
                         }
                     }
                 }
