@@ -339,7 +339,7 @@ template <int kMul> struct TileIter {
     const int* used;
     int q, q_last, lo, hi, hi_next, pos, end;
     int stop;                     // behind the query's last tile with a slot in use (kMul 2: hi or hi - 1)
-    int n_next;                   // kMul 2: slots in use of query q + 1
+    int n_cur, n_next;            // kMul 2: slots in use of queries q and q + 1
     __device__ __forceinline__ TileIter(const KParams& p, const WorkRange& w)
         : pre(p.tile_pre), used(p.n_used), q(w.q), q_last(p.q0 + p.nq), pos(w.begin * kMul), end(w.end * kMul) {
         lo = __ldcg(pre + q) * kMul;
@@ -351,7 +351,8 @@ template <int kMul> struct TileIter {
     __device__ __forceinline__ void set_stop() {
         stop = hi;
         if constexpr (kMul > 1) {
-            stop = lo + (n_next + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul);
+            n_cur = n_next;
+            stop = lo + (n_cur + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul);
             n_next = __ldcg(used + min(q + 1, q_last - 1));
         }
     }
@@ -652,11 +653,13 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         int stat_q = range.q;               // the query stat_next belongs to
         float stat_next = load_stat(stat_q);
         int gt = 0;
+        int n_used = 0;
         QMeta qm{};
         bool new_query = true;
         for (TileIter<1> it(p, range); it.more(); new_query = it.advance(), ++gt) {
             const int qg = it.q, tile = it.tile();
             if (new_query) {
+                n_used = __ldcg(p.n_used + qg);
                 qm = load_qmeta(p, qg);
                 if (stat_q != qg) stat_next = load_stat(qg);       // queries without a valid slot lay in between
                 asm volatile("bar.sync 1, 256;" ::: "memory");      // every softmax warp is done with the previous query
@@ -672,7 +675,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 const int b = gt & 1;
                 mbar_wait(bar_tfull + 8 * b, (gt >> 1) & 1, wc, kErrRecompute + 18, kPollSleepNs);
                 tc_fence_after_sync();
-                {
+                // this CTA's 128 keys are all behind the last slot in use: neither the dKV nor the dQ kernel reads them
+                if (tile * kTileKeys + static_cast<int>(rank) * 128 < n_used) {
                     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + b * C::kAccCols + g * 2 * NH;
                     // the 32 lanes hold consecutive keys: 32 x 16 bytes of consecutive addresses per store
                     const size_t off = static_cast<size_t>(p.scr0 + qg - p.q0) * p.topk_pad * HP + scratch_offset(key, g * NH, p.topk_pad);
@@ -1603,6 +1607,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (member == 0 && it.more()) fetch_idx(it.q, it.tile());
         for (uint32_t n = 0; it.more(); ++n) {      // n: tiles so far; unit 3 n + blk of the range belongs to group (n + blk) % 2
             const int tile = it.tile(), sq = p.scr0 + it.q - p.q0;
+            const int left = it.n_cur - tile * kTileKeys - 64 * e;      // slots in use from this warp's 64 keys on
             int* idx_s = idx_base + (n & 1) * 128;
             if (member == 0) {
                 idx_s[lane] = pf[0];
@@ -1630,6 +1635,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + us * 128 + 64 * e;
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
+                        if (left <= 32 * i) break;      // behind the last slot in use: a predicated-off reduction costs its issue
                         uint32_t r[32];
                         tmem_ld_32x32(taddr + 32 * i, r);
                         int ix[32];
