@@ -690,8 +690,8 @@ def run_ours(args):
             "config": _config(wname, w, args.s_q,
                               ("query+reduce_scatter" if query_sharded else "batch") if world > 1 else "none"),
             "stages": stages, "schedule": dict(zip(("chunks", "dkv_pairs"), op.get_schedule()),
-                                                note="chunks -1: chosen from the head count (64 heads: two overlapped parts; "
-                                                     "128: the kernels one after the other)"),
+                                                note="chunks -1: chosen by the library (one after the other above 64 heads "
+                                                     "or one 256-key tile)"),
             "clocks": clocks, "gpu_launches": n_launch, "kernels": kernels,
             "device_status": "ok" if not bad_status else "TIMEOUT in: " + "; ".join(bad_status),
         }
