@@ -766,7 +766,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // depends on timing, o and lse repeat bit for bit.
 // What bounds it: per tile and CTA 17 slots x 4 UMMAs x 64 cycles = 4352 cycles of tensor pipe; 275 KB of gathered rows
 // written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Measured (4096 queries x 128 heads x
-// top-k 2048): 8100 cycles a tile, 2.25 ms at the 1.65 GHz the power cap leaves, against 3.27 ms for two logit passes and
+// top-k 2048): 7800 cycles a tile, 2.24 ms at the 1.65 GHz the power cap leaves, against 3.27 ms for two logit passes and
 // an E.V pass; without the gathers 7000 cycles, without the softmax 6300, without both 6100.  The ring's depth does not
 // matter (five, six or seven slots: 2.32 / 2.32 / 2.31 ms).  Row gathers by TMA (tile::gather4 from eight warps) in place
 // of cp.async: 3.0 ms; two producer groups on alternate slots: 2.36 ms; one arrival per producer warp: 2.34 ms.
@@ -1412,15 +1412,15 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffMisc);
     const uint32_t bar_tfull = smem_u32(bars);                        // [2] tile stage landed (even CTA: in both CTAs)
     const uint32_t bar_tempty = bar_tfull + 8 * kTileStages;          // [2] the tile's UMMAs finished
-    const uint32_t bar_res = bar_tempty + 8 * kTileStages;            // 1  resident chunks landed (even CTA: in both CTAs)
-    const uint32_t bar_resfree = bar_res + 8;                         // 1  all UMMAs of the query finished
-    const uint32_t bar_ufull = bar_resfree + 8;                       // [kUnits] accumulator unit complete
+    const uint32_t bar_res = bar_tempty + 8 * kTileStages;            // [2] resident chunks of block 0 / of blocks 1 and 2 landed (even CTA: in both CTAs)
+    const uint32_t bar_resfree = bar_res + 16;                        // [2] the query's last UMMAs on them finished
+    const uint32_t bar_ufull = bar_resfree + 16;                      // [kUnits] accumulator unit complete
     const uint32_t bar_uempty = bar_ufull + 8 * kUnits;               // [kUnits] (even CTA) both CTAs have drained the unit
     const uint32_t bar_drain = bar_uempty + 8 * kUnits;               // 1  used only while winding down after an abort
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffMisc + 8 * (2 * kTileStages + 3 + 2 * kUnits));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffMisc + 8 * (2 * kTileStages + 5 + 2 * kUnits));
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 2);
-    static_assert(8 * (2 * kTileStages + 3 + 2 * kUnits) + 8 + sizeof(WorkRange) <= 256, "barrier area");
+    static_assert(8 * (2 * kTileStages + 5 + 2 * kUnits) + 8 + sizeof(WorkRange) <= 256, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
@@ -1429,8 +1429,10 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             mbar_init(bar_tfull + 8 * i, rank == 0 ? 2 : 1);   // own expect_tx arrival (+ the odd CTA's relayed one)
             mbar_init(bar_tempty + 8 * i, 1);
         }
-        mbar_init(bar_res, rank == 0 ? 2 : 1);
-        mbar_init(bar_resfree, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_res + 8 * i, rank == 0 ? 2 : 1);
+            mbar_init(bar_resfree + 8 * i, 1);
+        }
         mbar_init(bar_drain, 1);
         for (int i = 0; i < kUnits; ++i) {
             mbar_init(bar_ufull + 8 * i, 1);
@@ -1469,23 +1471,29 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int s = 0;
             uint32_t ph = 1, k = 0;        // ph: parity that means "stage free" in the current pass over the ring
             bool new_query = true;
-            for (Iter it(p, range); it.more(); new_query = it.advance()) {
-                if (new_query) {
-                    // the resident operands are replaced once the previous query's UMMAs are done; the drain warps
-                    // meanwhile still work through the accumulator ring, so the reductions do not pause
-                    if (k) mbar_wait(bar_resfree, (k - 1) & 1, wc, kErrDkv + 6, kPollSleepNs);
-                    ++k;
-                    mbar_arrive_expect_tx(bar_res, 9 * C::kChunk);
-                    const int row0 = it.q * p.h_q;
-                    for (int j = 0; j < 4; ++j) {          // slots 0..3: chunks {2r, 2r+1} of block 0 and block 1
-                        const int chunk = (j >> 1) * 4 + 2 * static_cast<int>(rank) + (j & 1);
-                        tma_load_2d_hint(s_base + C::kOffQ + j * C::kChunk, &tm_q, 64 * chunk, row0, bar_res, pol_stream);
-                        tma_load_2d_hint(s_base + C::kOffDO + j * C::kChunk, &tm_do, 64 * chunk, row0, bar_res, pol_stream);
+            // The resident operands are replaced in two parts, each as soon as the previous query's last UMMAs on it are done
+            // and behind the new query's first S / dS tile; the drain warps meanwhile still work through the accumulator ring.
+            // (All nine chunks at once, in front of the tile: 265 against 225 us for 1531 queries of at most three key tiles, 6.54 against
+            // 6.37 M cycles for 4096 queries of 16 tiles, 128 heads.)
+            auto load_resident = [&](int q) {
+                const int row0 = q * p.h_q;
+                for (int i = 0; i < 2; ++i) {              // slots 0 .. 3: chunks {2r, 2r+1} of block 0, of block 1
+                    if (k) mbar_wait(bar_resfree + 8 * i, (k - 1) & 1, wc, kErrDkv + 6 + i, kPollSleepNs);
+                    mbar_arrive_expect_tx(bar_res + 8 * i, (4 + i) * C::kChunk);
+                    for (int j = 2 * i; j < 2 * i + 2; ++j) {
+                        const int chunk = i * 4 + 2 * static_cast<int>(rank) + (j & 1);
+                        tma_load_2d_hint(s_base + C::kOffQ + j * C::kChunk, &tm_q, 64 * chunk, row0, bar_res + 8 * i, pol_stream);
+                        tma_load_2d_hint(s_base + C::kOffDO + j * C::kChunk, &tm_do, 64 * chunk, row0, bar_res + 8 * i, pol_stream);
                     }
-                    tma_load_2d_hint(s_base + C::kOffQ + 4 * C::kChunk, &tm_q, 64 * 8, row0, bar_res, pol_stream);
+                    if (i) tma_load_2d_hint(s_base + C::kOffQ + 4 * C::kChunk, &tm_q, 64 * 8, row0, bar_res + 8 * i, pol_stream);
                 }
-                if (!waited) {
+                ++k;
+            };
+            for (Iter it(p, range); it.more(); new_query = it.advance()) {
+                if (!waited) {                 // the first query's Q and dO do not wait for the kernel before this one
                     waited = true;
+                    load_resident(it.q);
+                    new_query = false;
                     pdl_wait();
                     pdl_trigger();
                 }
@@ -1497,6 +1505,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const int sq = p.scr0 + it.q - p.q0;
                 tma_load_4d_hint(dst, &tm_s, 0, kb, 0, sq, bar_tfull + 8 * s, pol_stream);
                 tma_load_4d_hint(dst + C::kHalfMat, &tm_ds, 0, kb, 0, sq, bar_tfull + 8 * s, pol_stream);
+                if (new_query) load_resident(it.q);
                 if (++s == kTileStages) {
                     s = 0;
                     ph ^= 1;
@@ -1517,13 +1526,15 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 uint32_t ph = 0, k = 0;
                 bool new_query = true;
                 for (Iter it(p, range); it.more(); new_query = it.advance()) {
-                    if (new_query) {
-                        mbar_wait(bar_res, k & 1, wc, kErrDkv + 10);
-                        mbar_arrive_cluster_relaxed(map_to_cta(bar_res, 0));
-                        ++k;
-                    }
                     mbar_spin(bar_tfull + 8 * s, ph, wc, kErrDkv + 11);
                     mbar_arrive_cluster_relaxed(map_to_cta(bar_tfull + 8 * s, 0));
+                    if (new_query) {
+                        for (int i = 0; i < 2; ++i) {
+                            mbar_wait(bar_res + 8 * i, k & 1, wc, kErrDkv + 10);
+                            mbar_arrive_cluster_relaxed(map_to_cta(bar_res + 8 * i, 0));
+                        }
+                        ++k;
+                    }
                     if (++s == kTileStages) {
                         s = 0;
                         ph ^= 1;
@@ -1536,13 +1547,14 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 uint32_t ph = 0, k = 0, unit = 0;
                 bool new_query = true;
                 for (Iter it(p, range); it.more();) {
-                    if (new_query) mbar_wait(bar_res, k++ & 1, wc, kErrDkv + 2);
+                    k += new_query;
                     const bool last = it.last_of_query();
                     mbar_wait(bar_tfull + 8 * s, ph, wc, kErrDkv + 4);
                     const uint32_t st_s = s_base + C::kOffStage + s * C::kStage;
                     const uint32_t st_ds = st_s + C::kHalfMat;
                     for (int blk = 0; blk < 3; ++blk, ++unit) {
                         const int us = unit % kUnits;
+                        if (new_query && blk < 2) mbar_wait(bar_res + 8 * blk, (k - 1) & 1, wc, kErrDkv + 2);
                         mbar_wait(bar_uempty + 8 * us, ((unit / kUnits) & 1) ^ 1, wc, kErrDkv + 3);
                         tc_fence_after_sync();
                         const uint32_t d = tmem + us * 128;
@@ -1562,9 +1574,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                          make_smem_desc(st_ds + ks * 2048, 1024, 128, kSwizzleNone), idesc,
                                          blk < 2 || ks != 0);
                         umma_commit_2cta_mask(bar_ufull + 8 * us, 3);
+                        if (last && blk != 1) umma_commit_2cta_mask(bar_resfree + 8 * (blk >> 1), 3);
                     }
                     umma_commit_2cta_mask(bar_tempty + 8 * s, 3);
-                    if (last) umma_commit_2cta_mask(bar_resfree, 3);
                     if (++s == kTileStages) {
                         s = 0;
                         ph ^= 1;
