@@ -1370,7 +1370,7 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
 //   from the slot pair (3, 4) in both CTAs: slot 4 holds chunk 8 in both, so both compute the same 64 real rows in
 //   lanes 64-127 (lanes 0-63 repeat chunk 3's rows and are dropped); CTA (tile & 1) drains them, which keeps the
 //   reductions of the two CTAs equal over two tiles.
-//   warp 0      producer: resident chunks per query; per 128-key tile this CTA's 64 keys of S and dS, two stages
+//   warp 0      producer: resident chunks per query; per 128-key tile this CTA's 64 keys of S and dS, two or four stages
 //   warp 1      even CTA: UMMA issuer for the pair; odd CTA: relays "my half landed" to the even CTA's barriers
 //   warps 2-17  drain, two groups of eight on alternate accumulator units (ring of four 128-column units per CTA):
 //               lane = d row, one predicated fp32 reduction per key = 128 contiguous bytes of dKV
@@ -1379,11 +1379,13 @@ namespace dp {
 constexpr int kThreads = 576;
 constexpr int kTileKeys = 128;
 constexpr int kUnits = 4;
-constexpr int kTileStages = 2;
 template <int HP> struct Cfg {
     static constexpr int kChunk = HP * 128;                 // resident chunk [HP heads x 64 d] bytes
     static constexpr int kHalfMat = HP * 128;               // S (or dS) of 64 keys: [HP/8][64 keys][8 heads]
     static constexpr int kStage = 2 * kHalfMat;             // S then dS
+    // What the resident chunks leave; 64 heads, 4096 queries of 16 tiles: 6.56 M cycles with two or three, 6.45 with four, 6.46
+    // with six or eight.  (A second set of resident chunks beside four stages: 6.50.)
+    static constexpr int kTileStages = HP == 64 ? 4 : 2;
     static constexpr int kOffQ = 0;                         // 5 slots
     static constexpr int kOffDO = 5 * kChunk;               // 4 slots
     static constexpr int kOffStage = 9 * kChunk;
@@ -1402,6 +1404,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     using namespace dp;
     using C = Cfg<HP>;
+    constexpr int kTileStages = C::kTileStages;
     const uint32_t rank = cluster_ctarank();
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform to the compiler
     const int lane = threadIdx.x & 31;
@@ -1410,8 +1413,8 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t s_base = smem_u32(smem);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffMisc);
-    const uint32_t bar_tfull = smem_u32(bars);                        // [2] tile stage landed (even CTA: in both CTAs)
-    const uint32_t bar_tempty = bar_tfull + 8 * kTileStages;          // [2] the tile's UMMAs finished
+    const uint32_t bar_tfull = smem_u32(bars);                        // [kTileStages] tile stage landed (even CTA: in both CTAs)
+    const uint32_t bar_tempty = bar_tfull + 8 * kTileStages;          // [kTileStages] the tile's UMMAs finished
     const uint32_t bar_res = bar_tempty + 8 * kTileStages;            // [2] resident chunks of block 0 / of blocks 1 and 2 landed (even CTA: in both CTAs)
     const uint32_t bar_resfree = bar_res + 16;                        // [2] the query's last UMMAs on them finished
     const uint32_t bar_ufull = bar_resfree + 16;                      // [kUnits] accumulator unit complete
