@@ -72,3 +72,26 @@ def test_query_table_on_the_gpu_equals_the_host_one(n_seq):
         want = op.query_meta_for(q0, lens, kv0, kv_lens, "cpu", q_start, 64, length)
         got = op.query_meta_for(q0, lens, kv0, kv_lens, DEV, q_start, 64, None if length is None else length.to(DEV))
         assert torch.equal(got.cpu(), want)
+
+
+# the last slot in use on, before and behind the edges of what is worked on as one: 32 keys (a drain warp's registers), 64 (a dQ
+# tile), 128 (a dKV tile, one CTA's half of a work tile), 256 (a work tile)
+EDGES = [1, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 160, 161, 255, 256, 257, 384, 385, 500]
+
+
+@pytest.mark.parametrize("h_q", [16, 64, 128])
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_last_slot_at_the_edges_of_the_key_groups(h_q, deterministic):
+    """What lies behind a query's last slot is neither computed nor added: a call with every slot in use leaves the scratch full
+    of other values first."""
+    from test_operator_b200 import op
+    s = make_sequence(Workload("edges", 1, 4 * len(EDGES), 900, h_q, 500, "uniform"), device=DEV, seed=53)
+    full = [s[k] for k in ("q", "kv", "dO", "lse", "O", "indices")]
+    op.mla_bwd(*full, q_start_index_s=None, deterministic=deterministic, check_device_status=True)
+    s["indices"] = s["indices"].clone()
+    for r in range(s["indices"].shape[0]):
+        s["indices"][r, EDGES[r % len(EDGES)]:] = -1
+    args = [s[k] for k in ("q", "kv", "dO", "lse", "O", "indices")]
+    ref = sparse_mla_bwd_ref(*args, q_start_index_s=None, chunk_s=16)
+    dq, dkv = op.mla_bwd(*args, q_start_index_s=None, deterministic=deterministic, check_device_status=True)
+    assert_backward_close(dq, dkv, *ref, "edges")
