@@ -796,6 +796,14 @@ constexpr int kPartFloats = kDV;           // a partial result: [HP heads][512] 
 static_assert(kSmemBytes <= 232448, "shared memory of one SM");
 }  // namespace ff
 
+// lse of a row that has a valid slot (the prep kernel writes the rows of a query that has none) from the reference of its
+// exponentials and their sum; o is O / sum.  What is not a number stays none, as in plain torch: a NaN logit makes the sum and
+// with it o and lse NaN; a logit of +inf gives o NaN, lse +inf; logits that are all -inf (sum 0) give o NaN, lse -inf.
+__device__ __forceinline__ float row_lse(float ref, float sum) {
+    const float inf = __int_as_float(0x7f800000);
+    return ref == inf ? inf : ref + __log2f(sum);
+}
+
 template <int HP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ff::kThreads, 1)
 smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
@@ -1224,14 +1232,12 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 // partial results: slot 2 c for a range that starts inside the query, 2 c + 1 for one that starts at or before it
                 const size_t prow = static_cast<size_t>((blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0)) * HP + head;
                 if (real && part == 0) {
-                    if (whole)
-                        p.lse_out[orow] = (total > 0.f ? ref + __log2f(total) : __int_as_float(0x7f800000)) * p.lse_out_mult;
-                    else
-                        p.part_ml[prow] = make_float2(ref, total);
+                    if (whole) p.lse_out[orow] = row_lse(ref, total) * p.lse_out_mult;
+                    else p.part_ml[prow] = make_float2(ref, total);
                 }
                 pending = true;
                 pend_whole = whole;
-                pend_inv = total > 0.f ? 1.f / total : 0.f;
+                pend_inv = 1.f / total;
                 pend_row = whole ? orow : prow;
             }
             new_query = next_query;
@@ -1295,7 +1301,7 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
         float weight[kHeads];
 #pragma unroll
         for (int h = 0; h < kHeads; ++h) {
-            const float m = ml[h].y > 0.f ? ml[h].x : ninf;     // no valid slot in this part
+            const float m = ml[h].x;                             // -inf: no valid slot in this part, or none above -inf
             float top = m;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
@@ -1315,16 +1321,17 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
             float wt[kFly][kHeads];
 #pragma unroll
             for (int u = 0; u < kFly; ++u) {
-                const int src = todo ? __ffs(todo) - 1 : 0;
+                const bool live = todo != 0;
+                const int src = live ? __ffs(todo) - 1 : 0;
                 const float4* o = reinterpret_cast<const float4*>(
                     reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), src))) + lane;
 #pragma unroll
                 for (int h = 0; h < kHeads; ++h) {
                     wt[u][h] = __shfl_sync(0xffffffffu, weight[h], src);
-                    if (!todo) wt[u][h] = 0.f;
+                    // (a part of weight 0 counts too: its O may hold a NaN)
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        v[u][h][i] = wt[u][h] > 0.f ? __ldcg(o + h * (kDV / 4) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[u][h][i] = live ? __ldcg(o + h * (kDV / 4) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 todo &= todo - 1;
             }
@@ -1345,10 +1352,10 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
 #pragma unroll
     for (int h = 0; h < kHeads; ++h) {
         if (head0 + h >= p.h_q) break;
-        const float inv = sum[h] > 0.f ? 1.f / sum[h] : 0.f;
+        const float inv = 1.f / sum[h];
         const size_t orow = static_cast<size_t>(q) * p.h_q + head0 + h;
         if (lane == 0 && half == 0)
-            p.lse_out[orow] = (sum[h] > 0.f ? ref[h] + __log2f(sum[h]) : __int_as_float(0x7f800000)) * p.lse_out_mult;
+            p.lse_out[orow] = row_lse(ref[h], sum[h]) * p.lse_out_mult;
         uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV + half * (kDV / 2)) + lane;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
