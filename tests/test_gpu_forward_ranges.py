@@ -68,3 +68,25 @@ def test_forward_with_a_workspace_too_small_to_spread_queries():
     o, lse = op.mla_fwd(*args, q_start_index_s=None, workspace_budget=4096, check_device_status=True)
     assert (lse - lse_ref * LOG2E).abs().max().item() <= 2e-4
     assert (o.float() - o_ref.float()).abs().max().item() <= 2 ** -6 * o_ref.float().abs().max().item()
+
+
+@pytest.mark.parametrize("h_q", [64, 128])
+def test_the_heaviest_slot_enters_unrounded(h_q):
+    """All rows of V are equal, so o / V is the sum of the weights.  The heaviest slot of the first tile and a heavier one (by 2^1.2
+    to 2^6.6) in the third enter as exactly 1 of their tile's maximum and are only scaled in fp32 afterwards; the other 698
+    slots weigh 2^-30 each.  So the sum is 1 to a few 2^-24, far from half a bf16 step, and o must be V bit for bit."""
+    from test_operator_b200 import op
+    s_q, topk, s_kv = 90, 700, 1024
+    g = torch.Generator(device=DEV).manual_seed(64)
+    kv = torch.zeros(s_kv, 576, device=DEV)
+    kv[:, :512] = torch.randn(512, generator=g, device=DEV)
+    kv[:, 512] = -500.0                                                     # times log2 e / 24 in the exponent
+    kv[:129, 512] = torch.arange(129, device=DEV).float()
+    kv = kv.bfloat16()
+    q = torch.zeros(s_q, h_q, 576, dtype=torch.bfloat16, device=DEV)
+    q[:, :, 512] = 1.0
+    idx = torch.arange(200, 200 + topk, device=DEV, dtype=torch.int32).repeat(s_q, 1)
+    idx[:, 5] = 0
+    idx[:, 600] = torch.arange(s_q, device=DEV, dtype=torch.int32) + 20
+    o, _ = op.mla_fwd(q, kv, idx, q_start_index_s=None, check_device_status=True)
+    assert torch.equal(o.view(torch.int16), kv[0, :512].expand_as(o).contiguous().view(torch.int16))
