@@ -22,7 +22,6 @@ namespace {
 using smla::KParams;
 
 constexpr size_t kAlign = 256;
-constexpr int kTicketWord = 16;     // word of a workspace's first 256 bytes that the prep kernel's blocks count on
 constexpr size_t kDefaultBudget = size_t(6) << 30;  // scratch budget when the caller gives none
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -172,7 +171,7 @@ struct Plan {
     int h_pad;       // heads padded to 64 or 128
     int topk_pad;    // top-k padded to a multiple of 256
     int q_chunk;     // queries per pass
-    size_t err_off, delta_off, used_off, pre_off, s_off, ds_off, total;
+    size_t err_off, delta_off, used_off, s_off, ds_off, total;
 };
 
 bool check_params(const smla_bwd_params* p) {
@@ -192,10 +191,9 @@ bool make_plan(const smla_bwd_params* p, size_t budget, Plan* pl) {
     const size_t per_q = size_t(pl->topk_pad) * pl->h_pad * 2 /*bf16*/ * 2 /*S and dS*/;
     pl->err_off = 0;
     pl->delta_off = kAlign;
-    // Delta, slots in use per query, prefix sum of the queries' tiles
+    // Delta, slots in use per query
     pl->used_off = align_up(pl->delta_off + size_t(p->s_q) * p->h_q * 4, 16);
-    pl->pre_off = pl->used_off + size_t(p->s_q) * 4;
-    const size_t fixed = align_up(pl->pre_off + (size_t(p->s_q) + 1) * 4, kAlign);
+    const size_t fixed = align_up(pl->used_off + size_t(p->s_q) * 4, kAlign);
     if (budget == 0) budget = kDefaultBudget;
     size_t qc = budget > fixed ? (budget - fixed) / per_q : 0;
     if (qc < 1) qc = 1;
@@ -351,7 +349,6 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     kp.lse = p->lse;
     kp.delta = delta;
     kp.n_used = reinterpret_cast<const int*>(ws + pl.used_off);
-    kp.tile_pre = reinterpret_cast<const int*>(ws + pl.pre_off);
     kp.s_scr = s_scr;
     kp.ds_scr = ds_scr;
     kp.dKV = p->dKV;
@@ -383,7 +380,6 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
         if (size_t(grid) < zero_blocks) grid = std::max(grid, int(zero_blocks < 8 * 148 ? zero_blocks : 8 * 148));
         launch(smla_prep_kernel, grid, kPrepThreads, 0, st, true, 1, reinterpret_cast<const uint4*>(p->O),
                reinterpret_cast<const uint4*>(p->dO), delta, reinterpret_cast<int*>(ws + pl.used_off),
-               reinterpret_cast<int*>(ws + pl.pre_off), reinterpret_cast<int*>(ws + pl.err_off) + kTicketWord,
                reinterpret_cast<uint4*>(p->dKV), zero_n, head_parts, kp);
     } else if (stages & SMLA_STAGE_ZERO) {
         if (cudaMemsetAsync(p->dKV, 0, size_t(p->s_kv) * kDQK * sizeof(float), st) != cudaSuccess) return SMLA_ERR_LAUNCH;
@@ -469,12 +465,12 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---- forward ---------------------------------------------------------------------------------------------
-// Workspace: error word | slots in use per query | prefix sum of the queries' tiles | partial results of the queries whose
+// Workspace: error word | slots in use per query | where each cluster's range begins | partial results of the queries whose
 // tiles are spread over several clusters, two per cluster.
 constexpr int kMaxFwdClusters = 80;
 struct FwdPlan {
     int h_pad, topk_pad, clusters;      // clusters: at most this many have room for their partial results
-    size_t err_off, used_off, pre_off, rq_off, ml_off, o_off, total;
+    size_t err_off, used_off, rq_off, ml_off, o_off, total;
 };
 
 bool check_fwd_params(const smla_fwd_params* p) {
@@ -493,9 +489,8 @@ bool make_fwd_plan(const smla_fwd_params* p, size_t bytes, FwdPlan* pl) {
     pl->topk_pad = (p->topk + smla::kWorkTileKeys - 1) / smla::kWorkTileKeys * smla::kWorkTileKeys;
     pl->err_off = 0;
     pl->used_off = kAlign;
-    pl->pre_off = pl->used_off + size_t(p->s_q) * 4;
-    pl->rq_off = align_up(pl->pre_off + (size_t(p->s_q) + 1) * 4, 16);
-    pl->ml_off = align_up(pl->rq_off + kMaxFwdClusters * 4, kAlign);
+    pl->rq_off = align_up(pl->used_off + size_t(p->s_q) * 4, 16);
+    pl->ml_off = align_up(pl->rq_off + kMaxFwdClusters * sizeof(int4), kAlign);
     const size_t per_cluster = 2 * size_t(pl->h_pad) * (SMLA_D_V + 2) * 4;
     const long long tiles = static_cast<long long>(p->s_q) * (pl->topk_pad / smla::kWorkTileKeys);
     long long c = std::min<long long>(kMaxFwdClusters, tiles);
@@ -524,8 +519,7 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     kp.kv = reinterpret_cast<const __nv_bfloat16*>(p->kv);
     kp.indices = p->indices;
     kp.n_used = reinterpret_cast<const int*>(ws + pl.used_off);
-    kp.tile_pre = reinterpret_cast<const int*>(ws + pl.pre_off);
-    kp.range_q = reinterpret_cast<int*>(ws + pl.rq_off);
+    kp.range_q = reinterpret_cast<int4*>(ws + pl.rq_off);
     kp.part_ml = reinterpret_cast<float2*>(ws + pl.ml_off);
     kp.part_o = reinterpret_cast<float*>(ws + pl.o_off);
     kp.lse_out = p->lse;
@@ -546,8 +540,7 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     kp.q0 = 0;
     kp.nq = p->s_q;
     launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, static_cast<const uint4*>(nullptr), static_cast<const uint4*>(nullptr),
-           static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), reinterpret_cast<int*>(ws + pl.pre_off),
-           reinterpret_cast<int*>(ws + pl.err_off) + kTicketWord, static_cast<uint4*>(nullptr), size_t(0), 1, kp);
+           static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), static_cast<uint4*>(nullptr), size_t(0), 1, kp);
     const int pairs = resident_pairs(smla_fwd_kernel<HP>, ff::kThreads, ff::kSmemBytes);
     if (pairs <= 0) return SMLA_ERR_LAUNCH;
     const int clusters = std::max(1, std::min(pairs, pl.clusters));

@@ -39,7 +39,6 @@ struct KParams {
     const float* lse;         // [s_q, h_q]
     const float* delta;       // [s_q, h_q]
     const int* n_used;        // [s_q] slots up to and including the query's last valid one
-    const int* tile_pre;      // [s_q + 1] exclusive prefix sum of ceil(n_used / 256) over the queries
     __nv_bfloat16* s_scr;     // [q_chunk][HP/8 head blocks][topk_pad keys][8 heads], see scratch_offset
     __nv_bfloat16* ds_scr;    // likewise
     float* dKV;               // [s_kv, 576]
@@ -50,7 +49,7 @@ struct KParams {
     float lse_out_mult;       // 1 (base 2) or ln 2 (natural log)
     float* part_o;            // partial results of queries spread over several clusters: [slot][HP][512]
     float2* part_ml;          // [slot][HP] {reference of the exponentials (log2), sum}
-    int* range_q;             // [clusters] first query of each cluster's range
+    int4* range_q;            // [clusters] {first query of the cluster's range, position of that query's first tile, tiles of the launch}
     __nv_bfloat16* gout;      // [s_q, h_q, 512] o (forward only)
     int* g_err;
     int q0;                   // first query (global row) of this launch
@@ -152,7 +151,6 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 //   block b < s_q   Delta of query b's rows (backward), and n_used[b]: the slots up to the query's last valid one (early tokens of a
 //                   causal sequence use a fraction of their top-k, the rest are out-of-range values at the end)
 //   every block     its share of dKV cleared (where the caller wants it cleared)
-//   last block      prefix sum of the queries' 256-key tiles, from which the persistent kernels take their ranges
 // Bound by HBM: O, dO and the indices read once, dKV written once.
 // =============================================================================================
 constexpr int kWorkTileKeys = 256;      // granularity of the work ranges: what the recompute kernel does per accumulator
@@ -182,10 +180,8 @@ __device__ __forceinline__ int block_exclusive_sum(int v, int* warp_sums, int* t
 
 __global__ void __launch_bounds__(kPrepThreads)
 smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, float* __restrict__ delta,
-                 int* __restrict__ n_used, int* __restrict__ tile_pre, int* ticket, uint4* __restrict__ zero_dst,
-                 size_t zero_n, int head_parts, const KParams p) {
-    __shared__ int red[32];
-    __shared__ int is_last;
+                 int* __restrict__ n_used, uint4* __restrict__ zero_dst, size_t zero_n, int head_parts, const KParams p) {
+    __shared__ int red[kPrepThreads / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kWarps = kPrepThreads / 32;
     pdl_wait();                   // (nothing above touches memory another kernel of the stream may still use)
@@ -201,18 +197,11 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
         if (lane == 0) red[warp] = last;
     }
     __syncthreads();
-    // The block that takes the last ticket sees every query's count and sums up the tiles at the end.  The ticket is drawn
-    // here so that its round trip runs under the loads below.
-    if (threadIdx.x == 0) {
-        if (q < p.s_q && hp == 0) {
-            int m = red[0];
+    if (threadIdx.x == 0 && q < p.s_q && hp == 0) {
+        int m = red[0];
 #pragma unroll
-            for (int w = 1; w < kWarps; ++w) m = max(m, red[w]);
-            n_used[q] = m + 1;
-        }
-        __threadfence();
-        is_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
-        __threadfence();
+        for (int w = 1; w < kWarps; ++w) m = max(m, red[w]);
+        n_used[q] = m + 1;
     }
     if (q < p.s_q && O == nullptr) {             // forward: a query without a valid slot is in nobody's range
         int m = -1;
@@ -250,31 +239,6 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
         const size_t z0 = zero_n * blockIdx.x / gridDim.x, z1 = zero_n * (blockIdx.x + 1) / gridDim.x;
         for (size_t i = z0 + threadIdx.x; i < z1; i += kPrepThreads) zero_dst[i] = make_uint4(0, 0, 0, 0);
     }
-    __syncthreads();
-    if (!is_last) return;
-    constexpr int kPer = 8;       // consecutive queries per thread and round
-    int carry = 0;
-    for (int base = 0; base < p.s_q; base += kPrepThreads * kPer) {
-        const int i0 = base + threadIdx.x * kPer;
-        int n[kPer], sum = 0;
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            n[i] = i0 + i < p.s_q ? (__ldcg(n_used + i0 + i) + kWorkTileKeys - 1) / kWorkTileKeys : 0;
-            sum += n[i];
-        }
-        int total;
-        int at = carry + block_exclusive_sum(sum, red, &total);
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            if (i0 + i < p.s_q) tile_pre[i0 + i] = at;
-            at += n[i];
-        }
-        carry += total;
-    }
-    if (threadIdx.x == 0) {
-        tile_pre[p.s_q] = carry;
-        *ticket = 0;
-    }
 }
 
 // Per-query table for packed sequences (KParams::qmeta) from a table of sequences that travels in the kernel's parameters:
@@ -304,57 +268,57 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 // tiles over 74 clusters as whole queries would be 56 queries for some and 55 for the others), a few long queries
 // spread over the whole chip, and tiles without a valid slot do not exist.  kMul: tiles of 256 / kMul keys.
 struct WorkRange {
-    int begin, end, q;            // positions in tile_pre's numbering; the query `begin` lies in
+    int begin, end;               // positions among the launch's tiles
+    int q, lo;                    // the query `begin` lies in; position of its first tile
 };
-__device__ __forceinline__ int range_start(int t0, int t1, int cluster, int n_clusters) {
-    return t0 + static_cast<int>(static_cast<long long>(t1 - t0) * cluster / n_clusters);
+__device__ __forceinline__ int work_tiles(int n_used) { return (n_used + kWorkTileKeys - 1) / kWorkTileKeys; }
+__device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clusters) {
+    return static_cast<int>(static_cast<long long>(n_tiles) * cluster / n_clusters);
 }
-// One warp: which range is this cluster's.  32-way search over the prefix sums (two rounds up to 1024 queries).
-__device__ __forceinline__ WorkRange find_range(const KParams& p, int cluster, int n_clusters) {
-    const int lane = threadIdx.x & 31;
-    const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
-    WorkRange w;
-    w.begin = range_start(t0, t1, cluster, n_clusters);
-    w.end = range_start(t0, t1, cluster + 1, n_clusters);
-    int lo = p.q0, n = p.nq;      // the last query in [lo, lo + n) whose first tile is at or before `begin`
-    while (n > 1) {
-        const int step = (n + 31) >> 5;
-        const int at = lane * step;
-        const bool before = at < n && (at == 0 || __ldcg(p.tile_pre + lo + at) <= w.begin);
-        const int k = 31 - __clz(__ballot_sync(0xffffffffu, before));
-        lo += k * step;
-        n = min(step, n - k * step);
+// Which range is this cluster's; called by the whole block, which passes a barrier before it reads *out.  Every block adds up
+// the slot counts itself (a few per thread: 8192 queries are 32 KB out of L2, all in flight at once), so that the ranges need
+// no prefix sum made by a kernel before and no counter that would have to survive from launch to launch.
+// scratch: one word of shared memory per warp.  Returns, in the one thread that wrote *out, the launch's tiles; -1 in the others.
+template <int kThreads>
+__device__ __forceinline__ int find_range(const KParams& p, int cluster, int n_clusters, int* scratch, WorkRange* out) {
+    const int* used = p.n_used + p.q0;
+    const int per = (p.nq + kThreads - 1) / kThreads;          // consecutive queries of a thread
+    const int i0 = min(static_cast<int>(threadIdx.x) * per, p.nq), i1 = min(i0 + per, p.nq);
+    int sum = 0, total;
+#pragma unroll 8
+    for (int i = i0; i < i1; ++i) sum += work_tiles(__ldcg(used + i));
+    int lo = block_exclusive_sum(sum, scratch, &total);
+    const int begin = range_start(total, cluster, n_clusters);
+    if (total == 0 ? threadIdx.x != 0 : begin < lo || begin >= lo + sum) return -1;
+    int q = i0;
+    if (total > 0) {
+        for (int n; begin >= lo + (n = work_tiles(__ldcg(used + q))); ++q) lo += n;
     }
-    w.q = lo;
-    return w;
+    *out = WorkRange{begin, range_start(total, cluster + 1, n_clusters), p.q0 + q, lo};
+    return total;
 }
 // Broadcast, so that the compiler knows the bounds of the loops below to be the same in all lanes: it then keeps what the
 // UMMAs of an issuing thread need (descriptors, addresses) in uniform registers, where tcgen05.mma takes its operands from.
 // With a loop bound or a ring position it takes for lane-dependent it moves every operand over first.
 __device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
-    return WorkRange{__shfl_sync(0xffffffffu, w.begin, 0), __shfl_sync(0xffffffffu, w.end, 0), __shfl_sync(0xffffffffu, w.q, 0)};
+    return WorkRange{__shfl_sync(0xffffffffu, w.begin, 0), __shfl_sync(0xffffffffu, w.end, 0), __shfl_sync(0xffffffffu, w.q, 0),
+                     __shfl_sync(0xffffffffu, w.lo, 0)};
 }
 template <int kMul> struct TileIter {
-    const int* pre;
     const int* used;
-    int q, q_last, lo, hi, hi_next, pos, end;
+    int q, q_last, lo, hi, pos, end;
     int stop;                     // behind the query's last tile with a slot in use (kMul 2: hi or hi - 1)
-    int n_cur, n_next;            // kMul 2: slots in use of queries q and q + 1
+    int n_cur, n_next;            // slots in use of queries q and q + 1 (one query ahead: the load is done when it is needed)
     __device__ __forceinline__ TileIter(const KParams& p, const WorkRange& w)
-        : pre(p.tile_pre), used(p.n_used), q(w.q), q_last(p.q0 + p.nq), pos(w.begin * kMul), end(w.end * kMul) {
-        lo = __ldcg(pre + q) * kMul;
-        hi = __ldcg(pre + q + 1) * kMul;
-        hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;      // one query ahead: the load is done when it is needed
-        if constexpr (kMul > 1) n_next = __ldcg(used + q);
-        set_stop();
+        : used(p.n_used), q(w.q), q_last(p.q0 + p.nq), lo(w.lo * kMul), pos(w.begin * kMul), end(w.end * kMul) {
+        n_next = __ldcg(used + q);
+        open_query();
     }
-    __device__ __forceinline__ void set_stop() {
-        stop = hi;
-        if constexpr (kMul > 1) {
-            n_cur = n_next;
-            stop = lo + (n_cur + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul);
-            n_next = __ldcg(used + min(q + 1, q_last - 1));
-        }
+    __device__ __forceinline__ void open_query() {
+        n_cur = n_next;
+        hi = lo + work_tiles(n_cur) * kMul;
+        stop = kMul > 1 ? lo + (n_cur + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul) : hi;
+        n_next = __ldcg(used + min(q + 1, q_last - 1));
     }
     __device__ __forceinline__ bool more() const { return pos < end; }
     __device__ __forceinline__ int tile() const { return pos - lo; }
@@ -366,9 +330,7 @@ template <int kMul> struct TileIter {
         while (pos < end) {
             ++q;
             lo = hi;
-            hi = hi_next;
-            hi_next = __ldcg(pre + min(q + 2, q_last)) * kMul;
-            set_stop();
+            open_query();
             if (hi > lo) break;
         }
         return true;
@@ -476,12 +438,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
         tmem_relinquish_2cta();
     }
-    pdl_wait();                  // tile counts and Delta of the prep kernel; the scratch's previous readers are done
+    pdl_wait();                  // slot counts and Delta of the prep kernel; the scratch's previous readers are done
     pdl_trigger();
-    if (warp == 17) {
-        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
-        if (lane == 0) *range_s = w;
-    }
+    find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(lse_s), range_s);   // (lse_s: not in use yet)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
@@ -868,15 +827,10 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         tmem_relinquish_2cta();
     }
     if (warp == 17 && lane == 0) tma_prefetch_desc(&tm_q);
-    pdl_wait();                  // the prep kernel's tile counts
+    pdl_wait();                  // the prep kernel's slot counts
     pdl_trigger();
-    if (warp == 17) {
-        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
-        if (lane == 0) {
-            *range_s = w;
-            if (rank == 0) p.range_q[blockIdx.x >> 1] = w.q;
-        }
-    }
+    const int total = find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + kOffStat), range_s);
+    if (total >= 0 && rank == 0) p.range_q[blockIdx.x >> 1] = make_int4(range_s->q, range_s->lo, total, 0);
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
@@ -1275,13 +1229,19 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
     const int half = (threadIdx.x >> 5) & 1;
     if (head0 >= p.h_q) return;
     const bool by_query = p.nq < n_clusters;
-    const int q = by_query ? p.q0 + item : __ldcg(p.range_q + item + 1);
-    const int t0 = __ldcg(p.tile_pre + p.q0), t1 = __ldcg(p.tile_pre + p.q0 + p.nq);
-    const int q_begin = __ldcg(p.tile_pre + q), q_end = __ldcg(p.tile_pre + q + 1);
+    const int4 boundary = __ldcg(p.range_q + (by_query ? 0 : item + 1));
+    const int q = by_query ? p.q0 + item : boundary.x, n_tiles = boundary.z;
+    int q_begin = boundary.y;
+    if (by_query) {                              // (fewer queries than clusters: at most three of them per lane)
+        q_begin = 0;
+        for (int i = lane; i < item; i += 32) q_begin += work_tiles(__ldcg(p.n_used + p.q0 + i));
+        q_begin = __reduce_add_sync(0xffffffffu, q_begin);
+    }
+    const int q_end = q_begin + work_tiles(__ldcg(p.n_used + q));
     if (q_begin >= q_end) return;                // no valid slot: the prep kernel has written o and lse
     // the cluster whose range holds the query's first tile: the largest k with range_start(k) <= q_begin
-    const int first = static_cast<int>((static_cast<long long>(q_begin - t0 + 1) * n_clusters - 1) / (t1 - t0));
-    if (range_start(t0, t1, first + 1, n_clusters) >= q_end || (!by_query && first != item)) return;
+    const int first = static_cast<int>((static_cast<long long>(q_begin + 1) * n_clusters - 1) / n_tiles);
+    if (range_start(n_tiles, first + 1, n_clusters) >= q_end || (!by_query && first != item)) return;
     const float ninf = __int_as_float(0xff800000);
     float ref[kHeads], sum[kHeads], acc[kHeads][8];
 #pragma unroll
@@ -1293,8 +1253,8 @@ __global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams 
     }
     for (int k0 = first; k0 < n_clusters; k0 += 32) {          // 32 parts at a time
         const int k = k0 + lane;
-        const int begin = k < n_clusters ? range_start(t0, t1, k, n_clusters) : t1;
-        const bool part = k < n_clusters && begin < q_end && begin < range_start(t0, t1, k + 1, n_clusters);
+        const int begin = k < n_clusters ? range_start(n_tiles, k, n_clusters) : n_tiles;
+        const bool part = k < n_clusters && begin < q_end && begin < range_start(n_tiles, k + 1, n_clusters);
         const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head0;
         float2 ml[kHeads];
 #pragma unroll
@@ -1457,12 +1417,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_relinquish_2cta();
     }
     // Behind the recompute kernel's trigger (it triggers after it has waited for the prep kernel) everything but S and dS is in
-    // place already: tile counts, indices, Q, dO, a cleared dKV.  Then only the first S / dS load waits.
+    // place already: slot counts, indices, Q, dO, a cleared dKV.  Then only the first S / dS load waits.
     if (!p.early_start) pdl_wait();
-    if (warp == 0) {
-        const WorkRange w = find_range(p, blockIdx.x >> 1, gridDim.x >> 1);
-        if (lane == 0) *range_s = w;
-    }
+    find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + C::kOffIdx), range_s);    // (index buffers: not in use yet)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
