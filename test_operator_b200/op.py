@@ -550,15 +550,21 @@ def mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor, sm_scale: 
                             NO_CAUSAL if q_start_index_s is None else int(q_start_index_s), 1 if lse_is_base2 else 0,
                             query_meta.data_ptr() if query_meta is not None else None)
         if workspace is None:
+            # allocated per call: the allocator keeps it apart from other threads' calls and gives it to a captured graph's pool
             need = _fwd_workspace_bytes(s_q, ks[0], h_q, ids[-1], workspace_budget)
             _check(need > 0, "unsupported shapes for the sparse MLA forward")
-            workspace = Workspace(need, q.device) if workspace_budget else _cached_workspace(need, q.device)
+            scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
+            if check_device_status:
+                scratch[:256].zero_()
+            ptr = scratch.data_ptr()
+        else:
+            ptr, need = workspace.ptr, workspace.nbytes
         stream = _raw_stream(index)
-        st = lib.smla_fwd_run(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream)
+        st = lib.smla_fwd_run(ctypes.byref(params), ptr, need, stream)
         if st:
             _raise_status(lib, st, "smla_fwd_run")
         if check_device_status:
-            _raise_status(lib, lib.smla_bwd_status(workspace.ptr, stream), "smla_fwd device status")
+            _raise_status(lib, lib.smla_bwd_status(ptr, stream), "smla_fwd device status")
     return o, lse
 
 
@@ -599,7 +605,7 @@ def index_inverse(indices: torch.Tensor, s_kv: int, q_start_index_s: Optional[in
     _check(need > 0, "unsupported shape (s_kv and topk positive, s_q * topk below 2^31)")
     index = indices.get_device()
     with _on_device(index):
-        ws = _cached_buffer("inverse", need, indices.device)
+        ws = torch.empty(need, dtype=torch.uint8, device=indices.device)
         row_ptr = torch.empty(s_kv + 1, dtype=torch.int32, device=indices.device)
         entries = torch.empty(s_q * topk, dtype=torch.int32, device=indices.device)
         st = lib.smla_index_inverse(indices.data_ptr(), s_q, topk, s_kv,
