@@ -5,9 +5,11 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <map>
+#include <memory>
 #include <mutex>
 #include <optional>
 #include <tuple>
@@ -18,20 +20,32 @@ namespace {
 
 // Scratch kept per (device, stream) so that the six-argument call does not allocate gigabytes every time
 // (the reference allocates only its small delta buffer per call, mla_bwd/mla_bwd.cu:1022-1025).  Calls queued
-// on different streams get different scratch; a larger problem replaces the entry.
-std::mutex g_ws_mutex;
-std::map<std::pair<int, void*>, torch::Tensor> g_ws;
+// on different streams get different scratch; a larger problem replaces the buffer.  A call holds the scratch's mutex
+// until all its kernels are queued, so that threads on one stream do not mix theirs on one buffer.
+struct Scratch {
+    std::mutex mutex;
+    torch::Tensor buf;
 
-torch::Tensor workspace_for(size_t need, const torch::Device& dev, void* stream) {
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    const std::pair<int, void*> key(dev.index(), stream);
-    auto it = g_ws.find(key);
-    if (it != g_ws.end() && static_cast<size_t>(it->second.numel()) >= need) return it->second;
-    if (it != g_ws.end()) g_ws.erase(it);     // let the smaller one go first
-    torch::Tensor buf = torch::empty({static_cast<int64_t>(need)}, torch::TensorOptions().dtype(torch::kUInt8).device(dev));
-    buf.narrow(0, 0, 256).zero_();            // the device error word starts clear; the kernels only ever set it
-    g_ws[key] = buf;
-    return buf;
+    torch::Tensor& of_size(size_t need, const torch::Device& dev) {
+        if (!buf.defined() || static_cast<size_t>(buf.numel()) < need) {
+            buf = torch::Tensor();                    // let the smaller one go first
+            buf = torch::empty({static_cast<int64_t>(need)}, torch::TensorOptions().dtype(torch::kUInt8).device(dev));
+            buf.narrow(0, 0, 256).zero_();            // the device error word starts clear; the kernels only ever set it
+        }
+        return buf;
+    }
+};
+std::mutex g_scratch_mutex;
+std::map<std::pair<int, void*>, std::shared_ptr<Scratch>> g_scratch;
+
+// While the stream is being captured, new scratch: a graph goes on using what it has recorded after a larger call has
+// replaced the kept buffer, so that one comes from the graph's own pool.
+std::shared_ptr<Scratch> scratch_for(const torch::Device& dev, void* stream) {
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return std::make_shared<Scratch>();
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    std::shared_ptr<Scratch>& s = g_scratch[{dev.index(), stream}];
+    if (!s) s = std::make_shared<Scratch>();
+    return s;
 }
 
 void check_input(const torch::Tensor& t, const char* name, const torch::Tensor& q, c10::ScalarType dtype) {
@@ -91,8 +105,14 @@ std::tuple<torch::Tensor, torch::Tensor> mla_bwd(const torch::Tensor& q, const t
     const size_t need = smla_bwd_workspace_size(&p, 0);
     TORCH_CHECK(need > 0, "unsupported shapes for the sparse MLA backward");
     cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-    torch::Tensor ws = workspace_for(need, q.device(), stream);
-    const int st = smla_bwd_run(&p, ws.data_ptr(), static_cast<size_t>(ws.numel()), stream);
+    int st;
+    {
+        pybind11::gil_scoped_release no_gil;          // a thread that waits for the mutex must not hold up the one that has it
+        std::shared_ptr<Scratch> scratch = scratch_for(q.device(), stream);
+        std::lock_guard<std::mutex> lock(scratch->mutex);
+        const torch::Tensor& ws = scratch->of_size(need, q.device());
+        st = smla_bwd_run(&p, ws.data_ptr(), static_cast<size_t>(ws.numel()), stream);
+    }
     TORCH_CHECK(st == SMLA_OK, "smla_bwd_run: ", smla_status_string(st), " (status ", st, ")");
     return {dQ, dKV};
 }
@@ -103,18 +123,26 @@ void check_device_status(int64_t device) {
     cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     torch::Tensor ws;
     {
-        std::lock_guard<std::mutex> lock(g_ws_mutex);
-        auto it = g_ws.find({static_cast<int>(device), stream});
-        if (it == g_ws.end()) return;
-        ws = it->second;
+        pybind11::gil_scoped_release no_gil;
+        std::shared_ptr<Scratch> scratch;
+        {
+            std::lock_guard<std::mutex> lock(g_scratch_mutex);
+            auto it = g_scratch.find({static_cast<int>(device), stream});
+            if (it == g_scratch.end()) return;
+            scratch = it->second;
+        }
+        std::lock_guard<std::mutex> lock(scratch->mutex);
+        if (!scratch->buf.defined()) return;
+        ws = scratch->buf;
     }
     const int st = smla_bwd_status(ws.data_ptr(), stream);
     TORCH_CHECK(st == SMLA_OK, "sparse MLA backward: ", smla_status_string(st), " (device code ", smla_bwd_last_device_code(), ")");
 }
 
 void release_workspaces() {
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    g_ws.clear();
+    std::map<std::pair<int, void*>, std::shared_ptr<Scratch>> gone;        // freed behind the lock
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    gone.swap(g_scratch);
 }
 
 }  // namespace

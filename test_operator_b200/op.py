@@ -220,47 +220,51 @@ class Workspace:
         self.ptr = self.buf.data_ptr()
 
 
-# Workspaces handed out when the caller passes none, one per (device, stream) so that calls queued on different
-# streams do not share scratch; kept (and grown when a larger problem comes) instead of allocating gigabytes per call.
-_ws_cache = {}
-_ws_cache_lock = threading.Lock()
+# Scratch of the backward calls that bring none, one set per (device, stream) so that calls queued on different streams do not
+# share any; kept (and grown when a larger problem comes) instead of allocating gigabytes per call.  A call holds the set's
+# lock until all its kernels are queued: two host threads that use one stream would otherwise mix theirs on one buffer.
+class _StreamScratch:
+    __slots__ = ("lock", "workspace", "staging")
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.workspace: Optional[Workspace] = None
+        self.staging: Optional[torch.Tensor] = None
+
+    def workspace_of(self, need: int, device) -> Workspace:
+        if self.workspace is None or self.workspace.nbytes < need:
+            self.workspace = None           # let the smaller one go before the larger one is allocated
+            self.workspace = Workspace(need, device)
+        return self.workspace
+
+    def staging_of(self, need: int, device) -> torch.Tensor:
+        if self.staging is None or self.staging.numel() < need:
+            self.staging = None
+            self.staging = torch.empty(need, dtype=torch.uint8, device=device)
+        return self.staging
 
 
-def _cached_workspace(need: int, device: torch.device) -> Workspace:
-    index = device.index if device.index is not None else torch.cuda.current_device()
+_scratch_cache = {}
+_scratch_cache_lock = threading.Lock()
+
+
+def _scratch_of_stream(index: int) -> _StreamScratch:
+    """The set of the current stream of device `index` (the current device).  While that stream is being captured, a new one:
+    the graph goes on using its buffers after a larger call has replaced the kept ones, so they come from the graph's own
+    pool, and what is only recorded (the clearing of a workspace's error word) must not pass for done in a later call."""
+    if torch.cuda.is_current_stream_capturing():
+        return _StreamScratch()
     key = (index, _raw_stream(index))
-    with _ws_cache_lock:
-        ws = _ws_cache.get(key)
-        if ws is None or ws.nbytes < need:
-            _ws_cache.pop(key, None)
-            ws = None                       # let the smaller one go before the larger one is allocated
-            ws = Workspace(need, device)
-            _ws_cache[key] = ws
-        return ws
-
-
-_buf_cache = {}
-
-
-def _cached_buffer(kind: str, need: int, device: torch.device) -> torch.Tensor:
-    """A byte buffer kept per (kind, device, stream) and grown on demand, like the workspaces."""
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (kind, index, _raw_stream(index))
-    with _ws_cache_lock:
-        buf = _buf_cache.get(key)
-        if buf is None or buf.numel() < need:
-            _buf_cache.pop(key, None)
-            buf = None
-            buf = torch.empty(need, dtype=torch.uint8, device=device)
-            _buf_cache[key] = buf
-        return buf
+    with _scratch_cache_lock:
+        if key not in _scratch_cache:
+            _scratch_cache[key] = _StreamScratch()
+        return _scratch_cache[key]
 
 
 def release_cached_workspaces() -> None:
     """Drop the workspaces and staging buffers kept for calls that pass none (they are re-created on demand)."""
-    with _ws_cache_lock:
-        _ws_cache.clear()
-        _buf_cache.clear()
+    with _scratch_cache_lock:
+        _scratch_cache.clear()
 
 
 def _make_params(q, kv2, dO, lse, O, idx2, dQ, dKV2, sm_scale, q_start_index_s, lse_is_base2,
@@ -392,26 +396,28 @@ def mla_bwd(
             _check_out(out_dkv, kv.numel(), torch.float32, q.device, "out_dkv")
             dKV = out_dkv
         params = _make_params(q, kv2, dO, lse, O, idx2, dQ, dKV, sm_scale, q_start_index_s, lse_is_base2, query_meta)
-        if workspace is None:
-            need = _bwd_workspace_bytes(params.s_q, params.s_kv, params.h_q, params.topk, workspace_budget)
-            _check(need > 0, "unsupported shapes for the sparse MLA backward")
-            # a budget asks for a particular size: do not serve it from a (possibly larger) cached one
-            workspace = Workspace(need, q.device) if workspace_budget else _cached_workspace(need, q.device)
-        stream = _raw_stream(index)
         stages = STAGE_ALL & ~STAGE_ZERO if accumulate else STAGE_ALL
-        if deterministic:
-            _check(query_meta is None, "deterministic=True handles one sequence per call (no query_meta)")
-            row_ptr, entries = index_inverse(idx2, kv2.shape[0], q_start_index_s)
-            per_q = lib.smla_bwd_staging_bytes_per_query(ctypes.byref(params))
-            n_stage = max(1, min(q.shape[0], max(int(staging_budget), per_q) // per_q))
-            staging = _cached_buffer("staging", n_stage * per_q, q.device)
-            det = _DetParams(row_ptr.data_ptr(), entries.data_ptr(), staging.data_ptr(), staging.numel())
-            st = lib.smla_bwd_run_deterministic(ctypes.byref(params), ctypes.byref(det), workspace.ptr, workspace.nbytes,
-                                                stream, stages)
-            for t in (row_ptr, entries):
-                t.record_stream(torch.cuda.current_stream())
-        else:
-            st = lib.smla_bwd_run_stages(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream, stages)
+        scratch = _scratch_of_stream(index) if workspace is None or deterministic else None
+        with scratch.lock if scratch else _NO_SWITCH:
+            if workspace is None:
+                need = _bwd_workspace_bytes(params.s_q, params.s_kv, params.h_q, params.topk, workspace_budget)
+                _check(need > 0, "unsupported shapes for the sparse MLA backward")
+                # a budget asks for a particular size: do not serve it from a (possibly larger) kept one
+                workspace = Workspace(need, q.device) if workspace_budget else scratch.workspace_of(need, q.device)
+            stream = _raw_stream(index)
+            if deterministic:
+                _check(query_meta is None, "deterministic=True handles one sequence per call (no query_meta)")
+                row_ptr, entries = index_inverse(idx2, kv2.shape[0], q_start_index_s)
+                per_q = lib.smla_bwd_staging_bytes_per_query(ctypes.byref(params))
+                n_stage = max(1, min(q.shape[0], max(int(staging_budget), per_q) // per_q))
+                staging = scratch.staging_of(n_stage * per_q, q.device)
+                det = _DetParams(row_ptr.data_ptr(), entries.data_ptr(), staging.data_ptr(), staging.numel())
+                st = lib.smla_bwd_run_deterministic(ctypes.byref(params), ctypes.byref(det), workspace.ptr, workspace.nbytes,
+                                                    stream, stages)
+                for t in (row_ptr, entries):
+                    t.record_stream(torch.cuda.current_stream())
+            else:
+                st = lib.smla_bwd_run_stages(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream, stages)
         _raise_status(lib, st, "smla_bwd_run")
         if check_device_status:
             _raise_status(lib, lib.smla_bwd_status(workspace.ptr, stream), "smla_bwd device status")

@@ -13,9 +13,14 @@ KEYS = ("q", "kv", "dO", "lse", "O", "indices")
 
 
 def _calls(op, s):
-    """Entry points that repeat bit for bit, by name."""
+    """Entry points that repeat bit for bit, by name (of the plain backward dQ does)."""
+    from tests.conftest import import_extension
     q, kv, idx = s["q"], s["kv"], s["indices"]
+    args = [s[k] for k in KEYS]
     return {
+        "bwd": lambda: op.mla_bwd(*args, q_start_index_s=None)[:1],
+        "repeatable": lambda: op.mla_bwd(*args, q_start_index_s=None, deterministic=True),
+        "module": lambda: import_extension().mla_bwd(*args, q_start_index_s=None)[:1],
         "fwd": lambda: op.mla_fwd(q, kv, idx, q_start_index_s=None),
         "inverse": lambda: op.index_inverse(idx, kv.shape[0]),
     }
@@ -32,7 +37,8 @@ def _same(a, b):
 SMALL, LARGE = (5, 700, 64, 300, 81), (300, 2000, 128, 600, 82)
 
 
-@pytest.mark.parametrize("names", [("fwd", "fwd"), ("inverse", "inverse"), ("fwd", "inverse")])
+@pytest.mark.parametrize("names", [("fwd", "fwd"), ("inverse", "inverse"), ("fwd", "inverse"), ("bwd", "bwd"), ("bwd", "fwd"),
+                                   ("repeatable", "repeatable"), ("repeatable", "bwd"), ("module", "module")])
 def test_two_threads_on_one_stream(names):
     from test_operator_b200 import op
     jobs = [_calls(op, _sequence(*shape))[n] for n, shape in zip(names, (SMALL, LARGE))]
@@ -56,7 +62,7 @@ def test_two_threads_on_one_stream(names):
     assert wrong == [0, 0]
 
 
-@pytest.mark.parametrize("name", ["fwd", "inverse"])
+@pytest.mark.parametrize("name", ["fwd", "inverse", "bwd", "repeatable", "module"])
 def test_a_graph_outlives_a_larger_call_on_its_stream(name):
     from test_operator_b200 import op
     small, large = (_calls(op, _sequence(*shape))[name] for shape in (SMALL, LARGE))
@@ -77,3 +83,24 @@ def test_a_graph_outlives_a_larger_call_on_its_stream(name):
             side.synchronize()
             assert _same(got, want)
         assert all(bool((t == 77).all()) for t in others)
+
+
+def test_a_backward_after_one_that_was_only_recorded():
+    """The first backward on a stream is recorded and not run; calls behind it on that stream get a workspace of their own."""
+    from test_operator_b200 import op
+    s = _sequence(*SMALL)
+    small = _calls(op, s)["bwd"]
+    want = small()
+    torch.cuda.synchronize()
+    op.release_cached_workspaces()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            recorded = small()
+        got = op.mla_bwd(*[s[k] for k in KEYS], q_start_index_s=None, check_device_status=True)
+        assert _same(got[:1], want)
+        graph.replay()
+        side.synchronize()
+        assert _same(recorded, want)
