@@ -494,11 +494,11 @@ bool make_fwd_plan(const smla_fwd_params* p, size_t bytes, FwdPlan* pl) {
     const size_t per_cluster = 2 * size_t(pl->h_pad) * (SMLA_D_V + 2) * 4;
     const long long tiles = static_cast<long long>(p->s_q) * (pl->topk_pad / smla::kWorkTileKeys);
     long long c = std::min<long long>(kMaxFwdClusters, tiles);
-    if (bytes) c = std::min<long long>(c, bytes > pl->ml_off + kAlign ? (bytes - pl->ml_off - kAlign) / per_cluster : 0);
+    if (bytes) c = std::min<long long>(c, bytes > pl->ml_off ? (bytes - pl->ml_off) / per_cluster : 0);
     if (c < 2) c = 0;                   // one cluster has every query whole
     pl->clusters = int(c);
-    pl->o_off = align_up(pl->ml_off + 2 * size_t(c) * pl->h_pad * 8, kAlign);
-    pl->total = pl->o_off + 2 * size_t(c) * pl->h_pad * SMLA_D_V * 4;
+    pl->o_off = pl->ml_off + 2 * size_t(c) * pl->h_pad * 8;      // (a multiple of kAlign: h_pad is 64 or 128)
+    pl->total = pl->ml_off + size_t(c) * per_cluster;            // what a size was asked for is enough for as many clusters again
     return true;
 }
 
