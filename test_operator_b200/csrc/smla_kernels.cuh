@@ -1061,6 +1061,9 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         bool pending = false, pend_whole = false;
         float pend_inv = 0.f;
         size_t pend_row = 0;
+        // o may start at any multiple of 16 bytes; where it is one of 32 it leaves in 32-byte stores (4096 queries x 128 heads x
+        // top-k 256: 488 us, 565 us in 16-byte stores)
+        const bool wide_o = (reinterpret_cast<uintptr_t>(p.gout) & 31) == 0;
         auto write_out = [&]() {
             pending = false;
             // lanes 0-63: columns [256 block, + 128), lanes 64-127: [256 block + 128, + 128)
@@ -1076,7 +1079,13 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
                         w[i] = pack_bf16x2(__uint_as_float(o[2 * i]) * pend_inv, __uint_as_float(o[2 * i + 1]) * pend_inv);
-                    st_global_v8(p.gout + at, w);
+                    if (wide_o) {
+                        st_global_v8(p.gout + at, w);
+                    } else {
+#pragma unroll
+                        for (int v = 0; v < 2; ++v)
+                            *reinterpret_cast<uint4*>(p.gout + at + 8 * v) = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+                    }
                 } else if (real) {
 #pragma unroll
                     for (int v = 0; v < 2; ++v) st_global_v8(p.part_o + at + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));

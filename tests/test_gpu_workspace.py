@@ -1,4 +1,5 @@
-"""What a workspace held before a call does not matter: not its scratch, and of its first 256 bytes only the error word does."""
+"""What a workspace held before a call does not matter: not its scratch, and of its first 256 bytes only the error word does.
+Tensors need no more than the alignment they are checked for."""
 import ctypes
 
 import pytest
@@ -42,3 +43,31 @@ def test_the_forward_gets_from_the_size_it_asked_for_what_it_gets_from_more(s_q,
     need = lib.smla_fwd_workspace_size(ctypes.byref(p), 0)
     (o1, lse1), (o2, lse2) = (op.mla_fwd(*args, q_start_index_s=None, workspace=op.Workspace(n, DEV)) for n in (need, 2 * need))
     assert torch.equal(o1.view(torch.int16), o2.view(torch.int16)) and torch.equal(lse1, lse2)
+
+
+@pytest.mark.parametrize("s_q,h_q", [(3, 128), (200, 64)])
+def test_tensors_at_the_smallest_alignment(s_q, h_q):
+    """Every tensor of the C ABI 16 bytes (bf16) or 4 bytes (indices, lse) off a larger power of two."""
+    from test_operator_b200 import op
+    lib = op.load_library()
+    s = make_sequence(Workload("align", 1, s_q, 900, h_q, 301, "uniform", invalid_frac=0.1), device=DEV, seed=72)
+
+    def off(t, elements):
+        room = torch.empty(t.numel() + 64, dtype=t.dtype, device=DEV)
+        view = room[elements:elements + t.numel()].view(t.shape)
+        assert view.data_ptr() % 512 == elements * t.element_size()
+        return view.copy_(t)
+
+    q, kv, dO, O, idx, lse = (off(s[k], n) for k, n in (("q", 8), ("kv", 8), ("dO", 8), ("O", 8), ("indices", 1), ("lse", 1)))
+    stream = torch.cuda.current_stream().cuda_stream
+    o_ref, lse_ref = op.mla_fwd(s["q"], s["kv"], s["indices"], q_start_index_s=None)
+    o, lse_out = off(torch.zeros_like(o_ref), 8), off(torch.zeros_like(lse_ref), 1)
+    ws = op.Workspace(64 << 20, DEV)
+    p = op._FwdParams(q.data_ptr(), kv.data_ptr(), idx.data_ptr(), o.data_ptr(), lse_out.data_ptr(), s_q, 900, h_q, 301, 0.0, op.NO_CAUSAL, 1, None)
+    assert lib.smla_fwd_run(ctypes.byref(p), ws.ptr, ws.nbytes, stream) == 0 and op.device_status(ws) == 0
+    assert torch.equal(o.view(torch.int16), o_ref.view(torch.int16)) and torch.equal(lse_out, lse_ref)
+    dq_ref, dkv_ref = op.mla_bwd(*[s[k] for k in KEYS], q_start_index_s=None)
+    dq, dkv = off(torch.zeros_like(dq_ref), 8), off(torch.zeros_like(dkv_ref), 4)
+    op.mla_bwd(q, kv, dO, lse, O, idx, q_start_index_s=None, out_dq=dq, out_dkv=dkv, check_device_status=True)
+    assert torch.equal(dq.view(torch.int16), dq_ref.view(torch.int16))
+    assert (dkv - dkv_ref).abs().max().item() <= 1e-5 * dkv_ref.abs().max().item()
