@@ -579,7 +579,7 @@ int static_workspace_ptr(void** out) {
 
 // ---- index inverse (CSR by kv row): layout and launches ------------------------------------------------------------
 inline size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
-struct InvLayout { size_t keys_a, keys_b, vals_a, vals_b, hist, totals, heads, total; };
+struct InvLayout { size_t keys_a, keys_b, vals_a, vals_b, hist, totals, heads, first, total; };
 inline InvLayout inv_layout(int64_t n, int32_t s_kv, const inv::Plan& pl) {
     InvLayout l;
     const size_t key_bytes = static_cast<size_t>(n) * (pl.key16 ? 2 : 4);
@@ -591,6 +591,7 @@ inline InvLayout inv_layout(int64_t n, int32_t s_kv, const inv::Plan& pl) {
     l.hist = off; off += up256(static_cast<size_t>(inv::kMaxRadix) * pl.n_blocks * 4);
     l.totals = off; off += up256(inv::kMaxRadix * 4);
     l.heads = off; off += up256((static_cast<size_t>(s_kv) + 1) * 4);
+    l.first = off; off += up256((static_cast<size_t>(s_kv) / inv::kRowTile + 1) * 4);
     l.total = off;
     return l;
 }
@@ -637,7 +638,13 @@ int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvL
                      : (last ? inv::scatter_kernel<KeyT, false, true, kItems> : inv::scatter_kernel<KeyT, false, false, kItems>),
                pl.n_blocks, inv::kThreads, kSmem, st, true, 1, kin, vin, src, kout, vout, hist, totals, n, shift, mask, pl.n_blocks, heads);
     }
-    launch(inv::row_ptr_kernel, src.s_kv / inv::kRowTile + 1, inv::kRowTile, 0, st, true, 1, heads, row_ptr, static_cast<int32_t>(n), src.s_kv);
+    const int row_blocks = src.s_kv / inv::kRowTile + 1;
+    int32_t* first = row_blocks > inv::kMaxLook ? reinterpret_cast<int32_t*>(ws + l.first) : nullptr;
+    if (first) {
+        launch(inv::row_min_kernel, row_blocks, inv::kRowTile, 0, st, true, 1, heads, first, src.s_kv);
+        launch(inv::suffix_min_kernel, 1, 1024, 0, st, true, 1, first, row_blocks);
+    }
+    launch(inv::row_ptr_kernel, row_blocks, inv::kRowTile, 0, st, true, 1, heads, first, row_ptr, static_cast<int32_t>(n), src.s_kv);
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 

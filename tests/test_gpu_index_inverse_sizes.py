@@ -36,3 +36,37 @@ def test_sizes(s_q, topk, s_kv, q_start, pattern):
     ref_ptr, ref_entries = index_inverse_ref(idx, s_kv, q_start)
     assert np.array_equal(row_ptr.cpu().numpy(), ref_ptr)
     assert np.array_equal(entries.cpu().numpy(), ref_entries)
+
+
+@pytest.mark.parametrize("s_kv", [65535, 65536, (1 << 20) - 1, 1 << 20, (1 << 20) + 5000])     # 64, 65, 1024, 1025, 1029 blocks of rows
+@pytest.mark.parametrize("used", ["first_rows", "last_row", "two_far_rows", "none"])
+def test_long_stretches_of_unused_rows(s_kv, used):
+    from test_operator_b200 import op
+    g = np.random.default_rng(s_kv)
+    idx = {"first_rows": lambda n: g.integers(-1, 700, n), "last_row": lambda n: np.full(n, s_kv - 1),
+           "two_far_rows": lambda n: np.where(g.integers(0, 2, n) == 0, 1023, s_kv * 2 // 3), "none": lambda n: np.full(n, -1)}[used]((9, 2000))
+    idx = idx.astype(np.int32)
+    row_ptr, entries = op.index_inverse(torch.from_numpy(idx).cuda(), s_kv)
+    ref_ptr, ref_entries = index_inverse_ref(idx, s_kv, None)
+    assert np.array_equal(row_ptr.cpu().numpy(), ref_ptr)
+    assert np.array_equal(entries.cpu().numpy(), ref_entries)
+
+
+def test_time_is_linear_in_the_rows():
+    """Slots on the first rows of a long kv pool only: four times the rows take about four times as long (42 and 78 us), not
+    sixteen times."""
+    from test_operator_b200 import op
+    idx = torch.randint(0, 1024, (16, 2048), dtype=torch.int32, device="cuda")
+
+    def best_us(s_kv):
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            op.index_inverse(idx, s_kv)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return min(times[1:])
+
+    assert best_us(1 << 22) < 8 * best_us(1 << 20)
