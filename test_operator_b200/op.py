@@ -797,8 +797,15 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
         s_in, s_out = torch.cuda.Stream(), torch.cuda.Stream()
         dev_in = [torch.empty(t.shape, dtype=t.dtype, device=dev) for t in host]
         kv_d = torch.empty(kv.shape, dtype=kv.dtype, device=dev)
+        if s_q:
+            _validate(dev_in[0], kv_d, *dev_in[1:])
         dkv_d = torch.empty(kv.shape, dtype=torch.float32, device=dev)
         dq_d = torch.empty(q.shape, dtype=torch.bfloat16, device=dev)
+        # said before the first copy: however this function ends, the allocator then waits for the copies still in flight
+        for t in dev_in + [kv_d]:
+            t.record_stream(s_in)
+        for t in (dkv_d, dq_d):
+            t.record_stream(s_out)
         s_in.wait_stream(s_comp)
         with torch.cuda.stream(s_in):
             kv_d.copy_(kv, non_blocking=True)
@@ -823,10 +830,6 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
         s_out.wait_stream(s_comp)
         with torch.cuda.stream(s_out):
             out_dkv.copy_(dkv_d, non_blocking=True)
-        for t in dev_in + [kv_d]:
-            t.record_stream(s_in)
-        for t in (dkv_d, dq_d):
-            t.record_stream(s_out)
         s_out.synchronize()
         s_comp.synchronize()
     return out_dq, out_dkv

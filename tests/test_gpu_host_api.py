@@ -5,6 +5,7 @@ import torch
 from test_operator_b200.inputs import Workload, make_sequence
 
 pytestmark = pytest.mark.gpu
+KEYS = ("q", "kv", "dO", "lse", "O", "indices")
 
 
 @pytest.mark.parametrize("q_start", [None, 40])
@@ -22,6 +23,33 @@ def test_host_entry_matches_device_entry(q_start):
     assert not dq_h.is_cuda and not dkv_h.is_cuda
     assert torch.equal(dq_h.view(torch.int16), dq_d.cpu().view(torch.int16))
     assert (dkv_h - dkv_d.cpu()).abs().max().item() <= 1e-5 * dkv_d.abs().max().item()
+
+
+@pytest.mark.parametrize("bad", ["lse_dtype", "dO_width", "heads", "indices_dtype", "transposed_q", "short_O", "kv_width"])
+def test_host_entry_refuses_before_anything_is_copied(bad, monkeypatch):
+    from test_operator_b200 import op
+    s = make_sequence(Workload("bad", 1, 24, 300, 16, 100, "uniform"), device="cpu", seed=22)
+    q, kv, dO, lse, O, idx = (s[k] for k in KEYS)
+    if bad == "lse_dtype":
+        lse = lse.double()
+    elif bad == "dO_width":
+        dO = dO[:, :, :256].contiguous()
+    elif bad == "heads":
+        q, dO, O, lse = (t[:, :12].contiguous() for t in (q, dO, O, lse))
+    elif bad == "indices_dtype":
+        idx = idx.long()
+    elif bad == "transposed_q":
+        q = q.transpose(0, 1).contiguous().transpose(0, 1)
+    elif bad == "short_O":
+        O = O[:20]
+    else:
+        kv = kv[:, :512].contiguous()
+    copies = []
+    real = torch.Tensor.copy_
+    monkeypatch.setattr(torch.Tensor, "copy_", lambda self, *a, **k: (copies.append(1), real(self, *a, **k))[1])
+    with pytest.raises(RuntimeError):
+        op.mla_bwd_host(q, kv, dO, lse, O, idx, device="cuda:0", q_start_index_s=None)
+    assert not copies
 
 
 def test_reduction_rate_probe_adds_what_it_claims():

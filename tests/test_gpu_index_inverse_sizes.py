@@ -53,7 +53,7 @@ def test_long_stretches_of_unused_rows(s_kv, used):
 
 
 def test_time_is_linear_in_the_rows():
-    """Slots on the first rows of a long kv pool only: four times the rows take about four times as long (42 and 78 us), not
+    """Slots on the first rows of a long kv pool only: four times the rows take at most about four times as long (42 and 78 us), not
     sixteen times."""
     from test_operator_b200 import op
     idx = torch.randint(0, 1024, (16, 2048), dtype=torch.int32, device="cuda")
