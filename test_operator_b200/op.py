@@ -774,10 +774,7 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
     """
     dev = torch.device(device)
     s_q = q.shape[0]
-    host = (q, dO, lse, O, indices)
-    for name, t in zip(("q", "dO", "lse", "O", "indices"), host):
-        _check(t.is_contiguous(), f"{name} must be contiguous")
-        _check(t.dim() > 0 and t.shape[0] == s_q, f"{name} first dim must equal s_q")
+    host = [t[:s_q] for t in (q, dO, lse, O, indices)]
     # A block costs the host about 80 us of calls, in which PCIe moves 4 MB.
     n_bytes = sum(t.numel() * t.element_size() for t in host)
     n_chunks = max(1, min(n_chunks, s_q, n_bytes // _HOST_BLOCK_BYTES))
@@ -795,8 +792,9 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
     with torch.cuda.device(dev):
         s_comp = torch.cuda.current_stream()
         s_in, s_out = torch.cuda.Stream(), torch.cuda.Stream()
-        dev_in = [torch.empty(t.shape, dtype=t.dtype, device=dev) for t in host]
-        kv_d = torch.empty(kv.shape, dtype=kv.dtype, device=dev)
+        # (as `.to` would make them: a strided input arrives contiguous)
+        dev_in = [torch.empty_like(t, device=dev) for t in host]
+        kv_d = torch.empty_like(kv, device=dev)
         if s_q:
             _validate(dev_in[0], kv_d, *dev_in[1:])
         dkv_d = torch.empty(kv.shape, dtype=torch.float32, device=dev)

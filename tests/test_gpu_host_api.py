@@ -25,6 +25,20 @@ def test_host_entry_matches_device_entry(q_start):
     assert (dkv_h - dkv_d.cpu()).abs().max().item() <= 1e-5 * dkv_d.abs().max().item()
 
 
+def test_host_entry_takes_strided_and_longer_inputs():
+    from test_operator_b200 import op
+    s = make_sequence(Workload("strided", 1, 40, 300, 16, 100, "uniform", invalid_frac=0.1), device="cpu", seed=21)
+    host = [s[k] for k in KEYS]
+    want = op.mla_bwd_host(*host, device="cuda:0", q_start_index_s=None)
+    q, kv, dO, lse, O, idx = host
+    wide = torch.zeros(40, 16, 600, dtype=torch.bfloat16)
+    wide[:, :, :576] = q
+    got = op.mla_bwd_host(wide[:, :, :576], kv, torch.cat([dO, dO]), torch.cat([lse, lse]), O, idx.repeat(2, 1), device="cuda:0",
+                          q_start_index_s=None)
+    assert torch.equal(got[0].view(torch.int16), want[0].view(torch.int16))
+    assert (got[1] - want[1]).abs().max().item() <= 1e-5 * want[1].abs().max().item()
+
+
 @pytest.mark.parametrize("bad", ["lse_dtype", "dO_width", "heads", "indices_dtype", "transposed_q", "short_O", "kv_width"])
 def test_host_entry_refuses_before_anything_is_copied(bad, monkeypatch):
     from test_operator_b200 import op
