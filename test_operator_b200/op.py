@@ -434,17 +434,14 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
     richer parameter block (`dq_test/dq_phase_capture.cuh:107-109`)."""
     n_seq = len(seq_q_len)
     device = torch.device(device)
-    if device.type == "cuda" and n_seq and all(
-            b == a + n for a, n, b in zip(seq_q_start, seq_q_len, seq_q_start[1:])):
-        t_q = sum(seq_q_len)
+    seq_q_start, seq_q_len, seq_kv_start, seq_kv_len = (list(v) for v in (seq_q_start, seq_q_len, seq_kv_start, seq_kv_len))
+    if device.type == "cuda" and _packed_from_row_0(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len):
+        t_q = int(sum(seq_q_len))
         if topk_length is not None:
             _check_topk_length(topk_length, t_q)
             topk_length = topk_length.reshape(-1).to(device=device, dtype=torch.int32).contiguous()
-        _check(seq_q_start[0] == 0, "the query rows of the sequences start at row 0")
         meta = torch.empty(t_q, 4, dtype=torch.int32, device=device)
-        if t_q == 0:
-            return meta
-        table = [(ctypes.c_int32 * n_seq)(*v) for v in (seq_q_start, seq_kv_start, seq_kv_len)]
+        table = [(ctypes.c_int32 * n_seq)(*(int(x) for x in v[:n_seq])) for v in (seq_q_start, seq_kv_start, seq_kv_len)]
         lib = load_library()
         index = meta.get_device()
         with _on_device(index):
@@ -452,13 +449,13 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
                                      topk_length.data_ptr() if topk_length is not None else None, _raw_stream(index))
         _raise_status(lib, st, "smla_query_meta")
         return meta
-    lens = torch.tensor(list(seq_q_len), dtype=torch.int64)
+    lens = torch.tensor(seq_q_len, dtype=torch.int64)
     seq_of_q = torch.repeat_interleave(torch.arange(n_seq), lens)
     t_q = int(lens.sum().item())
-    row_in_seq = torch.arange(t_q) - torch.tensor(list(seq_q_start), dtype=torch.int64)[seq_of_q]
+    row_in_seq = torch.arange(t_q) - torch.tensor(seq_q_start, dtype=torch.int64)[seq_of_q]
     meta = torch.empty(t_q, 4, dtype=torch.int32)
-    meta[:, 0] = torch.tensor(list(seq_kv_start), dtype=torch.int32)[seq_of_q]
-    meta[:, 1] = torch.tensor(list(seq_kv_len), dtype=torch.int32)[seq_of_q]
+    meta[:, 0] = torch.tensor(seq_kv_start, dtype=torch.int32)[seq_of_q]
+    meta[:, 1] = torch.tensor(seq_kv_len, dtype=torch.int32)[seq_of_q]
     meta[:, 2] = (row_in_seq + (q_start_index_s or 0)).to(torch.int32)
     meta[:, 3] = topk
     meta = meta.to(device)
@@ -466,6 +463,20 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
         _check_topk_length(topk_length, t_q)
         meta[:, 3] = topk_length.reshape(-1).to(device=device, dtype=torch.int32).clamp(0, topk)
     return meta.contiguous()
+
+
+def _packed_from_row_0(q_start, q_len, kv_start, kv_len) -> bool:
+    """What the table kernel can do: sequences one behind the other from query row 0, some query, values of 32 bits.  The rest
+    (the shard of a sequence that starts at a negative row, say) is put together on the host."""
+    n = len(q_len)
+    if n == 0 or min(len(q_start), len(kv_start), len(kv_len)) < n:
+        return False
+    row = 0
+    for a, length in zip(q_start, q_len):
+        if a != row or length < 0 or int(length) != length:
+            return False
+        row += int(length)
+    return 0 < row < 1 << 31 and all(-(1 << 31) <= v < 1 << 31 for v in kv_start[:n] + kv_len[:n])
 
 
 def _check_topk_length(topk_length: torch.Tensor, t_q: int) -> None:

@@ -74,6 +74,29 @@ def test_query_table_on_the_gpu_equals_the_host_one(n_seq):
         assert torch.equal(got.cpu(), want)
 
 
+@pytest.mark.parametrize("q0,lens,kv0,kv_lens", [
+    ([-100], [28], [0], [300]),                              # the shard of a sequence that begins 100 queries earlier
+    ([5, 8], [3, 4], [0, 40], [40, 50]),                     # rows counted from elsewhere
+    ([0, 3, 7], [3, 4], [0, 40, 90], [40, 50, 0]),           # offsets with the end behind them, as cu_seqlens are
+    (torch.tensor([0, 3]), torch.tensor([3, 4]), torch.tensor([0, 40]), torch.tensor([40, 50])),
+    ([0, 0], [0, 0], [0, 0], [1, 1]),
+])
+def test_query_table_of_other_forms_equals_the_host_one(q0, lens, kv0, kv_lens):
+    from test_operator_b200 import op
+    want = op.query_meta_for(q0, lens, kv0, kv_lens, "cpu", 7, 64)
+    got = op.query_meta_for(q0, lens, kv0, kv_lens, DEV, 7, 64)
+    assert got.is_cuda and torch.equal(got.cpu(), want)
+
+
+def test_query_table_refuses_what_the_host_one_refuses():
+    from test_operator_b200 import op
+    for bad in (dict(kv_lens=[40]), dict(kv0=[0, 1 << 31]), dict(lens=[3, -4])):
+        args = {**dict(q0=[0, 3], lens=[3, 4], kv0=[0, 40], kv_lens=[40, 50]), **bad}
+        for device in ("cpu", DEV):
+            with pytest.raises((RuntimeError, IndexError, ValueError)):
+                op.query_meta_for(*args.values(), device, 0, 64)
+
+
 # the last slot in use on, before and behind the edges of what is worked on as one: 32 keys (a drain warp's registers), 64 (a dQ
 # tile), 128 (a dKV tile, one CTA's half of a work tile), 256 (a work tile)
 EDGES = [1, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 160, 161, 255, 256, 257, 384, 385, 500]
