@@ -117,8 +117,8 @@ size_t smla_bwd_staging_bytes_per_query(const smla_bwd_params* p);
  * fragments the pool), or a latency-bound loop that cannot take the device-wide synchronisation an
  * allocation or free may imply.  Such a caller still owns q, kv, dO, lse, O, indices, dQ and dKV; what it cannot
  * provide is the scratch for Delta and the bf16 S / dS.  This entry point takes that scratch from a
- * 32 MiB array compiled into the library (smla_bwd_noalloc_capacity()), resident on every GPU that loads
- * the library until the process exits.  It calls no cudaMalloc / cudaFree and no allocating library routine.
+ * 32 MiB array compiled into the library (smla_bwd_noalloc_capacity(); 4 MiB behind it hold a slot count per query), resident
+ * on every GPU that loads the library until the process exits.  It calls no cudaMalloc / cudaFree and no allocating library routine.
  *
  * Limits and rules:
  *  - 256 + 4*s_q*h_q bytes of Delta plus the S/dS of at least one query (4 * topk_pad * h_pad bytes, topk
@@ -128,7 +128,7 @@ size_t smla_bwd_staging_bytes_per_query(const smla_bwd_params* p);
  *  - The first call on a device looks up the array's device address (cudaGetSymbolAddress, with that
  *    device current) and caches it; make that first call before any stream capture begins.
  *  - All calls on a device share the one array.  It keeps whatever the previous call left; every byte that
- *    is read is rewritten first (Delta and the S/dS rows of a pass are fully overwritten before use; the
+ *    is read is rewritten first (Delta, the slot counts and the S/dS rows of a pass are written before use; the
  *    error word starts at zero with the library image and is cleared again when a timeout has been reported).  Two calls whose kernels overlap on the GPU (different streams, or threads)
  *    race on it: serialise them.
  *  - Status of the last call: smla_bwd_noalloc_status(stream) (synchronises the stream). */

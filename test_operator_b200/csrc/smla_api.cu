@@ -555,9 +555,12 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
 }
 
 // ---- workspace that lives in the library image (smla_bwd_run_noalloc) -----------------------------------
-// Every GPU that loads the library carries these bytes until the process exits.
+// Every GPU that loads the library carries these bytes until the process exits: what the limit of the entry point is counted
+// in (error word, Delta, S and dS), and behind it room for the slot counts of as many queries as that limit lets through (Delta
+// has at least 32 bytes a query), so that the counts take nothing away from it.
 constexpr size_t kStaticWorkspaceBytes = size_t(32) << 20;
-static __device__ __align__(256) unsigned char g_static_workspace[kStaticWorkspaceBytes];
+constexpr size_t kStaticCountBytes = kStaticWorkspaceBytes / 32 * 4 + 2 * kAlign;
+static __device__ __align__(256) unsigned char g_static_workspace[kStaticWorkspaceBytes + kStaticCountBytes];
 
 std::mutex g_static_ws_mutex;
 void* g_static_ws_ptr[kMaxDevices] = {};   // device address of g_static_workspace, per device ordinal
@@ -748,13 +751,15 @@ int smla_bwd_run_noalloc(const smla_bwd_params* p, void* stream) {
     g_last_launches = 0;
     Plan pl;
     if (!check_params(p)) return SMLA_ERR_BAD_ARG;
-    // the fixed part (error word, Delta) plus the S / dS scratch of at least one query must fit the built-in array
-    if (!plan_for_workspace(p, kStaticWorkspaceBytes, &pl)) return SMLA_ERR_TOO_LARGE_FOR_STATIC;
+    // the fixed part (error word, Delta) plus the S / dS scratch of at least one query must fit the built-in array's 32 MiB
+    if (!make_plan(p, 1, &pl)) return SMLA_ERR_BAD_ARG;
+    const size_t counts = pl.s_off - align_up(kAlign + size_t(p->s_q) * p->h_q * 4, kAlign);
+    if (counts > kStaticCountBytes || !plan_for_workspace(p, kStaticWorkspaceBytes + counts, &pl)) return SMLA_ERR_TOO_LARGE_FOR_STATIC;
     void* ws = nullptr;
     const int st = static_workspace_ptr(&ws);
     if (st != SMLA_OK) return st;
     // one stream only: this entry point creates nothing, streams and events included
-    return run_stages_impl(p, ws, kStaticWorkspaceBytes, stream, SMLA_STAGE_ALL, false);
+    return run_stages_impl(p, ws, kStaticWorkspaceBytes + counts, stream, SMLA_STAGE_ALL, false);
 }
 
 size_t smla_bwd_noalloc_capacity(void) { return kStaticWorkspaceBytes; }

@@ -103,6 +103,19 @@ def test_workspace_size_and_bad_arguments_without_a_gpu():
     assert b"workspace" in lib.smla_status_string(3)
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the accepted calls would be run")
+@pytest.mark.parametrize("h_q", [8, 64, 72, 128])
+def test_noalloc_limit_counts_delta_and_one_query(h_q):
+    """256 + 4 s_q h_q bytes of Delta and one query's S / dS within 32 MiB: the largest s_q is let through (and then finds no
+    device here, status 2), the next one is refused (status 5)."""
+    lib = op.load_library()
+    one_query = 256 * (64 if h_q <= 64 else 128) * 4
+    most = ((32 << 20) - one_query - 256) // 256 * 256 // (4 * h_q)
+    for s_q, want in ((most, 2), (most + 256 // (4 * h_q) + 1, 5), (1000, 2)):
+        p = op._Params(256, 256, 256, 256, 256, 256, 256, 256, s_q, 1024, h_q, 64, 0.0, 0, 1)
+        assert lib.smla_bwd_run_noalloc(ctypes.byref(p), None) == want, (s_q, want)
+
+
 def test_operator_rejects_what_the_reference_rejects():
     w = Workload("v", 1, 2, 32, 16, 8, "uniform")
     s = make_sequence(w, device="cpu", seed=1)
