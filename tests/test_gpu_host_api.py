@@ -9,18 +9,35 @@ KEYS = ("q", "kv", "dO", "lse", "O", "indices")
 
 
 @pytest.mark.parametrize("q_start", [None, 40])
-def test_host_entry_matches_device_entry(q_start):
+def test_host_entry_matches_device_entry(q_start, monkeypatch):
     from test_operator_b200 import op
-    w = Workload("host", 1, 37, 512, 64, 128, "uniform", invalid_frac=0.1)
+    w = Workload("host", 1, 130, 512, 64, 128, "uniform", invalid_frac=0.1)       # 27 MB of inputs: blocks are of 4 MB at least
     s = make_sequence(w, device="cpu", seed=19)
     host = [s[k].pin_memory() for k in ("q", "kv", "dO", "lse", "O", "indices")]
+    real, blocks = op.mla_bwd, []
+    monkeypatch.setattr(op, "mla_bwd", lambda *a, **k: (blocks.append(a[0].shape[0]), real(*a, **k))[1])
     dq_h, dkv_h = op.mla_bwd_host(*host, device="cuda:0", q_start_index_s=q_start, n_chunks=5)
+    assert len(blocks) == 5 and sum(blocks) == 130
     dev = [t.to("cuda:0") for t in host]
     dq_d, dkv_d = op.mla_bwd(*dev, q_start_index_s=q_start, check_device_status=True)
     from oracle.sparse_mla_ref import sparse_mla_bwd_ref
     from tests.metrics import assert_backward_close
     assert_backward_close(dq_d.cpu(), dkv_d.cpu(), *sparse_mla_bwd_ref(*host, q_start_index_s=q_start))
     assert not dq_h.is_cuda and not dkv_h.is_cuda
+    assert torch.equal(dq_h.view(torch.int16), dq_d.cpu().view(torch.int16))
+    assert (dkv_h - dkv_d.cpu()).abs().max().item() <= 1e-5 * dkv_d.abs().max().item()
+
+
+@pytest.mark.parametrize("s_q,n_chunks", [(1, 8), (2, 2), (5, 8), (11, 7), (30, 30)])
+def test_host_entry_with_fewer_rows_than_parts(s_q, n_chunks, monkeypatch):
+    """Blocks of a few rows and of none."""
+    from test_operator_b200 import op
+    monkeypatch.setattr(op, "_HOST_BLOCK_BYTES", 1)
+    s = make_sequence(Workload("rows", 1, s_q, 300, 16, 100, "uniform", invalid_frac=0.1), device="cuda:0", seed=20)
+    dev = [s[k] for k in KEYS]
+    host = [t.cpu().pin_memory() for t in dev]
+    dq_h, dkv_h = op.mla_bwd_host(*host, device="cuda:0", q_start_index_s=None, n_chunks=n_chunks)
+    dq_d, dkv_d = op.mla_bwd(*dev, q_start_index_s=None, check_device_status=True)
     assert torch.equal(dq_h.view(torch.int16), dq_d.cpu().view(torch.int16))
     assert (dkv_h - dkv_d.cpu()).abs().max().item() <= 1e-5 * dkv_d.abs().max().item()
 
