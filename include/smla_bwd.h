@@ -196,13 +196,12 @@ int smla_bwd_last_device_code(void);
 /* How one pass of the backward is scheduled.  chunks = 0: the kernels one after another on the caller's stream.
  * chunks >= 2: the queries of a pass are cut into that many parts and the dKV kernel of a part runs on a second
  * stream owned by the library, on `dkv_pairs` 2-SM clusters (0: chosen by the library from the head count), beside
- * the recompute and dQ kernels of the next part: the dKV kernel keeps the load/store path busy and the tensor cores
- * a third of the time, the other two the reverse.  chunks = -1 (the default): chosen by the library - two overlapped
- * parts up to 64 heads and top-k 256, one after another otherwise, which is what measures faster on B200.
+ * the recompute and dQ kernels of the next part.  chunks = -1 (the default): chosen by the library - one after another,
+ * which is what measures faster on B200 at every size tried.
  * A pass falls back to one-after-the-other when it has too few queries to keep every cluster busy in every part.
  * The second stream and its events are created by the first call that needs them on a device: make that call before a
  * stream capture begins.  Process-wide; the environment variable SMLA_SCHEDULE="chunks,dkv_pairs" sets the initial
- * value.  smla_bwd_get_schedule returns what was set (-1 for automatic), not what a head count resolves to. */
+ * value.  smla_bwd_get_schedule returns what was set (-1 for automatic). */
 int smla_bwd_set_schedule(int chunks, int dkv_pairs);
 void smla_bwd_get_schedule(int* chunks, int* dkv_pairs);
 

@@ -33,13 +33,17 @@ thread_local int g_last_device_code = 0;
 // chunks == 0: the four kernels one after another on the caller's stream.
 // chunks >= 2: the queries of a pass are cut into `chunks` parts; recompute and dq of part c run on the caller's
 //   stream while the dkv kernel of part c - 1 runs on a second (internal, higher-priority) stream with a grid of
-//   `dkv_pairs` clusters, the recompute kernels taking the remaining clusters.  The dkv kernel is bound by the
-//   chip's fp32 reduction rate, not by its SMs, so it loses little on fewer SMs, and the SMs it leaves do the
-//   tensor-core work of the other two kernels meanwhile.
+//   `dkv_pairs` clusters, the recompute kernels taking the remaining clusters.
+// chunks == -1 (automatic): one after another, which measures faster everywhere on B200 (alternating the two on one GPU, back to
+//   back, one after another / two parts): 128 heads, 4096 queries x top-k 2048 8.04 / 8.40 ms; 64 heads at top-k 2048
+//   6.23 / 6.32 ms, 512 1.84 / 1.85, 256 1.05 / 1.18, 128 0.73 / 0.89, 64 0.61 / 0.75; 16 heads at 256 0.90 / 1.00; 1400
+//   queries x 64 heads x 256 0.35 / 0.41, 8192 queries 2.16 / 2.35.  The dKV kernel's reductions and the other kernels'
+//   gathers share the L2, so running them side by side gives the sum of their times, and a part's kernels do not start
+//   under one another's tails.
 constexpr int kMaxChunks = 16;
-std::atomic<int> g_sched_chunks{-2};      // -2: not yet read from the environment; -1: chosen per head count
+std::atomic<int> g_sched_chunks{-2};      // -2: not yet read from the environment
 std::atomic<int> g_sched_dkv_pairs{0};
-constexpr int kDefaultChunks = -1;        // chosen from the head count, see auto_chunks
+constexpr int kDefaultChunks = -1;
 constexpr int kDefaultDkvPairs = 0;       // 0: chosen from the head count, see auto_dkv_pairs
 std::atomic<long long> g_wait_limit{smla::kWaitLimitCycles};
 
@@ -62,15 +66,9 @@ void schedule(int* chunks, int* dkv_pairs) {
     *dkv_pairs = g_sched_dkv_pairs.load();
 }
 
-// Clusters for the dkv kernel when the caller leaves the choice to the library: its share of the three kernels'
-// time, measured with each kernel alone on a whole B200 (top-k 2048; dkv 3.8 ms at either head count, recompute +
-// dq 3.4 ms at 128 heads and 2.65 ms at 64).  The step time is flat within +-3 clusters of these.
-// Measured on B200, alternating the schedules on one GPU over a second of calls: one kernel after the other is the faster
-// form with 128 heads (8.04 against 8.40 ms on 4096 queries x top-k 2048) and with 64 (6.23 against 6.32 ms at top-k 2048,
-// 1.84 / 1.85 at 512, 0.436 / 0.448 on 777 queries x 600): the dKV kernel's reductions and the other kernels' gathers share
-// the L2, so running them side by side gives the sum of their times.  The overlapped form stays for queries of one tile.
-int auto_chunks(int h_pad, int topk_pad) { return h_pad > 64 || topk_pad > smla::kWorkTileKeys ? 0 : 2; }
-
+// Clusters for the dkv kernel of the overlapped form when the caller leaves the choice to the library: its share of the
+// three kernels' time with each alone on a whole B200 (top-k 2048; dkv 3.7 ms with 128 heads, recompute + dq 3.2 ms; 3.5 and
+// 2.1 ms with 64).  The time of a call is flat within +-3 clusters of these.
 int auto_dkv_pairs(int h_pad, int resident) {
     const double share = h_pad > 64 ? 0.50 : 0.60;
     int n = static_cast<int>(resident * share + 0.5);
@@ -417,7 +415,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
 
     int chunks = 0, dkv_pairs = 0;
     schedule(&chunks, &dkv_pairs);
-    if (chunks < 0) chunks = auto_chunks(HP, pl.topk_pad);
+    if (chunks < 0) chunks = 0;
     const int all = SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ;
     if (dkv_pairs <= 0) dkv_pairs = auto_dkv_pairs(HP, pairs_d < pairs_r ? pairs_d : pairs_r);
     if (!allow_overlap || det || (stages & all) != all || dkv_pairs >= pairs_d || dkv_pairs >= pairs_r) chunks = 0;

@@ -54,20 +54,20 @@ def test_overlapped_schedule_replays_from_a_cuda_graph():
         op.set_schedule(*before)
 
 
-def test_default_schedule_follows_the_head_count():
-    """Automatic (-1): two overlapped parts with 64 heads, the kernels one after the other with 128."""
+def test_default_schedule_is_one_after_the_other_at_every_head_count():
+    """Automatic (-1): the kernels one after the other; two overlapped parts with 64 heads only where they are asked for."""
     from test_operator_b200 import op
     before = op.get_schedule()
-    op.set_schedule(-1, 0)
     try:
-        for h_q, launches in ((64, 1 + 3 * 2), (128, 1 + 3)):
+        for h_q, chunks, launches in ((64, -1, 1 + 3), (64, 2, 1 + 3 * 2), (128, -1, 1 + 3)):
+            op.set_schedule(chunks, 0)
             w = Workload("sched_auto", 1, 1400, 2048, h_q, 256, "uniform", invalid_frac=0.1)
             s = make_sequence(w, device=DEV, seed=39)
             args = [s[k] for k in KEYS]
             dq, dkv = op.mla_bwd(*args, q_start_index_s=None, check_device_status=True)
             assert op.last_launch_count() == launches
             dq_ref, dkv_ref = sparse_mla_bwd_ref(*args, q_start_index_s=None, chunk_s=16)
-            assert_backward_close(dq, dkv, dq_ref, dkv_ref, f"automatic schedule, {h_q} heads")
+            assert_backward_close(dq, dkv, dq_ref, dkv_ref, f"schedule {chunks}, {h_q} heads")
     finally:
         op.set_schedule(*before)
 
