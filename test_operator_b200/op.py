@@ -9,8 +9,10 @@ There is no CPU or eager fallback: if the library is missing and cannot be built
 """
 from __future__ import annotations
 
+import array
 import ctypes
 import functools
+import itertools
 import math
 import os
 import threading
@@ -182,6 +184,7 @@ def _on_device(index: int):
     return _NO_SWITCH if torch.cuda.current_device() == index else torch.cuda.device(index)
 
 
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", None) or torch.cuda.is_current_stream_capturing
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
@@ -252,7 +255,7 @@ def _scratch_of_stream(index: int) -> _StreamScratch:
     """The set of the current stream of device `index` (the current device).  While that stream is being captured, a new one:
     the graph goes on using its buffers after a larger call has replaced the kept ones, so they come from the graph's own
     pool, and what is only recorded (the clearing of a workspace's error word) must not pass for done in a later call."""
-    if torch.cuda.is_current_stream_capturing():
+    if _capturing():
         return _StreamScratch()
     key = (index, _raw_stream(index))
     with _scratch_cache_lock:
@@ -435,17 +438,17 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
     n_seq = len(seq_q_len)
     device = torch.device(device)
     seq_q_start, seq_q_len, seq_kv_start, seq_kv_len = (list(v) for v in (seq_q_start, seq_q_len, seq_kv_start, seq_kv_len))
-    if device.type == "cuda" and _packed_from_row_0(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len):
-        t_q = int(sum(seq_q_len))
+    packed = _packed_tables(n_seq, seq_q_start, seq_q_len, seq_kv_start, seq_kv_len) if device.type == "cuda" else None
+    if packed is not None:
+        t_q, table = packed
         if topk_length is not None:
             _check_topk_length(topk_length, t_q)
             topk_length = topk_length.reshape(-1).to(device=device, dtype=torch.int32).contiguous()
         meta = torch.empty(t_q, 4, dtype=torch.int32, device=device)
-        table = [(ctypes.c_int32 * n_seq)(*(int(x) for x in v[:n_seq])) for v in (seq_q_start, seq_kv_start, seq_kv_len)]
         lib = load_library()
         index = meta.get_device()
         with _on_device(index):
-            st = lib.smla_query_meta(meta.data_ptr(), n_seq, *table, t_q, q_start_index_s or 0, topk,
+            st = lib.smla_query_meta(meta.data_ptr(), n_seq, *(t.buffer_info()[0] for t in table), t_q, q_start_index_s or 0, topk,
                                      topk_length.data_ptr() if topk_length is not None else None, _raw_stream(index))
         _raise_status(lib, st, "smla_query_meta")
         return meta
@@ -465,18 +468,18 @@ def query_meta_for(seq_q_start, seq_q_len, seq_kv_start, seq_kv_len, device, q_s
     return meta.contiguous()
 
 
-def _packed_from_row_0(q_start, q_len, kv_start, kv_len) -> bool:
-    """What the table kernel can do: sequences one behind the other from query row 0, some query, values of 32 bits.  The rest
-    (the shard of a sequence that starts at a negative row, say) is put together on the host."""
-    n = len(q_len)
-    if n == 0 or min(len(q_start), len(kv_start), len(kv_len)) < n:
-        return False
-    row = 0
-    for a, length in zip(q_start, q_len):
-        if a != row or length < 0 or int(length) != length:
-            return False
-        row += int(length)
-    return 0 < row < 1 << 31 and all(-(1 << 31) <= v < 1 << 31 for v in kv_start[:n] + kv_len[:n])
+def _packed_tables(n, q_start, q_len, kv_start, kv_len):
+    """The sequences as the table kernel takes them - one behind the other from query row 0, some query, whole lists of values of
+    32 bits - or None: the rest (the shard of a sequence that starts at a negative row, say) is put together on the host."""
+    if min(len(q_start), len(kv_start), len(kv_len)) < n or min(q_len, default=-1) < 0:
+        return None
+    *rows, t_q = itertools.accumulate(q_len, initial=0)
+    if rows != q_start[:n] or not 0 < t_q < 1 << 31:
+        return None
+    try:
+        return int(t_q), [array.array("i", v) for v in (rows, kv_start[:n], kv_len[:n])]
+    except (TypeError, OverflowError):
+        return None
 
 
 def _check_topk_length(topk_length: torch.Tensor, t_q: int) -> None:
