@@ -33,10 +33,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// True in exactly one lane of a converged warp.  A branch on this (not on lane == 0) is how the compiler learns that a
-// single thread runs the block: the operands of tcgen05.mma / commit live in uniform registers, and behind a lane
-// comparison every one of those instructions is wrapped in a loop over the lanes (measured with a standalone probe: 94 -
-// 102 cycles per UMMA issued behind lane == 0 whatever its size, the tensor pipe's own 43 - 64 behind elect.sync).
+// True in exactly one lane of a converged warp.  The threads that issue UMMAs are picked with it and not with lane == 0:
+// measured, 94 - 102 cycles per UMMA of N <= 128 behind a lane comparison, the tensor pipe's own 43 - 64 behind elect.sync.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -96,10 +94,8 @@ __device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, const W
     if (mbar_test_wait(bar, parity)) return true;
     return mbar_spin_slow(bar, parity, ctx, code);
 }
-// The consumer's place in a ring of slots, with the barrier of the NEXT slot polled while the current one is worked on: a
-// poll takes a few hundred cycles behind a busy load/store pipe, which a thread that issues UMMAs (or forwards signals)
-// one slot at a time cannot afford per slot (standalone probe, idle SM, slots of four 64-cycle UMMAs: 300 cycles per slot
-// polling when the slot is due, 259 polling ahead).
+// The consumer's place in a ring of slots, with the barrier of the NEXT slot polled while the current one is worked on, so
+// that a poll's latency is not added to every slot of a thread that issues UMMAs (or forwards signals) one slot at a time.
 template <int kSlots> struct RingReader {
     uint32_t full0;               // barrier of slot 0
     uint32_t slot = 0, phase = 0;

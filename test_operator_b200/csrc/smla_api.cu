@@ -270,7 +270,7 @@ void launch(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t 
 // passes; a query of one work tile (256 keys) is never split.
 int dq_key_split(int s_q, int topk_pad, int parts) {
     int z = 1;
-    while (z < 8 && 2 * z <= topk_pad / smla::kWorkTileKeys && s_q <= 148 / (parts * 2 * z)) z *= 2;
+    while (z < 8 && 2 * z <= topk_pad / smla::kWorkTileKeys && s_q <= smla::kSmCount / (parts * 2 * z)) z *= 2;
     return z;
 }
 
@@ -373,9 +373,9 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
         const size_t zero_blocks = (zero_n + kPrepThreads * 16 - 1) / (kPrepThreads * 16);
         // (34 queries x 128 heads: 14 us with one block per query, 6.6 us so)
         int head_parts = 1;
-        while (static_cast<long long>(p->s_q) * head_parts * 2 <= 8 * 148 && p->h_q / (head_parts * 2) >= 16) head_parts *= 2;
+        while (static_cast<long long>(p->s_q) * head_parts * 2 <= 8 * kSmCount && p->h_q / (head_parts * 2) >= 16) head_parts *= 2;
         int grid = p->s_q * head_parts;
-        if (size_t(grid) < zero_blocks) grid = std::max(grid, int(zero_blocks < 8 * 148 ? zero_blocks : 8 * 148));
+        if (size_t(grid) < zero_blocks) grid = std::max(grid, int(std::min<size_t>(zero_blocks, 8 * kSmCount)));
         launch(smla_prep_kernel, grid, kPrepThreads, 0, st, true, 1, reinterpret_cast<const uint4*>(p->O),
                reinterpret_cast<const uint4*>(p->dO), delta, reinterpret_cast<int*>(ws + pl.used_off),
                reinterpret_cast<uint4*>(p->dKV), zero_n, head_parts, kp);

@@ -3,7 +3,7 @@
 // The backward of one query token is a chain of five contractions around a softmax-gradient
 // step.  It is split into four kernels that hand bf16 S / dS through a scratch buffer:
 //
-//   delta      Delta[q,h] = sum_j O[q,h,j] * dO[q,h,j]                         (HBM-bound)
+//   prep       Delta[q,h] = sum_j O[q,h,j] * dO[q,h,j], slots in use per query, dKV cleared   (HBM-bound)
 //   recompute  P^T = K_g Q^T, dP^T = V_g dO^T  (tcgen05, keys on the M axis),
 //              S = exp2(P*scale*log2e - lse), dS = S*(dP - Delta)*scale -> bf16 scratch
 //   dkv        dKV^T[d, key] = dO^T S + Q^T dS (tcgen05, d on the M axis), then one coalesced
@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(256) smla_delta_kernel(const uint4* __restrict
 //   every block     its share of dKV cleared (where the caller wants it cleared)
 // Bound by HBM: O, dO and the indices read once, dKV written once.
 // =============================================================================================
+constexpr int kSmCount = 148;           // of a B200: for splits of small grids
 constexpr int kWorkTileKeys = 256;      // granularity of the work ranges: what the recompute kernel does per accumulator
 constexpr int kPrepThreads = 256;
 
@@ -297,9 +298,7 @@ __device__ __forceinline__ int find_range(const KParams& p, int cluster, int n_c
     *out = WorkRange{begin, range_start(total, cluster + 1, n_clusters), p.q0 + q, lo};
     return total;
 }
-// Broadcast, so that the compiler knows the bounds of the loops below to be the same in all lanes: it then keeps what the
-// UMMAs of an issuing thread need (descriptors, addresses) in uniform registers, where tcgen05.mma takes its operands from.
-// With a loop bound or a ring position it takes for lane-dependent it moves every operand over first.
+// Broadcast, so that the bounds of the loops around the UMMAs are warp-uniform to the compiler as well (see elect_one).
 __device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
     return WorkRange{__shfl_sync(0xffffffffu, w.begin, 0), __shfl_sync(0xffffffffu, w.end, 0), __shfl_sync(0xffffffffu, w.q, 0),
                      __shfl_sync(0xffffffffu, w.lo, 0)};
@@ -729,11 +728,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // repeat bit for bit.
 // What bounds it: per tile and CTA 17 slots x 4 UMMAs x 64 cycles = 4352 cycles of tensor pipe; 275 KB of gathered rows
 // written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Measured (4096 queries x 128 heads x
-// top-k 2048): 7800 cycles a tile, 2.24 ms at the 1.65 GHz the power cap leaves, against 3.27 ms for two logit passes and
-// an E.V pass; without the gathers 7000 cycles, without the softmax 6300, without both 6100.  The ring's depth does not
-// matter (five, six or seven slots: 2.32 / 2.32 / 2.31 ms).  Row gathers by TMA (tile::gather4 from eight warps) in place
-// of cp.async: 3.0 ms; two producer groups on alternate slots: 2.36 ms; one arrival per producer warp: 2.34 ms.
-// With 64 heads half of the UMMAs' rows are zeros: 2.4 ms.
+// top-k 2048, a launch's cycles by its tiles): 8330 cycles a tile, 2.24 ms at the 1.65 GHz the power cap leaves in ten calls,
+// 2.5 ms at 1.47 in sixty (3.27 ms for two logit passes and an E.V pass); 64 heads, half of the UMMAs' rows zeros, 8140 cycles,
+// 2.24 - 2.3 ms.  Five, six or seven ring slots: 2.48 / 2.47 / 2.48 ms back to back, 64 heads 2.27 / 2.28 / 2.29.
 // A query whose tiles lie in several clusters' ranges leaves unnormalised partial results, which
 // smla_fwd_combine_kernel adds up.
 // =============================================================================================
@@ -754,7 +751,6 @@ constexpr int kOffStat = kOffRows + 3 * kTileKeys * 4;        // [2 tile paritie
 constexpr int kOffMisc = kOffStat + 2 * 4 * 64 * 4;
 constexpr int kSmemBytes = kOffMisc + 512 + 1024;             // barriers + alignment slack
 constexpr int kTmemO = 0, kTmemS = 256;
-constexpr int kPartFloats = kDV;           // a partial result: [HP heads][512] fp32 and [HP heads]{reference, sum}
 static_assert(kSmemBytes <= 232448, "shared memory of one SM");
 }  // namespace ff
 

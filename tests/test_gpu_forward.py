@@ -147,9 +147,8 @@ def test_forward_over_packed_sequences_with_a_query_table():
 
 
 def test_forward_many_queries_repeats_bit_for_bit_and_matches_oracle():
-    """More queries than SMs: every CTA of the logits kernels walks through several queries with its ring, accumulator
-    buffers and counters running on, and four threads issue its UMMAs (two per tile stream, handing over through a
-    counter).  o and lse must come out bit-identical in every run, and all queries are compared with the oracle
+    """More queries than SMs: every CTA of the forward kernel walks through several queries with its ring, accumulator
+    buffers and barrier phases running on.  o and lse must come out bit-identical in every run, and all queries are compared with the oracle
     (the same fp32 arithmetic on the GPU)."""
     from test_operator_b200 import op
     w = Workload("fwd_repeat", 1, 700, 1024, 128, 512, "uniform", invalid_frac=0.1)
