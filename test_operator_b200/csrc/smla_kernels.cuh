@@ -715,10 +715,10 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // Both gathers go through one ring of 16 KB slots in the order the UMMAs consume them: K of tile n + 1 (nine slots of
 // [128 keys x 64 columns]), then V of tile n (eight slots of [64 keys x 128 columns]); a slot feeds four UMMAs of 64
 // cycles either way, and the softmax of tile n runs under the UMMAs of S n + 1.
-//   warps 0-7   softmax: warp w reads lane quarter w % 4, columns [64 (w / 4), + 64) of S: one head, 64 keys per thread
-//   warps 8-15  gather producers (cp.async 16 B, swizzled)
-//   warp 16     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full"
-//   warp 17     TMA of the CTA's Q chunks
+//   warps 0-15  softmax: warp w reads lane quarter w % 4, columns [32 (w / 4), + 32) of S: one head, 32 keys per thread
+//   warps 16-23 gather producers (cp.async 16 B, swizzled)
+//   warp 24     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full" and "my P is written"
+//   warp 25     TMA of the CTA's Q chunks
 // The exponentials of a tile are taken against the maximum of the row so far; where a tile raises it, O and the sum are
 // rescaled.  A reference that lags behind the maximum (moved only when exceeded by 2^8) makes most of the rescaling
 // unnecessary and is 3 % faster (128 heads, 2.34 against 2.42 ms), but the heaviest probabilities then lose in their rounding
@@ -727,16 +727,21 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // 1.930 / 1.665 / 1.695e-3 with logits eight times as large (2048 slots, 128 heads).  Nothing depends on timing, o and lse
 // repeat bit for bit.
 // What bounds it: per tile and CTA 17 slots x 4 UMMAs x 64 cycles = 4352 cycles of tensor pipe; 275 KB of gathered rows
-// written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Measured (4096 queries x 128 heads x
-// top-k 2048, a launch's cycles by its tiles): 8330 cycles a tile, 2.24 ms at the 1.65 GHz the power cap leaves in ten calls,
-// 2.5 ms at 1.47 in sixty (3.27 ms for two logit passes and an E.V pass); 64 heads, half of the UMMAs' rows zeros, 8140 cycles,
-// 2.24 - 2.3 ms.  Five, six or seven ring slots: 2.48 / 2.47 / 2.48 ms back to back, 64 heads 2.27 / 2.28 / 2.29.
+// written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Eight softmax warps of 64 keys a thread were
+// busy 95 % of a launch, the issuer waiting 1900 cycles a tile for P (8330 cycles a tile, 128 heads).  Sixteen warps of 32 keys
+// hide each other's latency, P is announced by a local arrival that the odd CTA's relay thread forwards (a cluster-scope release
+// by every warp held it for hundreds of cycles): the issuer's wait for P is below 100 cycles, what is left are waits for gathered
+// slots.  4096 queries x 128 heads x top-k 2048: 2657 -> 2250 us on a cool GPU, 2521 -> 2445 back to back, where the power cap
+// holds the clock down.  Five, six or seven ring slots made no difference before.
 // A query whose tiles lie in several clusters' ranges leaves unnormalised partial results, which
 // smla_fwd_combine_kernel adds up.
 // =============================================================================================
 namespace ff {
-constexpr int kThreads = 576;
+constexpr int kSoftmaxWarps = 16;
 constexpr int kProducerThreads = 256;
+constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 64;
+constexpr int kIssueWarp = kThreads / 32 - 2, kLoadWarp = kThreads / 32 - 1;
+constexpr int kParts = 8;                  // a head's 256 keys of a tile over eight warps
 constexpr int kTileKeys = 256;             // per pair; 128 per CTA
 constexpr int kSlotBytes = 16384;
 constexpr int kStages = 7;
@@ -747,8 +752,8 @@ constexpr int kOffQ = 0;
 constexpr int kOffP = kQChunks * kQChunk;
 constexpr int kOffRing = kOffP + 4 * kPChunk;
 constexpr int kOffRows = kOffRing + kStages * kSlotBytes;     // [3 tiles][256] kv rows
-constexpr int kOffStat = kOffRows + 3 * kTileKeys * 4;        // [2 tile parities][4 key quarters][64 heads] row maxima / sums
-constexpr int kOffMisc = kOffStat + 2 * 4 * 64 * 4;
+constexpr int kOffStat = kOffRows + 3 * kTileKeys * 4;        // [2 tile parities][8 key parts][64 heads] row maxima / sums
+constexpr int kOffMisc = kOffStat + 2 * kParts * 64 * 4;
 constexpr int kSmemBytes = kOffMisc + 512 + 1024;             // barriers + alignment slack
 constexpr int kTmemO = 0, kTmemS = 256;
 static_assert(kSmemBytes <= 232448, "shared memory of one SM");
@@ -767,7 +772,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ff::kThreads, 1)
 smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     using namespace ff;
     constexpr int NH = HP / 2;               // heads of this CTA (of the 64 rows the UMMAs compute)
-    constexpr int kSoftmaxWarps = NH / 8;    // with 64 heads a CTA's rows 32-63 do not exist: the warps of that lane quarter idle
+    constexpr int kBusyWarps = NH / 4;       // with 64 heads a CTA's rows 32-63 do not exist: the warps of those lane quarters idle
     const uint32_t rank = cluster_ctarank();
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
@@ -782,7 +787,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     const uint32_t bar_qfree = bar_qfull + 8 * kQChunks;    // [9] the query's last UMMAs on the chunk finished
     const uint32_t bar_tfull = bar_qfree + 8 * kQChunks;    // [2] S buffer complete
     const uint32_t bar_tempty = bar_tfull + 16;             // [2] (even CTA) both CTAs have read the S buffer
-    const uint32_t bar_pfull = bar_tempty + 16;             // (even CTA) P of the tile written in both CTAs
+    const uint32_t bar_pfull = bar_tempty + 16;             // P of the tile written (even CTA: in both CTAs)
     const uint32_t bar_pv = bar_pfull + 8;                  // O += P V of the tile finished
     const uint32_t bar_drain = bar_pv + 8;                  // used only while winding down after an abort
     constexpr int kBars = 2 * kStages + 2 * kQChunks + 7;
@@ -804,9 +809,9 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(bar_tfull + 8 * i, 1);
-            mbar_init(bar_tempty + 8 * i, 2 * kSoftmaxWarps);
+            mbar_init(bar_tempty + 8 * i, 2 * kBusyWarps);
         }
-        mbar_init(bar_pfull, 2 * kSoftmaxWarps);
+        mbar_init(bar_pfull, kBusyWarps + (rank == 0 ? 1 : 0));      // + the odd CTA's forwarded arrival
         mbar_init(bar_pv, 1);
         mbar_init(bar_drain, 1);
         fence_mbar_init();
@@ -818,11 +823,11 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         }
         fence_proxy_async_smem();
     }
-    if (warp == 16) {
+    if (warp == kIssueWarp) {
         tmem_alloc_2cta(smem_u32(tmem_slot), 512);
         tmem_relinquish_2cta();
     }
-    if (warp == 17 && lane == 0) tma_prefetch_desc(&tm_q);
+    if (warp == kLoadWarp && lane == 0) tma_prefetch_desc(&tm_q);
     pdl_wait();                  // the prep kernel's slot counts
     pdl_trigger();
     const int total = find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + kOffStat), range_s);
@@ -835,9 +840,9 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     const WorkRange range = uniform_range(*range_s);
     const int n_tiles = range.end - range.begin;
 
-    if (warp >= 8 && warp < 16) {
+    if (warp >= kSoftmaxWarps && warp < kIssueWarp) {
         // ------------------------------------------------------------------ gather producers
-        const int pt = threadIdx.x - 256;   // 0..255
+        const int pt = threadIdx.x - kSoftmaxWarps * 32;   // 0..255
         const char* kvb = reinterpret_cast<const char*>(p.kv);
         const uint64_t pol_keep = l2_policy_evict_last();
         int* rows = reinterpret_cast<int*>(smem + kOffRows);
@@ -911,7 +916,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 }
             }
         }
-    } else if (warp == 17) {
+    } else if (warp == kLoadWarp) {
         // ------------------------------------------------------------------ Q chunks of this CTA's heads
         if (lane == 0) {
             const uint64_t pol_stream = l2_policy_evict_first();
@@ -927,7 +932,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 while (!it.advance()) {}
             }
         }
-    } else if (warp == 16) {
+    } else if (warp == kIssueWarp) {
         if (elect_one()) {
             if (rank == 1) {
                 // -------------------------------------------------------------- forward slot-full to the even CTA
@@ -940,6 +945,11 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     const int k_slots = n + 1 < n_tiles ? kQChunks : 0;
                     const int slots = k_slots + (n >= 0 ? kVSlots : 0);
                     for (int j = 0; j < slots; ++j) {
+                        if (j == k_slots) {          // P of tile n, in front of the V it is multiplied with
+                            mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
+                            fence_proxy_async_smem();
+                            mbar_arrive_cluster_relaxed(map_to_cta(bar_pfull, 0));
+                        }
                         // this CTA's half of Q is part of what "full" promises
                         if (j < k_slots && new_query) mbar_wait(bar_qfull + 8 * j, qpar, wc, kErrFwd + 15);
                         ring.wait(wc, kErrFwd + 17);
@@ -1027,27 +1037,24 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             }
         }
     } else if ((warp & 1) * 32 < NH) {
-        // ------------------------------------------------------------------ softmax (one head, 64 keys of the tile per thread)
-        const int quarter = warp & 3, ch = warp >> 2;
-        const int part = (quarter >> 1) * 2 + ch;                // which 64 keys of the tile: its 64-key chunk of P
+        // ------------------------------------------------------------------ softmax (one head, 32 keys of the tile per thread)
+        const int quarter = warp & 3, cg = warp >> 2;
+        const int part = (quarter >> 1) * 4 + cg;                // which 32 keys of the tile
         const int row = (quarter & 1) * 32 + lane;               // head row of this CTA
         const int head = static_cast<int>(rank) * NH + row;
         const bool real = head < p.h_q;
         const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
-        const uint32_t tempty0 = map_to_cta(bar_tempty, 0), pfull0 = map_to_cta(bar_pfull, 0);
-        const uint32_t p_row = s_base + kOffP + part * kPChunk + row * 128;
-        const int bar_id = 1 + (quarter & 1);                    // the four warps that share 32 rows
-        float* stat = reinterpret_cast<float*>(smem + kOffStat);
+        const uint32_t tempty0 = map_to_cta(bar_tempty, 0);
+        const uint32_t p_row = s_base + kOffP + (part >> 1) * kPChunk + row * 128;
+        const int bar_id = 1 + (quarter & 1);                    // the eight warps that share 32 rows
+        float* stat = reinterpret_cast<float*>(smem + kOffStat) + row;
         const float ninf = __int_as_float(0xff800000);
         TileIter<1> it(p, range);
         QMeta qm = load_qmeta(p, range.q);
-        // which of the warp's 64 keys are valid: one bit per key, loaded a tile ahead
-        int idx0 = -1, idx1 = -1;
+        int idx = -1;                        // of the lane's key, loaded a tile ahead
         auto load_idx = [&]() {
-            const int key = it.tile() * kTileKeys + part * 64 + lane;
-            const int32_t* src = p.indices + static_cast<size_t>(it.q) * p.topk + key;
-            idx0 = it.more() && key < p.topk ? __ldg(src) : -1;
-            idx1 = it.more() && key + 32 < p.topk ? __ldg(src + 32) : -1;
+            const int key = it.tile() * kTileKeys + part * 32 + lane;
+            idx = it.more() && key < p.topk ? __ldg(p.indices + static_cast<size_t>(it.q) * p.topk + key) : -1;
         };
         load_idx();
         bool new_query = true;
@@ -1060,39 +1067,40 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         // o may start at any multiple of 16 bytes; where it is one of 32 it leaves in 32-byte stores (4096 queries x 128 heads x
         // top-k 256: 488 us, 565 us in 16-byte stores)
         const bool wide_o = (reinterpret_cast<uintptr_t>(p.gout) & 31) == 0;
+        const uint32_t o_cols = tmem + lanes + kTmemO + cg * 32;         // this warp's 32 columns of either d-block
         auto write_out = [&]() {
             pending = false;
             // lanes 0-63: columns [256 block, + 128), lanes 64-127: [256 block + 128, + 128)
 #pragma unroll 1
-            for (int c = 0; c < 8; ++c) {
-                const int blk = c >> 2, e = (c & 3) * 16;
-                uint32_t o[16];
-                tmem_ld_32x16(tmem + lanes + kTmemO + blk * 128 + ch * 64 + e, o);
+            for (int blk = 0; blk < 2; ++blk) {
+                uint32_t o[32];
+                tmem_ld_32x32(o_cols + blk * 128, o);
                 tmem_ld_wait();
-                const size_t at = pend_row * kDV + blk * 256 + (quarter >> 1) * 128 + ch * 64 + e;
+                const size_t at = pend_row * kDV + blk * 256 + (quarter >> 1) * 128 + cg * 32;
                 if (real && pend_whole) {
-                    uint32_t w[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        w[i] = pack_bf16x2(__uint_as_float(o[2 * i]) * pend_inv, __uint_as_float(o[2 * i + 1]) * pend_inv);
-                    if (wide_o) {
-                        st_global_v8(p.gout + at, w);
-                    } else {
+                    for (int e = 0; e < 2; ++e) {
+                        uint32_t w[8];
 #pragma unroll
-                        for (int v = 0; v < 2; ++v)
-                            *reinterpret_cast<uint4*>(p.gout + at + 8 * v) = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+                        for (int i = 0; i < 8; ++i)
+                            w[i] = pack_bf16x2(__uint_as_float(o[16 * e + 2 * i]) * pend_inv, __uint_as_float(o[16 * e + 2 * i + 1]) * pend_inv);
+                        if (wide_o) {
+                            st_global_v8(p.gout + at + 16 * e, w);
+                        } else {
+#pragma unroll
+                            for (int v = 0; v < 2; ++v)
+                                *reinterpret_cast<uint4*>(p.gout + at + 16 * e + 8 * v) = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+                        }
                     }
                 } else if (real) {
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) st_global_v8(p.part_o + at + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
+                    for (int v = 0; v < 4; ++v) st_global_v8(p.part_o + at + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
                 }
             }
         };
         int seg_begin = 0;
         for (int n = 0; n < n_tiles; ++n) {
-            const int key = it.tile() * kTileKeys + part * 64 + lane;
-            const uint32_t mask0 = __ballot_sync(0xffffffffu, slot_valid(idx0, key, qm, p));
-            const uint32_t mask1 = __ballot_sync(0xffffffffu, slot_valid(idx1, key + 32, qm, p));
+            const uint32_t mask = __ballot_sync(0xffffffffu, slot_valid(idx, it.tile() * kTileKeys + part * 32 + lane, qm, p));
             if (new_query) {
                 ref = ninf;
                 sum = 0.f;
@@ -1108,34 +1116,32 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             const int b = n & 1;
             mbar_wait(bar_tfull + 8 * b, (n >> 1) & 1, wc, kErrFwd + 18, kPollSleepNs);
             tc_fence_after_sync();
-            uint32_t sv[64];
-            tmem_ld_32x32(tmem + lanes + kTmemS + b * 128 + ch * 64, *reinterpret_cast<uint32_t(*)[32]>(sv));
-            tmem_ld_32x32(tmem + lanes + kTmemS + b * 128 + ch * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(sv + 32));
+            uint32_t sv[32];
+            tmem_ld_32x32(tmem + lanes + kTmemS + b * 128 + cg * 32, sv);
             tmem_ld_wait();
             tc_fence_before_sync();
             __syncwarp();
             // the S buffer has been read (tcgen05.wait::ld), which is all the issuer needs to know
             if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * b);
-            if ((mask0 & mask1) != 0xffffffffu) {            // warp-uniform
+            if (mask != 0xffffffffu) {                       // warp-uniform
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    if (!((mask0 >> i) & 1u)) sv[i] = 0xff800000u;
-                    if (!((mask1 >> i) & 1u)) sv[32 + i] = 0xff800000u;
-                }
+                for (int i = 0; i < 32; ++i)
+                    if (!((mask >> i) & 1u)) sv[i] = 0xff800000u;
             }
             float m[4] = {ninf, ninf, ninf, ninf};
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
+            for (int i = 0; i < 32; i += 4) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) m[k] = fmaxf(m[k], __uint_as_float(sv[i + k]));
             }
-            stat[(b * 4 + part) * 64 + row] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
-            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+            stat[(b * kParts + part) * 64] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+            asm volatile("bar.sync %0, 256;" ::"r"(bar_id) : "memory");
             float scale_o = 1.f;
             bool rescale = false;
-            uint32_t pk[32];
-            const float* st = stat + b * 4 * 64 + row;
-            const float top = fmaxf(fmaxf(st[0], st[64]), fmaxf(st[128], st[192])) * p.scale_log2e;
+            float top = ninf;
+#pragma unroll
+            for (int i = 0; i < kParts; ++i) top = fmaxf(top, stat[(b * kParts + i) * 64]);
+            top *= p.scale_log2e;
             if (top > ref) {             // (first valid tile: O and the sum are still empty)
                 rescale = ref > ninf;
                 if (rescale) scale_o = ex2_approx(ref - top);
@@ -1144,8 +1150,9 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             const float neg = ref == ninf ? 0.f : -ref;
             sum *= scale_o;
             float add[2] = {0.f, 0.f};
+            uint32_t pk[16];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
+            for (int i = 0; i < 16; ++i) {
                 const float x = ex2_approx(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2e, neg));
                 const float y = ex2_approx(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2e, neg));
                 add[0] += x;
@@ -1156,39 +1163,38 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             // P of the previous tile has been consumed and O is at rest
             if (n > 0) mbar_wait(bar_pv, (n - 1) & 1, wc, kErrFwd + 20, kPollSleepNs);
             tc_fence_after_sync();
-            if (pending) write_out();
-            if (__any_sync(0xffffffffu, rescale)) {          // this warp's half of the columns of both d-blocks
-#pragma unroll 1
-                for (int c = 0; c < 256; c += 128) {
-#pragma unroll 1
-                    for (int e = 0; e < 64; e += 16) {
-                        const uint32_t at = tmem + lanes + kTmemO + c + ch * 64 + e;
-                        uint32_t o[16];
-                        tmem_ld_32x16(at, o);
-                        tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale_o);
-                        tmem_st_32x16(at, o);
-                    }
+            for (int u = 0; u < 4; ++u)
+                st_shared_v4(p_row + ((((part & 1) * 4 + u) ^ (row & 7)) << 4), pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
+            fence_proxy_async_smem();
+            if (pending) write_out();
+            if (__any_sync(0xffffffffu, rescale)) {          // this warp's quarter of the columns of both d-blocks
+#pragma unroll 1
+                for (int blk = 0; blk < 2; ++blk) {
+                    uint32_t o[32];
+                    tmem_ld_32x32(o_cols + blk * 128, o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale_o);
+                    tmem_st_32x32(o_cols + blk * 128, o);
                 }
                 tmem_st_wait();
             }
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                st_shared_v4(p_row + ((u ^ (row & 7)) << 4), pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
-            fence_proxy_async_smem();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_release(pfull0);
+            // Local arrival, forwarded by the odd CTA's relay thread: a cluster-scope release costs hundreds of cycles a tile.
+            if (lane == 0) mbar_arrive(bar_pfull);
 
             if (last) {
                 // ---- the query's (or the range's) last tile: lse now, o once its P V is done - or an unnormalised part of them
                 const bool whole = seg_begin == q_lo && seg_end == q_hi;
-                stat[(4 * ((n + 1) & 1) + part) * 64 + row] = sum;
-                asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-                const float* sums = stat + 4 * ((n + 1) & 1) * 64 + row;
-                const float total = (sums[0] + sums[64]) + (sums[128] + sums[192]);
-                asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // the next tile's maxima go to the same place
+                float* sums = stat + kParts * ((n + 1) & 1) * 64;
+                sums[part * 64] = sum;
+                asm volatile("bar.sync %0, 256;" ::"r"(bar_id) : "memory");
+                float total = 0.f;
+#pragma unroll
+                for (int i = 0; i < kParts; ++i) total += sums[i * 64];
+                asm volatile("bar.sync %0, 256;" ::"r"(bar_id) : "memory");      // the next tile's maxima go to the same place
                 const size_t orow = static_cast<size_t>(qg) * p.h_q + head;
                 // partial results: slot 2 c for a range that starts inside the query, 2 c + 1 for one that starts at or before it
                 const size_t prow = static_cast<size_t>((blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0)) * HP + head;
@@ -1213,7 +1219,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // neither CTA leaves while the other may still signal it or read its operands
-    if (warp == 16) tmem_dealloc_2cta(tmem, 512);
+    if (warp == kIssueWarp) tmem_dealloc_2cta(tmem, 512);
 }
 
 // Queries whose tiles were spread over several clusters: o = sum of 2^(ref_i - ref) O_i over the parts, divided by the sum
