@@ -426,6 +426,27 @@ __device__ __forceinline__ void st_global_v8(void* addr, const uint32_t (&v)[8])
                  : "memory");
 }
 
+// (read once, written by the kernel before: not through L1)
+__device__ __forceinline__ void ld_global_v8(const void* addr, uint32_t (&v)[8]) {
+    asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(addr)
+                 : "memory");
+}
+// Barrier of `threads` threads of the block that also tells whether `v` was true in any of them.
+__device__ __forceinline__ bool bar_or(int id, int threads, bool v) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(static_cast<uint32_t>(v)), "r"(id), "r"(threads)
+        : "memory");
+    return any != 0;
+}
+
 // ---- small helpers -----------------------------------------------------------------------------
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;

@@ -460,6 +460,11 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 
+// No cluster has more than one tile, whatever the indices are (KParams::every_slot).
+bool at_most_a_tile_each(int queries, int tiles_per_query, int clusters) {
+    return static_cast<long long>(queries) * tiles_per_query <= clusters;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---- forward ---------------------------------------------------------------------------------------------
@@ -537,17 +542,19 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     kp.wait_limit = g_wait_limit.load();
     kp.q0 = 0;
     kp.nq = p->s_q;
-    launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, static_cast<const uint4*>(nullptr), static_cast<const uint4*>(nullptr),
-           static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), static_cast<uint4*>(nullptr), size_t(0), 1, kp);
     const int pairs = resident_pairs(smla_fwd_kernel<HP>, ff::kThreads, ff::kSmemBytes);
     if (pairs <= 0) return SMLA_ERR_LAUNCH;
     const int clusters = std::max(1, std::min(pairs, pl.clusters));
+    const int q_tiles = pl.topk_pad / kWorkTileKeys;
+    if (at_most_a_tile_each(p->s_q, q_tiles, clusters))
+        kp.every_slot = p->topk;
+    else
+        launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, static_cast<const uint4*>(nullptr), static_cast<const uint4*>(nullptr),
+               static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), static_cast<uint4*>(nullptr), size_t(0), 1, kp);
     launch(smla_fwd_kernel<HP>, 2 * clusters, ff::kThreads, ff::kSmemBytes, st, true, 1, tm_q, kp);
-    if (clusters > 1) {
-        if (p->s_q < clusters)
-            launch(smla_fwd_combine_kernel<1>, p->s_q * ((p->h_q + 3) / 4), 256, 0, st, true, 1, kp, clusters, HP);
-        else
-            launch(smla_fwd_combine_kernel<4>, (clusters - 1) * ((p->h_q + 15) / 16), 256, 0, st, true, 1, kp, clusters, HP);
+    if (clusters > 1 && (!kp.every_slot || q_tiles > 1)) {
+        const int items = p->s_q < clusters ? p->s_q : clusters - 1;
+        launch(smla_fwd_combine_kernel, items * ((p->h_q + 31) / 32 * 4), 256, 0, st, true, 1, kp, clusters, HP);
     }
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }

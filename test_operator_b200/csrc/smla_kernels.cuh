@@ -61,7 +61,8 @@ struct KParams {
     const int4* qmeta;        // optional per query {first kv row of its sequence, kv rows of its sequence,
                               // position for the causal rule, top-k slots in use}; null: one sequence
     long long wait_limit;     // cycles a bounded wait may take
-    int early_start;          // dkv, dq: launched behind the trigger of the kernel before in the same call (see there)
+    int early_start;          // launched behind the trigger of the kernel before in the same call (see the kernels)
+    int every_slot;           // > 0 (topk): count every slot of every query as used and do not read n_used (slots_used)
 };
 
 // What a query may attend to: rows [kv_base, kv_base + kv_len) of kv, index values relative to kv_base.
@@ -268,13 +269,21 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 // many equal contiguous ranges as there are clusters: every cluster gets the same number of tiles (4096 queries of eight
 // tiles over 74 clusters as whole queries would be 56 queries for some and 55 for the others), a few long queries
 // spread over the whole chip, and tiles without a valid slot do not exist.  kMul: tiles of 256 / kMul keys.
+//
+// A call whose queries have no more tiles than there are clusters takes as long as one tile takes, whether or not some of the
+// tiles are empty.  There the ranges are cut as if every slot were in use (every_slot): nothing has to look at the indices
+// first, which saves the forward its prep kernel: eight queries x 128 heads x top-k 2048 25.1 -> 19.5 us a call (prep kernel,
+// its hand-over and the 5700 cycles that the ranges took from its counts; 128 blocks with one tile each either way).  From the
+// next tile on some cluster has two, and an empty tile would cost as much as a full one.
+__device__ __forceinline__ int slots_used(const KParams& p, int q) { return p.every_slot ? p.every_slot : __ldcg(p.n_used + q); }
 struct WorkRange {
     int begin, end;               // positions among the launch's tiles
     int q, lo;                    // the query `begin` lies in; position of its first tile
 };
 __device__ __forceinline__ int work_tiles(int n_used) { return (n_used + kWorkTileKeys - 1) / kWorkTileKeys; }
-__device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clusters) {
-    return static_cast<int>(static_cast<long long>(n_tiles) * cluster / n_clusters);
+__device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clusters) {     // n_tiles * cluster / n_clusters in 32 bits
+    const uint32_t n = n_tiles, c = cluster, m = n_clusters;
+    return static_cast<int>(n / m * c + n % m * c / m);
 }
 // Which range is this cluster's; called by the whole block, which passes a barrier before it reads *out.  Every block adds up
 // the slot counts itself (a few per thread: 8192 queries are 32 KB out of L2, all in flight at once), so that the ranges need
@@ -282,6 +291,12 @@ __device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clust
 // scratch: one word of shared memory per warp.  Returns, in the one thread that wrote *out, the launch's tiles; -1 in the others.
 template <int kThreads>
 __device__ __forceinline__ int find_range(const KParams& p, int cluster, int n_clusters, int* scratch, WorkRange* out) {
+    if (p.every_slot) {
+        if (threadIdx.x != 0) return -1;
+        const int tiles = work_tiles(p.every_slot), total = p.nq * tiles, begin = range_start(total, cluster, n_clusters);
+        *out = WorkRange{begin, range_start(total, cluster + 1, n_clusters), p.q0 + begin / tiles, begin / tiles * tiles};
+        return total;
+    }
     const int* used = p.n_used + p.q0;
     const int per = (p.nq + kThreads - 1) / kThreads;          // consecutive queries of a thread
     const int i0 = min(static_cast<int>(threadIdx.x) * per, p.nq), i1 = min(i0 + per, p.nq);
@@ -305,19 +320,21 @@ __device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
 }
 template <int kMul> struct TileIter {
     const int* used;
+    int every_slot;               // KParams::every_slot
     int q, q_last, lo, hi, pos, end;
     int stop;                     // behind the query's last tile with a slot in use (kMul 2: hi or hi - 1)
     int n_cur, n_next;            // slots in use of queries q and q + 1 (one query ahead: the load is done when it is needed)
     __device__ __forceinline__ TileIter(const KParams& p, const WorkRange& w)
-        : used(p.n_used), q(w.q), q_last(p.q0 + p.nq), lo(w.lo * kMul), pos(w.begin * kMul), end(w.end * kMul) {
-        n_next = __ldcg(used + q);
+        : used(p.n_used), every_slot(p.every_slot), q(w.q), q_last(p.q0 + p.nq), lo(w.lo * kMul), pos(w.begin * kMul), end(w.end * kMul) {
+        n_next = slots(q);
         open_query();
     }
+    __device__ __forceinline__ int slots(int query) const { return every_slot ? every_slot : __ldcg(used + query); }
     __device__ __forceinline__ void open_query() {
         n_cur = n_next;
         hi = lo + work_tiles(n_cur) * kMul;
         stop = kMul > 1 ? lo + (n_cur + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul) : hi;
-        n_next = __ldcg(used + min(q + 1, q_last - 1));
+        n_next = slots(min(q + 1, q_last - 1));
     }
     __device__ __forceinline__ bool more() const { return pos < end; }
     __device__ __forceinline__ int tile() const { return pos - lo; }
@@ -617,7 +634,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         for (TileIter<1> it(p, range); it.more(); new_query = it.advance(), ++gt) {
             const int qg = it.q, tile = it.tile();
             if (new_query) {
-                n_used = __ldcg(p.n_used + qg);
+                n_used = slots_used(p, qg);
                 qm = load_qmeta(p, qg);
                 if (stat_q != qg) stat_next = load_stat(qg);       // queries without a valid slot lay in between
                 asm volatile("bar.sync 1, 256;" ::: "memory");      // every softmax warp is done with the previous query
@@ -767,6 +784,10 @@ __device__ __forceinline__ float row_lse(float ref, float sum) {
     return ref == inf ? inf : ref + __log2f(sum);
 }
 
+// lse of a query without a valid slot, and the row sum that marks partial results without one (a sum is never negative).
+__device__ __forceinline__ float no_slot_lse(const KParams& p) { return __int_as_float(0x7f800000) * p.lse_out_mult; }
+constexpr float kNoSlot = -1.f;
+
 template <int HP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ff::kThreads, 1)
 smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
@@ -828,10 +849,12 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         tmem_relinquish_2cta();
     }
     if (warp == kLoadWarp && lane == 0) tma_prefetch_desc(&tm_q);
-    pdl_wait();                  // the prep kernel's slot counts
-    pdl_trigger();
+    if (!p.every_slot) {
+        pdl_wait();              // the prep kernel's slot counts
+        pdl_trigger();
+    }
     const int total = find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + kOffStat), range_s);
-    if (total >= 0 && rank == 0) p.range_q[blockIdx.x >> 1] = make_int4(range_s->q, range_s->lo, total, 0);
+    if (total >= 0 && rank == 0 && !p.every_slot) p.range_q[blockIdx.x >> 1] = make_int4(range_s->q, range_s->lo, total, 0);
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
@@ -839,6 +862,10 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
     const int n_tiles = range.end - range.begin;
+    if (p.every_slot) {          // nothing of the caller's has been touched so far
+        pdl_wait();
+        pdl_trigger();
+    }
 
     if (warp >= kSoftmaxWarps && warp < kIssueWarp) {
         // ------------------------------------------------------------------ gather producers
@@ -1059,11 +1086,12 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         load_idx();
         bool new_query = true;
         float ref = ninf, sum = 0.f;         // reference of the row's exponentials (log2 units), sum over this thread's keys
+        bool any_valid = false;              // the query has had a valid slot (only every_slot gives tiles to one that has none)
         // A query's O leaves when the next tile's exponentials are done: waiting for the last P V right behind its P held
         // up the next query's softmax, and the tensor pipe with it, by about 4000 cycles a query.
         bool pending = false, pend_whole = false;
         float pend_inv = 0.f;
-        size_t pend_row = 0;
+        size_t pend_row = 0;                 // row of o, or slot of the partial results
         // o may start at any multiple of 16 bytes; where it is one of 32 it leaves in 32-byte stores (4096 queries x 128 heads x
         // top-k 256: 488 us, 565 us in 16-byte stores)
         const bool wide_o = (reinterpret_cast<uintptr_t>(p.gout) & 31) == 0;
@@ -1076,7 +1104,8 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 uint32_t o[32];
                 tmem_ld_32x32(o_cols + blk * 128, o);
                 tmem_ld_wait();
-                const size_t at = pend_row * kDV + blk * 256 + (quarter >> 1) * 128 + cg * 32;
+                const int col = blk * 256 + (quarter >> 1) * 128 + cg * 32;
+                const size_t at = pend_row * kDV + col;
                 if (real && pend_whole) {
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
@@ -1094,7 +1123,8 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     }
                 } else if (real) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) st_global_v8(p.part_o + at + 8 * v, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
+                    for (int v = 0; v < 4; ++v)      // [slot][8 columns][heads]: a warp's store is 1 KB in one piece
+                        st_global_v8(p.part_o + ((pend_row * (kDV / 8) + (col >> 3) + v) * HP + head) * 8, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * v));
                 }
             }
         };
@@ -1104,6 +1134,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             if (new_query) {
                 ref = ninf;
                 sum = 0.f;
+                any_valid = false;
                 seg_begin = it.pos;
             }
             const int qg = it.q, q_lo = it.lo, q_hi = it.hi;
@@ -1135,7 +1166,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 for (int k = 0; k < 4; ++k) m[k] = fmaxf(m[k], __uint_as_float(sv[i + k]));
             }
             stat[(b * kParts + part) * 64] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
-            asm volatile("bar.sync %0, 256;" ::"r"(bar_id) : "memory");
+            any_valid = bar_or(bar_id, 256, mask != 0u) || any_valid;
             float scale_o = 1.f;
             bool rescale = false;
             float top = ninf;
@@ -1197,15 +1228,15 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 asm volatile("bar.sync %0, 256;" ::"r"(bar_id) : "memory");      // the next tile's maxima go to the same place
                 const size_t orow = static_cast<size_t>(qg) * p.h_q + head;
                 // partial results: slot 2 c for a range that starts inside the query, 2 c + 1 for one that starts at or before it
-                const size_t prow = static_cast<size_t>((blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0)) * HP + head;
+                const size_t slot = (blockIdx.x >> 1) * 2 + (seg_begin == q_lo ? 1 : 0);
                 if (real && part == 0) {
-                    if (whole) p.lse_out[orow] = row_lse(ref, total) * p.lse_out_mult;
-                    else p.part_ml[prow] = make_float2(ref, total);
+                    if (whole) p.lse_out[orow] = any_valid ? row_lse(ref, total) * p.lse_out_mult : no_slot_lse(p);
+                    else p.part_ml[slot * HP + head] = make_float2(ref, any_valid ? total : kNoSlot);
                 }
                 pending = true;
                 pend_whole = whole;
-                pend_inv = 1.f / total;
-                pend_row = whole ? orow : prow;
+                pend_inv = any_valid ? 1.f / total : 0.f;        // no valid slot: O is 0
+                pend_row = whole ? orow : slot;
             }
             new_query = next_query;
         }
@@ -1225,116 +1256,104 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 // Queries whose tiles were spread over several clusters: o = sum of 2^(ref_i - ref) O_i over the parts, divided by the sum
 // of their weighted row sums.  The items are the queries where there are at most as many as boundaries between ranges, else
 // the boundaries (the one that is its query's first does the work; the forward kernel has noted each range's first
-// query).  One warp per (item, kHeads heads, half of the columns): lane i takes the references and sums of part i, all
-// weights are known before the first row of O is loaded, and the rows are added in the order of the parts.  Bound by the
-// latency of its dependent rounds of loads: eight tokens of eight parts each 20 us with a block per boundary and a round
-// per part, 7.6 us so (kHeads 1); 94 queries over 73 boundaries 35 us with a search of the query in every block and a
-// warp per head, 15 us so (kHeads 4).
-template <int kHeads>
-__global__ void __launch_bounds__(256, 4) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
+// query).  A lane takes one head and sixteen columns: the parts lie as [8 columns][heads][8], so a warp loads a part in pieces of
+// 1 KB, and a lane's weights need no other lane.  The first parts' O is asked for together with all references and sums.
+// Parts are added in their order.  Bound by the latency of its dependent loads; eight queries of eight parts: 5.5 us of a call,
+// 7.6 us with a warp per head and half of the columns, whose weights took two rounds of loads before the first row.
+constexpr int kCombineFly = 4;                   // parts in flight
+__global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
     pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const int per_item = (p.h_q + 4 * kHeads - 1) / (4 * kHeads);
-    const int item = static_cast<int>(blockIdx.x) / per_item;
-    const int head0 = (static_cast<int>(blockIdx.x) % per_item * 4 + (threadIdx.x >> 6)) * kHeads;
-    const int half = (threadIdx.x >> 5) & 1;
-    if (head0 >= p.h_q) return;
-    const bool by_query = p.nq < n_clusters;
-    const int4 boundary = __ldcg(p.range_q + (by_query ? 0 : item + 1));
-    const int q = by_query ? p.q0 + item : boundary.x, n_tiles = boundary.z;
-    int q_begin = boundary.y;
-    if (by_query) {                              // (fewer queries than clusters: at most three of them per lane)
-        q_begin = 0;
-        for (int i = lane; i < item; i += 32) q_begin += work_tiles(__ldcg(p.n_used + p.q0 + i));
-        q_begin = __reduce_add_sync(0xffffffffu, q_begin);
+    const int per_item = (p.h_q + 31) / 32 * 4;  // blocks: eight of the 32 column groups each
+    const int item = static_cast<int>(blockIdx.x) / per_item, in_item = static_cast<int>(blockIdx.x) % per_item;
+    const int head = in_item / 4 * 32 + lane, col = (in_item % 4 * 8 + static_cast<int>(threadIdx.x >> 5)) * 16;
+    int q, n_tiles, q_begin, q_end;
+    if (p.every_slot) {
+        const int tiles = work_tiles(p.every_slot);
+        q = p.q0 + item;
+        n_tiles = p.nq * tiles;
+        q_begin = item * tiles;
+        q_end = q_begin + tiles;
+    } else {
+        const bool by_query = p.nq < n_clusters;
+        const int4 boundary = __ldcg(p.range_q + (by_query ? 0 : item + 1));
+        q = by_query ? p.q0 + item : boundary.x;
+        n_tiles = boundary.z;
+        q_begin = boundary.y;
+        if (by_query) {                          // (fewer queries than clusters: at most three of them per lane)
+            q_begin = 0;
+            for (int i = lane; i < item; i += 32) q_begin += work_tiles(__ldcg(p.n_used + p.q0 + i));
+            q_begin = __reduce_add_sync(0xffffffffu, q_begin);
+        }
+        q_end = q_begin + work_tiles(__ldcg(p.n_used + q));
+        if (q_begin >= q_end) return;            // no valid slot: the prep kernel has written o and lse
     }
-    const int q_end = q_begin + work_tiles(__ldcg(p.n_used + q));
-    if (q_begin >= q_end) return;                // no valid slot: the prep kernel has written o and lse
-    // the cluster whose range holds the query's first tile: the largest k with range_start(k) <= q_begin
+    // the clusters whose ranges hold a tile t: the largest k with range_start(k) <= t
     const int first = static_cast<int>((static_cast<long long>(q_begin + 1) * n_clusters - 1) / n_tiles);
-    if (range_start(n_tiles, first + 1, n_clusters) >= q_end || (!by_query && first != item)) return;
+    const int last = static_cast<int>((static_cast<long long>(q_end) * n_clusters - 1) / n_tiles);
+    if (first == last || (!p.every_slot && p.nq >= n_clusters && first != item)) return;
+    if (head >= p.h_q) return;
+    // part k: its slot, -1 where the range is empty
+    auto slot_of = [&](int k) {
+        const int begin = range_start(n_tiles, k, n_clusters);
+        return begin == range_start(n_tiles, k + 1, n_clusters) ? -1 : 2 * k + (begin <= q_begin ? 1 : 0);
+    };
+    auto load_part = [&](int k, uint32_t (&v)[2][8], float2& ml) {
+        const int slot = k <= last ? slot_of(k) : -1;
+        ml = make_float2(__int_as_float(0xff800000), kNoSlot);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i / 8][i % 8] = 0u;
+        if (slot >= 0) {
+            const float* o = p.part_o + ((static_cast<size_t>(slot) * (kDV / 8) + (col >> 3)) * h_pad + head) * 8;
+            ml = __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head);
+            ld_global_v8(o, v[0]);
+            ld_global_v8(o + h_pad * 8, v[1]);
+        }
+    };
     const float ninf = __int_as_float(0xff800000);
-    float ref[kHeads], sum[kHeads], acc[kHeads][8];
+    uint32_t v[kCombineFly][2][8];
+    float2 ml[kCombineFly];
 #pragma unroll
-    for (int h = 0; h < kHeads; ++h) {
-        ref[h] = ninf;
-        sum[h] = 0.f;
+    for (int u = 0; u < kCombineFly; ++u) load_part(first + u, v[u], ml[u]);
+    float ref = ninf, sum = 0.f, acc[16];
+    bool any = false;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[h][i] = 0.f;
+    for (int u = 0; u < kCombineFly; ++u) {
+        ref = fmaxf(ref, ml[u].x);               // -inf: no valid slot in this part, or none above -inf
+        any = any || ml[u].y != kNoSlot;
     }
-    for (int k0 = first; k0 < n_clusters; k0 += 32) {          // 32 parts at a time
-        const int k = k0 + lane;
-        const int begin = k < n_clusters ? range_start(n_tiles, k, n_clusters) : n_tiles;
-        const bool part = k < n_clusters && begin < q_end && begin < range_start(n_tiles, k + 1, n_clusters);
-        const size_t row = static_cast<size_t>(2 * k + (begin <= q_begin ? 1 : 0)) * h_pad + head0;
-        float2 ml[kHeads];
+    for (int k = first + kCombineFly; k <= last; ++k) {
+        const int slot = slot_of(k);
+        if (slot < 0) continue;
+        const float2 x = __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head);
+        ref = fmaxf(ref, x.x);
+        any = any || x.y != kNoSlot;
+    }
 #pragma unroll
-        for (int h = 0; h < kHeads; ++h)
-            ml[h] = part && head0 + h < p.h_q ? __ldcg(p.part_ml + row + h) : make_float2(ninf, 0.f);
-        float weight[kHeads];
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+    for (int k = first;;) {
 #pragma unroll
-        for (int h = 0; h < kHeads; ++h) {
-            const float m = ml[h].x;                             // -inf: no valid slot in this part, or none above -inf
-            float top = m;
+        for (int u = 0; u < kCombineFly; ++u) {
+            const float w = ml[u].x > ninf ? ex2_approx(ml[u].x - ref) : 0.f;
+            sum = fmaf(w, ml[u].y, sum);
+            // (a part of weight 0 counts too: its O may hold a NaN)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            top = fmaxf(top, ref[h]);
-            weight[h] = m > ninf ? ex2_approx(m - top) : 0.f;
-            const float keep = ref[h] > ninf ? ex2_approx(ref[h] - top) : 0.f;
-            sum[h] = sum[h] * keep + warp_sum(weight[h] * ml[h].y);
-            ref[h] = top;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[h][i] *= keep;
+            for (int i = 0; i < 16; ++i) acc[i] = fmaf(__uint_as_float(v[u][i / 8][i % 8]), w, acc[i]);
         }
-        uint32_t todo = __ballot_sync(0xffffffffu, part);
-        const float* mine = p.part_o + row * kDV + half * (kDV / 2);
-        constexpr int kFly = 4 / kHeads;                       // parts in flight (times kHeads rows of 1 KB)
-        while (todo) {
-            float4 v[kFly][kHeads][2];
-            float wt[kFly][kHeads];
+        k += kCombineFly;
+        if (k > last) break;
 #pragma unroll
-            for (int u = 0; u < kFly; ++u) {
-                const bool live = todo != 0;
-                const int src = live ? __ffs(todo) - 1 : 0;
-                const float4* o = reinterpret_cast<const float4*>(
-                    reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), src))) + lane;
-#pragma unroll
-                for (int h = 0; h < kHeads; ++h) {
-                    wt[u][h] = __shfl_sync(0xffffffffu, weight[h], src);
-                    // (a part of weight 0 counts too: its O may hold a NaN)
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        v[u][h][i] = live ? __ldcg(o + h * (kDV / 4) + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                todo &= todo - 1;
-            }
-#pragma unroll
-            for (int u = 0; u < kFly; ++u)
-#pragma unroll
-                for (int h = 0; h < kHeads; ++h)
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        acc[h][4 * i] = fmaf(v[u][h][i].x, wt[u][h], acc[h][4 * i]);
-                        acc[h][4 * i + 1] = fmaf(v[u][h][i].y, wt[u][h], acc[h][4 * i + 1]);
-                        acc[h][4 * i + 2] = fmaf(v[u][h][i].z, wt[u][h], acc[h][4 * i + 2]);
-                        acc[h][4 * i + 3] = fmaf(v[u][h][i].w, wt[u][h], acc[h][4 * i + 3]);
-                    }
-        }
-        if (__shfl_sync(0xffffffffu, begin, 31) >= q_end) break;
+        for (int u = 0; u < kCombineFly; ++u) load_part(k + u, v[u], ml[u]);
     }
+    const size_t orow = static_cast<size_t>(q) * p.h_q + head;
+    if (col == 0) p.lse_out[orow] = any ? row_lse(ref, sum) * p.lse_out_mult : no_slot_lse(p);
+    const float inv = any ? 1.f / sum : 0.f;
+    uint4* out = reinterpret_cast<uint4*>(p.gout + orow * kDV + col);
 #pragma unroll
-    for (int h = 0; h < kHeads; ++h) {
-        if (head0 + h >= p.h_q) break;
-        const float inv = 1.f / sum[h];
-        const size_t orow = static_cast<size_t>(q) * p.h_q + head0 + h;
-        if (lane == 0 && half == 0)
-            p.lse_out[orow] = row_lse(ref[h], sum[h]) * p.lse_out_mult;
-        uint2* out = reinterpret_cast<uint2*>(p.gout + orow * kDV + half * (kDV / 2)) + lane;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            out[32 * i] = make_uint2(pack_bf16x2(acc[h][4 * i] * inv, acc[h][4 * i + 1] * inv),
-                                     pack_bf16x2(acc[h][4 * i + 2] * inv, acc[h][4 * i + 3] * inv));
-    }
+    for (int i = 0; i < 2; ++i)
+        out[i] = make_uint4(pack_bf16x2(acc[8 * i] * inv, acc[8 * i + 1] * inv), pack_bf16x2(acc[8 * i + 2] * inv, acc[8 * i + 3] * inv),
+                            pack_bf16x2(acc[8 * i + 4] * inv, acc[8 * i + 5] * inv), pack_bf16x2(acc[8 * i + 6] * inv, acc[8 * i + 7] * inv));
 }
 
 // =============================================================================================
@@ -1824,7 +1843,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     // waited for the recompute kernel), so its CTAs fill whatever SMs the dKV kernel leaves; the last CTA then holds the
     // grid open until the dKV kernel is done, so that "dq done" still means "all done" to whatever follows.
     if (!p.early_start) pdl_wait();
-    const int n_all = __shfl_sync(0xffffffffu, (__ldcg(p.n_used + qg) + kTileKeys - 1) / kTileKeys, 0);
+    const int n_all = __shfl_sync(0xffffffffu, (slots_used(p, qg) + kTileKeys - 1) / kTileKeys, 0);
     const int tile0 = n_all * z / nz, n_tiles = n_all * (z + 1) / nz - tile0;
 
     if (warp >= 4 && warp < 12) {
