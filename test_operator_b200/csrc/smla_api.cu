@@ -309,6 +309,11 @@ int resident_pairs(K kernel, int threads, int smem_bytes) {
     return n;
 }
 
+// No cluster has more than one tile, whatever the indices are (KParams::every_slot).
+bool at_most_a_tile_each(int queries, int tiles_per_query, int clusters) {
+    return static_cast<long long>(queries) * tiles_per_query <= clusters;
+}
+
 template <int HP>
 int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStream_t st, int stages, bool allow_overlap,
                  const smla_bwd_det_params* det = nullptr) {
@@ -388,9 +393,11 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     const int pairs_d = resident_pairs(smla_dkv_pair_kernel<HP>, dp::kThreads, dp::Cfg<HP>::kSmemBytes);
     if (pairs_r <= 0 || pairs_d <= 0) return SMLA_ERR_LAUNCH;
     const int q_tiles = pl.topk_pad / kWorkTileKeys;          // at most; the kernels know how many are in use
+    if (at_most_a_tile_each(p->s_q, q_tiles, std::min(pairs_r, pairs_d))) kp.every_slot = p->topk;
     auto grid_of = [&](int pairs) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * q_tiles)); };
     // `pdl`: start under the previous kernel's tail (one-stream schedules only)
     auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
+        kp.early_start = pdl && kp.every_slot && (stages & SMLA_STAGE_DELTA) && kp.q0 == 0;     // (right behind the prep kernel)
         launch(smla_recompute_pair_kernel<HP>, grid_of(pairs), rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
     auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl, bool after_recompute) {
@@ -458,11 +465,6 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             return SMLA_ERR_LAUNCH;
     }
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
-}
-
-// No cluster has more than one tile, whatever the indices are (KParams::every_slot).
-bool at_most_a_tile_each(int queries, int tiles_per_query, int clusters) {
-    return static_cast<long long>(queries) * tiles_per_query <= clusters;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -454,8 +454,13 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
         tmem_relinquish_2cta();
     }
-    pdl_wait();                  // slot counts and Delta of the prep kernel; the scratch's previous readers are done
-    pdl_trigger();
+    // Slot counts and Delta of the prep kernel.  Behind that kernel's trigger (it triggers once it has waited itself) all but
+    // Delta is in place where the ranges need no counts: then only the softmax warps wait.  64 queries x 16 heads x top-k 64:
+    // 24.9 -> 21.2 us a call.
+    if (!p.early_start) {
+        pdl_wait();
+        pdl_trigger();
+    }
     find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(lse_s), range_s);   // (lse_s: not in use yet)
     tc_fence_before_sync();
     __syncthreads();
@@ -625,6 +630,10 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             const size_t o = static_cast<size_t>(qg) * p.h_q + h;
             return t < HP ? p.lse[o] * p.lse_mult : p.delta[o] * p.sm_scale;
         };
+        if (p.early_start) {                // Delta; and nobody's scratch is written before this
+            pdl_wait();
+            pdl_trigger();
+        }
         int stat_q = range.q;               // the query stat_next belongs to
         float stat_next = load_stat(stat_q);
         int gt = 0;

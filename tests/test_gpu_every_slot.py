@@ -5,6 +5,7 @@ import torch
 
 from oracle.sparse_mla_ref import cosine, sparse_mla_bwd_ref, sparse_mla_fwd_ref
 from test_operator_b200.inputs import LOG2E, Workload, make_sequence
+from tests.metrics import assert_backward_close
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -53,3 +54,21 @@ def test_forward_logits_of_minus_infinity():
     o, lse = op.mla_fwd(q, kv, idx, q_start_index_s=None, check_device_status=True)
     assert torch.all(torch.isneginf(lse[[0, 2, 3]])) and torch.all(torch.isnan(o[[0, 2, 3], :, 0].float()))
     assert torch.all(torch.isposinf(lse[1])) and torch.all(o[1] == 0)
+
+
+@pytest.mark.parametrize("holes", [False, True], ids=["full", "holes"])
+@pytest.mark.parametrize("h_q", [16, 128])
+# (not one slot a query: its softmax is constant, dP - Delta is 0 up to the rounding of two sums, and so is all of dQ)
+@pytest.mark.parametrize("s_q,topk", [(1, 3)] + SIZES[1:])
+def test_backward(s_q, topk, h_q, holes):
+    from test_operator_b200 import op
+    s, idx, s_kv = _inputs(s_q, topk, h_q, holes)
+    args = (s["q"], s["kv"], s["dO"], s["lse"], s["O"], idx)
+    ref = sparse_mla_bwd_ref(*args, q_start_index_s=None, chunk_s=16)
+    dkv_dirty = torch.full((s_kv, 576), 7.0, device=DEV)          # cleared beside the kernel that computes S and dS
+    for out_dkv in (None, dkv_dirty):
+        dq, dkv = op.mla_bwd(*args, q_start_index_s=None, check_device_status=True, out_dkv=out_dkv)
+        assert_backward_close(dq, dkv, *ref)
+    unused = torch.ones(s_kv, dtype=torch.bool, device=DEV)
+    unused[idx[(idx >= 0) & (idx < s_kv)].long()] = False
+    assert torch.all(dkv[unused] == 0) and torch.all(dq[((idx < 0) | (idx >= s_kv)).all(dim=1)] == 0)
