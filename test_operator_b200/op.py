@@ -12,10 +12,13 @@ from __future__ import annotations
 import array
 import ctypes
 import functools
+import importlib.machinery
+import importlib.util
 import itertools
 import math
 import os
 import threading
+import warnings
 from typing import Optional, Tuple
 
 import torch
@@ -166,9 +169,53 @@ def load_library() -> ctypes.CDLL:
         return lib
 
 
-# Host path of a call.  The smallest calls take the GPU some tens of microseconds, so what Python does per call counts:
-# the current device is only switched when it has to be, the stream is taken as the raw handle, workspace sizes are
-# remembered per shape, and a call that passes one quick look at its tensors skips the itemised checks.
+# Host path of a call.  The smallest calls take the GPU 15 - 20 us, so what Python does per call counts: a call that passes one
+# quick look at its arguments is checked, given its outputs and queued by a small compiled module (csrc/smla_host.cpp); everything
+# else takes the way below, with the itemised checks and their messages.
+class _NoNativeHost:
+    """Without the compiled host module (no compiler, say) every call takes the Python way."""
+
+    @staticmethod
+    def fwd(*_):
+        return None
+
+    @staticmethod
+    def bwd_need(*_):
+        return 0
+
+
+_native = None
+
+
+def _host():
+    """The compiled host module, bound to the loaded library's entry points."""
+    global _native
+    if _native is None:
+        lib = load_library()
+        with _lib_lock:
+            if _native is None:
+                _native = _load_host(lib)
+    return _native
+
+
+def _load_host(lib):
+    try:
+        if _build.host_needs_build():
+            _build.build_host()
+    except Exception as e:
+        if not os.path.exists(_build.HOST_PATH):
+            warnings.warn(f"the compiled host module could not be built, calls take some 8 us longer: {e}")
+            return _NoNativeHost
+    loader = importlib.machinery.ExtensionFileLoader("_smla_host", _build.HOST_PATH)
+    module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("_smla_host", loader, origin=_build.HOST_PATH))
+    loader.exec_module(module)
+    module.init(*(ctypes.cast(f, ctypes.c_void_p).value for f in
+                  (lib.smla_fwd_run, lib.smla_fwd_workspace_size, lib.smla_bwd_run_stages, lib.smla_bwd_workspace_size)))
+    return module
+
+
+# Here the current device is only switched when it has to be, the stream is taken as the raw handle, and workspace sizes are
+# remembered per shape.
 class _NoSwitch:
     def __enter__(self):
         return None
@@ -297,26 +344,6 @@ def _check_out(t, like_shape_numel, dtype, device, name) -> None:
            and t.numel() == like_shape_numel, f"{name} must be a contiguous {dtype} CUDA tensor of {like_shape_numel} elements on {device}")
 
 
-def _plainly_valid(q, kv, dO, lse, O, indices) -> bool:
-    """True for what nearly every call passes: accepts only what `_validate` accepts, which has the error messages."""
-    try:
-        s_q, h_q, d = q.shape
-        s_kv, d_kv = kv.shape
-        n, topk = indices.shape
-        index = q.get_device()
-        want = (s_q, h_q, D_V)
-        return (d == D_QK and d_kv == D_QK and n == s_q and topk > 0 and 0 < h_q <= 128 and h_q % 8 == 0 and index >= 0
-                and dO.shape == want and O.shape == want and lse.shape == (s_q, h_q)
-                and q.dtype is torch.bfloat16 and kv.dtype is torch.bfloat16 and dO.dtype is torch.bfloat16
-                and O.dtype is torch.bfloat16 and lse.dtype is torch.float32 and indices.dtype is torch.int32
-                and kv.get_device() == index and dO.get_device() == index and lse.get_device() == index
-                and O.get_device() == index and indices.get_device() == index and q.is_cuda
-                and q.is_contiguous() and kv.is_contiguous() and dO.is_contiguous() and lse.is_contiguous()
-                and O.is_contiguous() and indices.is_contiguous())
-    except (AttributeError, TypeError, ValueError):
-        return False
-
-
 def _validate(q, kv, dO, lse, O, indices):
     """The reference's TORCH_CHECKs (`mla_bwd/mla_bwd.cu:975-1015`), widened to h_q in {8..128} and 3-D kv/indices."""
     for name, t in (("q", q), ("kv", kv), ("dO", dO), ("lse", lse), ("O", O), ("indices", indices)):
@@ -379,9 +406,32 @@ def mla_bwd(
     bytes per slot), for runs that must repeat exactly.  The call enqueues on the current stream and does not
     synchronise unless `check_device_status=True`, which also raises if a kernel reported a timed-out wait.
     """
-    if not _plainly_valid(q, kv, dO, lse, O, indices):
+    host = _host()
+    native_need = host.bwd_need(q, kv, dO, lse, O, indices)
+    if not native_need:
         _validate(q, kv, dO, lse, O, indices)
     _check_query_meta(query_meta, q)
+    if native_need and not (deterministic or workspace_budget):
+        if out_dq is not None:
+            _check_out(out_dq, q.numel(), torch.bfloat16, q.device, "out_dq")
+        if out_dkv is not None:
+            _check_out(out_dkv, kv.numel(), torch.float32, q.device, "out_dkv")
+        else:
+            _check(not accumulate, "accumulate=True needs out_dkv")
+        index = q.get_device()
+        with _on_device(index):
+            scratch = _scratch_of_stream(index) if workspace is None else None
+            with scratch.lock if scratch else _NO_SWITCH:
+                ws = workspace if scratch is None else scratch.workspace_of(native_need, q.device)
+                out = host.bwd(q, kv, dO, lse, O, indices, sm_scale, q_start_index_s, 1 if lse_is_base2 else 0, out_dq, out_dkv, query_meta,
+                               ws.ptr, ws.nbytes, STAGE_ALL & ~STAGE_ZERO if accumulate else STAGE_ALL)
+            if out is not None:
+                lib = load_library()
+                if type(out) is int:
+                    _raise_status(lib, out, "smla_bwd_run")
+                if check_device_status:
+                    _raise_status(lib, lib.smla_bwd_status(ws.ptr, _raw_stream(index)), "smla_bwd device status")
+                return (out[0] if out_dq is None else out_dq, out[1] if out_dkv is None else out_dkv)
     lib = load_library()
     kv2 = kv if kv.dim() == 2 else kv.reshape(kv.shape[0], D_QK)
     idx2 = indices if indices.dim() == 2 else indices.reshape(indices.shape[0], indices.shape[-1])
@@ -547,6 +597,12 @@ def mla_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor, sm_scale: 
     (`dq_test/test_dq_phase.py:53-59`).  Defaults mirror `mla_bwd` (causal rule with query start 0, base-2
     lse) so that `mla_bwd(q, kv, dO, lse, o, indices)` can consume the outputs directly.
     """
+    if workspace is None and query_meta is None and not (workspace_budget or check_device_status):
+        out = _host().fwd(q, kv, indices, sm_scale, q_start_index_s, 1 if lse_is_base2 else 0)
+        if type(out) is tuple:
+            return out
+        if out is not None:
+            _raise_status(load_library(), out, "smla_fwd_run")
     for name, t in (("q", q), ("kv", kv), ("indices", indices)):
         if not (isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous()):
             raise RuntimeError(f"{name} must be a contiguous CUDA tensor")
