@@ -341,6 +341,12 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
                  : "memory");
     return v;
 }
+// A value into another CTA's shared memory; its arrival counts 4 bytes on that CTA's barrier (addresses from map_to_cta).
+__device__ __forceinline__ void st_async_f32(uint32_t cluster_addr, float v, uint32_t cluster_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr),
+                 "r"(__float_as_uint(v)), "r"(cluster_bar)
+                 : "memory");
+}
 // All threads of both CTAs: arrive + wait on the hardware cluster barrier.
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -372,9 +372,26 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     kp.wait_limit = g_wait_limit.load();
     kp.staging = det ? det->staging : nullptr;
 
-    if (stages & SMLA_STAGE_DELTA) {
+    const int pairs_r = resident_pairs(smla_recompute_pair_kernel<HP>, rp::kThreads, rp::Cfg<HP>::kSmemBytes);
+    const int pairs_d = resident_pairs(smla_dkv_pair_kernel<HP>, dp::kThreads, dp::Cfg<HP>::kSmemBytes);
+    if (pairs_r <= 0 || pairs_d <= 0) return SMLA_ERR_LAUNCH;
+    const int q_tiles = pl.topk_pad / kWorkTileKeys;          // at most; the kernels know how many are in use
+    if (at_most_a_tile_each(p->s_q, q_tiles, std::min(pairs_r, pairs_d))) kp.every_slot = p->topk;
+    const size_t zero_n = (stages & SMLA_STAGE_ZERO) ? size_t(p->s_kv) * (kDQK / 4) : 0;     // 16-byte pieces
+    // One tile per cluster and one pass: the recompute kernel's softmax warps find Delta and clear dKV while their only tile is
+    // gathered and multiplied, with no prep kernel in front.
+    constexpr int kBoth = SMLA_STAGE_DELTA | SMLA_STAGE_RECOMPUTE;
+    if (kp.every_slot && (stages & kBoth) == kBoth && pl.q_chunk >= p->s_q) {
+        kp.own_prep = 1;
+        kp.o_in = reinterpret_cast<const uint4*>(p->O);
+        kp.do_in = reinterpret_cast<const uint4*>(p->dO);
+        kp.delta_out = delta;
+        kp.zero_n = zero_n;
+    }
+    if (kp.own_prep) {
+        // nothing to launch
+    } else if (stages & SMLA_STAGE_DELTA) {
         // one block per query, more where few queries come with a large dKV to clear
-        const size_t zero_n = (stages & SMLA_STAGE_ZERO) ? size_t(p->s_kv) * (kDQK / 4) : 0;     // 16-byte pieces
         const size_t zero_blocks = (zero_n + kPrepThreads * 16 - 1) / (kPrepThreads * 16);
         // (34 queries x 128 heads: 14 us with one block per query, 6.6 us so)
         int head_parts = 1;
@@ -389,16 +406,12 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     }
     if (!(stages & (SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ)))
         return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
-    const int pairs_r = resident_pairs(smla_recompute_pair_kernel<HP>, rp::kThreads, rp::Cfg<HP>::kSmemBytes);
-    const int pairs_d = resident_pairs(smla_dkv_pair_kernel<HP>, dp::kThreads, dp::Cfg<HP>::kSmemBytes);
-    if (pairs_r <= 0 || pairs_d <= 0) return SMLA_ERR_LAUNCH;
-    const int q_tiles = pl.topk_pad / kWorkTileKeys;          // at most; the kernels know how many are in use
-    if (at_most_a_tile_each(p->s_q, q_tiles, std::min(pairs_r, pairs_d))) kp.every_slot = p->topk;
     auto grid_of = [&](int pairs) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * q_tiles)); };
     // `pdl`: start under the previous kernel's tail (one-stream schedules only)
     auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
-        kp.early_start = pdl && kp.every_slot && (stages & SMLA_STAGE_DELTA) && kp.q0 == 0;     // (right behind the prep kernel)
-        launch(smla_recompute_pair_kernel<HP>, grid_of(pairs), rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
+        // (own_prep: further clusters, without a tile, where dKV is large: 16 KB of it a block)
+        const int grid = !kp.own_prep ? grid_of(pairs) : std::max(grid_of(pairs), 2 * int(std::min<size_t>(pairs, zero_n / 2048)));
+        launch(smla_recompute_pair_kernel<HP>, grid, rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
     auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl, bool after_recompute) {
         kp.early_start = after_recompute;

@@ -61,8 +61,13 @@ struct KParams {
     const int4* qmeta;        // optional per query {first kv row of its sequence, kv rows of its sequence,
                               // position for the causal rule, top-k slots in use}; null: one sequence
     long long wait_limit;     // cycles a bounded wait may take
-    int early_start;          // launched behind the trigger of the kernel before in the same call (see the kernels)
+    int early_start;          // dkv, dq: launched behind the trigger of the kernel before in the same call (see there)
     int every_slot;           // > 0 (topk): count every slot of every query as used and do not read n_used (slots_used)
+    // recompute without a prep kernel in front (own_prep, only with every_slot): O, dO and the 16-byte pieces of dKV to clear
+    int own_prep;
+    const uint4 *o_in, *do_in;
+    float* delta_out;         // (for calls of single stages that follow)
+    size_t zero_n;
 };
 
 // What a query may attend to: rows [kv_base, kv_base + kv_len) of kv, index values relative to kv_base.
@@ -180,6 +185,26 @@ __device__ __forceinline__ int block_exclusive_sum(int v, int* warp_sums, int* t
     return before + incl - v;
 }
 
+// Delta of `kRows` (query, head) rows, row[i] of [rows, 512] each: 4 kRows 16-byte loads of a lane in flight.  Returned in every lane.
+template <int kRows>
+__device__ __forceinline__ void delta_rows(const uint4* O, const uint4* dO, const size_t (&row)[kRows], float (&out)[kRows]) {
+    const int lane = threadIdx.x & 31;
+    uint4 a[2 * kRows], b[2 * kRows];
+#pragma unroll
+    for (int i = 0; i < 2 * kRows; ++i) {
+        const size_t at = row[i >> 1] * (kDV / 8) + 32 * (i & 1) + lane;
+        a[i] = ld_stream_v4(O + at);
+        b[i] = ld_stream_v4(dO + at);
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) out[i] = warp_sum(dot8_bf16(a[2 * i + 1], b[2 * i + 1], dot8_bf16(a[2 * i], b[2 * i], 0.f)));
+}
+// This block's share of dKV cleared, by `threads` of its threads.
+__device__ __forceinline__ void clear_share(uint4* dst, size_t n, int thread, int threads) {
+    const size_t z0 = n * blockIdx.x / gridDim.x, z1 = n * (blockIdx.x + 1) / gridDim.x;
+    for (size_t i = z0 + thread; i < z1; i += threads) dst[i] = make_uint4(0, 0, 0, 0);
+}
+
 __global__ void __launch_bounds__(kPrepThreads)
 smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, float* __restrict__ delta,
                  int* __restrict__ n_used, uint4* __restrict__ zero_dst, size_t zero_n, int head_parts, const KParams p) {
@@ -216,31 +241,20 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
                 p.lse_out[static_cast<size_t>(q) * p.h_q + h] = __int_as_float(0x7f800000) * p.lse_out_mult;
         }
     } else if (q < p.s_q) {
-        const uint4* o = O + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
-        const uint4* g = dO + static_cast<size_t>(q) * p.h_q * (kDV / 8) + lane;
-        // two rows at a time: eight 16-byte loads of a lane in flight
+        const size_t row0 = static_cast<size_t>(q) * p.h_q;
         const int h_end = p.h_q * (hp + 1) / head_parts;
         for (int h = p.h_q * hp / head_parts + warp; h < h_end; h += 2 * kWarps) {
             const int h2 = h + kWarps < h_end ? h + kWarps : h;
-            uint4 a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int at = (i < 2 ? h : h2) * (kDV / 8) + 32 * (i & 1);
-                a[i] = ld_stream_v4(o + at);
-                b[i] = ld_stream_v4(g + at);
-            }
-            const float s0 = warp_sum(dot8_bf16(a[1], b[1], dot8_bf16(a[0], b[0], 0.f)));
-            const float s1 = warp_sum(dot8_bf16(a[3], b[3], dot8_bf16(a[2], b[2], 0.f)));
+            const size_t row[2] = {row0 + h, row0 + h2};
+            float d[2];
+            delta_rows(O, dO, row, d);
             if (lane == 0) {
-                delta[static_cast<size_t>(q) * p.h_q + h] = s0;
-                delta[static_cast<size_t>(q) * p.h_q + h2] = s1;
+                delta[row[0]] = d[0];
+                delta[row[1]] = d[1];
             }
         }
     }
-    if (zero_n) {
-        const size_t z0 = zero_n * blockIdx.x / gridDim.x, z1 = zero_n * (blockIdx.x + 1) / gridDim.x;
-        for (size_t i = z0 + threadIdx.x; i < z1; i += kPrepThreads) zero_dst[i] = make_uint4(0, 0, 0, 0);
-    }
+    if (zero_n) clear_share(zero_dst, zero_n, threadIdx.x, kPrepThreads);
 }
 
 // Per-query table for packed sequences (KParams::qmeta) from a table of sequences that travels in the kernel's parameters:
@@ -272,8 +286,8 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 //
 // A call whose queries have no more tiles than there are clusters takes as long as one tile takes, whether or not some of the
 // tiles are empty.  There the ranges are cut as if every slot were in use (every_slot): nothing has to look at the indices
-// first, which saves the forward its prep kernel: eight queries x 128 heads x top-k 2048 25.1 -> 19.5 us a call (prep kernel,
-// its hand-over and the 5700 cycles that the ranges took from its counts; 128 blocks with one tile each either way).  From the
+// first, which saves both directions their prep kernel (own_prep in the backward).  Eight queries x 128 heads x top-k 2048, forward:
+// 25.1 -> 19.5 us a call (prep kernel, its hand-over and the 5700 cycles that the ranges took from its counts).  From the
 // next tile on some cluster has two, and an empty tile would cost as much as a full one.
 __device__ __forceinline__ int slots_used(const KParams& p, int q) { return p.every_slot ? p.every_slot : __ldcg(p.n_used + q); }
 struct WorkRange {
@@ -423,8 +437,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 1024 + 8 * (2 * kStages + 2 * kQChunks + 4));
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t bar_drain = smem_u32(tmem_slot + 2);     // used only while winding down after an abort
-    WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 4);
-    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 16 + sizeof(WorkRange) <= 512, "barrier area");
+    const uint32_t bar_delta = smem_u32(tmem_slot + 4);     // (own_prep) the other CTA's heads' Delta has arrived
+    WorkRange* range_s = reinterpret_cast<WorkRange*>(tmem_slot + 6);
+    static_assert(8 * (2 * kStages + 2 * kQChunks + 4) + 24 + sizeof(WorkRange) <= 512, "barrier area");
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, map_to_cta(smem_u32(tmem_slot + 1), rank ^ 1)};
 
     if (threadIdx.x == 0) {
@@ -443,7 +458,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             mbar_init(bar_tempty + 8 * i, 16);   // 8 softmax warps in each CTA
         }
         mbar_init(bar_drain, 1);
+        mbar_init(bar_delta, 1);
         fence_mbar_init();
+        if (p.own_prep) mbar_arrive_expect_tx(bar_delta, 4 * max(0, min(NH, p.h_q - NH * static_cast<int>(rank ^ 1))));
     }
     {   // zero block standing in for the dO half of column chunk 8 (never overwritten)
         uint4* z = reinterpret_cast<uint4*>(smem + C::kOffB + 8 * C::kBChunk + C::kBHalf);
@@ -454,10 +471,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
         tmem_relinquish_2cta();
     }
-    // Slot counts and Delta of the prep kernel.  Behind that kernel's trigger (it triggers once it has waited itself) all but
-    // Delta is in place where the ranges need no counts: then only the softmax warps wait.  64 queries x 16 heads x top-k 64:
-    // 24.9 -> 21.2 us a call.
-    if (!p.early_start) {
+    if (!p.own_prep) {           // slot counts and Delta of the prep kernel; the scratch's previous readers are done
         pdl_wait();
         pdl_trigger();
     }
@@ -469,6 +483,10 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
     static_assert(kTileKeys == kWorkTileKeys, "one work tile per accumulator");
+    if (p.own_prep) {            // nothing of the caller's has been touched so far
+        pdl_wait();
+        pdl_trigger();
+    }
 
     if (warp >= 8 && warp < 16) {
         // ------------------------------------------------------------------ gather producers
@@ -628,11 +646,35 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             if (t >= 2 * HP) return 0.f;
             if (h >= p.h_q) return t < HP ? __int_as_float(0x7f800000) : 0.f;
             const size_t o = static_cast<size_t>(qg) * p.h_q + h;
+            if (t >= HP && p.own_prep) return delta_s[h];
             return t < HP ? p.lse[o] * p.lse_mult : p.delta[o] * p.sm_scale;
         };
-        if (p.early_start) {                // Delta; and nobody's scratch is written before this
-            pdl_wait();
-            pdl_trigger();
+        if (p.own_prep) {
+            // Delta of the one query this cluster works on: each CTA its half of the heads, four rows a warp at a time, written to both
+            // CTAs; it is done before the tile's logits are.  One launch less in a chain of four, host and GPU: 64 queries x 16 heads
+            // x top-k 64 21.2 -> 20.6 us with this kernel behind the prep kernel's trigger before; on its own 24.9 -> 20.6.
+            if (range.begin < range.end) {
+                const uint32_t peer_delta = map_to_cta(smem_u32(delta_s), rank ^ 1), peer_bar = map_to_cta(bar_delta, rank ^ 1);
+                const int h0 = NH * static_cast<int>(rank), h1 = min(p.h_q, h0 + NH);
+                for (int h = h0 + warp; h < h1; h += 32) {
+                    size_t at[4];
+                    float d[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) at[i] = static_cast<size_t>(range.q) * p.h_q + (h + 8 * i < h1 ? h + 8 * i : h);
+                    delta_rows(p.o_in, p.do_in, at, d);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (lane == i && h + 8 * i < h1) {
+                            delta_s[h + 8 * i] = d[i] * p.sm_scale;
+                            st_async_f32(peer_delta + 4 * (h + 8 * i), d[i] * p.sm_scale, peer_bar);
+                            p.delta_out[at[i]] = d[i];
+                        }
+                    }
+                }
+            }
+            if (p.zero_n) clear_share(reinterpret_cast<uint4*>(p.dKV), p.zero_n, t, 256);
+            if (range.begin < range.end) mbar_wait(bar_delta, 0, wc, kErrRecompute + 19, kPollSleepNs);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
         }
         int stat_q = range.q;               // the query stat_next belongs to
         float stat_next = load_stat(stat_q);

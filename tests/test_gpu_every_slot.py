@@ -15,7 +15,7 @@ SIZES = [(1, 1), (1, 256), (74, 200), (75, 200), (37, 300), (38, 300), (9, 2048)
 
 
 def _inputs(s_q, topk, h_q, holes):
-    s_kv = max(2 * topk, 64)
+    s_kv = 40000 if topk == 3 else max(2 * topk, 64)       # (a large dKV to clear beside a single tile)
     s = make_sequence(Workload("every_slot", 1, s_q, s_kv, h_q, topk, "uniform", invalid_frac=0.0), device=DEV, seed=17)
     idx = s["indices"]
     if holes:
@@ -69,6 +69,10 @@ def test_backward(s_q, topk, h_q, holes):
     for out_dkv in (None, dkv_dirty):
         dq, dkv = op.mla_bwd(*args, q_start_index_s=None, check_device_status=True, out_dkv=out_dkv)
         assert_backward_close(dq, dkv, *ref)
+    dkv2 = torch.ones_like(dkv)
+    op.mla_bwd(*args, q_start_index_s=None, out_dkv=dkv2, accumulate=True)
+    # added to ones: rounded to 2^-24 of the sum's size at every addition
+    assert (dkv2 - 1 - dkv).abs().max().item() <= (dkv.abs().max().item() + 1) * 2.0 ** -24 * (s_q + 2) * 2
     unused = torch.ones(s_kv, dtype=torch.bool, device=DEV)
     unused[idx[(idx >= 0) & (idx < s_kv)].long()] = False
     assert torch.all(dkv[unused] == 0) and torch.all(dq[((idx < 0) | (idx >= s_kv)).all(dim=1)] == 0)
