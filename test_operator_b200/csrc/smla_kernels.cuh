@@ -1823,32 +1823,33 @@ constexpr int kThreads = 448;
 constexpr int kProducerWarps = 8;
 constexpr int kTileKeys = 64;
 constexpr int kParts = kQChunks / kDqChunks;
-template <int HP> struct Cfg {
-    static constexpr int kStages = HP == 64 ? 3 : 2;        // what fits twice into an SM's shared memory
+// kDeep: one CTA per SM with as many stages as its shared memory holds, for launches that do not give every SM two CTAs: with
+// two stages a CTA alone on its SM waits for its gathers, 1300 cycles a tile against 625 of shared-memory traffic.  Calls of 37 queries
+// x 128 heads x top-k 2048 117.4 -> 104.9 us, 27 x 64 heads 96.0 -> 91.8, 12 x 128 heads 58.1 -> 54.9, 3 x 128 40.2 -> 38.8.
+template <int HP, bool kDeep> struct Cfg {
+    static constexpr int kStages = kDeep ? (HP == 64 ? 6 : 5) : HP == 64 ? 3 : 2;      // (not deep: what fits twice into an SM's shared memory)
     static constexpr int kKgBytes = kDqChunks * 8192;
     static constexpr int kDsBytes = (HP / 64) * 8192;
     static constexpr int kStage = kKgBytes + kDsBytes;     // dS right after Kg
     static constexpr int kOffMisc = kStages * kStage;
     // the A operand always spans 128 heads: with HP = 64 its upper half reads 8 KB past the dS tile
     static constexpr int kSmemBytes = kOffMisc + 256 + 1024 + (HP == 64 ? 8192 : 0);
-    static_assert(2 * (kSmemBytes + 1024) <= 233472, "two CTAs per SM");
+    static_assert((kDeep ? 1 : 2) * (kSmemBytes + 1024) <= 233472, "one or two CTAs per SM");
     static constexpr int kTmemCols = 256;                  // up to 256 columns of d; two CTAs share the SM's 512
     static constexpr int kRowBytes = kDqChunks * 128 + 16;    // epilogue staging of one head's row
     static_assert(128 * kRowBytes <= kOffMisc, "the epilogue stages its rows in the pipeline's memory");
-    // keys of a query split over a cluster: every CTA leaves its fp32 accumulator [heads][columns] behind the barriers for
-    // the others to read (rows 16 bytes apart modulo 128: conflict-free 16-byte accesses); one CTA per SM then
+    // keys of a query split over a cluster: every CTA leaves its fp32 accumulator [heads][columns] in the pipeline's memory for
+    // the others to read (rows 16 bytes apart modulo 128: conflict-free 16-byte accesses)
     static constexpr int kPartPitch = kDqChunks * 64 + 4;
-    static constexpr int kOffPart = kOffMisc + 256;
-    static constexpr int kSplitSmemBytes = kOffPart + 128 * kPartPitch * 4 + 1024;
-    static_assert(kSplitSmemBytes <= 232448, "shared memory of one SM");
+    static_assert(!kDeep || HP * kPartPitch * 4 <= kOffMisc, "the accumulator of a split query");
 };
 }  // namespace dq
 
-template <int HP>
-__global__ void __launch_bounds__(dq::kThreads, 2)
+template <int HP, bool kDeep>
+__global__ void __launch_bounds__(dq::kThreads, kDeep ? 1 : 2)
 smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     using namespace dq;
-    using C = Cfg<HP>;
+    using C = Cfg<HP, kDeep>;
     constexpr int kStages = C::kStages;
     // the CTAs of a cluster (usually one) share a (query, d-part) and split its keys
     const int nz = static_cast<int>(cluster_nctas()), z = static_cast<int>(cluster_ctarank());
@@ -2005,9 +2006,9 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         const int head = quarter * 32 + lane;
         const uint32_t row_s = s_base + head * kRowBytes;
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-        if (nz > 1) {
+        if (kDeep && nz > 1) {
             if (quarter * 32 < p.h_q) {
-                const uint32_t part_s = s_base + C::kOffPart + head * (C::kPartPitch * 4);
+                const uint32_t part_s = s_base + head * (C::kPartPitch * 4);
 #pragma unroll 1
                 for (int cg = 0; cg < kDqChunks * 4; ++cg) {
                     uint32_t r[16];
@@ -2049,14 +2050,14 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     if (p.early_start && blockIdx.x == gridDim.x - 1) pdl_wait();
     tc_fence_before_sync();
     __syncthreads();
-    if (nz > 1) {
+    if (kDeep && nz > 1) {
         // every CTA adds up its share of the heads, always in rank order
         cluster_sync_all();
         constexpr int kGroups = kDqChunks * 8;   // 8 columns at a time
         const int h0 = p.h_q * z / nz, h1 = p.h_q * (z + 1) / nz;
         for (int i = threadIdx.x; i < (h1 - h0) * kGroups; i += kThreads) {
             const int h = h0 + i / kGroups, c = (i % kGroups) * 8;
-            const uint32_t at = s_base + C::kOffPart + (h * C::kPartPitch + c) * 4;
+            const uint32_t at = s_base + (h * C::kPartPitch + c) * 4;
             float acc[8] = {};
             for (int r = 0; r < nz; ++r) {
                 const uint32_t a = map_to_cta(at, r);
