@@ -377,40 +377,34 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     if (pairs_r <= 0 || pairs_d <= 0) return SMLA_ERR_LAUNCH;
     const int q_tiles = pl.topk_pad / kWorkTileKeys;          // at most; the kernels know how many are in use
     if (at_most_a_tile_each(p->s_q, q_tiles, std::min(pairs_r, pairs_d))) kp.every_slot = p->topk;
-    const size_t zero_n = (stages & SMLA_STAGE_ZERO) ? size_t(p->s_kv) * (kDQK / 4) : 0;     // 16-byte pieces
-    // One tile per cluster and one pass: the recompute kernel's softmax warps find Delta and clear dKV while their only tile is
-    // gathered and multiplied, with no prep kernel in front.
+    // (cleared by the recompute kernel of the first pass where there is one)
+    const size_t dkv_bytes = size_t(p->s_kv) * kDQK * sizeof(float);
+    const size_t clear_bytes = (stages & SMLA_STAGE_ZERO) && (stages & SMLA_STAGE_RECOMPUTE) ? dkv_bytes : 0;
+    if ((stages & SMLA_STAGE_ZERO) && !clear_bytes && cudaMemsetAsync(p->dKV, 0, dkv_bytes, st) != cudaSuccess) return SMLA_ERR_LAUNCH;
+    // One tile per cluster and one pass: the recompute kernel's softmax warps find Delta while their only tile is gathered and
+    // multiplied, with no prep kernel in front.
     constexpr int kBoth = SMLA_STAGE_DELTA | SMLA_STAGE_RECOMPUTE;
     if (kp.every_slot && (stages & kBoth) == kBoth && pl.q_chunk >= p->s_q) {
         kp.own_prep = 1;
         kp.o_in = reinterpret_cast<const uint4*>(p->O);
         kp.do_in = reinterpret_cast<const uint4*>(p->dO);
         kp.delta_out = delta;
-        kp.zero_n = zero_n;
     }
-    if (kp.own_prep) {
-        // nothing to launch
-    } else if (stages & SMLA_STAGE_DELTA) {
-        // one block per query, more where few queries come with a large dKV to clear
-        const size_t zero_blocks = (zero_n + kPrepThreads * 16 - 1) / (kPrepThreads * 16);
-        // (34 queries x 128 heads: 14 us with one block per query, 6.6 us so)
+    if ((stages & SMLA_STAGE_DELTA) && !kp.own_prep) {
+        // one block per query, more for few queries (34 queries x 128 heads: 14 us with one block per query, 6.6 us so)
         int head_parts = 1;
         while (static_cast<long long>(p->s_q) * head_parts * 2 <= 8 * kSmCount && p->h_q / (head_parts * 2) >= 16) head_parts *= 2;
-        int grid = p->s_q * head_parts;
-        if (size_t(grid) < zero_blocks) grid = std::max(grid, int(std::min<size_t>(zero_blocks, 8 * kSmCount)));
-        launch(smla_prep_kernel, grid, kPrepThreads, 0, st, true, 1, reinterpret_cast<const uint4*>(p->O),
-               reinterpret_cast<const uint4*>(p->dO), delta, reinterpret_cast<int*>(ws + pl.used_off),
-               reinterpret_cast<uint4*>(p->dKV), zero_n, head_parts, kp);
-    } else if (stages & SMLA_STAGE_ZERO) {
-        if (cudaMemsetAsync(p->dKV, 0, size_t(p->s_kv) * kDQK * sizeof(float), st) != cudaSuccess) return SMLA_ERR_LAUNCH;
+        launch(smla_prep_kernel, p->s_q * head_parts, kPrepThreads, 0, st, true, 1, reinterpret_cast<const uint4*>(p->O),
+               reinterpret_cast<const uint4*>(p->dO), delta, reinterpret_cast<int*>(ws + pl.used_off), head_parts, kp);
     }
     if (!(stages & (SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ)))
         return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
     auto grid_of = [&](int pairs) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * q_tiles)); };
     // `pdl`: start under the previous kernel's tail (one-stream schedules only)
     auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
-        // (own_prep: further clusters, without a tile, where dKV is large: 16 KB of it a block)
-        const int grid = !kp.own_prep ? grid_of(pairs) : std::max(grid_of(pairs), 2 * int(std::min<size_t>(pairs, zero_n / 2048)));
+        kp.clear_bytes = kp.q0 == 0 ? clear_bytes : 0;
+        // (further clusters, without a tile, where few queries come with a large dKV: 16 KB of it a block)
+        const int grid = std::max(grid_of(pairs), 2 * int(std::min<size_t>(pairs, kp.clear_bytes >> 15)));
         launch(smla_recompute_pair_kernel<HP>, grid, rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
     auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl, bool after_recompute) {
@@ -569,7 +563,7 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
         kp.every_slot = p->topk;
     else
         launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, static_cast<const uint4*>(nullptr), static_cast<const uint4*>(nullptr),
-               static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), static_cast<uint4*>(nullptr), size_t(0), 1, kp);
+               static_cast<float*>(nullptr), reinterpret_cast<int*>(ws + pl.used_off), 1, kp);
     launch(smla_fwd_kernel<HP>, 2 * clusters, ff::kThreads, ff::kSmemBytes, st, true, 1, tm_q, kp);
     if (clusters > 1 && (!kp.every_slot || q_tiles > 1)) {
         const int items = p->s_q < clusters ? p->s_q : clusters - 1;
