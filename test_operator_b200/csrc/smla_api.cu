@@ -618,19 +618,19 @@ inline InvLayout inv_layout(int64_t n, int32_t s_kv, const inv::Plan& pl) {
 }
 
 // Two passes (up to 65535 rows) on 8.4 M slots and 32768 rows: 214 us with keys formed by a kernel of their own, read twice by
-// every scatter, carried as 32 bits and written by the last pass for a binary search per row; 139 us in this form.
-template <typename KeyT, int kItems>
+// every scatter, carried as 32 bits and written by the last pass for a binary search per row; 134 us in this form.
+template <typename KeyT, int kItems, bool kMasks>
 int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvLayout& l, uint8_t* ws, int64_t n64, int32_t* row_ptr,
                          int32_t* entries, cudaStream_t st) {
     const uint32_t n = static_cast<uint32_t>(n64);
     constexpr int kSmem = inv::scatter_smem<KeyT, kItems>();
     static std::atomic<bool> attr_done[kMaxDevices];
     if (!once_per_device(attr_done, [] {
-            bool ok = set_smem(inv::scatter_kernel<KeyT, true, true, kItems>, kSmem);
-            ok &= set_smem(inv::scatter_kernel<KeyT, true, false, kItems>, kSmem);
-            ok &= set_smem(inv::scatter_kernel<KeyT, false, true, kItems>, kSmem);
-            ok &= set_smem(inv::scatter_kernel<KeyT, false, false, kItems>, kSmem);
-            if (kItems == inv::kItemsLarge) ok &= set_smem(inv::small_sort_kernel<KeyT>, kSmem);
+            bool ok = set_smem(inv::scatter_kernel<KeyT, true, true, kItems, kMasks>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, true, false, kItems, kMasks>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, false, true, kItems, kMasks>, kSmem);
+            ok &= set_smem(inv::scatter_kernel<KeyT, false, false, kItems, kMasks>, kSmem);
+            ok &= set_smem(inv::small_sort_kernel<KeyT>, inv::scatter_smem<KeyT, inv::kItemsSmall>());
             return ok;
         }))
         return SMLA_ERR_LAUNCH;
@@ -640,7 +640,7 @@ int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvL
     uint32_t* totals = reinterpret_cast<uint32_t*>(ws + l.totals);
     int32_t* heads = reinterpret_cast<int32_t*>(ws + l.heads);
     if (n64 <= inv::kSmallInput) {
-        launch(inv::small_sort_kernel<KeyT>, 1, inv::kThreads, kSmem, st, true, 1, src, keys[0], entries, n, pl.passes, pl.digit_bits);
+        launch(inv::small_sort_kernel<KeyT>, 1, inv::kThreads, inv::scatter_smem<KeyT, inv::kItemsSmall>(), st, true, 1, src, keys[0], entries, n, pl.passes, pl.digit_bits);
         launch(inv::small_row_ptr_kernel<KeyT>, src.s_kv / 256 + 1, 256, 0, st, true, 1, keys[0], row_ptr, static_cast<int32_t>(n), src.s_kv);
         return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
     }
@@ -655,8 +655,8 @@ int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvL
         launch(first ? inv::histogram_kernel<KeyT, true, kItems> : inv::histogram_kernel<KeyT, false, kItems>, pl.n_blocks, inv::kThreads, 0, st, true, 1, kin,
                src, hist, n, shift, mask, pl.n_blocks, heads);
         launch(inv::scan_rows_kernel, static_cast<int>(mask) + 1, 1024, 0, st, true, 1, hist, totals, pl.n_blocks);
-        launch(first ? (last ? inv::scatter_kernel<KeyT, true, true, kItems> : inv::scatter_kernel<KeyT, true, false, kItems>)
-                     : (last ? inv::scatter_kernel<KeyT, false, true, kItems> : inv::scatter_kernel<KeyT, false, false, kItems>),
+        launch(first ? (last ? inv::scatter_kernel<KeyT, true, true, kItems, kMasks> : inv::scatter_kernel<KeyT, true, false, kItems, kMasks>)
+                     : (last ? inv::scatter_kernel<KeyT, false, true, kItems, kMasks> : inv::scatter_kernel<KeyT, false, false, kItems, kMasks>),
                pl.n_blocks, inv::kThreads, kSmem, st, true, 1, kin, vin, src, kout, vout, hist, totals, n, shift, mask, pl.n_blocks, heads);
     }
     const int row_blocks = src.s_kv / inv::kRowTile + 1;
@@ -667,6 +667,13 @@ int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvL
     }
     launch(inv::row_ptr_kernel, row_blocks, inv::kRowTile, 0, st, true, 1, heads, first, row_ptr, static_cast<int32_t>(n), src.s_kv);
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
+}
+
+template <int kItems, bool kMasks>
+int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvLayout& l, uint8_t* ws, int64_t n, int32_t* row_ptr,
+                         int32_t* entries, cudaStream_t st) {
+    return pl.key16 ? launch_index_inverse<uint16_t, kItems, kMasks>(src, pl, l, ws, n, row_ptr, entries, st)
+                    : launch_index_inverse<uint32_t, kItems, kMasks>(src, pl, l, ws, n, row_ptr, entries, st);
 }
 
 inline bool inv_shape_ok(int32_t s_q, int32_t topk, int32_t s_kv) {
@@ -900,10 +907,9 @@ int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_
     src.causal = q_start_index_s != SMLA_NO_CAUSAL;
     src.q_start = src.causal ? q_start_index_s : 0;
     if (pl.items == inv::kItemsMid)
-        return pl.key16 ? launch_index_inverse<uint16_t, inv::kItemsMid>(src, pl, l, ws, n, row_ptr, entries, st)
-                        : launch_index_inverse<uint32_t, inv::kItemsMid>(src, pl, l, ws, n, row_ptr, entries, st);
-    return pl.key16 ? launch_index_inverse<uint16_t, inv::kItemsLarge>(src, pl, l, ws, n, row_ptr, entries, st)
-                    : launch_index_inverse<uint32_t, inv::kItemsLarge>(src, pl, l, ws, n, row_ptr, entries, st);
+        return launch_index_inverse<inv::kItemsMid, true>(src, pl, l, ws, n, row_ptr, entries, st);
+    return pl.by_masks ? launch_index_inverse<inv::kItemsLarge, true>(src, pl, l, ws, n, row_ptr, entries, st)
+                       : launch_index_inverse<inv::kItemsLarge, false>(src, pl, l, ws, n, row_ptr, entries, st);
 }
 
 // ---- sum of the ranks' partial dKV over NVLink (query-sharded runs) ---------------------------------------------

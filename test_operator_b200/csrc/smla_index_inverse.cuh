@@ -24,12 +24,12 @@ namespace inv {
 
 constexpr int kThreads = 512;
 // Entries per thread; a block's entries are contiguous, a warp's are (32 kItems of them): (warp, step, lane) order is flat
-// order.  Large inputs take sixteen (long runs on the way out; 8.4 M slots: 139 us with sixteen, 144 with twelve, 159 with
-// eight).  Below kLargeInput they take four, so that there are blocks for all SMs (270,000 slots: 46 us with sixteen, 29 with
-// eight).
-constexpr int kItemsLarge = 16, kItemsMid = 4;
+// order.  Large inputs take fourteen: long runs on the way out, and 8.4 M slots are 4.0 rounds of blocks on 148 SMs (3.5 with
+// sixteen; 159 us with eight, 144 with twelve, 139 with sixteen, 137 with fourteen).  Below kLargeInput they take four, so that
+// there are blocks for all SMs (270,000 slots: 46 us with sixteen, 29 with eight).
+constexpr int kItemsLarge = 14, kItemsMid = 4, kItemsSmall = 16;
 constexpr int64_t kLargeInput = 1 << 20;
-constexpr int kSmallInput = kThreads * kItemsLarge;     // one block sorts this many alone
+constexpr int kSmallInput = kThreads * kItemsSmall;     // one block sorts this many alone
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxRadix = 256;
 constexpr int kRowTile = 1024;                   // rows per block of the row_ptr kernel
@@ -37,6 +37,7 @@ constexpr int kRowTile = 1024;                   // rows per block of the row_pt
 // themselves, a block at a time: one step where slots are spread, 0.28 us a step where the rows behind are unused.  With more
 // of them two small kernels prepare it (see row_min_kernel): 32 K slots all in the first 1024 of 4 M rows 9.4 ms by looking.
 constexpr int kMaxLook = 64;
+constexpr int kResidentBlocks = 2 * 148;         // scatter blocks that a B200 runs at once
 
 struct Plan {
     int passes;      // 1..4
@@ -44,6 +45,7 @@ struct Plan {
     int items;       // entries per thread
     int n_blocks;
     bool key16;      // keys fit 16 bits
+    bool by_masks;   // block_rank's kMasks (large form; the others always)
 };
 
 inline Plan make_plan(int64_t n, int32_t s_kv) {
@@ -55,6 +57,7 @@ inline Plan make_plan(int64_t n, int32_t s_kv) {
     pl.items = n > kSmallInput && n < kLargeInput ? kItemsMid : kItemsLarge;
     pl.n_blocks = static_cast<int>((n + kThreads * pl.items - 1) / (kThreads * pl.items));
     pl.key16 = s_kv < 65536;
+    pl.by_masks = pl.n_blocks <= kResidentBlocks;
     return pl;
 }
 
@@ -181,32 +184,51 @@ struct RankShared {
 // entries 32 at a time against its own running counts, with no counting round before, as two chains with counts of their
 // own (a step's read of a count waits for the step before it; two chains hide that); the counts then are
 // prefixed over the runs and the digits.  Ends with all threads past a barrier.
-template <int kItems>
+//
+// kMasks: the lanes of a step that share a digit are found by each setting its bit in the digit's word of shared memory
+// (`words`, kRuns * kMaxRadix of them), not by eight ballots.  That is a third of the instructions and the shorter chain, but more
+// shared-memory traffic: faster while every block runs at once, slower where many wait for an SM.  10 x 512 slots 17.6 us by ballots,
+// 15.0 by masks; 0.9 M slots (450 small blocks) 49.6 / 46.0; 2.1 M of 8192 rows (293 blocks) 42.2 / 38.3; 8.4 M of 32768 (1171
+// blocks) 134.1 / 136.3; 16.8 M of 65000 258 / 275.
+template <bool kMasks, int kItems>
 __device__ __forceinline__ void block_rank(const uint32_t (&keys)[kItems], int shift, uint32_t mask, uint32_t first, uint32_t n,
-                                           RankShared& sh, uint32_t (&pos)[kItems]) {
+                                           RankShared& sh, uint32_t* words, uint32_t (&pos)[kItems]) {
     static_assert(kChains == 2 && kThreads == 2 * kMaxRadix, "two threads per digit below");
     constexpr int kSteps = kItems / kChains;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lanes_below = (1u << lane) - 1u;
     uint16_t* mine = sh.count[warp * kChains];
+    uint32_t* same = words + warp * kChains * kMaxRadix;
     for (int d = lane; d < kChains * kMaxRadix / 2; d += 32) reinterpret_cast<uint32_t*>(mine)[d] = 0;
+    if (kMasks) {
+        for (int d = lane; d < kChains * kMaxRadix; d += 32) same[d] = 0;
+    }
     __syncwarp();
 #pragma unroll
     for (int t = 0; t < kSteps; ++t) {
-        uint32_t d[kChains], peers[kChains], before[kChains];
+        uint32_t at[kChains], peers[kChains], before[kChains];
 #pragma unroll
         for (int c = 0; c < kChains; ++c) {
             const int e = c * kSteps + t;
-            d[c] = digit_of(keys[e], shift, mask);
-            peers[c] = same_digit_lanes(d[c], first + e * 32 < n);
-            before[c] = mine[c * kMaxRadix + d[c]];
-            pos[e] = before[c] + __popc(peers[c] & lanes_below);
+            const uint32_t d = digit_of(keys[e], shift, mask);
+            at[c] = c * kMaxRadix + d;
+            if (!kMasks) peers[c] = same_digit_lanes(d, first + e * 32 < n);
+            else if (first + e * 32 < n) atomicOr(&same[at[c]], 1u << lane);
+        }
+        if (kMasks) __syncwarp();
+#pragma unroll
+        for (int c = 0; c < kChains; ++c) {
+            if (kMasks) peers[c] = same[at[c]];
+            before[c] = mine[at[c]];
+            pos[c * kSteps + t] = before[c] + __popc(peers[c] & lanes_below);
         }
         __syncwarp();
 #pragma unroll
         for (int c = 0; c < kChains; ++c)
-            if (first + (c * kSteps + t) * 32 < n && (peers[c] & lanes_below) == 0)
-                mine[c * kMaxRadix + d[c]] = static_cast<uint16_t>(before[c] + __popc(peers[c]));
+            if (first + (c * kSteps + t) * 32 < n && (peers[c] & lanes_below) == 0) {     // the lowest of them
+                mine[at[c]] = static_cast<uint16_t>(before[c] + __popc(peers[c]));
+                if (kMasks) same[at[c]] = 0;
+            }
         __syncwarp();
     }
     __syncthreads();
@@ -239,16 +261,24 @@ __device__ __forceinline__ void block_rank(const uint32_t (&keys)[kItems], int s
 // consecutive addresses inside a digit's run instead of 32 different lines per warp instruction).
 // kFirst: keys from the indices, values are the flat positions themselves.  kLast: keys are not written; the head of every
 // run of equal keys lowers its row's row_ptr to its position.
-// What bounds it: instruction issue, shared-memory bank conflicts of the ranked accesses and latency, about a third each;
-// occupancy and block size change little.  8.4 M slots, 32768 rows: 76 -> 55 us per pass.
-template <typename KeyT, int kItems> constexpr int scatter_smem() { return kThreads * kItems * static_cast<int>(4 + sizeof(KeyT)); }
+// In the first pass with 16-bit keys a value is its position, so key and position inside the block share a staged word (139 -> 134 us
+// for the whole sort, with fourteen entries a thread).
+// What bounds it: instruction issue (0.5 a cycle and scheduler), shared-memory bank conflicts of the ranked accesses and latency, about
+// a third each.  8.4 M slots, 32768 rows: 76 -> 52 us per pass.
+template <typename KeyT, int kItems> constexpr int scatter_smem() {
+    constexpr int kEntries = kThreads * kItems * static_cast<int>(4 + sizeof(KeyT)), kWords = kRuns * kMaxRadix * 4;
+    return kEntries > kWords ? kEntries : kWords;      // staged entries; before them block_rank's words
+}
 
-template <typename KeyT, bool kFirst, bool kLast, int kItems>
+template <typename KeyT, bool kFirst, bool kLast, int kItems, bool kMasks>
 __global__ void __launch_bounds__(kThreads, 2)
 scatter_kernel(const KeyT* __restrict__ keys_in, const int32_t* __restrict__ vals_in, const Source src, KeyT* __restrict__ keys_out,
                int32_t* __restrict__ vals_out, const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, uint32_t n,
                int shift, uint32_t mask, int n_blocks, int32_t* __restrict__ row_ptr) {
     constexpr int kBlockItems = kThreads * kItems, kWarpItems = 32 * kItems;
+    // in the first pass a value is its position: key and position inside the block share a word
+    constexpr bool kPacked = kFirst && sizeof(KeyT) == 2;
+    static_assert(kBlockItems <= 65536, "positions inside a block in 16 bits");
     extern __shared__ __align__(16) uint32_t staged[];
     int32_t* svals = reinterpret_cast<int32_t*>(staged);
     KeyT* skeys = reinterpret_cast<KeyT*>(staged + kBlockItems);
@@ -274,25 +304,29 @@ scatter_kernel(const KeyT* __restrict__ keys_in, const int32_t* __restrict__ val
         for (int t = 0; t < kItems; ++t) keys[t] = src.key(first + t * 32, static_cast<int>(keys[t]));
     }
     const uint32_t digit0 = block_exclusive_scan(tot, sh.warp_sums, &sh.total);
-    block_rank(keys, shift, mask, first, n, sh, pos);
+    block_rank<kMasks>(keys, shift, mask, first, n, sh, staged, pos);
     if (threadIdx.x < radix) out_base[threadIdx.x] = digit0 + blk - sh.local_base[threadIdx.x];
 #pragma unroll
     for (int t = 0; t < kItems; ++t) {
         const uint32_t i = first + t * 32;
         if (i < n) {
-            skeys[pos[t]] = static_cast<KeyT>(keys[t]);
-            svals[pos[t]] = kFirst ? static_cast<int32_t>(i) : __ldg(vals_in + i);
+            if constexpr (kPacked) {
+                staged[pos[t]] = keys[t] << 16 | (i - block0);
+            } else {
+                skeys[pos[t]] = static_cast<KeyT>(keys[t]);
+                svals[pos[t]] = kFirst ? static_cast<int32_t>(i) : __ldg(vals_in + i);
+            }
         }
     }
     __syncthreads();
     const uint32_t count = min(n - block0, static_cast<uint32_t>(kBlockItems));
 #pragma unroll 8
     for (uint32_t j = threadIdx.x; j < count; j += kThreads) {
-        const uint32_t key = skeys[j];
+        const uint32_t key = kPacked ? staged[j] >> 16 : skeys[j];
         const uint32_t at = out_base[digit_of(key, shift, mask)] + j;
-        vals_out[at] = svals[j];
+        vals_out[at] = kPacked ? static_cast<int32_t>(block0 + (staged[j] & 0xffffu)) : svals[j];
         if (!kLast) keys_out[at] = static_cast<KeyT>(key);
-        else if (j == 0 || skeys[j - 1] != key) atomicMin(row_ptr + key, static_cast<int32_t>(at));
+        else if (j == 0 || (kPacked ? staged[j - 1] >> 16 : skeys[j - 1]) != key) atomicMin(row_ptr + key, static_cast<int32_t>(at));
     }
 }
 
@@ -382,7 +416,7 @@ row_ptr_kernel(const int32_t* __restrict__ heads, const int32_t* __restrict__ fi
 template <typename KeyT>
 __global__ void __launch_bounds__(kThreads, 1)
 small_sort_kernel(const Source src, KeyT* __restrict__ keys_out, int32_t* __restrict__ vals_out, uint32_t n, int passes, int digit_bits) {
-    constexpr int kItems = kItemsLarge, kBlockItems = kSmallInput, kWarpItems = 32 * kItems;
+    constexpr int kItems = kItemsSmall, kBlockItems = kSmallInput, kWarpItems = 32 * kItems;
     extern __shared__ __align__(16) uint32_t staged[];
     int32_t* svals = reinterpret_cast<int32_t*>(staged);
     KeyT* skeys = reinterpret_cast<KeyT*>(staged + kBlockItems);
@@ -400,7 +434,7 @@ small_sort_kernel(const Source src, KeyT* __restrict__ keys_out, int32_t* __rest
         vals[t] = i;
     }
     for (int pass = 0; pass < passes; ++pass) {
-        block_rank(keys, pass * digit_bits, mask, first, n, sh, pos);
+        block_rank<true>(keys, pass * digit_bits, mask, first, n, sh, staged, pos);
 #pragma unroll
         for (int t = 0; t < kItems; ++t)
             if (first + t * 32 < n) {
