@@ -801,9 +801,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // [128 keys x 64 columns]), then V of tile n (eight slots of [64 keys x 128 columns]); a slot feeds four UMMAs of 64
 // cycles either way, and the softmax of tile n runs under the UMMAs of S n + 1.
 //   warps 0-15  softmax: warp w reads lane quarter w % 4, columns [32 (w / 4), + 32) of S: one head, 32 keys per thread
-//   warps 16-23 gather producers (cp.async 16 B, swizzled)
-//   warp 24     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full" and "my P is written"
-//   warp 25     TMA of the CTA's Q chunks
+//   warps 16-19 gather producers (cp.async 16 B, swizzled)
+//   warp 20     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full" and "my P is written"
+//   warp 21     TMA of the CTA's Q chunks
 // The exponentials of a tile are taken against the maximum of the row so far; where a tile raises it, O and the sum are
 // rescaled.  A reference that lags behind the maximum (moved only when exceeded by 2^8) makes most of the rescaling
 // unnecessary and is 3 % faster (128 heads, 2.34 against 2.42 ms), but the heaviest probabilities then lose in their rounding
@@ -823,7 +823,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // =============================================================================================
 namespace ff {
 constexpr int kSoftmaxWarps = 16;
-constexpr int kProducerThreads = 256;
+constexpr int kProducerThreads = 128;
 constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 64;
 constexpr int kIssueWarp = kThreads / 32 - 2, kLoadWarp = kThreads / 32 - 1;
 constexpr int kParts = 8;                  // a head's 256 keys of a tile over eight warps
@@ -832,7 +832,6 @@ constexpr int kSlotBytes = 16384;
 constexpr int kStages = 7;
 constexpr int kQChunk = 64 * 128;          // [64 head rows x 64 columns]
 constexpr int kPChunk = 64 * 128;          // [64 head rows x 64 keys]
-constexpr int kVSlots = 8;                 // per tile: four groups of 64 keys x two d-blocks
 constexpr int kOffQ = 0;
 constexpr int kOffP = kQChunks * kQChunk;
 constexpr int kOffRing = kOffP + 4 * kPChunk;
@@ -842,6 +841,11 @@ constexpr int kOffMisc = kOffStat + 2 * kParts * 64 * 4;
 constexpr int kSmemBytes = kOffMisc + 512 + 1024;             // barriers + alignment slack
 constexpr int kTmemO = 0, kTmemS = 256;
 static_assert(kSmemBytes <= 232448, "shared memory of one SM");
+// Groups of 64 keys (two slots each) up to the last slot in use of the iterator's tile: what lies behind takes no part in P V.  4096
+// queries x 128 heads x top-k 100 418 -> 370 us, 3000 x 64 heads x 330 428 -> 388, 4000 x 128 heads of a causal prefix 2268 -> 2079; full
+// tiles alike (128 heads) or 2.5 % faster (64).  It takes loops with variable ends, and with eight producer warps (72 registers a
+// thread) those spilled: full tiles 2 - 13 % slower.  Four producer warps leave 80 registers.
+__device__ __forceinline__ int v_groups(const TileIter<1>& it) { return (min(kTileKeys, it.n_cur - it.tile() * kTileKeys) + 63) >> 6; }
 }  // namespace ff
 
 // lse of a row that has a valid slot (the prep kernel writes the rows of a query that has none) from the reference of its
@@ -937,7 +941,8 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 
     if (warp >= kSoftmaxWarps && warp < kIssueWarp) {
         // ------------------------------------------------------------------ gather producers
-        const int pt = threadIdx.x - kSoftmaxWarps * 32;   // 0..255
+        const int pt = threadIdx.x - kSoftmaxWarps * 32;   
+        constexpr int kRowsK = kProducerThreads / 8, kRowsV = kProducerThreads / 16;     // rows that the producers copy side by side
         const char* kvb = reinterpret_cast<const char*>(p.kv);
         const uint64_t pol_keep = l2_policy_evict_last();
         int* rows = reinterpret_cast<int*>(smem + kOffRows);
@@ -953,11 +958,16 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         // key pt of every tile: raw index loaded one tile ahead, turned into a kv row when it is published
         TileIter<1> it(p, range);
         QMeta qm = load_qmeta(p, range.q);
+        constexpr int kKeys = kTileKeys / kProducerThreads;
+        int idx_next[kKeys];
         auto load_idx = [&]() {
-            const int key = it.tile() * kTileKeys + pt;
-            return it.more() && key < p.topk ? __ldg(p.indices + static_cast<size_t>(it.q) * p.topk + key) : -1;
+#pragma unroll
+            for (int i = 0; i < kKeys; ++i) {
+                const int key = it.tile() * kTileKeys + pt + i * kProducerThreads;
+                idx_next[i] = it.more() && key < p.topk ? __ldg(p.indices + static_cast<size_t>(it.q) * p.topk + key) : -1;
+            }
         };
-        int idx_next = load_idx();
+        load_idx();
         auto next_slot = [&]() {
             cp_async_mbar_arrive_noinc(bar_full + 8 * s);
             if (++s == kStages) {
@@ -965,19 +975,22 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 ph ^= 1;
             }
         };
-        for (int n = -1; n < n_tiles; ++n) {            // K of tile n + 1, then V of tile n
+        int groups = 0, groups_next = 0;                // V's groups of 64 keys: of tile n, of tile n + 1
+        for (int n = -1; n < n_tiles; ++n, groups = groups_next) {            // K of tile n + 1, then V of tile n
             if (n + 1 < n_tiles) {
                 // three buffers: the one written now was last read two steps ago, before the previous step's barrier
                 int* mine = rows + (n + 1) % 3 * kTileKeys;
-                mine[pt] = gather_row(idx_next, qm, p);
-                if (it.advance() && it.more()) qm = load_qmeta(p, it.q);
-                idx_next = load_idx();
-                asm volatile("bar.sync 3, 256;" ::: "memory");
-                const char* src[4];
-                uint32_t nb[4];             // 0: slot out of range, read nothing and land zeros
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = mine[rank * 128 + rk + 32 * i];
+                for (int i = 0; i < kKeys; ++i) mine[pt + i * kProducerThreads] = gather_row(idx_next[i], qm, p);
+                groups_next = v_groups(it);
+                if (it.advance() && it.more()) qm = load_qmeta(p, it.q);
+                load_idx();
+                asm volatile("bar.sync 3, %0;" ::"n"(kProducerThreads) : "memory");
+                const char* src[128 / kRowsK];
+                uint32_t nb[128 / kRowsK];  // 0: slot out of range, read nothing and land zeros
+#pragma unroll
+                for (int i = 0; i < 128 / kRowsK; ++i) {
+                    const int row = mine[rank * 128 + rk + kRowsK * i];
                     nb[i] = row >= 0 ? 16u : 0u;
                     src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2) + uk * 16;
                 }
@@ -985,18 +998,19 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     mbar_wait(bar_empty + 8 * s, ph, wc, kErrFwd + 11, kPollSleepNs);
                     const uint32_t d = dst_k + s * kSlotBytes;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cp_async16_zfill_hint(d + i * 32 * 128, src[i] + j * 128, nb[i], pol_keep);
+                    for (int i = 0; i < 128 / kRowsK; ++i) cp_async16_zfill_hint(d + i * kRowsK * 128, src[i] + j * 128, nb[i], pol_keep);
                     next_slot();
                 }
             }
             if (n >= 0) {
                 const int* mine = rows + n % 3 * kTileKeys;
-                for (int g = 0; g < 4; ++g) {
-                    const char* src[4];
-                    uint32_t nb[4];
+#pragma unroll 1
+                for (int g = 0; g < groups; ++g) {
+                    const char* src[64 / kRowsV];
+                    uint32_t nb[64 / kRowsV];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int row = mine[g * 64 + rv + 16 * i];
+                    for (int i = 0; i < 64 / kRowsV; ++i) {
+                        const int row = mine[g * 64 + rv + kRowsV * i];
                         nb[i] = row >= 0 ? 16u : 0u;
                         src[i] = src_v + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
                     }
@@ -1005,7 +1019,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                         mbar_wait(bar_empty + 8 * s, ph, wc, kErrFwd + 11, kPollSleepNs);
                         const uint32_t d = dst_v + s * kSlotBytes;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cp_async16_zfill_hint(d + i * 16 * 128, src[i] + b * 512, nb[i], pol_keep);
+                        for (int i = 0; i < 64 / kRowsV; ++i) cp_async16_zfill_hint(d + i * kRowsV * 128, src[i] + b * 512, nb[i], pol_keep);
                         next_slot();
                     }
                 }
@@ -1036,9 +1050,10 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 uint32_t qpar = 0;
                 TileIter<1> it(p, range);
                 bool new_query = true;
-                for (int n = -1; n < n_tiles; ++n) {
+                int groups = 0, groups_next = 0;
+                for (int n = -1; n < n_tiles; ++n, groups = groups_next) {
                     const int k_slots = n + 1 < n_tiles ? kQChunks : 0;
-                    const int slots = k_slots + (n >= 0 ? kVSlots : 0);
+                    const int slots = k_slots + 2 * groups;
                     for (int j = 0; j < slots; ++j) {
                         if (j == k_slots) {          // P of tile n, in front of the V it is multiplied with
                             mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
@@ -1057,6 +1072,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                         mbar_arrive_cluster_relaxed(full_even + 8 * s);
                     }
                     if (k_slots) {
+                        groups_next = v_groups(it);
                         new_query = it.advance();
                         if (new_query) qpar ^= 1;
                     }
@@ -1076,14 +1092,15 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 TileIter<1> it(p, range);
                 bool new_query = true;
                 uint32_t first_bits = 0;      // bit n & 1: tile n is its query's first in this range
-                for (int n = -1; n < n_tiles; ++n) {
+                int groups = 0, groups_next = 0;
+                for (int n = -1; n < n_tiles; ++n, groups = groups_next) {
                     if (n + 1 < n_tiles) {
                         // S of tile n + 1
                         const int t = n + 1, b = t & 1;
                         const bool last = it.last_of_query();
                         mbar_wait(bar_tempty + 8 * b, ((t >> 1) & 1) ^ 1, wc, kErrFwd + 13);
                         const uint32_t d = tmem + kTmemS + b * 128;
-#pragma unroll
+#pragma unroll 1
                         for (int j = 0; j < kQChunks; ++j) {
                             if (new_query) mbar_wait(bar_qfull + 8 * j, qpar, wc, kErrFwd + 12);
                             ring.wait(wc, kErrFwd + 14);
@@ -1099,6 +1116,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                             if (last) umma_commit_2cta_mask(bar_qfree + 8 * j, 3);   // the next query's chunk may come in
                         }
                         umma_commit_2cta_mask(bar_tfull + 8 * b, 3);
+                        groups_next = v_groups(it);
                         first_bits = (first_bits & ~(1u << b)) | (static_cast<uint32_t>(new_query) << b);
                         new_query = it.advance();
                         if (new_query) qpar ^= 1;
@@ -1107,20 +1125,22 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                         // O += P V of tile n
                         const uint32_t acc0 = ((first_bits >> (n & 1)) & 1u) ^ 1u;
                         mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 19);
+#pragma unroll 1
+                        for (int g = 0; g < groups; ++g) {
 #pragma unroll
-                        for (int v = 0; v < kVSlots; ++v) {
-                            const int g = v >> 1, b = v & 1;
-                            ring.wait(wc, kErrFwd + 14);
-                            const uint32_t s = ring.slot;
-                            ring.next();
-                            fence_proxy_async_smem();        // the slot was written by cp.async, the tensor core reads it
-                            tc_fence_after_sync();
-                            const uint32_t a = p_lo + g * (kPChunk >> 4), bb = v_lo + s * (kSlotBytes >> 4);
+                            for (int b = 0; b < 2; ++b) {
+                                ring.wait(wc, kErrFwd + 14);
+                                const uint32_t s = ring.slot;
+                                ring.next();
+                                fence_proxy_async_smem();        // the slot was written by cp.async, the tensor core reads it
+                                tc_fence_after_sync();
+                                const uint32_t a = p_lo + g * (kPChunk >> 4), bb = v_lo + s * (kSlotBytes >> 4);
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)   // 16 keys: 32 bytes along P's rows, 16 rows (2 KB) of V
-                                umma_ss_2cta(tmem + kTmemO + b * 128, k_hi | (a + 2 * kk), v_hi | (bb + kk * (2048 >> 4)), idesc_o,
-                                             (g | kk) != 0 ? 1u : acc0);
-                            umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                                for (int kk = 0; kk < 4; ++kk)   // 16 keys: 32 bytes along P's rows, 16 rows (2 KB) of V
+                                    umma_ss_2cta(tmem + kTmemO + b * 128, k_hi | (a + 2 * kk), v_hi | (bb + kk * (2048 >> 4)), idesc_o,
+                                                 (g | kk) != 0 ? 1u : acc0);
+                                umma_commit_2cta_mask(bar_empty + 8 * s, 3);
+                            }
                         }
                         umma_commit_2cta_mask(bar_pv, 3);
                     }
