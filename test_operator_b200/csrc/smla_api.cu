@@ -567,7 +567,11 @@ int launch_fwd_chain(const smla_fwd_params* p, const FwdPlan& pl, uint8_t* ws, c
     launch(smla_fwd_kernel<HP>, 2 * clusters, ff::kThreads, ff::kSmemBytes, st, true, 1, tm_q, kp);
     if (clusters > 1 && (!kp.every_slot || q_tiles > 1)) {
         const int items = p->s_q < clusters ? p->s_q : clusters - 1;
-        launch(smla_fwd_combine_kernel, items * ((p->h_q + 31) / 32 * 4), 256, 0, st, true, 1, kp, clusters, HP);
+        const int grid = items * ((p->h_q + 31) / 32 * (1024 / kCombineThreads));
+        // (as many queries as clusters, of about equal length: a query lies in two ranges, seldom in three)
+        const bool two_parts = kp.every_slot ? q_tiles <= 2 : p->s_q >= clusters;
+        if (two_parts) launch(smla_fwd_combine_kernel<2>, grid, kCombineThreads, 0, st, true, 1, kp, clusters, HP);
+        else launch(smla_fwd_combine_kernel<4>, grid, kCombineThreads, 0, st, true, 1, kp, clusters, HP);
     }
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }

@@ -1348,14 +1348,20 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 // 1 KB, and a lane's weights need no other lane.  The first parts' O is asked for together with all references and sums.
 // Parts are added in their order.  Bound by the latency of its dependent loads; eight queries of eight parts: 5.5 us of a call,
 // 7.6 us with a warp per head and half of the columns, whose weights took two rounds of loads before the first row.
-constexpr int kCombineFly = 4;                   // parts in flight
-__global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
+// Blocks are small, so that many of them are in place beside the forward kernel's last blocks when it ends.  kFly: parts in flight, two
+// where no query has more (72 registers a thread instead of 112).  30 queries x 128 heads x top-k 512 18.2 us a call with blocks of
+// 256 and four parts, 17.4 so; 90 queries x 600 41.6 / 39.4; one query x 2048 (eight parts) 15.4 / 14.9; eight x 2048 alike, and
+// 19.4 -> 22.9 with two parts in flight.
+constexpr int kCombineThreads = 64;
+template <int kFly>
+__global__ void __launch_bounds__(kCombineThreads) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const int per_item = (p.h_q + 31) / 32 * 4;  // blocks: eight of the 32 column groups each
+    constexpr int kCols = kCombineThreads / 32, kBlocks = 32 / kCols;      // column groups of a block, blocks of 32 heads
+    const int per_item = (p.h_q + 31) / 32 * kBlocks;
     const int item = static_cast<int>(blockIdx.x) / per_item, in_item = static_cast<int>(blockIdx.x) % per_item;
-    const int head = in_item / 4 * 32 + lane, col = (in_item % 4 * 8 + static_cast<int>(threadIdx.x >> 5)) * 16;
+    const int head = in_item / kBlocks * 32 + lane, col = (in_item % kBlocks * kCols + static_cast<int>(threadIdx.x >> 5)) * 16;
     int q, n_tiles, q_begin, q_end;
     if (p.every_slot) {
         const int tiles = work_tiles(p.every_slot);
@@ -1400,18 +1406,18 @@ __global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, 
         }
     };
     const float ninf = __int_as_float(0xff800000);
-    uint32_t v[kCombineFly][2][8];
-    float2 ml[kCombineFly];
+    uint32_t v[kFly][2][8];
+    float2 ml[kFly];
 #pragma unroll
-    for (int u = 0; u < kCombineFly; ++u) load_part(first + u, v[u], ml[u]);
+    for (int u = 0; u < kFly; ++u) load_part(first + u, v[u], ml[u]);
     float ref = ninf, sum = 0.f, acc[16];
     bool any = false;
 #pragma unroll
-    for (int u = 0; u < kCombineFly; ++u) {
+    for (int u = 0; u < kFly; ++u) {
         ref = fmaxf(ref, ml[u].x);               // -inf: no valid slot in this part, or none above -inf
         any = any || ml[u].y != kNoSlot;
     }
-    for (int k = first + kCombineFly; k <= last; ++k) {
+    for (int k = first + kFly; k <= last; ++k) {
         const int slot = slot_of(k);
         if (slot < 0) continue;
         const float2 x = __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head);
@@ -1422,17 +1428,17 @@ __global__ void __launch_bounds__(256) smla_fwd_combine_kernel(const KParams p, 
     for (int i = 0; i < 16; ++i) acc[i] = 0.f;
     for (int k = first;;) {
 #pragma unroll
-        for (int u = 0; u < kCombineFly; ++u) {
+        for (int u = 0; u < kFly; ++u) {
             const float w = ml[u].x > ninf ? ex2_approx(ml[u].x - ref) : 0.f;
             sum = fmaf(w, ml[u].y, sum);
             // (a part of weight 0 counts too: its O may hold a NaN)
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[i] = fmaf(__uint_as_float(v[u][i / 8][i % 8]), w, acc[i]);
         }
-        k += kCombineFly;
+        k += kFly;
         if (k > last) break;
 #pragma unroll
-        for (int u = 0; u < kCombineFly; ++u) load_part(k + u, v[u], ml[u]);
+        for (int u = 0; u < kFly; ++u) load_part(k + u, v[u], ml[u]);
     }
     const size_t orow = static_cast<size_t>(q) * p.h_q + head;
     if (col == 0) p.lse_out[orow] = any ? row_lse(ref, sum) * p.lse_out_mult : no_slot_lse(p);
