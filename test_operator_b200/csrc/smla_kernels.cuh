@@ -81,10 +81,14 @@ __device__ __forceinline__ QMeta load_qmeta(const KParams& p, int q_global) {
     }
     return QMeta{0, p.s_kv, p.q_start + q_global, p.topk};
 }
-// kv row a slot gathers from, -1 when the index is outside the query's sequence (nothing is read then)
-__device__ __forceinline__ int gather_row(int idx, const QMeta& m, const KParams& p) {
-    const int row = m.kv_base + idx;
-    return (idx >= 0 && idx < m.kv_len && row < p.s_kv) ? row : -1;
+__device__ __forceinline__ bool slot_valid(int idx, int key, const QMeta& m, const KParams& p) {
+    return key < m.topk_len && idx >= 0 && idx < m.kv_len && m.kv_base + idx < p.s_kv && (!p.causal || idx <= m.q_pos);
+}
+// kv row a slot gathers from, -1 for one that takes no part (nothing is read then, zeros land).  The whole rule, not the range alone:
+// the contractions over keys multiply a masked slot's row by an exact 0, and a masked slot may name a row that holds NaN or an
+// infinity (one of a cache that has not been written yet).
+__device__ __forceinline__ int gather_row(int idx, int key, const QMeta& m, const KParams& p) {
+    return slot_valid(idx, key, m, p) ? m.kv_base + idx : -1;
 }
 // After a bounded wait has given up: let this thread's own cp.async land and leave in-flight TMA loads (they
 // depend on nothing and complete within microseconds) the time to land before the CTA gives up its shared memory.
@@ -106,10 +110,6 @@ __device__ __forceinline__ size_t scratch_offset(int key, int head, int topk_pad
 
 // error codes recorded by bounded waits: 100*kernel + site
 enum { kErrRecompute = 100, kErrDkv = 200, kErrDq = 300, kErrFwd = 400 };
-
-__device__ __forceinline__ bool slot_valid(int idx, int key, const QMeta& m, const KParams& p) {
-    return key < m.topk_len && idx >= 0 && idx < m.kv_len && m.kv_base + idx < p.s_kv && (!p.causal || idx <= m.q_pos);
-}
 
 __device__ __forceinline__ float dot8_bf16(const uint4& a, const uint4& b, float acc) {
     const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
@@ -505,14 +505,14 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         int s = 0;
         uint32_t ph = 1;                    // parity that means "slot free" for the current pass over the ring
         while (it.more()) {
-            // A slot whose index is out of range reads nothing and lands as zeros (its S, dS are forced to 0
+            // A slot that takes no part reads nothing and lands as zeros (its S, dS are forced to 0
             // anyway).  Sending all of them to one stand-in row instead would make that row's cache lines a
             // hot spot that every SM queues on.
             const char* src[4];
             uint32_t nb[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int row = gather_row(idx_next[i], qm_next, p);
+                const int row = gather_row(idx_next[i], it.tile() * kTileKeys + static_cast<int>(rank) * 128 + r0 + 32 * i, qm_next, p);
                 nb[i] = row >= 0 ? 16u : 0u;
                 src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
             }
@@ -981,13 +981,16 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                 // three buffers: the one written now was last read two steps ago, before the previous step's barrier
                 int* mine = rows + (n + 1) % 3 * kTileKeys;
 #pragma unroll
-                for (int i = 0; i < kKeys; ++i) mine[pt + i * kProducerThreads] = gather_row(idx_next[i], qm, p);
+                for (int i = 0; i < kKeys; ++i) {
+                    const int at = pt + i * kProducerThreads;
+                    mine[at] = gather_row(idx_next[i], it.tile() * kTileKeys + at, qm, p);
+                }
                 groups_next = v_groups(it);
                 if (it.advance() && it.more()) qm = load_qmeta(p, it.q);
                 load_idx();
                 asm volatile("bar.sync 3, %0;" ::"n"(kProducerThreads) : "memory");
                 const char* src[128 / kRowsK];
-                uint32_t nb[128 / kRowsK];  // 0: slot out of range, read nothing and land zeros
+                uint32_t nb[128 / kRowsK];  // 0: the slot takes no part, read nothing and land zeros
 #pragma unroll
                 for (int i = 0; i < 128 / kRowsK; ++i) {
                     const int row = mine[rank * 128 + rk + kRowsK * i];
@@ -1967,10 +1970,10 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         uint32_t ph = 1;                    // parity that means "stage free" for the current pass over the ring
         for (int tile = 0; tile < n_tiles; ++tile) {
             const char* src[2];
-            uint32_t nb[2];   // 0: slot out of range, read nothing and land zeros (no shared stand-in row: it would be a hot spot)
+            uint32_t nb[2];   // 0: the slot takes no part, read nothing and land zeros (no shared stand-in row: it would be a hot spot)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int row = gather_row(idx_next[i], qm, p);
+                const int row = gather_row(idx_next[i], (tile0 + tile) * kTileKeys + r0 + 32 * i, qm, p);
                 nb[i] = row >= 0 ? 16u : 0u;
                 src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
             }
