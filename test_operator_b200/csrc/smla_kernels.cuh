@@ -463,10 +463,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         tmem_alloc_2cta(smem_u32(tmem_slot), C::kTmemCols);
         tmem_relinquish_2cta();
     }
-    if (!p.own_prep) {           // slot counts and Delta of the prep kernel; the scratch's previous readers are done
-        pdl_wait();
-        pdl_trigger();
-    }
+    if (!p.own_prep) pdl_wait();     // slot counts and Delta of the prep kernel; the scratch's previous readers are done
     find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(lse_s), range_s);   // (lse_s: not in use yet)
     tc_fence_before_sync();
     __syncthreads();
@@ -475,10 +472,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
     static_assert(kTileKeys == kWorkTileKeys, "one work tile per accumulator");
-    if (p.own_prep) {            // nothing of the caller's has been touched so far
-        pdl_wait();
-        pdl_trigger();
-    }
+    if (p.own_prep) pdl_wait();      // nothing of the caller's has been touched so far
+    pdl_trigger();                   // (the tensor memory is this CTA's: see the dq kernel)
 
     if (warp >= 8 && warp < 16) {
         // ------------------------------------------------------------------ gather producers
@@ -921,10 +916,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
         tmem_relinquish_2cta();
     }
     if (warp == kLoadWarp && lane == 0) tma_prefetch_desc(&tm_q);
-    if (!p.every_slot) {
-        pdl_wait();              // the prep kernel's slot counts
-        pdl_trigger();
-    }
+    if (!p.every_slot) pdl_wait();   // the prep kernel's slot counts
     const int total = find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + kOffStat), range_s);
     if (total >= 0 && rank == 0 && !p.every_slot) p.range_q[blockIdx.x >> 1] = make_int4(range_s->q, range_s->lo, total, 0);
     tc_fence_before_sync();
@@ -934,10 +926,8 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
     const int n_tiles = range.end - range.begin;
-    if (p.every_slot) {          // nothing of the caller's has been touched so far
-        pdl_wait();
-        pdl_trigger();
-    }
+    if (p.every_slot) pdl_wait();    // nothing of the caller's has been touched so far
+    pdl_trigger();                   // (the tensor memory is this CTA's: see the dq kernel)
 
     if (warp >= kSoftmaxWarps && warp < kIssueWarp) {
         // ------------------------------------------------------------------ gather producers
@@ -1919,9 +1909,6 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const WaitCtx wc{p.g_err, s_abort, p.wait_limit, 0u};
 
-    // A chain of small kernels ends here: the next one of the stream may come up to its own wait (64 queries x 16 heads x top-k 64:
-    // 20.6 -> 19.6 us).  Large grids keep their SMs to themselves: 37 queries x 128 heads x 2048 116 -> 119 us with it.
-    if (p.every_slot) pdl_trigger();
     if (threadIdx.x == 0) {
         *s_abort = 0;
         for (int i = 0; i < kStages; ++i) {
@@ -1940,6 +1927,11 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    // A chain of small kernels ends here: the next one of the stream may come up to its own wait (64 queries x 16 heads x top-k 64:
+    // 20.6 -> 19.6 us).  Large grids keep their SMs to themselves: 37 queries x 128 heads x 2048 116 -> 119 us with it.
+    // Not before this CTA has its tensor memory: a block of the next kernel that fits beside it could take all of it and then wait for
+    // this grid to end, which waits for its share.
+    if (p.every_slot) pdl_trigger();
     // Behind the dKV kernel's trigger everything this kernel reads is in place already (that kernel triggers after it has
     // waited for the recompute kernel), so its CTAs fill whatever SMs the dKV kernel leaves; the last CTA then holds the
     // grid open until the dKV kernel is done, so that "dq done" still means "all done" to whatever follows.
