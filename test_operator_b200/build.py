@@ -5,10 +5,12 @@
 """
 from __future__ import annotations
 
+import hashlib
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -17,7 +19,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libsmla_bwd.so")
 
 HOST_SOURCE = os.path.join(CSRC, "smla_host.cpp")
-HOST_PATH = os.path.join(LIB_DIR, "_smla_host.so")
+HOST_HEADER = os.path.join(ROOT, "include", "smla_bwd.h")
 
 SOURCES = ["smla_api.cu"]
 HEADERS = ["sm100_ptx.cuh", "smla_kernels.cuh", "smla_index_inverse.cuh"]
@@ -38,49 +40,60 @@ def _nvcc() -> str:
 
 
 def needs_build() -> bool:
-    return _older(LIB_PATH, [os.path.join(CSRC, f) for f in SOURCES + HEADERS])
-
-
-def host_needs_build() -> bool:
-    return _older(HOST_PATH, [HOST_SOURCE])
-
-
-def _older(path: str, sources) -> bool:
-    if not os.path.exists(path):
+    if not os.path.exists(LIB_PATH):
         return True
-    t = os.path.getmtime(path)
-    return any(os.path.getmtime(d) > t for d in [*sources, os.path.join(ROOT, "include", "smla_bwd.h")])
+    t = os.path.getmtime(LIB_PATH)
+    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.join(ROOT, "include", "smla_bwd.h")]
+    return any(os.path.getmtime(d) > t for d in deps)
+
+
+def host_path() -> str:
+    """Where the host module for this interpreter, this torch and these sources lies.  All of them are in its name: it goes by torch's
+    C++ interface and by the structs of the C header, so one that was built for others must not be loaded."""
+    import torch
+    tag = hashlib.sha256(torch.__version__.encode())
+    for path in (HOST_SOURCE, HOST_HEADER):
+        with open(path, "rb") as f:
+            tag.update(f.read())
+    return os.path.join(LIB_DIR, "_smla_host." + tag.hexdigest()[:16] + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if force or needs_build():
-        _run([_nvcc()] + NVCC_FLAGS + [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB_PATH], "build.log", verbose)
-    if force or host_needs_build():
+        _compile([_nvcc()] + NVCC_FLAGS + [os.path.join(CSRC, s) for s in SOURCES], LIB_PATH, "build.log", verbose)
+    if force or not os.path.exists(host_path()):
         build_host(verbose)
     return LIB_PATH
 
 
 def build_host(verbose: bool = False) -> str:
     """The CPython module of csrc/smla_host.cpp (no kernels in it): the host compiler against torch's headers."""
-    import sysconfig
-
     from torch.utils import cpp_extension
+    path = host_path()
     cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
     inc = [sysconfig.get_paths()["include"], os.path.join(cuda_home, "include"), *cpp_extension.include_paths()]
-    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", *(f"-I{d}" for d in inc), HOST_SOURCE, "-o", HOST_PATH,
-           *(f"-L{d}" for d in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
-    _run(cmd, "build_host.log", verbose)
-    return HOST_PATH
+    _compile([shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", *(f"-I{d}" for d in inc), HOST_SOURCE,
+              *(f"-L{d}" for d in cpp_extension.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"], path,
+             "build_host.log", verbose)
+    return path
 
 
-def _run(cmd, log_name: str, verbose: bool) -> None:
+def _compile(cmd, path: str, log_name: str, verbose: bool) -> None:
+    """Runs the compiler.  `path` shows up when the file is whole: ranks that start together may all build it, and load it meanwhile."""
     os.makedirs(LIB_DIR, exist_ok=True)
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    log = res.stdout + res.stderr
-    with open(os.path.join(LIB_DIR, log_name), "w") as f:
-        f.write(" ".join(cmd) + "\n" + log)
-    if res.returncode != 0:
-        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + log[-4000:])
+    part = f"{path}.{os.getpid()}.part"
+    cmd = [*cmd, "-o", part]
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        log = res.stdout + res.stderr
+        with open(os.path.join(LIB_DIR, log_name), "w") as f:
+            f.write(" ".join(cmd) + "\n" + log)
+        if res.returncode != 0:
+            raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + log[-4000:])
+        os.replace(part, path)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
     if verbose:
         print(log)
 

@@ -173,7 +173,7 @@ def load_library() -> ctypes.CDLL:
 # quick look at its arguments is checked, given its outputs and queued by a small compiled module (csrc/smla_host.cpp); everything
 # else takes the way below, with the itemised checks and their messages.
 class _NoNativeHost:
-    """Without the compiled host module (no compiler, say) every call takes the Python way."""
+    """Where the compiled host module cannot be built or loaded (no compiler, say) every call takes the Python way."""
 
     @staticmethod
     def fwd(*_):
@@ -200,18 +200,18 @@ def _host():
 
 def _load_host(lib):
     try:
-        if _build.host_needs_build():
+        path = _build.host_path()
+        if not os.path.exists(path):
             _build.build_host()
+        loader = importlib.machinery.ExtensionFileLoader("_smla_host", path)
+        module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("_smla_host", loader, origin=path))
+        loader.exec_module(module)
+        module.init(*(ctypes.cast(f, ctypes.c_void_p).value for f in
+                      (lib.smla_fwd_run, lib.smla_fwd_workspace_size, lib.smla_bwd_run_stages, lib.smla_bwd_workspace_size)))
+        return module
     except Exception as e:
-        if not os.path.exists(_build.HOST_PATH):
-            warnings.warn(f"the compiled host module could not be built, calls take some 8 us longer: {e}")
-            return _NoNativeHost
-    loader = importlib.machinery.ExtensionFileLoader("_smla_host", _build.HOST_PATH)
-    module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("_smla_host", loader, origin=_build.HOST_PATH))
-    loader.exec_module(module)
-    module.init(*(ctypes.cast(f, ctypes.c_void_p).value for f in
-                  (lib.smla_fwd_run, lib.smla_fwd_workspace_size, lib.smla_bwd_run_stages, lib.smla_bwd_workspace_size)))
-    return module
+        warnings.warn(f"the compiled host module cannot be used, calls take some 8 us longer: {e}")
+        return _NoNativeHost
 
 
 # Here the current device is only switched when it has to be, the stream is taken as the raw handle, and workspace sizes are
