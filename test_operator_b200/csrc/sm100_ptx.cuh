@@ -353,13 +353,17 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Arrive on a barrier of another CTA with the cluster-scope release (address from map_to_cta).
+__device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 // Address of the same shared-memory location in CTA `rank` of the cluster (shared::cluster window).
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
-// Same without the cluster-scope release: that release costs the issuing thread about a thousand cycles per
+// mbar_arrive_cluster_release without the release: that release costs the issuing thread about a thousand cycles per
 // call, which a thread relaying one signal per pipeline step cannot afford.  Only for signals whose data is
 // already in place by other means: shared memory of the signalling CTA filled by copies this thread has seen
 // complete (and fenced to the async proxy), or tensor-memory reads this warp has waited for.
@@ -367,7 +371,7 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
 // on the two cases above and on measurement (a build with -DSMLA_RELEASE_ARRIVE gives bit-identical S, dS and dQ).
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_bar) {
 #ifdef SMLA_RELEASE_ARRIVE
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+    mbar_arrive_cluster_release(cluster_bar);
 #else
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 #endif

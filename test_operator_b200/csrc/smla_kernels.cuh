@@ -797,8 +797,9 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // cycles either way, and the softmax of tile n runs under the UMMAs of S n + 1.
 //   warps 0-15  softmax: warp w reads lane quarter w % 4, columns [32 (w / 4), + 32) of S: one head, 32 keys per thread
 //   warps 16-19 gather producers (cp.async 16 B, swizzled)
-//   warp 20     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full" and "my P is written"
+//   warp 20     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full"
 //   warp 21     TMA of the CTA's Q chunks
+//   warp 22     odd CTA: forwards "my P is written" (even CTA: idle)
 // The exponentials of a tile are taken against the maximum of the row so far; where a tile raises it, O and the sum are
 // rescaled.  A reference that lags behind the maximum (moved only when exceeded by 2^8) makes most of the rescaling
 // unnecessary and is 3 % faster (128 heads, 2.34 against 2.42 ms), but the heaviest probabilities then lose in their rounding
@@ -809,18 +810,19 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // What bounds it: per tile and CTA 17 slots x 4 UMMAs x 64 cycles = 4352 cycles of tensor pipe; 275 KB of gathered rows
 // written and 408 KB of operands read in shared memory, 5350 cycles at 128 B/clk.  Eight softmax warps of 64 keys a thread were
 // busy 95 % of a launch, the issuer waiting 1900 cycles a tile for P (8330 cycles a tile, 128 heads).  Sixteen warps of 32 keys
-// hide each other's latency, P is announced by a local arrival that the odd CTA's relay thread forwards (a cluster-scope release
-// by every warp held it for hundreds of cycles): the issuer's wait for P is below 100 cycles, what is left are waits for gathered
-// slots.  4096 queries x 128 heads x top-k 2048: 2657 -> 2250 us on a cool GPU, 2521 -> 2445 back to back, where the power cap
-// holds the clock down.  Five, six or seven ring slots made no difference before.
+// hide each other's latency, P is announced by a local arrival that a thread of the odd CTA forwards (a cluster-scope release by
+// every warp held it for hundreds of cycles): what is left are waits for gathered slots.  4096 queries x 128 heads x top-k 2048
+// back to back, where the power cap holds the clock down: 2568 us with eight warps, 2458 with sixteen and a forwarded arrival that
+// released nothing, 2 % above that as it is (see warp 22).  Five, six and seven ring slots were compared with eight warps only (2.48 /
+// 2.47 / 2.48 ms), when the ring was not what the issuer waited for.
 // A query whose tiles lie in several clusters' ranges leaves unnormalised partial results, which
 // smla_fwd_combine_kernel adds up.
 // =============================================================================================
 namespace ff {
 constexpr int kSoftmaxWarps = 16;
 constexpr int kProducerThreads = 128;
-constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 64;
-constexpr int kIssueWarp = kThreads / 32 - 2, kLoadWarp = kThreads / 32 - 1;
+constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 96;
+constexpr int kIssueWarp = kThreads / 32 - 3, kLoadWarp = kThreads / 32 - 2, kRelayWarp = kThreads / 32 - 1;
 constexpr int kParts = 8;                  // a head's 256 keys of a tile over eight warps
 constexpr int kTileKeys = 256;             // per pair; 128 per CTA
 constexpr int kSlotBytes = 16384;
@@ -1048,11 +1050,6 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     const int k_slots = n + 1 < n_tiles ? kQChunks : 0;
                     const int slots = k_slots + 2 * groups;
                     for (int j = 0; j < slots; ++j) {
-                        if (j == k_slots) {          // P of tile n, in front of the V it is multiplied with
-                            mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
-                            fence_proxy_async_smem();
-                            mbar_arrive_cluster_relaxed(map_to_cta(bar_pfull, 0));
-                        }
                         // this CTA's half of Q is part of what "full" promises
                         if (j < k_slots && new_query) mbar_wait(bar_qfull + 8 * j, qpar, wc, kErrFwd + 15);
                         ring.wait(wc, kErrFwd + 17);
@@ -1142,6 +1139,23 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     umma_commit_2cta_mask(bar_drain, 1);
                     mbar_wait_drain(bar_drain, 0, p.wait_limit);
                 }
+            }
+        }
+    } else if (warp == kRelayWarp) {
+        // ------------------------------------------------------------------ odd CTA: "my P is written" for the issuer
+        // P is plain stores of this CTA's softmax warps, and they have rescaled its O and read it out: none of that is a case for a
+        // relaxed arrival, so it is released at cluster scope, once a tile and in a warp of its own.  That costs a tile's latency where a
+        // cluster has one tile and 1 - 2 % where it has many: 8 tokens x 128 heads x 2048 19.6 us without the release, 20.3 with it;
+        // 4096 x 128 heads x 256 410 / 412, x 2048 2361 / 2398.  By the thread that forwards the slots, whose next slot waits for it:
+        // 20.1, 448, 2429.  A wait at cluster scope in the issuer on top: 20.2, 451, 2482.
+        if (rank == 1 && elect_one()) {
+            const uint32_t pfull_even = map_to_cta(bar_pfull, 0);
+            for (int n = 0; n < n_tiles; ++n) {
+                mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
+                tc_fence_after_sync();
+                fence_proxy_async_smem();
+                tc_fence_before_sync();
+                mbar_arrive_cluster_release(pfull_even);
             }
         }
     } else if ((warp & 1) * 32 < NH) {
@@ -1294,7 +1308,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             }
             tc_fence_before_sync();
             __syncwarp();
-            // Local arrival, forwarded by the odd CTA's relay thread: a cluster-scope release costs hundreds of cycles a tile.
+            // Local arrival, forwarded by warp 22 of the odd CTA: a cluster-scope release would hold this warp for hundreds of cycles.
             if (lane == 0) mbar_arrive(bar_pfull);
 
             if (last) {

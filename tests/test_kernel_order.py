@@ -40,3 +40,17 @@ def test_no_trigger_before_the_tensor_memory_is_allocated(name):
     alloc = re.search(r"\btmem_alloc\w*\(", body).start()
     allocated = body.index("__syncthreads()", alloc)
     assert all(m.start() > allocated for m in re.finditer(r"\bpdl_trigger\(\)", body))
+
+
+def test_p_of_the_odd_cta_is_released_to_the_issuer():
+    """What the odd CTA's softmax warps have written (P by plain stores, the rescaled O into tensor memory) reaches the UMMAs that the
+    even CTA issues through one forwarding thread: ordered behind the tensor-memory accesses, fenced to the async proxy, and released at
+    cluster scope."""
+    body = _kernels()["smla_fwd_kernel"]
+    waits = [m.end() for m in re.finditer(r"mbar_wait\(bar_pfull,[^;]*;", body)]
+    calls = [re.findall(r"\b(\w+)\(", body[at:])[:4] for at in waits]
+    assert ["tc_fence_after_sync", "fence_proxy_async_smem", "tc_fence_before_sync", "mbar_arrive_cluster_release"] in calls
+    assert len(waits) == 2 and not re.search(r"mbar_arrive_cluster_relaxed\([^;]*pfull", body)
+    with open(os.path.join(os.path.dirname(SOURCE), "sm100_ptx.cuh")) as f:
+        ptx = f.read()
+    assert "mbarrier.arrive.release.cluster" in ptx.split("void mbar_arrive_cluster_release")[1].split("}")[0]
