@@ -798,8 +798,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 //   warps 0-15  softmax: warp w reads lane quarter w % 4, columns [32 (w / 4), + 32) of S: one head, 32 keys per thread
 //   warps 16-19 gather producers (cp.async 16 B, swizzled)
 //   warp 20     even CTA: the UMMA issuer (one elected thread); odd CTA: forwards "my slot is full"
-//   warp 21     TMA of the CTA's Q chunks
-//   warp 22     odd CTA: forwards "my P is written" (even CTA: idle)
+//   warp 21     TMA of the CTA's Q chunks; odd CTA: forwards "my P is written"
 // The exponentials of a tile are taken against the maximum of the row so far; where a tile raises it, O and the sum are
 // rescaled.  A reference that lags behind the maximum (moved only when exceeded by 2^8) makes most of the rescaling
 // unnecessary and is 3 % faster (128 heads, 2.34 against 2.42 ms), but the heaviest probabilities then lose in their rounding
@@ -813,7 +812,7 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // hide each other's latency, P is announced by a local arrival that a thread of the odd CTA forwards (a cluster-scope release by
 // every warp held it for hundreds of cycles): what is left are waits for gathered slots.  4096 queries x 128 heads x top-k 2048
 // back to back, where the power cap holds the clock down: 2568 us with eight warps, 2458 with sixteen and a forwarded arrival that
-// released nothing, 2 % above that as it is (see warp 22).  Five, six and seven ring slots were compared with eight warps only (2.48 /
+// released nothing, 2 % above that as it is (see warp 21).  Five, six and seven ring slots were compared with eight warps only (2.48 /
 // 2.47 / 2.48 ms), when the ring was not what the issuer waited for.
 // A query whose tiles lie in several clusters' ranges leaves unnormalised partial results, which
 // smla_fwd_combine_kernel adds up.
@@ -821,8 +820,8 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 namespace ff {
 constexpr int kSoftmaxWarps = 16;
 constexpr int kProducerThreads = 128;
-constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 96;
-constexpr int kIssueWarp = kThreads / 32 - 3, kLoadWarp = kThreads / 32 - 2, kRelayWarp = kThreads / 32 - 1;
+constexpr int kThreads = kSoftmaxWarps * 32 + kProducerThreads + 64;
+constexpr int kIssueWarp = kThreads / 32 - 2, kLoadWarp = kThreads / 32 - 1;
 constexpr int kParts = 8;                  // a head's 256 keys of a tile over eight warps
 constexpr int kTileKeys = 256;             // per pair; 128 per CTA
 constexpr int kSlotBytes = 16384;
@@ -1021,19 +1020,38 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             }
         }
     } else if (warp == kLoadWarp) {
-        // ------------------------------------------------------------------ Q chunks of this CTA's heads
+        // ------------------------------------------------------------------ Q chunks of this CTA's heads; odd CTA: "my P is written"
         if (lane == 0) {
             const uint64_t pol_stream = l2_policy_evict_first();
+            const uint32_t pfull_even = map_to_cta(bar_pfull, 0);
             uint32_t qpar = 1;              // parity of "chunk free" left by the previous query
-            bool first = true;
-            for (TileIter<1> it(p, range); it.more(); first = false, qpar ^= 1) {
-                const int row0 = it.q * p.h_q + NH * static_cast<int>(rank);
-                for (int j = 0; j < kQChunks; ++j) {
-                    if (!first) mbar_wait(bar_qfree + 8 * j, qpar, wc, kErrFwd + 16, kPollSleepNs);
-                    mbar_arrive_expect_tx(bar_qfull + 8 * j, NH * 128);
-                    tma_load_2d_hint(s_base + kOffQ + j * kQChunk, &tm_q, 64 * j, row0, bar_qfull + 8 * j, pol_stream);
+            TileIter<1> it(p, range);
+            bool new_query = true;
+            for (int n = -1; n < n_tiles; ++n) {
+                if (new_query && it.more()) {                 // of tile n + 1: free once the logits of tile n are done
+                    const int row0 = it.q * p.h_q + NH * static_cast<int>(rank);
+                    for (int j = 0; j < kQChunks; ++j) {
+                        if (n >= 0) mbar_wait(bar_qfree + 8 * j, qpar, wc, kErrFwd + 16, kPollSleepNs);
+                        mbar_arrive_expect_tx(bar_qfull + 8 * j, NH * 128);
+                        tma_load_2d_hint(s_base + kOffQ + j * kQChunk, &tm_q, 64 * j, row0, bar_qfull + 8 * j, pol_stream);
+                    }
+                    qpar ^= 1;
                 }
-                while (!it.advance()) {}
+                if (it.more()) new_query = it.advance();
+                // P is plain stores of this CTA's softmax warps, and they have rescaled its O and read it out: none of that is a case
+                // for a relaxed arrival, so it is released for the issuer at cluster scope, once a tile.
+                // That adds a tile's latency where a cluster has one tile and 1 - 2 % where it has many (without the release / with it):
+                // 8 tokens x 128 heads x 2048 19.4 / 19.9 us, 74 x 256 12.3 / 12.9, 4096 x 256 408 / 416, x 2048 2383 / 2407.  By the thread
+                // that forwards the slots, whose next slot waits for it: 20.1, -, 448, 2429; a wait at cluster scope in the issuer on
+                // top of that: 20.2, -, 451, 2482.  By a warp of its own the block leaves no room for one of the combine kernel beside
+                // it: 20.0, 13.1, 417, 2423, and one query x 18944 slots 52.6 us against 39.1.
+                if (rank == 1 && n >= 0) {
+                    mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
+                    tc_fence_after_sync();
+                    fence_proxy_async_smem();
+                    tc_fence_before_sync();
+                    mbar_arrive_cluster_release(pfull_even);
+                }
             }
         }
     } else if (warp == kIssueWarp) {
@@ -1139,23 +1157,6 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
                     umma_commit_2cta_mask(bar_drain, 1);
                     mbar_wait_drain(bar_drain, 0, p.wait_limit);
                 }
-            }
-        }
-    } else if (warp == kRelayWarp) {
-        // ------------------------------------------------------------------ odd CTA: "my P is written" for the issuer
-        // P is plain stores of this CTA's softmax warps, and they have rescaled its O and read it out: none of that is a case for a
-        // relaxed arrival, so it is released at cluster scope, once a tile and in a warp of its own.  That costs a tile's latency where a
-        // cluster has one tile and 1 - 2 % where it has many: 8 tokens x 128 heads x 2048 19.6 us without the release, 20.3 with it;
-        // 4096 x 128 heads x 256 410 / 412, x 2048 2361 / 2398.  By the thread that forwards the slots, whose next slot waits for it:
-        // 20.1, 448, 2429.  A wait at cluster scope in the issuer on top: 20.2, 451, 2482.
-        if (rank == 1 && elect_one()) {
-            const uint32_t pfull_even = map_to_cta(bar_pfull, 0);
-            for (int n = 0; n < n_tiles; ++n) {
-                mbar_wait(bar_pfull, n & 1, wc, kErrFwd + 22);
-                tc_fence_after_sync();
-                fence_proxy_async_smem();
-                tc_fence_before_sync();
-                mbar_arrive_cluster_release(pfull_even);
             }
         }
     } else if ((warp & 1) * 32 < NH) {
@@ -1308,7 +1309,7 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
             }
             tc_fence_before_sync();
             __syncwarp();
-            // Local arrival, forwarded by warp 22 of the odd CTA: a cluster-scope release would hold this warp for hundreds of cycles.
+            // Local arrival, forwarded by warp 21 of the odd CTA: a cluster-scope release would hold this warp for hundreds of cycles.
             if (lane == 0) mbar_arrive(bar_pfull);
 
             if (last) {
