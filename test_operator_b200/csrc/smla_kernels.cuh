@@ -1353,16 +1353,18 @@ smla_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const KParams p) {
 // of their weighted row sums.  The items are the queries where there are at most as many as boundaries between ranges, else
 // the boundaries (the one that is its query's first does the work; the forward kernel has noted each range's first
 // query).  A lane takes one head and sixteen columns: the parts lie as [8 columns][heads][8], so a warp loads a part in pieces of
-// 1 KB, and a lane's weights need no other lane.  The first parts' O is asked for together with all references and sums.
+// 1 KB, and a lane's weights need no other lane.  The first parts' O is on its way while the others' references and sums are read.
 // Parts are added in their order.  Bound by the latency of its dependent loads; eight queries of eight parts: 5.5 us of a call,
 // 7.6 us with a warp per head and half of the columns, whose weights took two rounds of loads before the first row.
 // Blocks are small, so that many of them are in place beside the forward kernel's last blocks when it ends.  kFly: parts in flight, two
-// where no query has more (72 registers a thread instead of 112).  30 queries x 128 heads x top-k 512 18.2 us a call with blocks of
+// where no query has more (80 registers a thread instead of 110).  30 queries x 128 heads x top-k 512 18.2 us a call with blocks of
 // 256 and four parts, 17.4 so; 90 queries x 600 41.6 / 39.4; one query x 2048 (eight parts) 15.4 / 14.9; eight x 2048 alike, and
-// 19.4 -> 22.9 with two parts in flight.
+// 19.4 -> 22.9 with two parts in flight.  112 registers at most: a block then fits beside one of the forward kernel, by the register file's
+// four parts (16384 each; six warps of 80 x 32 there and one of these).  With 118 all blocks come up on the first SMs that are free, and
+// one query x 18944 slots takes 49.5 us, 31.9 so.
 constexpr int kCombineThreads = 64;
 template <int kFly>
-__global__ void __launch_bounds__(kCombineThreads) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
+__global__ void __maxnreg__(112) smla_fwd_combine_kernel(const KParams p, int n_clusters, int h_pad) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
@@ -1395,46 +1397,70 @@ __global__ void __launch_bounds__(kCombineThreads) smla_fwd_combine_kernel(const
     const int first = static_cast<int>((static_cast<long long>(q_begin + 1) * n_clusters - 1) / n_tiles);
     const int last = static_cast<int>((static_cast<long long>(q_end) * n_clusters - 1) / n_tiles);
     if (first == last || (!p.every_slot && p.nq >= n_clusters && first != item)) return;
-    if (head >= p.h_q) return;
-    // part k: its slot, -1 where the range is empty
-    auto slot_of = [&](int k) {
+    const float ninf = __int_as_float(0xff800000);
+    // Lane i: the slot of part k0 + i, -1 where its range is empty or there is no such part.  (Once for all: the two divisions a
+    // part took a good part of the kernel's time.)  All lanes stay to the end, those of heads beyond h_q with rows of the padding.
+    auto slots_from = [&](int k0) {
+        const int k = k0 + lane;
+        if (k > last) return -1;
         const int begin = range_start(n_tiles, k, n_clusters);
         return begin == range_start(n_tiles, k + 1, n_clusters) ? -1 : 2 * k + (begin <= q_begin ? 1 : 0);
     };
-    auto load_part = [&](int k, uint32_t (&v)[2][8], float2& ml) {
-        const int slot = k <= last ? slot_of(k) : -1;
-        ml = make_float2(__int_as_float(0xff800000), kNoSlot);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i / 8][i % 8] = 0u;
-        if (slot >= 0) {
-            const float* o = p.part_o + ((static_cast<size_t>(slot) * (kDV / 8) + (col >> 3)) * h_pad + head) * 8;
-            ml = __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head);
-            ld_global_v8(o, v[0]);
-            ld_global_v8(o + h_pad * 8, v[1]);
-        }
-    };
-    const float ninf = __int_as_float(0xff800000);
+    auto load_ml = [&](int slot) { return __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head); };
     uint32_t v[kFly][2][8];
     float2 ml[kFly];
+    auto load_part = [&](int u, int slot) {
+        const float* o = p.part_o + ((static_cast<size_t>(slot) * (kDV / 8) + (col >> 3)) * h_pad + head) * 8;
+        ml[u] = load_ml(slot);
+        ld_global_v8(o, v[u][0]);
+        ld_global_v8(o + h_pad * 8, v[u][1]);
+    };
+    auto no_part = [&](int u) {
+        ml[u] = make_float2(ninf, kNoSlot);
 #pragma unroll
-    for (int u = 0; u < kFly; ++u) load_part(first + u, v[u], ml[u]);
+        for (int i = 0; i < 16; ++i) v[u][i / 8][i % 8] = 0u;
+    };
+    int slots = slots_from(first);
+#pragma unroll
+    for (int u = 0; u < kFly; ++u) {
+        const int slot = __shfl_sync(0xffffffffu, slots, u);
+        no_part(u);
+        if (slot >= 0) load_part(u, slot);
+    }
     float ref = ninf, sum = 0.f, acc[16];
     bool any = false;
+    // The other parts: their references first.  Those without a valid slot (every_slot counts their tiles as used) hold zeros and are
+    // passed over:
+    // one query x 128 heads x 18944 slots of which 300 are in use 38.7 -> 17.2 us, 8 x 2048 with 100 20.1 -> 17.8; all in use 38.8 -> 31.9
+    // (the divisions of slots_from), 20.2 and 20.2.
+    uint32_t live = 0;                           // lane w: bit i says that part first + kFly + 32 w + i has a valid slot (of all heads or of none)
+#pragma unroll 1
+    for (int w = 0, k0 = first + kFly; k0 <= last; ++w, k0 += 32) {
+        slots = slots_from(k0);
+        const uint32_t word = __ballot_sync(0xffffffffu, slots >= 0 && __ldcg(&p.part_ml[static_cast<size_t>(slots) * h_pad].y) != kNoSlot);
+        if (lane == w) live = word;
+        any = any || word;
+        constexpr int kBatch = 8;
+        for (uint32_t todo = word; todo;) {
+            float x[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {   // (the first again where there are no more)
+                const int slot = __shfl_sync(0xffffffffu, slots, __ffs(todo ? todo : word) - 1);
+                x[u] = load_ml(slot).x;
+                todo &= todo - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) ref = fmaxf(ref, x[u]);
+        }
+    }
 #pragma unroll
     for (int u = 0; u < kFly; ++u) {
         ref = fmaxf(ref, ml[u].x);               // -inf: no valid slot in this part, or none above -inf
         any = any || ml[u].y != kNoSlot;
     }
-    for (int k = first + kFly; k <= last; ++k) {
-        const int slot = slot_of(k);
-        if (slot < 0) continue;
-        const float2 x = __ldcg(p.part_ml + static_cast<size_t>(slot) * h_pad + head);
-        ref = fmaxf(ref, x.x);
-        any = any || x.y != kNoSlot;
-    }
 #pragma unroll
     for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    for (int k = first;;) {
+    auto add_parts = [&]() {
 #pragma unroll
         for (int u = 0; u < kFly; ++u) {
             const float w = ml[u].x > ninf ? ex2_approx(ml[u].x - ref) : 0.f;
@@ -1443,11 +1469,33 @@ __global__ void __launch_bounds__(kCombineThreads) smla_fwd_combine_kernel(const
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[i] = fmaf(__uint_as_float(v[u][i / 8][i % 8]), w, acc[i]);
         }
-        k += kFly;
-        if (k > last) break;
+    };
+    add_parts();
+#pragma unroll 1
+    for (int w = 0, k0 = first + kFly; k0 <= last; ++w, k0 += 32) {
+        uint32_t todo = __shfl_sync(0xffffffffu, live, w);
+        if (todo == 0) continue;
+        if (last - first - kFly >= 32) slots = slots_from(k0);       // (else they are the ones from before)
+        while (__popc(todo) >= kFly) {
 #pragma unroll
-        for (int u = 0; u < kFly; ++u) load_part(k + u, v[u], ml[u]);
+            for (int u = 0; u < kFly; ++u) {
+                load_part(u, __shfl_sync(0xffffffffu, slots, __ffs(todo) - 1));
+                todo &= todo - 1;
+            }
+            add_parts();
+        }
+        if (todo) {
+#pragma unroll
+            for (int u = 0; u < kFly; ++u) {
+                const int slot = __shfl_sync(0xffffffffu, slots, todo ? __ffs(todo) - 1 : 0);
+                no_part(u);
+                if (todo) load_part(u, slot);
+                todo &= todo - 1;
+            }
+            add_parts();
+        }
     }
+    if (head >= p.h_q) return;
     const size_t orow = static_cast<size_t>(q) * p.h_q + head;
     if (col == 0) p.lse_out[orow] = any ? row_lse(ref, sum) * p.lse_out_mult : no_slot_lse(p);
     const float inv = any ? 1.f / sum : 0.f;
