@@ -912,6 +912,9 @@ int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_
     src.q_start = src.causal ? q_start_index_s : 0;
     if (pl.items == inv::kItemsMid)
         return launch_index_inverse<inv::kItemsMid, true>(src, pl, l, ws, n, row_ptr, entries, st);
+    if (pl.items == inv::kItemsFewerRounds)
+        return pl.by_masks ? launch_index_inverse<inv::kItemsFewerRounds, true>(src, pl, l, ws, n, row_ptr, entries, st)
+                           : launch_index_inverse<inv::kItemsFewerRounds, false>(src, pl, l, ws, n, row_ptr, entries, st);
     return pl.by_masks ? launch_index_inverse<inv::kItemsLarge, true>(src, pl, l, ws, n, row_ptr, entries, st)
                        : launch_index_inverse<inv::kItemsLarge, false>(src, pl, l, ws, n, row_ptr, entries, st);
 }

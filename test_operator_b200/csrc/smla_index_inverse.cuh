@@ -24,10 +24,14 @@ namespace inv {
 
 constexpr int kThreads = 512;
 // Entries per thread; a block's entries are contiguous, a warp's are (32 kItems of them): (warp, step, lane) order is flat
-// order.  Large inputs take fourteen: long runs on the way out, and 8.4 M slots are 4.0 rounds of blocks on 148 SMs (3.5 with
-// sixteen; 159 us with eight, 144 with twelve, 139 with sixteen, 137 with fourteen).  Below kLargeInput they take four, so that
-// there are blocks for all SMs (270,000 slots: 46 us with sixteen, 29 with eight).
-constexpr int kItemsLarge = 14, kItemsMid = 4, kItemsSmall = 16;
+// order.  Large inputs take fourteen (8.4 M slots: 159 us with eight, 144 with twelve, 139 with sixteen, 137 with fourteen), or sixteen
+// where the last round of blocks on the 148 SMs would be nearly empty otherwise: where rounds x entries, the entries that a thread
+// goes through one after the other, are fewer with sixteen.  Fourteen / sixteen measured (us; * what the rule takes): 2.1 M slots
+// 38.9* / 41.4, 2.4 M 54.4 / 43.2* (two rounds against one), 3.0 M 56.3* / 62.5, 4.3 M 85.3 / 80.3* (three against two), 5.2 M 86.2* / 95.2,
+// 7.1 M 117.4 / 115.5*, 8.4 M 134.5* / 135.4, 9.0 M 148.7 / 150.2* (70 entries against 64; the one range where it is wrong, by 1 %), 9.6 M
+// 160.9 / 153.2*, 10.7 M 176.6 / 169.9*, 12 M 194.1 / 190.7*, 14.5 M 226.4 / 227.2*, 16.8 M 258.9* / 264.5.  Below kLargeInput they take four,
+// so that there are blocks for all SMs (270,000 slots: 46 us with sixteen, 29 with eight).
+constexpr int kItemsLarge = 14, kItemsFewerRounds = 16, kItemsMid = 4, kItemsSmall = 16;
 constexpr int64_t kLargeInput = 1 << 20;
 constexpr int kSmallInput = kThreads * kItemsSmall;     // one block sorts this many alone
 constexpr int kWarps = kThreads / 32;
@@ -54,8 +58,11 @@ inline Plan make_plan(int64_t n, int32_t s_kv) {
     Plan pl;
     pl.passes = (bits + 7) / 8;
     pl.digit_bits = (bits + pl.passes - 1) / pl.passes;
-    pl.items = n > kSmallInput && n < kLargeInput ? kItemsMid : kItemsLarge;
-    pl.n_blocks = static_cast<int>((n + kThreads * pl.items - 1) / (kThreads * pl.items));
+    const auto blocks = [n](int items) { return (n + kThreads * items - 1) / (kThreads * items); };
+    const auto steps = [&](int items) { return (blocks(items) + kResidentBlocks - 1) / kResidentBlocks * items; };
+    if (n > kSmallInput && n < kLargeInput) pl.items = kItemsMid;
+    else pl.items = steps(kItemsFewerRounds) < steps(kItemsLarge) ? kItemsFewerRounds : kItemsLarge;
+    pl.n_blocks = static_cast<int>(blocks(pl.items));
     pl.key16 = s_kv < 65536;
     pl.by_masks = pl.n_blocks <= kResidentBlocks;
     return pl;
@@ -186,10 +193,12 @@ struct RankShared {
 // prefixed over the runs and the digits.  Ends with all threads past a barrier.
 //
 // kMasks: the lanes of a step that share a digit are found by each setting its bit in the digit's word of shared memory
-// (`words`, kRuns * kMaxRadix of them), not by eight ballots.  That is a third of the instructions and the shorter chain, but more
-// shared-memory traffic: faster while every block runs at once, slower where many wait for an SM.  10 x 512 slots 17.6 us by ballots,
-// 15.0 by masks; 0.9 M slots (450 small blocks) 49.6 / 46.0; 2.1 M of 8192 rows (293 blocks) 42.2 / 38.3; 8.4 M of 32768 (1171
-// blocks) 134.1 / 136.3; 16.8 M of 65000 258 / 275.
+// (`words`, kRuns * kMaxRadix of them; the atomic-or match known from radix sorts by ranking), not by eight ballots.  That is a third of
+// the instructions and the shorter chain, but more shared-memory traffic: clearly faster while every block runs at once, slower where a
+// great many wait for an SM.  By ballots / by masks, us: 10 x 512 slots 17.6 / 15.0; 0.9 M slots (450 small blocks) 49.6 / 46.0; 2.1 M
+// (293 blocks) 42.8 / 38.9; then, in fourteens, 3.0 M (419) 56.2 / 54.7, 5.2 M (726) 86.1 / 84.0, 8.4 M (1171) 134.5 / 134.6, 12 M (1674)
+// 194.1 / 201.8, 16.8 M (2341) 258.8 / 275.2; with 32-bit keys 3.0 M 85.8 / 81.6, 9.0 M 214.8 / 202.4, 16.8 M 373.7 / 366.3.  The line lies at
+// the blocks that run at once, where masks win by a tenth whatever the keys.
 template <bool kMasks, int kItems>
 __device__ __forceinline__ void block_rank(const uint32_t (&keys)[kItems], int shift, uint32_t mask, uint32_t first, uint32_t n,
                                            RankShared& sh, uint32_t* words, uint32_t (&pos)[kItems]) {
