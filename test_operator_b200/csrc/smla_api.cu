@@ -455,8 +455,8 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
         std::lock_guard<std::mutex> lock(g_dev_sched_mutex);
         DevSched* ds = dev_sched_locked();
         if (!ds) return SMLA_ERR_LAUNCH;
-        // the second stream starts behind everything the caller's stream holds so far (dKV cleared, Delta, the
-        // previous pass's readers of the scratch)
+        // the second stream starts behind everything the caller's stream holds so far (Delta, the previous pass's readers of the
+        // scratch); dKV is cleared by the first part's recompute kernel, which ev_part[0] stands behind
         if (cudaEventRecord(ds->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(ds->side, ds->ev_fork, 0) != cudaSuccess)
             return SMLA_ERR_LAUNCH;
         for (int c = 0; c < parts; ++c) {

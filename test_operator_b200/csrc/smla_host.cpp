@@ -3,8 +3,8 @@
 // loaded hands its entry points over (init).
 //
 // Why: the smallest calls keep the GPU busy for 15 - 20 us, and a call's way through Python took the host as long.  Host time of a
-// call: backward 21.8 -> 15.4 us (10.3 of them four launches), forward of eight tokens 19.8 -> 10.1 us (two launches, 5.6); from
-// an idle GPU to the result 77 -> 52 us (64 queries x 16 heads x top-k 64, backward) and 58 -> 38 us (8 tokens x 128 heads, forward).
+// call, through Python / so: backward of 64 queries x 16 heads x top-k 64 (three launches) 23.7 / 12.4 us, forward of eight tokens x 128
+// heads (two) 17.0 / 8.0; from an idle GPU to the result 46.1 / 34.9 and 42.0 / 33.3.
 //
 // It takes what nearly every call passes and answers None (or a size of 0) for anything else - other argument types, tensor
 // subclasses, wrapped tensors, wrong shapes - which op.py then handles itself, error messages included.

@@ -85,10 +85,16 @@ __device__ __forceinline__ bool slot_valid(int idx, int key, const QMeta& m, con
     return key < m.topk_len && idx >= 0 && idx < m.kv_len && m.kv_base + idx < p.s_kv && (!p.causal || idx <= m.q_pos);
 }
 // kv row a slot gathers from, -1 for one that takes no part (nothing is read then, zeros land).  The whole rule, not the range alone:
-// the contractions over keys multiply a masked slot's row by an exact 0, and a masked slot may name a row that holds NaN or an
-// infinity (one of a cache that has not been written yet).
+// the contractions over keys (forward, dQ) multiply a masked slot's row by an exact 0, and a masked slot may name a row that holds NaN or
+// an infinity (one of a cache that has not been written yet).
 __device__ __forceinline__ int gather_row(int idx, int key, const QMeta& m, const KParams& p) {
     return slot_valid(idx, key, m, p) ? m.kv_base + idx : -1;
+}
+// The same by the range alone, for the recompute kernel: there a row meets its own slot's S and dS only, which are masked bit by bit.
+// (64 queries x 16 heads x top-k 64 19.57 us a call with the whole rule, 19.45 so.)
+__device__ __forceinline__ int gather_row_in_range(int idx, const QMeta& m, const KParams& p) {
+    const int row = m.kv_base + idx;
+    return idx >= 0 && idx < m.kv_len && row < p.s_kv ? row : -1;
 }
 // After a bounded wait has given up: let this thread's own cp.async land and leave in-flight TMA loads (they
 // depend on nothing and complete within microseconds) the time to land before the CTA gives up its shared memory.
@@ -276,11 +282,16 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 // tiles over 74 clusters as whole queries would be 56 queries for some and 55 for the others), a few long queries
 // spread over the whole chip, and tiles without a valid slot do not exist.  kMul: tiles of 256 / kMul keys.
 //
-// A call whose queries have no more tiles than there are clusters takes as long as one tile takes, whether or not some of the
-// tiles are empty.  There the ranges are cut as if every slot were in use (every_slot): nothing has to look at the indices
-// first, which saves both directions their prep kernel (own_prep in the backward).  Eight queries x 128 heads x top-k 2048, forward:
-// 25.1 -> 19.5 us a call (prep kernel, its hand-over and the 5700 cycles that the ranges took from its counts).  From the
-// next tile on some cluster has two, and an empty tile would cost as much as a full one.
+// In a call whose queries have no more tiles than there are clusters no cluster has more than one tile, and the kernels that go by
+// these ranges take as long as one tile takes, whether or not some of the tiles are empty.  There the ranges are cut as if every slot
+// were in use (every_slot): nothing has to look at the indices first, which saves both directions their prep kernel (own_prep in the
+// backward).  From the next tile on some cluster has two, and an empty tile would cost as much as a full one.
+// The dQ kernel, where a CTA goes through a query's tiles, does work on empty ones.  128 heads, with a prep kernel / so, us:
+//   8 queries x top-k 2048, slots in use   2048          700           100           1
+//   forward                                25.6 / 20.2   22.7 / 20.3   18.6 / 17.8   19.2 / 17.8
+//   backward                               45.0 / 35.9   39.4 / 34.6   32.1 / 33.0   28.4 / 32.8
+// The last two of the backward are what it costs.  A dQ kernel that looked for the last valid slot first took 32.1 and 31.8 there, and
+// 36.9 with all in use (37 queries x 512 31.1 -> 31.8).
 __device__ __forceinline__ int slots_used(const KParams& p, int q) { return p.every_slot ? p.every_slot : __ldcg(p.n_used + q); }
 struct WorkRange {
     int begin, end;               // positions among the launch's tiles
@@ -500,14 +511,14 @@ smla_recompute_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         int s = 0;
         uint32_t ph = 1;                    // parity that means "slot free" for the current pass over the ring
         while (it.more()) {
-            // A slot that takes no part reads nothing and lands as zeros (its S, dS are forced to 0
+            // A slot whose index is out of range reads nothing and lands as zeros (its S, dS are forced to 0
             // anyway).  Sending all of them to one stand-in row instead would make that row's cache lines a
             // hot spot that every SM queues on.
             const char* src[4];
             uint32_t nb[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int row = gather_row(idx_next[i], it.tile() * kTileKeys + static_cast<int>(rank) * 128 + r0 + 32 * i, qm_next, p);
+                const int row = gather_row_in_range(idx_next[i], qm_next, p);
                 nb[i] = row >= 0 ? 16u : 0u;
                 src[i] = kvb + static_cast<size_t>(row >= 0 ? row : 0) * (kDQK * 2);
             }
@@ -1596,8 +1607,9 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_alloc_2cta(smem_u32(tmem_slot), 512);
         tmem_relinquish_2cta();
     }
-    // Behind the recompute kernel's trigger (it triggers after it has waited for the prep kernel) everything but S and dS is in
-    // place already: slot counts, indices, Q, dO, a cleared dKV.  Then only the first S / dS load waits.
+    // Behind the recompute kernel's trigger (it triggers after it has waited for what was before it) slot counts, indices, Q and dO
+    // are in place.  S, dS and a cleared dKV are not, before that kernel has ended: the first S / dS load waits for that, and no
+    // reduction can be issued before UMMAs on what it has loaded.
     if (!p.early_start) pdl_wait();
     find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + C::kOffIdx), range_s);    // (index buffers: not in use yet)
     tc_fence_before_sync();

@@ -210,7 +210,7 @@ def _load_host(lib):
                       (lib.smla_fwd_run, lib.smla_fwd_workspace_size, lib.smla_bwd_run_stages, lib.smla_bwd_workspace_size)))
         return module
     except Exception as e:
-        warnings.warn(f"the compiled host module cannot be used, calls take some 8 us longer: {e}")
+        warnings.warn(f"the compiled host module cannot be used, calls take some 10 us longer: {e}")
         return _NoNativeHost
 
 
