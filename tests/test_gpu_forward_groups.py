@@ -17,14 +17,15 @@ def test_last_slot_at_the_edges_of_the_groups(h_q, topk):
     s_q, s_kv = 300, 2048                      # several queries a cluster
     s = make_sequence(Workload("groups", 1, s_q, s_kv, h_q, topk, "uniform", invalid_frac=0.1), device=DEV, seed=31, with_forward=False)
     q, kv, idx = s["q"], s["kv"], s["indices"]
-    kv[-1] = float("nan")                      # named by no slot
-    idx[idx == s_kv - 1] = 0
+    kv[-1] = float("nan")                      # named by slots that the causal rule masks
+    start = s_kv - 400
+    idx[idx > start] = 0
     last = [n for n in (1, 63, 64, 65, 128, 129, 192, 193, 256, 257, 320, 321, 449, 512) if n <= topk]
     for r in range(s_q):
         idx[r, last[r % len(last)] - 1] = r    # the last slot in use is a valid one
-        idx[r, last[r % len(last)]:] = -1
-    o_ref, lse_ref = sparse_mla_fwd_ref(q, torch.nan_to_num(kv), idx, q_start_index_s=None)
-    o, lse = op.mla_fwd(q, kv, idx, q_start_index_s=None, check_device_status=True)
+        idx[r, last[r % len(last)]:] = -1 if r % 2 else s_kv - 1
+    o_ref, lse_ref = sparse_mla_fwd_ref(q, torch.nan_to_num(kv), idx, q_start_index_s=start)
+    o, lse = op.mla_fwd(q, kv, idx, q_start_index_s=start, check_device_status=True)
     assert (lse - lse_ref * LOG2E).abs().max().item() <= 2e-4
     assert (o.float() - o_ref.float()).abs().max().item() <= 2 ** -6 * o_ref.float().abs().max().item()
     assert cosine(o.float().cpu(), o_ref.float().cpu()) > 0.9999

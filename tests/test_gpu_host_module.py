@@ -70,8 +70,9 @@ def test_both_ways_agree(form, monkeypatch):
         pytest.skip("the host module is not built")
     bwd = lambda **kw: op.mla_bwd(*a.values(), **scal, **kw)                               # noqa: E731
     fwd = lambda: op.mla_fwd(a["q"], a["kv"], a["indices"], **scal)                        # noqa: E731
-    # (the kernels' order of additions into dKV varies: one query per row of dKV would be needed to compare it bit for bit)
-    calls = [fwd, lambda: bwd()[:1], lambda: bwd(accumulate=True),
+    # (the kernels' order of additions into dKV varies: one query per row of dKV would be needed to compare it bit for bit; here its
+    # shape and type)
+    calls = [fwd, lambda: bwd()[:1], lambda: (torch.zeros_like(bwd()[1]),), lambda: bwd(accumulate=True),
              lambda: (bwd(out_dq=torch.empty_like(a["q"]), out_dkv=torch.empty(a["kv"].shape, device=DEV))[0],)]
     got = [_outcome(c) for c in calls]
     assert (native.fwd(a["q"], a["kv"], a["indices"], scal["sm_scale"], scal["q_start_index_s"], 1) is not None) == taken
