@@ -604,9 +604,15 @@ int static_workspace_ptr(void** out) {
 
 // ---- index inverse (CSR by kv row): layout and launches ------------------------------------------------------------
 inline size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
-struct InvLayout { size_t keys_a, keys_b, vals_a, vals_b, hist, totals, heads, first, total; };
+struct InvLayout { size_t keys_a, keys_b, vals_a, vals_b, hist, totals, heads, first, counts, total; };
 inline InvLayout inv_layout(int64_t n, int32_t s_kv, const inv::Plan& pl) {
-    InvLayout l;
+    InvLayout l{};
+    if (pl.groups) {             // direct form
+        l.counts = 0;
+        l.totals = up256(static_cast<size_t>(pl.groups) * pl.rows_pad * 4);
+        l.total = l.totals + up256((static_cast<size_t>(pl.rows_pad) / inv::kScanRows + 1) * 4);
+        return l;
+    }
     const size_t key_bytes = static_cast<size_t>(n) * (pl.key16 ? 2 : 4);
     size_t off = 0;
     l.keys_a = off; off += up256(key_bytes);
@@ -678,6 +684,22 @@ int launch_index_inverse(const inv::Source& src, const inv::Plan& pl, const InvL
                          int32_t* entries, cudaStream_t st) {
     return pl.key16 ? launch_index_inverse<uint16_t, kItems, kMasks>(src, pl, l, ws, n, row_ptr, entries, st)
                     : launch_index_inverse<uint32_t, kItems, kMasks>(src, pl, l, ws, n, row_ptr, entries, st);
+}
+
+// The direct form: counts per group of queries, positions, entries.
+int launch_index_inverse_direct(const inv::Source& src, const inv::Plan& pl, const InvLayout& l, uint8_t* ws, int32_t s_q, int32_t* row_ptr,
+                                int32_t* entries, cudaStream_t st) {
+    static std::atomic<bool> attr_done[kMaxDevices];
+    if (!once_per_device(attr_done, [] { return set_smem(inv::group_count_kernel, inv::kPlaceRows * 4) && set_smem(inv::place_kernel, inv::kPlaceRows * 4); }))
+        return SMLA_ERR_LAUNCH;
+    uint32_t* counts = reinterpret_cast<uint32_t*>(ws + l.counts);
+    uint32_t* totals = reinterpret_cast<uint32_t*>(ws + l.totals);
+    const int smem = pl.rows_pad * 4, scan_blocks = (pl.rows_pad + inv::kScanRows - 1) / inv::kScanRows;
+    launch(inv::group_count_kernel, pl.groups, inv::kPlaceThreads, smem, st, true, 1, src, counts, entries, s_q, pl.per_group, pl.rows_pad);
+    launch(inv::group_scan_kernel, scan_blocks, inv::kPlaceThreads, 0, st, true, 1, counts, totals, pl.groups, pl.rows_pad);
+    launch(inv::place_kernel, pl.groups, inv::kPlaceThreads, smem, st, true, 1, src, counts, totals, row_ptr, entries, s_q, pl.per_group, pl.rows_pad,
+           scan_blocks);
+    return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }
 
 inline bool inv_shape_ok(int32_t s_q, int32_t topk, int32_t s_kv) {
@@ -885,7 +907,9 @@ size_t smla_index_inverse_workspace_size(int32_t s_q, int32_t topk, int32_t s_kv
     if (!inv_shape_ok(s_q, topk, s_kv)) return 0;
     const int64_t n = static_cast<int64_t>(s_q) * topk;
     // (never less than twelve bytes a slot, what the documentation promises to be about the size)
-    return std::max(inv_layout(n, s_kv, inv::make_plan(n, s_kv)).total, static_cast<size_t>(n) * 12) + 256;
+    size_t total = static_cast<size_t>(n) * 12;
+    for (bool direct : {false, true}) total = std::max(total, inv_layout(n, s_kv, inv::make_plan(s_q, topk, s_kv, direct)).total);
+    return total + 256;
 }
 
 int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_t s_kv, int32_t q_start_index_s,
@@ -900,8 +924,12 @@ int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_
     }
     if (!indices || !entries || !workspace) return SMLA_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return SMLA_ERR_BAD_ARG;
-    const inv::Plan pl = inv::make_plan(n, s_kv);
-    const InvLayout l = inv_layout(n, s_kv, pl);
+    inv::Plan pl = inv::make_plan(s_q, topk, s_kv);
+    InvLayout l = inv_layout(n, s_kv, pl);
+    if (pl.groups && workspace_bytes < l.total) {        // the sort may need less
+        pl = inv::make_plan(s_q, topk, s_kv, false);
+        l = inv_layout(n, s_kv, pl);
+    }
     if (workspace_bytes < l.total) return SMLA_ERR_WORKSPACE;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     inv::Source src;
@@ -910,6 +938,7 @@ int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_
     src.s_kv = s_kv;
     src.causal = q_start_index_s != SMLA_NO_CAUSAL;
     src.q_start = src.causal ? q_start_index_s : 0;
+    if (pl.groups) return launch_index_inverse_direct(src, pl, l, ws, s_q, row_ptr, entries, st);
     if (pl.items == inv::kItemsMid)
         return launch_index_inverse<inv::kItemsMid, true>(src, pl, l, ws, n, row_ptr, entries, st);
     if (pl.items == inv::kItemsFewerRounds)

@@ -10,10 +10,13 @@
 // where s_kv fits, and are not written by the last pass.  row_ptr: the last pass takes, for every row, the smallest
 // position at which a run of its key begins (integer minimum: order does not matter), and a last kernel (with two small ones
 // before it for many rows) gives rows without a slot the next row's position.  Inputs of at most one block (8192 slots) are sorted by that block in shared memory.
+// Where the rows' counters fit into shared memory and the slots are many enough for them, no sort: a count per row and group of queries,
+// then every slot goes to its place at once (direct form, below).
 // All kernels are launched behind their predecessor's start (programmatic dependent launch).
 //
 // The reference has no such operator; the validity rule is the one of its kernel (mla_bwd/mla_bwd.cu:765-789).
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <climits>
 #include <cuda_runtime.h>
@@ -43,6 +46,13 @@ constexpr int kRowTile = 1024;                   // rows per block of the row_pt
 constexpr int kMaxLook = 64;
 constexpr int kResidentBlocks = 2 * 148;         // scatter blocks that a B200 runs at once
 
+// Direct form (see there): one block per SM, the counters that fit into its shared memory, slots and queries of a batch at most, and
+// where the position begins in a counter.
+constexpr int kMaxGroups = 148;
+constexpr int kPlaceRows = 53248;
+constexpr int kPlaceThreads = 1024, kPlaceItems = 8, kBatch = kPlaceThreads * kPlaceItems;
+constexpr int kQueryBits = 6, kPosShift = kQueryBits + 1;
+
 struct Plan {
     int passes;      // 1..4
     int digit_bits;  // <= 8
@@ -50,9 +60,30 @@ struct Plan {
     int n_blocks;
     bool key16;      // keys fit 16 bits
     bool by_masks;   // block_rank's kMasks (large form; the others always)
+    int groups;      // direct form: groups of queries, 0 where the sort is taken
+    int per_group;   // queries of a group
+    int rows_pad;    // s_kv + 1, padded
 };
 
-inline Plan make_plan(int64_t n, int32_t s_kv) {
+// Whether the direct form is taken.  What it costs beyond its slots is the counters, three passes over [groups][rows], 0.36 us per 1024
+// rows, and 2 us per batch that a group goes through; the sort costs more per slot from 2 M slots on.  Sort / direct, us, distinct rows
+// (* what the rule takes), 32768 rows unless given: 16 x 2048 slots on 8192 rows 26.7 / 17.8*, 128 x 2048 26.3 / 22.7*, 256 x 2048
+// 26.4 / 24.3*, 257 x 999 on 44000 26.9* / 28.0, 512 x 2048 39.5 / 28.2*, 8192 x 128 on 4096 35.8* / 40.1, 1024 x 2048 41.7 / 37.3*, on
+// 52000 42.7* / 45.2, 2000 x 1000 on 40000 42.2* / 43.3, 4096 x 512 41.7* / 42.8, on 8192 39.1 / 35.0*, 8192 x 256 on 8192 39.1* / 46.2, 2048 x
+// 2048 72.5 / 55.0*, 4096 x 2048 134.8 / 87.9*, on 52000 135.1 / 103.8*, on 8192 129.4 / 78.8*, 8192 x 2048 on 16384 254 / 195*.
+// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 152, on 8192
+// 129 / 177; every slot the same row 138 / 275.  The slots a top-k selects are distinct, and nothing known before the launch tells.
+inline bool direct_form(int32_t s_q, int32_t topk, int32_t s_kv) {
+    const int64_t n = static_cast<int64_t>(s_q) * topk;
+    if (n <= kSmallInput || s_kv >= kPlaceRows - 4 || n >= int64_t{1} << (32 - kPosShift)) return false;
+    const int64_t per_group = (s_q + kMaxGroups - 1) / kMaxGroups;
+    const int64_t batches = topk > kBatch ? per_group * ((topk + kBatch - 1) / kBatch)
+                                          : (per_group + std::min(kQueryBits, kBatch / topk) - 1) / std::min(kQueryBits, kBatch / topk);
+    return s_kv / 1024 * 9 + 50 * batches <= 412 + 175 * std::max<int64_t>(0, (n >> 20) - 2);      // units of 0.04 us
+}
+
+inline Plan make_plan(int32_t s_q, int32_t topk, int32_t s_kv, bool may_be_direct = true) {
+    const int64_t n = static_cast<int64_t>(s_q) * topk;
     int bits = 1;
     while ((static_cast<int64_t>(1) << bits) <= static_cast<int64_t>(s_kv)) ++bits;   // keys are 0..s_kv inclusive
     Plan pl;
@@ -65,6 +96,12 @@ inline Plan make_plan(int64_t n, int32_t s_kv) {
     pl.n_blocks = static_cast<int>(blocks(pl.items));
     pl.key16 = s_kv < 65536;
     pl.by_masks = pl.n_blocks <= kResidentBlocks;
+    pl.groups = pl.per_group = 0;
+    pl.rows_pad = (s_kv + 1 + 3) & ~3;
+    if (may_be_direct && direct_form(s_q, topk, s_kv)) {
+        pl.per_group = (s_q + kMaxGroups - 1) / kMaxGroups;
+        pl.groups = (s_q + pl.per_group - 1) / pl.per_group;
+    }
     return pl;
 }
 
@@ -419,6 +456,298 @@ row_ptr_kernel(const int32_t* __restrict__ heads, const int32_t* __restrict__ fi
     if (lane > warp) m = min(m, warp_min[lane]);
     m = __reduce_min_sync(0xffffffffu, m);
     if (r <= s_kv) row_ptr[r] = min(v, m);
+}
+
+// ---- direct form: a counter per kv row in shared memory, no sort ----------------------------------------------------------
+// The queries are cut into groups of consecutive ones, one block each.  place_kernel goes through its group in batches of up to six
+// queries.  A row's word in shared memory holds the position in `entries` of the row's next slot and one bit per query of the
+// batch: every slot sets its query's bit in its row's word, in any order, and behind a barrier finds its position as the word's
+// position plus the bits of the queries before its own.  So what order the atomics take does not matter, as long as the slots of one
+// query name different rows.  Rows that a query names twice get a flag in their word, and their slots are placed one after the other
+// (place_repeated).  The words start at the rows' positions: group_count_kernel counts every group's slots per row, group_scan_kernel
+// turns these [group][row] counts into positions.
+// What bounds it: place_kernel (61 of 88 us with 8.4 M slots and 32768 rows; the sort: 135) stores four bytes at a time all over `entries`, a
+// sector a cycle and SM (56000 cycles), and its phases between barriers take turns with that.  With 512 threads of sixteen slots 147 us, with one
+// query a batch 91; counting 10, positions 8.
+constexpr int kPlaceWarps = kPlaceThreads / 32;
+constexpr uint32_t kQueryMask = (1u << kQueryBits) - 1u, kRepeated = 1u << kQueryBits;
+constexpr uint32_t kNoRow = 0xffffffffu;
+constexpr int kScanRows = 128, kScanSegs = kPlaceThreads / kScanRows;       // a block of group_scan_kernel: rows x pieces of the groups
+constexpr int kHeads = 1024;
+constexpr uint32_t kNoNode = 2047;
+static_assert(kPlaceThreads <= kNoNode, "eleven bits");
+
+struct PlaceShared {
+    uint32_t none[kPlaceItems * kPlaceWarps];  // per step of 32 slots: unused ones, then the position of the first of them
+    uint32_t none_at;                          // position of the group's next unused slot
+    uint32_t items;                            // place_repeated: which items have a slot of a repeated row
+    // place_repeated: lists, by row modulo kHeads, of nodes; a node stands for the lanes of a warp that name the same row
+    uint32_t head[kHeads];
+    uint32_t node[kPlaceThreads];              // row, next node (kNoNode: none), slots less one: 16, 11, 5 bits
+    uint32_t warp_sums[32];
+    uint32_t total;
+};
+
+// counts[group][row] of the group's slots; row s_kv: its unused ones.  `entries` is cleared, so that its lines are in the L2, whole, when
+// place_kernel stores four bytes at a time into them: on lines that are not there these stores fetch their sectors (buffers that were
+// not in the L2, 8.4 M slots: 112.8 us without the clearing, 92.4 with it).
+__global__ void __launch_bounds__(kPlaceThreads, 1)
+group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __restrict__ entries, int s_q, int per_group, int rows_pad) {
+    extern __shared__ __align__(16) uint32_t cnt[];
+    for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    __syncthreads();
+    const uint32_t q0 = blockIdx.x * per_group, q1 = min(q0 + per_group, static_cast<uint32_t>(s_q));
+    const uint32_t end = q1 * src.topk;
+    uint32_t none = 0;
+    int next[kPlaceItems];
+    auto load = [&](uint32_t i0) {
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) next[k] = i0 + k * kPlaceThreads < end ? __ldg(src.indices + i0 + k * kPlaceThreads) : -1;
+    };
+    load(q0 * src.topk + threadIdx.x);
+    for (uint32_t i0 = q0 * src.topk + threadIdx.x; i0 < end; i0 += kBatch) {
+        int idx[kPlaceItems];
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) idx[k] = next[k];
+        load(i0 + kBatch);
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) {
+            const uint32_t i = i0 + k * kPlaceThreads;
+            if (i < end) entries[i] = 0;
+            const uint32_t key = i < end ? src.key(i, idx[k]) : 0u;
+            if (i < end && key != static_cast<uint32_t>(src.s_kv)) atomicAdd(&cnt[key], 1u);
+            else none += i < end;
+        }
+    }
+    none = __reduce_add_sync(0xffffffffu, none);
+    if ((threadIdx.x & 31) == 0 && none) atomicAdd(&cnt[src.s_kv], none);
+    __syncthreads();
+    uint4* out = reinterpret_cast<uint4*>(counts + static_cast<size_t>(blockIdx.x) * rows_pad);
+    for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) out[i] = reinterpret_cast<uint4*>(cnt)[i];
+}
+
+// counts[group][row] -> position of the group's first entry of the row, counted from the first entry of the block's rows; totals[block]:
+// entries of the block's rows.  "Row" s_kv, the unused slots, is the last one and so lands behind all others.
+__global__ void __launch_bounds__(kPlaceThreads)
+group_scan_kernel(uint32_t* __restrict__ counts, uint32_t* __restrict__ totals, int n_groups, int rows_pad) {
+    constexpr int kPer = (kMaxGroups + kScanSegs - 1) / kScanSegs;
+    __shared__ uint32_t seg_sum[kScanSegs][kScanRows];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t total;
+    const int r = threadIdx.x % kScanRows, seg = threadIdx.x / kScanRows, row = blockIdx.x * kScanRows + r;
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    uint32_t* mine = counts + static_cast<size_t>(seg * kPer) * rows_pad + row;
+    const int n = row < rows_pad ? min(kPer, n_groups - seg * kPer) : 0;
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) c[i] = i < n ? mine[static_cast<size_t>(i) * rows_pad] : 0u;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) sum += c[i];
+    seg_sum[seg][r] = sum;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int s = 0; s < kScanSegs; ++s) {
+        const uint32_t x = seg_sum[s][r];
+        if (s < seg) before += x;
+        all += x;
+    }
+    // rows before this one: segment 0's threads hold one row each
+    const uint32_t at = block_exclusive_scan(seg == 0 ? all : 0u, warp_sums, &total);
+    if (seg == 0) seg_sum[0][r] = at;
+    __syncthreads();
+    before += seg_sum[0][r];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        if (i < n) mine[static_cast<size_t>(i) * rows_pad] = before;
+        before += c[i];
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+
+// Slots of rows that some query of the batch names more than once: 1024 at a time (an item of every thread), in flat order.  A slot's
+// position is its row's, plus the slots of the row in the warps before and in the lanes before; a row has at most one node a warp, so
+// the walk is short however many slots repeat it.  row: as in place_kernel, kNoRow for all other slots.
+__device__ __noinline__ void place_repeated(const uint32_t (&row)[kPlaceItems], uint32_t begin, uint32_t* word, PlaceShared& sh,
+                                            int32_t* __restrict__ entries) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < kPlaceItems; ++k) mine |= static_cast<uint32_t>(row[k] != kNoRow) << k;
+    mine = __reduce_or_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicOr(&sh.items, mine);
+    __syncthreads();
+    const uint32_t items = sh.items;
+#pragma unroll
+    for (int k = 0; k < kPlaceItems; ++k) {
+        if (!((items >> k) & 1u)) continue;              // (the same in the whole block)
+        const bool member = row[k] != kNoRow;
+        const uint32_t r = row[k] & 0xffffu;
+        uint32_t peers = __ballot_sync(0xffffffffu, member);
+        for (uint32_t rest = peers; rest;) {             // a step per row (`match.any` takes a warp at a time, some 64 cycles each)
+            const uint32_t lead = __shfl_sync(0xffffffffu, r, __ffs(rest) - 1);
+            const uint32_t same = __ballot_sync(0xffffffffu, member && r == lead);
+            if ((same >> lane) & 1u) peers = same;
+            rest &= ~same;
+        }
+        const bool first = member && (peers & below) == 0;
+        if (first) {
+            sh.node[threadIdx.x] = r | atomicExch(&sh.head[r % kHeads], threadIdx.x) << 16 | (__popc(peers) - 1) << 27;
+        }
+        __syncthreads();
+        uint32_t before = 0, all = 0, pos = 0;
+        if (member) {
+            for (uint32_t at = sh.head[r % kHeads]; at != kNoNode;) {
+                const uint32_t node = sh.node[at], size = (node & 0xffffu) == r ? (node >> 27) + 1 : 0u;
+                all += size;
+                if (at / 32 < threadIdx.x / 32) before += size;
+                at = node >> 16 & 2047u;
+            }
+            pos = word[r] >> kPosShift;
+            entries[pos + before + __popc(peers & below)] = static_cast<int32_t>(begin + k * kPlaceThreads + threadIdx.x);
+        }
+        __syncthreads();
+        if (first) {
+            sh.head[r % kHeads] = kNoNode;
+            if (before == 0) word[r] = (pos + all) << kPosShift;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) sh.items = 0;
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPlaceThreads, 1)
+place_kernel(const Source src, const uint32_t* __restrict__ counts, const uint32_t* __restrict__ totals, int32_t* __restrict__ row_ptr,
+             int32_t* __restrict__ entries, int s_q, int per_group, int rows_pad, int n_scan_blocks) {
+    extern __shared__ __align__(16) uint32_t word[];
+    __shared__ PlaceShared sh;
+    __shared__ uint32_t base[kPlaceRows / kScanRows + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    static_assert(kPlaceRows / kScanRows + 1 <= kPlaceThreads && kHeads <= kPlaceThreads, "one a thread");
+    sh.head[threadIdx.x] = kNoNode;
+    if (threadIdx.x == 0) sh.items = 0;
+    // batches: as many whole queries as there are bits and slots, or a piece of one query
+    const uint32_t q0 = blockIdx.x * per_group, q1 = min(q0 + per_group, static_cast<uint32_t>(s_q));
+    const uint32_t end = q1 * src.topk;
+    const uint32_t pieces = (src.topk + kBatch - 1) / kBatch;                // of a query
+    const uint32_t n_q = pieces > 1 ? 1u : min(static_cast<uint32_t>(kQueryBits), kBatch / src.topk);
+    const float inv_topk = 1.f / static_cast<float>(src.topk);
+    struct Batch { uint32_t q, begin, end; };
+    auto batch_at = [&](uint32_t b) {
+        const uint32_t q = q0 + b / pieces * n_q, begin = q * src.topk + b % pieces * kBatch;
+        return Batch{q, begin, min(min(begin + kBatch, (q + n_q) * src.topk), end)};
+    };
+    smla::pdl_wait();
+    smla::pdl_trigger();
+    int next[kPlaceItems];
+    auto load = [&](const Batch& t) {
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) {
+            const uint32_t i = t.begin + k * kPlaceThreads + threadIdx.x;
+            next[k] = i < t.end ? __ldg(src.indices + i) : -1;
+        }
+    };
+    const uint32_t n_batches = (q1 - q0 + n_q - 1) / n_q * pieces;
+    Batch t = batch_at(0);
+    load(t);
+    const uint32_t at = block_exclusive_scan(static_cast<int>(threadIdx.x) < n_scan_blocks ? totals[threadIdx.x] : 0u, sh.warp_sums, &sh.total);
+    if (static_cast<int>(threadIdx.x) < n_scan_blocks) base[threadIdx.x] = at;
+    __syncthreads();
+    const uint4* in = reinterpret_cast<const uint4*>(counts + static_cast<size_t>(blockIdx.x) * rows_pad);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) {
+        const uint4 v = __ldcg(in + i);
+        const uint32_t b = base[i / (kScanRows / 4)];
+        reinterpret_cast<uint4*>(word)[i] = make_uint4((v.x + b) << kPosShift, (v.y + b) << kPosShift, (v.z + b) << kPosShift, (v.w + b) << kPosShift);
+    }
+    // row_ptr: where group 0's entries of the row begin; every block writes its share
+    for (int r = blockIdx.x * kPlaceThreads + threadIdx.x; r <= src.s_kv; r += gridDim.x * kPlaceThreads)
+        row_ptr[r] = static_cast<int32_t>(__ldcg(counts + r) + base[r / kScanRows]);
+    if (threadIdx.x == 0) sh.none_at = __ldcg(counts + static_cast<size_t>(blockIdx.x) * rows_pad + src.s_kv) + base[src.s_kv / kScanRows];
+    __syncthreads();
+    for (uint32_t b = 0; b < n_batches; ++b) {
+        const Batch cur = t;
+        uint32_t row[kPlaceItems];                               // with the query's number in the batch above it; kNoRow: no valid slot
+        bool repeated = false;
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) {
+            const uint32_t j = k * kPlaceThreads + threadIdx.x;
+            // (j + 1/2) / topk is at least 1 / (2 topk) away from every whole number, 6e-5 for a batch of more than one query
+            const uint32_t ql = pieces > 1 ? 0u : static_cast<uint32_t>((static_cast<float>(j) + 0.5f) * inv_topk);
+            const bool valid = next[k] >= 0 && next[k] < src.s_kv && (!src.causal || next[k] <= src.q_start + static_cast<int>(cur.q + ql));
+            row[k] = valid ? static_cast<uint32_t>(next[k]) | ql << 16 : kNoRow;
+            const uint32_t none = __ballot_sync(0xffffffffu, !valid && cur.begin + j < cur.end);
+            if (lane == 0) sh.none[k * kPlaceWarps + warp] = __popc(none);
+            // neighbours with one row set its bit once: a row that fills a query's slots would have them all wait for one word
+            const bool again = __shfl_up_sync(0xffffffffu, row[k], 1) == row[k] && lane > 0;
+            if (valid) {
+                uint32_t old = 1u << ql;
+                if (!again) old &= atomicOr(&word[next[k]], old);
+                if (old) {
+                    atomicOr(&word[next[k]], kRepeated);
+                    repeated = true;
+                }
+            }
+        }
+        if (b + 1 < n_batches) {
+            t = batch_at(b + 1);
+            load(t);
+        }
+        const bool any_repeated = __syncthreads_or(repeated);
+        if (warp == 0) {                                         // positions of the unused slots: exclusive sum over the steps
+            constexpr int kPer = kPlaceItems * kPlaceWarps / 32;
+            uint32_t c[kPer], sum = 0;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) sum += c[i] = sh.none[lane * kPer + i];
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            uint32_t a = sh.none_at + incl - sum;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                sh.none[lane * kPer + i] = a;
+                a += c[i];
+            }
+            __syncwarp();
+            if (lane == 31) sh.none_at = a;
+        }
+        uint32_t w[kPlaceItems];
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) w[k] = row[k] != kNoRow ? word[row[k] & 0xffffu] : kRepeated;
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) {
+            if (w[k] & kRepeated) continue;
+            const uint32_t before = w[k] & ((1u << (row[k] >> 16)) - 1u);
+            entries[(w[k] >> kPosShift) + __popc(before)] = static_cast<int32_t>(cur.begin + k * kPlaceThreads + threadIdx.x);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPlaceItems; ++k) {
+            const uint32_t i = cur.begin + k * kPlaceThreads + threadIdx.x;
+            const bool unused = row[k] == kNoRow && i < cur.end;
+            const uint32_t none = __ballot_sync(0xffffffffu, unused);
+            if (unused) entries[sh.none[k * kPlaceWarps + warp] + __popc(none & below)] = static_cast<int32_t>(i);
+            // the row's last query of the batch moves its position on and clears the bits
+            if (!(w[k] & kRepeated) && (w[k] & kQueryMask) >> (row[k] >> 16) == 1u)
+                word[row[k] & 0xffffu] = ((w[k] >> kPosShift) + __popc(w[k] & kQueryMask)) << kPosShift;
+        }
+        __syncthreads();
+        if (any_repeated) {
+#pragma unroll
+            for (int k = 0; k < kPlaceItems; ++k)
+                if (!(w[k] & kRepeated)) row[k] = kNoRow;
+            place_repeated(row, cur.begin, word, sh, entries);
+        }
+    }
 }
 
 // ---- at most one block's worth of slots: every pass in shared memory -----------------------------------------------------
