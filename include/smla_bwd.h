@@ -86,6 +86,10 @@ int smla_bwd_run(const smla_bwd_params* p, void* workspace, size_t workspace_byt
  * dKV over several calls) and lets tests and profilers run one kernel at a time. */
 int smla_bwd_run_stages(const smla_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream,
                         int stage_mask);
+/* Same for a caller that has Delta = rowsum(O * dO) already: `delta` [s_q, h_q] fp32 on the device, in the place of O, which is not read
+ * and may be null.  SMLA_STAGE_DELTA then only finds the slots in use. */
+int smla_bwd_run_given_delta(const smla_bwd_params* p, const float* delta, void* workspace, size_t workspace_bytes, void* stream,
+                             int stage_mask);
 
 /* Whole backward with a REPRODUCIBLE dKV: the same inputs give the same bits in every run.  (No counterpart in the
  * reference, whose scatter is an order-dependent reduce-add as well: mla_bwd/mla_bwd.cu:23-26,527-537.)

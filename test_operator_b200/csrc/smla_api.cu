@@ -316,7 +316,7 @@ bool at_most_a_tile_each(int queries, int tiles_per_query, int clusters) {
 
 template <int HP>
 int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStream_t st, int stages, bool allow_overlap,
-                 const smla_bwd_det_params* det = nullptr) {
+                 const smla_bwd_det_params* det = nullptr, const float* given_delta = nullptr) {
     using namespace smla;
     if (!bind_context()) return SMLA_ERR_LAUNCH;
     __nv_bfloat16* s_scr = reinterpret_cast<__nv_bfloat16*>(ws + pl.s_off);
@@ -350,7 +350,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     kp.kv = reinterpret_cast<const __nv_bfloat16*>(p->kv);
     kp.indices = p->indices;
     kp.lse = p->lse;
-    kp.delta = delta;
+    kp.delta = given_delta ? given_delta : delta;
     kp.n_used = reinterpret_cast<const int*>(ws + pl.used_off);
     kp.s_scr = s_scr;
     kp.ds_scr = ds_scr;
@@ -384,13 +384,16 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     // One tile per cluster and one pass: the recompute kernel's softmax warps find Delta while their only tile is gathered and
     // multiplied, with no prep kernel in front.
     constexpr int kBoth = SMLA_STAGE_DELTA | SMLA_STAGE_RECOMPUTE;
-    if (kp.every_slot && (stages & kBoth) == kBoth && pl.q_chunk >= p->s_q) {
+    if (kp.every_slot && (stages & kBoth) == kBoth && pl.q_chunk >= p->s_q && !given_delta) {
         kp.own_prep = 1;
         kp.o_in = reinterpret_cast<const uint4*>(p->O);
         kp.do_in = reinterpret_cast<const uint4*>(p->dO);
         kp.delta_out = delta;
     }
-    if ((stages & SMLA_STAGE_DELTA) && !kp.own_prep) {
+    if (given_delta) {
+        if ((stages & SMLA_STAGE_DELTA) && !kp.every_slot)       // the slots in use alone
+            launch(smla_prep_kernel, p->s_q, kPrepThreads, 0, st, true, 1, nullptr, nullptr, nullptr, reinterpret_cast<int*>(ws + pl.used_off), 1, kp);
+    } else if ((stages & SMLA_STAGE_DELTA) && !kp.own_prep) {
         // one block per query, more for few queries (34 queries x 128 heads: 14 us with one block per query, 6.6 us so)
         int head_parts = 1;
         while (static_cast<long long>(p->s_q) * head_parts * 2 <= 8 * kSmCount && p->h_q / (head_parts * 2) >= 16) head_parts *= 2;
@@ -734,10 +737,10 @@ int smla_bwd_get_workspace_layout(const smla_bwd_params* p, size_t workspace_byt
 
 namespace {
 int run_stages_impl(const smla_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream, int stage_mask,
-                    bool allow_overlap, const smla_bwd_det_params* det = nullptr) {
+                    bool allow_overlap, const smla_bwd_det_params* det = nullptr, const float* given_delta = nullptr) {
     g_last_launches = 0;
     if (!check_params(p) || !workspace) return SMLA_ERR_BAD_ARG;
-    if (!p->q || !p->kv || !p->dO || !p->lse || !p->O || !p->indices || !p->dQ || !p->dKV) return SMLA_ERR_BAD_ARG;
+    if (!p->q || !p->kv || !p->dO || !p->lse || (!p->O && !given_delta) || !p->indices || !p->dQ || !p->dKV) return SMLA_ERR_BAD_ARG;
     // TMA needs 16-byte aligned bases; vector loads/stores need the same for the rest
     if (!aligned16(p->q) || !aligned16(p->kv) || !aligned16(p->dO) || !aligned16(p->O) || !aligned16(p->dQ) ||
         !aligned16(p->dKV) || (reinterpret_cast<uintptr_t>(workspace) & (kAlign - 1)))
@@ -754,10 +757,15 @@ int run_stages_impl(const smla_bwd_params* p, void* workspace, size_t workspace_
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-    return pl.h_pad == 64 ? launch_chain<64>(p, pl, ws, st, stage_mask, allow_overlap, det)
-                          : launch_chain<128>(p, pl, ws, st, stage_mask, allow_overlap, det);
+    return pl.h_pad == 64 ? launch_chain<64>(p, pl, ws, st, stage_mask, allow_overlap, det, given_delta)
+                          : launch_chain<128>(p, pl, ws, st, stage_mask, allow_overlap, det, given_delta);
 }
 }  // namespace
+
+int smla_bwd_run_given_delta(const smla_bwd_params* p, const float* delta, void* workspace, size_t workspace_bytes, void* stream, int stage_mask) {
+    if (!delta || (reinterpret_cast<uintptr_t>(delta) & 3)) return SMLA_ERR_BAD_ARG;
+    return run_stages_impl(p, workspace, workspace_bytes, stream, stage_mask, true, nullptr, delta);
+}
 
 int smla_bwd_run_deterministic(const smla_bwd_params* p, const smla_bwd_det_params* det, void* workspace,
                                size_t workspace_bytes, void* stream, int stage_mask) {

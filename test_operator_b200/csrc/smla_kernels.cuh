@@ -229,8 +229,9 @@ smla_prep_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, floa
         for (int w = 1; w < kWarps; ++w) m = max(m, red[w]);
         n_used[q] = m + 1;
     }
-    if (q < p.s_q && O == nullptr) {             // forward: a query without a valid slot is in nobody's range
-        int m = -1;
+    if (O == nullptr) {                          // forward, or a backward that is given Delta
+        if (q >= p.s_q || p.gout == nullptr) return;
+        int m = -1;                              // a query without a valid slot is in nobody's range
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) m = max(m, red[w]);
         if (m < 0) {

@@ -107,6 +107,9 @@ def load_library() -> ctypes.CDLL:
         lib.smla_bwd_run_stages.restype = ctypes.c_int
         lib.smla_bwd_run_stages.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p,
                                             ctypes.c_int]
+        lib.smla_bwd_run_given_delta.restype = ctypes.c_int
+        lib.smla_bwd_run_given_delta.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p,
+                                                 ctypes.c_int]
         lib.smla_query_meta.restype = ctypes.c_int
         lib.smla_query_meta.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
@@ -177,6 +180,10 @@ class _NoNativeHost:
 
     @staticmethod
     def fwd(*_):
+        return None
+
+    @staticmethod
+    def delta_start(*_):
         return None
 
     @staticmethod
@@ -390,6 +397,7 @@ def mla_bwd(
     query_meta: Optional[torch.Tensor] = None,
     deterministic: bool = False,
     staging_budget: int = 2 << 30,
+    delta: Optional[torch.Tensor] = None,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Sparse MLA attention backward.  Returns (dQ bf16 [s_q,h_q,576], dKV fp32 shaped like kv).
 
@@ -403,7 +411,8 @@ def mla_bwd(
     (device, stream).  `deterministic=True` makes dKV reproducible bit for bit (dQ always is): the index inverse of the
     sparse pattern is built (`index_inverse`), every slot's contribution goes to a staging buffer of at most about
     `staging_budget` bytes and is added per kv row in a fixed order - slower (one extra write and read of 2304
-    bytes per slot), for runs that must repeat exactly.  The call enqueues on the current stream and does not
+    bytes per slot), for runs that must repeat exactly.  `delta` (fp32 [s_q, h_q] on the device): rowsum(O * dO) for a caller that has
+    it already; what O holds is not read then.  The call enqueues on the current stream and does not
     synchronise unless `check_device_status=True`, which also raises if a kernel reported a timed-out wait.
     """
     host = _host()
@@ -411,7 +420,10 @@ def mla_bwd(
     if not native_need:
         _validate(q, kv, dO, lse, O, indices)
     _check_query_meta(query_meta, q)
-    if native_need and not (deterministic or workspace_budget):
+    if delta is not None:
+        _check(not deterministic, "deterministic=True finds Delta itself")
+        _check_out(delta, lse.numel(), torch.float32, q.device, "delta")
+    if native_need and not (deterministic or workspace_budget or delta is not None):
         if out_dq is not None:
             _check_out(out_dq, q.numel(), torch.bfloat16, q.device, "out_dq")
         if out_dkv is not None:
@@ -469,6 +481,8 @@ def mla_bwd(
                                                     stream, stages)
                 for t in (row_ptr, entries):
                     t.record_stream(torch.cuda.current_stream())
+            elif delta is not None:
+                st = lib.smla_bwd_run_given_delta(ctypes.byref(params), delta.data_ptr(), workspace.ptr, workspace.nbytes, stream, stages)
             else:
                 st = lib.smla_bwd_run_stages(ctypes.byref(params), workspace.ptr, workspace.nbytes, stream, stages)
         _raise_status(lib, st, "smla_bwd_run")
@@ -829,6 +843,9 @@ def last_launch_count() -> int:
 
 
 _HOST_BLOCK_BYTES = 4 << 20
+# Threads that find Delta on the host, where torch may use that many: 1024 queries x 128 heads on pinned buffers 11.0 ms with O copied, 12.0 with
+# three threads, 10.0 with four, 9.05 with five or six, 9.15 with eight, 9.45 with twelve (they take the host's memory from the copies).
+_HOST_DELTA_THREADS = 6
 
 
 def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] = None,
@@ -839,7 +856,8 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
 
     The query dimension is cut into at most `n_chunks` blocks (of a few MB of inputs at least) and pipelined over three
     streams: block i+1 is copied to `device` while block i runs and the dQ of block i-1 travels back; every block adds into
-    one fp32 dKV on the device, which returns last.  Returns (dQ, dKV) as host tensors (written into
+    one fp32 dKV on the device, which returns last.  With several blocks Delta is found on the host, by threads that end with the call, and
+    O does not cross PCIe (contiguous inputs, and a torch that may use six threads: `torch.set_num_threads`).  Returns (dQ, dKV) as host tensors (written into
     `out_dq` / `out_dkv` when given) and synchronises before returning.
     """
     dev = torch.device(device)
@@ -874,21 +892,49 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
             t.record_stream(s_in)
         for t in (dkv_d, dq_d):
             t.record_stream(s_out)
+        # O is needed for Delta alone: where the host finds that fast enough, O stays where it is.
+        job = None
+        if n_chunks > 1 and torch.get_num_threads() >= _HOST_DELTA_THREADS:
+            delta = torch.empty(lse[:s_q].shape, dtype=torch.float32, pin_memory=True)
+            job = _host().delta_start(host[3], host[1], delta, _HOST_DELTA_THREADS)
+        if job is not None:
+            delta_d = torch.empty(delta.shape, dtype=torch.float32, device=dev)
+            delta_d.record_stream(s_in)
         s_in.wait_stream(s_comp)
         with torch.cuda.stream(s_in):
             kv_d.copy_(kv, non_blocking=True)
         first = True
-        for r0, r1 in zip(bounds, bounds[1:]):
-            if r1 == r0:
-                continue
-            blk = [d[r0:r1] for d in dev_in]
+        blocks = [(r0, r1) for r0, r1 in zip(bounds, bounds[1:]) if r1 > r0]
+
+        def copy_in(i):
+            r0, r1 = blocks[i]
             with torch.cuda.stream(s_in):
-                for d, t in zip(blk, host):
-                    d.copy_(t[r0:r1], non_blocking=True)
-            s_comp.wait_event(s_in.record_event())
+                for k, (d, t) in enumerate(zip(dev_in, host)):
+                    if k != 3 or job is None:
+                        d[r0:r1].copy_(t[r0:r1], non_blocking=True)
+
+        for i, (r0, r1) in enumerate(blocks):
+            given = {}
+            if i == 0 or job is None:
+                copy_in(i)
+            if job is not None:
+                # (PCIe does not wait for a Delta that is not ready: the next block's copies go first then)
+                rows = r1 * lse.shape[1]
+                ahead = i + 1 < len(blocks) and not _host().delta_wait(job, rows, False)
+                if ahead:
+                    copy_in(i + 1)
+                _host().delta_wait(job, rows, True)
+                with torch.cuda.stream(s_in):
+                    delta_d[r0:r1].copy_(delta[r0:r1], non_blocking=True)
+                given["delta"] = delta_d[r0:r1]
+            arrived = s_in.record_event()
+            if job is not None and i + 1 < len(blocks) and not ahead:
+                copy_in(i + 1)
+            blk = [d[r0:r1] for d in dev_in]
+            s_comp.wait_event(arrived)
             qs = None if q_start_index_s is None else q_start_index_s + r0
             mla_bwd(blk[0], kv_d, blk[1], blk[2], blk[3], blk[4], sm_scale=sm_scale, q_start_index_s=qs,
-                    lse_is_base2=lse_is_base2, out_dkv=dkv_d, accumulate=not first, workspace=workspace, out_dq=dq_d[r0:r1])
+                    lse_is_base2=lse_is_base2, out_dkv=dkv_d, accumulate=not first, workspace=workspace, out_dq=dq_d[r0:r1], **given)
             first = False
             s_out.wait_event(s_comp.record_event())
             with torch.cuda.stream(s_out):
