@@ -1919,15 +1919,16 @@ __global__ void __launch_bounds__(256) smla_dkv_segment_sum_kernel(const int* __
 // =============================================================================================
 // dq: one CTA per (query, d-part of three column chunks); 14 warps; two CTAs per SM, so that one's start-up (TMEM,
 // first gathers) and epilogue run under the other's tiles.
-//   warps 0-3   epilogue: TMEM -> bf16 -> dQ[q, head, d]; lane = head, so a thread stores whole 64-byte pieces of
-//               its head's row
+//   warps 0-3   epilogue: TMEM -> bf16 -> dQ[q, head, d]; lane = head (64 heads: sixteen in the lower lanes of every warp), so a
+//               thread stores whole 64-byte pieces of its head's row
 //   warps 4-11  producers: per 64-key tile the part's columns of the kv rows picked by index (16-byte
 //               cp.async into the swizzled layout)
 //   warp 13     TMA: the dS scratch tile
 //   warp 12     UMMA issuer: acc[128 heads, d of the part] += dS^T . Kg  (both operands MN-major: the key index is
 //               the contraction and runs along shared-memory rows).  Heads are the M side so that N can be the 192
-//               columns of the part.  With HP = 64 the upper 64 accumulator rows are computed from whatever follows the
-//               dS tile in shared memory and never read.
+//               columns of the part.  64 heads use M = 64: as fast in cycles as M = 128 with 64 rows to spare, but these
+//               cost power, and long calls run at the power cap: 4096 queries x 64 heads x top-k 2048 back to back 1207 ->
+//               1048 us for the kernel, 6073 -> 5885 for the call; 777 x 64 x 600 402 -> 388.
 // With few queries a cluster of up to eight CTAs splits the keys of one (query, d-part) and adds up in rank order.
 // =============================================================================================
 namespace dq {
@@ -1944,8 +1945,7 @@ template <int HP, bool kDeep> struct Cfg {
     static constexpr int kDsBytes = (HP / 64) * 8192;
     static constexpr int kStage = kKgBytes + kDsBytes;     // dS right after Kg
     static constexpr int kOffMisc = kStages * kStage;
-    // the A operand always spans 128 heads: with HP = 64 its upper half reads 8 KB past the dS tile
-    static constexpr int kSmemBytes = kOffMisc + 256 + 1024 + (HP == 64 ? 8192 : 0);
+    static constexpr int kSmemBytes = kOffMisc + 256 + 1024;
     static_assert((kDeep ? 1 : 2) * (kSmemBytes + 1024) <= 233472, "one or two CTAs per SM");
     static constexpr int kTmemCols = 256;                  // up to 256 columns of d; two CTAs share the SM's 512
     static constexpr int kRowBytes = kDqChunks * 128 + 16;    // epilogue staging of one head's row
@@ -2079,7 +2079,7 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         }
     } else if (warp == 12) {
         if (elect_one()) {
-            constexpr uint32_t idesc1 = make_idesc_bf16(128, kDqChunks * 64, 1, 1);     // N = the part's columns in one UMMA
+            constexpr uint32_t idesc1 = make_idesc_bf16(HP, kDqChunks * 64, 1, 1);     // N = the part's columns in one UMMA
             // A = dS^T: [HP/8 head blocks][64 keys][8 heads], 8-key groups 128 B apart, head blocks 1 KB apart.
             // Descriptors: the fixed fields once, the address (16-byte units, the low 14 bits) added per UMMA.
             const uint64_t a_hi = make_smem_desc(0, 128, 1024, kSwizzleNone) & 0xFFFFFFFF00000000ull;
@@ -2117,11 +2117,14 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
         // spread over all banks) and sends it off as one bulk copy: whole cache lines instead of 32 scattered
         // 16-byte pieces per store instruction.
         constexpr int kRowBytes = C::kRowBytes;
-        const int head = quarter * 32 + lane;
+        // 128 heads: one per lane; 64 (UMMAs of M = 64): sixteen in the lower lanes of every quarter
+        constexpr int kQuarterHeads = HP / 4;
+        const int head = quarter * kQuarterHeads + (lane & (kQuarterHeads - 1));
+        const bool real = lane < kQuarterHeads && head < p.h_q;
         const uint32_t row_s = s_base + head * kRowBytes;
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
         if (kDeep && nz > 1) {
-            if (quarter * 32 < p.h_q) {
+            if (quarter * kQuarterHeads < p.h_q) {
                 const uint32_t part_s = s_base + head * (C::kPartPitch * 4);
 #pragma unroll 1
                 for (int cg = 0; cg < kDqChunks * 4; ++cg) {
@@ -2130,11 +2133,12 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                     tmem_ld_wait();
 #pragma unroll
                     for (int v = 0; v < 4; ++v)
-                        st_shared_v4(part_s + cg * 64 + v * 16, r[4 * v] & zero_mask, r[4 * v + 1] & zero_mask, r[4 * v + 2] & zero_mask,
-                                     r[4 * v + 3] & zero_mask);
+                        if (lane < kQuarterHeads)
+                            st_shared_v4(part_s + cg * 64 + v * 16, r[4 * v] & zero_mask, r[4 * v + 1] & zero_mask, r[4 * v + 2] & zero_mask,
+                                         r[4 * v + 3] & zero_mask);
                 }
             }
-        } else if (quarter * 32 < p.h_q) {        // warp-uniform: heads are padded to a multiple of 8 only
+        } else if (quarter * kQuarterHeads < p.h_q) {        // warp-uniform: heads are padded to a multiple of 8 only
 #pragma unroll 1
             // 32 columns at a time: two CTAs per SM leave 64 registers a thread (16 at a time: 64 queries x 16 heads x top-k 64
             // 19.64 against 19.43 us, larger calls alike)
@@ -2146,13 +2150,13 @@ smla_dq_kernel(const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
                 for (int i = 0; i < 32; ++i) r[i] &= zero_mask;
 #pragma unroll
                 for (int v = 0; v < 4; ++v)
-                    st_shared_v4(row_s + cg * 64 + v * 16,
+                    if (lane < kQuarterHeads) st_shared_v4(row_s + cg * 64 + v * 16,
                                  pack_bf16x2(__uint_as_float(r[8 * v]), __uint_as_float(r[8 * v + 1])),
                                  pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3])),
                                  pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5])),
                                  pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7])));
             }
-            if (head < p.h_q) {
+            if (real) {
                 fence_proxy_async_smem();         // this thread's row only: no one else touches it
                 bulk_store(p.dQ + (static_cast<size_t>(qg) * p.h_q + head) * kDQK + chunk0 * 64, row_s, kDqChunks * 128);
                 bulk_commit();
