@@ -1705,6 +1705,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             } else {
                 // -------------------------------------------------------------- UMMA issuer for the pair
                 constexpr uint32_t idesc = make_idesc_bf16(256, 128, 1, 0);   // A MN-major (d contiguous), B K-major
+                constexpr uint32_t idesc2 = make_idesc_bf16(128, 128, 1, 0);  // block 2: 64 rows per CTA
                 int s = 0;
                 uint32_t ph = 0, k = 0, unit = 0;
                 bool new_query = true;
@@ -1720,8 +1721,8 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         mbar_wait(bar_uempty + 8 * us, ((unit / kUnits) & 1) ^ 1, wc, kErrDkv + 3);
                         tc_fence_after_sync();
                         const uint32_t d = tmem + us * 128;
-                        // each CTA's 128 rows: slot pair (0,1), (2,3) or, for block 2, (3,4)
-                        const int slot = blk == 2 ? 3 : 2 * blk;
+                        // each CTA's 128 rows: slot pair (0,1) or (2,3); for block 2 the 64 rows of slot 4, the same in both
+                        const int slot = blk == 2 ? 4 : 2 * blk;
                         if (blk < 2) {
                             const uint32_t a_do = s_base + C::kOffDO + slot * C::kChunk;
 #pragma unroll
@@ -1733,7 +1734,7 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
                         for (int ks = 0; ks < HP / 16; ++ks)
                             umma_ss_2cta(d, make_smem_desc(a_q + ks * 2048, C::kChunk, 1024, kSwizzle128),
-                                         make_smem_desc(st_ds + ks * 2048, 1024, 128, kSwizzleNone), idesc,
+                                         make_smem_desc(st_ds + ks * 2048, 1024, 128, kSwizzleNone), blk < 2 ? idesc : idesc2,
                                          blk < 2 || ks != 0);
                         umma_commit_2cta_mask(bar_ufull + 8 * us, 3);
                         if (last && blk != 1) umma_commit_2cta_mask(bar_resfree + 8 * (blk >> 1), 3);
@@ -1795,18 +1796,19 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const int us = unit % kUnits;
                 mbar_wait(bar_ufull + 8 * us, (unit / kUnits) & 1, wc, kErrDkv + 5, kPollSleepNs);
                 tc_fence_after_sync();
-                // blocks 0, 1: every row is real (d = 256 blk + 128 rank + row).  Block 2: rows 64..127 are d 512..575
-                // in both CTAs; the CTA whose turn it is drains them.
-                const bool mine = blk < 2 || (quarter >= 2 && (n & 1) == rank);
+                // Blocks 0, 1: every row is real (d = 256 blk + 128 rank + row).  Block 2: 64 rows, d 512..575 in both CTAs; lanes 0-63 hold
+                // them for the first 64 keys of the tile, lanes 64-127 for the others.  Each CTA drains one half, the warps that have
+                // that half's indices; which one changes from tile to tile, so that the four sub-partitions have the same to do.
+                const int half = (static_cast<int>(n) ^ static_cast<int>(rank)) & 1;
+                const bool mine = blk < 2 || (e == half && (quarter >> 1) == half);
                 if (mine) {
-                    const int d0 = blk < 2 ? 256 * blk + 128 * static_cast<int>(rank) : 512 - 64;
-                    float* out = p.dKV + d0 + quarter * 32 + lane;
+                    const int d = blk < 2 ? 256 * blk + 128 * static_cast<int>(rank) + quarter * 32 + lane : 512 + (quarter & 1) * 32 + lane;
+                    float* out = p.dKV + d;
                     // staged form: the row of slot (query, first key of this warp's 64) in the staging buffer
                     float* sout = nullptr;
                     if constexpr (kStaged)
-                        sout = p.staging + (static_cast<size_t>(sq) * p.topk_pad + tile * kTileKeys + 64 * e) * kDQK +
-                               d0 + quarter * 32 + lane;
-                    const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + us * 128 + 64 * e;
+                        sout = p.staging + (static_cast<size_t>(sq) * p.topk_pad + tile * kTileKeys + 64 * e) * kDQK + d;
+                    const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + us * 128 + (blk < 2 ? 64 * e : 0);
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         if (left <= 32 * i) break;      // behind the last slot in use: a predicated-off reduction costs its issue
