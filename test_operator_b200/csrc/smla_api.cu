@@ -417,7 +417,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             // of this pass in CSR order
             launch(smla_dkv_pair_kernel<HP, true>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s,
                    tm_ds, kp);
-            launch(smla_dkv_segment_sum_kernel, (p->s_kv + 7) / 8, 256, 0, s_, false, 1, det->row_ptr, det->entries, det->staging, p->dKV,
+            launch(smla_dkv_segment_sum_kernel, std::min((p->s_kv + kSegThreads / 32 - 1) / (kSegThreads / 32), 2 * kSmCount), kSegThreads, 0, s_, true, 1, det->row_ptr, det->entries, det->staging, p->dKV,
                    p->s_kv, p->topk, pl.topk_pad, kp.q0, kp.q0 + kp.nq);
             return;
         }
@@ -452,7 +452,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             kp.scr0 = 0;
             if (stages & SMLA_STAGE_RECOMPUTE) launch_recompute(st, pairs_r, true);
             if (stages & SMLA_STAGE_DKV) launch_dkv(st, pairs_d, true, stages & SMLA_STAGE_RECOMPUTE);
-            if (stages & SMLA_STAGE_DQ) launch_dq(st, true, (stages & SMLA_STAGE_DKV) && !det);
+            if (stages & SMLA_STAGE_DQ) launch_dq(st, true, stages & SMLA_STAGE_DKV);
             continue;
         }
         std::lock_guard<std::mutex> lock(g_dev_sched_mutex);
@@ -753,7 +753,9 @@ int run_stages_impl(const smla_bwd_params* p, void* workspace, size_t workspace_
         const size_t per_q = size_t(pl.topk_pad) * SMLA_D_QK * sizeof(float);
         const size_t fit = det->staging_bytes / per_q;
         if (fit < 1) return SMLA_ERR_WORKSPACE;
-        if (size_t(pl.q_chunk) > fit) pl.q_chunk = int(fit);
+        // passes of equal size (1024 queries of 2048 slots, 455 of which fit: three of 342, not two and one of 114)
+        const int passes = int((p->s_q + std::min<size_t>(pl.q_chunk, fit) - 1) / std::min<size_t>(pl.q_chunk, fit));
+        pl.q_chunk = (p->s_q + passes - 1) / passes;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);

@@ -1855,66 +1855,72 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // CSR segment (found by binary search), and passes follow one another in a fixed order.  Bound by reading the staging
 // rows once: four rows of 2304 bytes in flight per warp (with two, in 4-byte loads: 4.3 TB/s; now 5.7).
 // =============================================================================================
+// Two blocks an SM go through the rows: all of them are there from the start, so the dQ kernel behind this one, which needs nothing of it,
+// comes up beside the last rows.  1024 queries x 64 heads x top-k 2048 2677 -> 2590 us, 300 x 128 x 1000 572 -> 548, 40 x 128 x 512 84.8 ->
+// 73.4, 1000 x 64 x 128 on 60000 rows 428 -> 380.  With one block, and dQ CTAs beside it throughout, too little is in flight (3147).
 constexpr int kFlight = 4;
-__global__ void __launch_bounds__(256) smla_dkv_segment_sum_kernel(const int* __restrict__ row_ptr,
-                                                                   const int* __restrict__ entries,
-                                                                   const float* __restrict__ staging, float* __restrict__ dKV,
-                                                                   int s_kv, int topk, int topk_pad, int q_lo, int q_hi) {
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+constexpr int kSegThreads = 256;
+__global__ void __launch_bounds__(kSegThreads) smla_dkv_segment_sum_kernel(const int* __restrict__ row_ptr,
+                                                                           const int* __restrict__ entries,
+                                                                           const float* __restrict__ staging, float* __restrict__ dKV,
+                                                                           int s_kv, int topk, int topk_pad, int q_lo, int q_hi) {
     const int lane = threadIdx.x & 31;
-    if (row >= s_kv) return;
-    const int b = __ldg(row_ptr + row), e = __ldg(row_ptr + row + 1);
-    auto lower = [&](long long flat) {      // first position in [b, e) whose flat slot id is >= flat
-        int lo = b, hi = e;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (__ldg(entries + mid) < flat) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo;
-    };
-    const int i0 = lower(static_cast<long long>(q_lo) * topk), i1 = lower(static_cast<long long>(q_hi) * topk);
-    if (i1 <= i0) return;
-    constexpr int kPer = kDQK / 64;          // nine pairs of elements per lane
-    float2 acc[kPer];
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) acc[k] = make_float2(0.f, 0.f);
-    for (int c = i0; c < i1; c += 32) {      // a lane locates one of the next 32 slots, the warp adds them in order
-        const int n = min(32, i1 - c);
-        unsigned long long mine = 0;
-        if (lane < n) {
-            const int flat = __ldg(entries + c + lane);
-            const int q = flat / topk;
-            mine = reinterpret_cast<unsigned long long>(staging + (static_cast<size_t>(q - q_lo) * topk_pad + (flat - q * topk)) * kDQK);
-        }
-        for (int j = 0; j < n; j += kFlight) {
-            float2 v[kFlight][kPer];
-#pragma unroll
-            for (int u = 0; u < kFlight; ++u) {
-                const unsigned long long src = __shfl_sync(0xffffffffu, mine, min(j + u, 31));
-                if (j + u < n) {
-#pragma unroll
-                    for (int k = 0; k < kPer; ++k) v[u][k] = __ldcs(reinterpret_cast<const float2*>(src) + lane + 32 * k);
-                }
+    pdl_wait();                   // the staging rows
+    pdl_trigger();
+    for (int row = blockIdx.x * (kSegThreads / 32) + (threadIdx.x >> 5); row < s_kv; row += gridDim.x * (kSegThreads / 32)) {
+        const int b = __ldg(row_ptr + row), e = __ldg(row_ptr + row + 1);
+        auto lower = [&](long long flat) {      // first position in [b, e) whose flat slot id is >= flat
+            int lo = b, hi = e;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (__ldg(entries + mid) < flat) lo = mid + 1;
+                else hi = mid;
             }
+            return lo;
+        };
+        const int i0 = lower(static_cast<long long>(q_lo) * topk), i1 = lower(static_cast<long long>(q_hi) * topk);
+        if (i1 <= i0) continue;
+        constexpr int kPer = kDQK / 64;          // nine pairs of elements per lane
+        float2 acc[kPer];
 #pragma unroll
-            for (int u = 0; u < kFlight; ++u)
-                if (j + u < n) {
+        for (int k = 0; k < kPer; ++k) acc[k] = make_float2(0.f, 0.f);
+        for (int c = i0; c < i1; c += 32) {      // a lane locates one of the next 32 slots, the warp adds them in order
+            const int n = min(32, i1 - c);
+            unsigned long long mine = 0;
+            if (lane < n) {
+                const int flat = __ldg(entries + c + lane);
+                const int q = flat / topk;
+                mine = reinterpret_cast<unsigned long long>(staging + (static_cast<size_t>(q - q_lo) * topk_pad + (flat - q * topk)) * kDQK);
+            }
+            for (int j = 0; j < n; j += kFlight) {
+                float2 v[kFlight][kPer];
 #pragma unroll
-                    for (int k = 0; k < kPer; ++k) {
-                        acc[k].x += v[u][k].x;
-                        acc[k].y += v[u][k].y;
+                for (int u = 0; u < kFlight; ++u) {
+                    const unsigned long long src = __shfl_sync(0xffffffffu, mine, min(j + u, 31));
+                    if (j + u < n) {
+#pragma unroll
+                        for (int k = 0; k < kPer; ++k) v[u][k] = __ldcs(reinterpret_cast<const float2*>(src) + lane + 32 * k);
                     }
                 }
-        }
-    }
-    float2* out = reinterpret_cast<float2*>(dKV + static_cast<size_t>(row) * kDQK) + lane;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        float2 x = out[32 * k];
-        x.x += acc[k].x;
-        x.y += acc[k].y;
-        out[32 * k] = x;
+                for (int u = 0; u < kFlight; ++u)
+                    if (j + u < n) {
+#pragma unroll
+                        for (int k = 0; k < kPer; ++k) {
+                            acc[k].x += v[u][k].x;
+                            acc[k].y += v[u][k].y;
+                        }
+                    }
+            }
+        }
+        float2* out = reinterpret_cast<float2*>(dKV + static_cast<size_t>(row) * kDQK) + lane;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            float2 x = out[32 * k];
+            x.x += acc[k].x;
+            x.y += acc[k].y;
+            out[32 * k] = x;
+        }
     }
 }
 
