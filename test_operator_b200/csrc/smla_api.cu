@@ -340,6 +340,7 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             bool done = set_smem(smla_recompute_pair_kernel<HP>, rp::Cfg<HP>::kSmemBytes);
             done &= set_smem(smla_dkv_pair_kernel<HP>, dp::Cfg<HP>::kSmemBytes);
             done &= set_smem(smla_dkv_pair_kernel<HP, true>, dp::Cfg<HP>::kSmemBytes);
+            done &= set_smem(smla_dkv_pair_kernel<HP, false, true>, dp::Cfg<HP>::kSmemBytes);
             done &= set_smem(smla_dq_kernel<HP, false>, dq::Cfg<HP, false>::kSmemBytes);
             done &= set_smem(smla_dq_kernel<HP, true>, dq::Cfg<HP, true>::kSmemBytes);
             return done;
@@ -402,12 +403,12 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
     }
     if (!(stages & (SMLA_STAGE_RECOMPUTE | SMLA_STAGE_DKV | SMLA_STAGE_DQ)))
         return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
-    auto grid_of = [&](int pairs) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * q_tiles)); };
+    auto grid_of = [&](int pairs, int tiles) { return 2 * int(std::min<long long>(pairs, static_cast<long long>(kp.nq) * tiles)); };
     // `pdl`: start under the previous kernel's tail (one-stream schedules only)
     auto launch_recompute = [&](cudaStream_t s_, int pairs, bool pdl) {
         kp.clear_bytes = kp.q0 == 0 ? clear_bytes : 0;
         // (further clusters, without a tile, where few queries come with a large dKV: 16 KB of it a block)
-        const int grid = std::max(grid_of(pairs), 2 * int(std::min<size_t>(pairs, kp.clear_bytes >> 15)));
+        const int grid = std::max(grid_of(pairs, q_tiles), 2 * int(std::min<size_t>(pairs, kp.clear_bytes >> 15)));
         launch(smla_recompute_pair_kernel<HP>, grid, rp::kThreads, rp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qnh, tm_donh, kp);
     };
     auto launch_dkv = [&](cudaStream_t s_, int pairs, bool pdl, bool after_recompute) {
@@ -415,13 +416,18 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
         if (det) {
             // reproducible form: per-slot contributions to the staging rows, then one warp per kv row adds its slots
             // of this pass in CSR order
-            launch(smla_dkv_pair_kernel<HP, true>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s,
+            launch(smla_dkv_pair_kernel<HP, true>, grid_of(pairs, q_tiles), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s,
                    tm_ds, kp);
             launch(smla_dkv_segment_sum_kernel, std::min((p->s_kv + kSegThreads / 32 - 1) / (kSegThreads / 32), 2 * kSmCount), kSegThreads, 0, s_, true, 1, det->row_ptr, det->entries, det->staging, p->dKV,
                    p->s_kv, p->topk, pl.topk_pad, kp.q0, kp.q0 + kp.nq);
             return;
         }
-        launch(smla_dkv_pair_kernel<HP>, grid_of(pairs), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s, tm_ds, kp);
+        const int tiles = (p->topk + dp::kTileKeys - 1) / dp::kTileKeys;
+        if (tiles > 1)
+            launch(smla_dkv_pair_kernel<HP, false, true>, grid_of(pairs, tiles), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp,
+                   tm_s, tm_ds, kp);
+        else
+            launch(smla_dkv_pair_kernel<HP>, grid_of(pairs, tiles), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s, tm_ds, kp);
     };
     const int dq_split = dq_key_split(p->s_q, pl.topk_pad, dq::kParts);
     auto launch_dq = [&](cudaStream_t s_, bool pdl, bool after_dkv) {

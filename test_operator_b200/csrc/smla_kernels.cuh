@@ -298,7 +298,7 @@ struct WorkRange {
     int begin, end;               // positions among the launch's tiles
     int q, lo;                    // the query `begin` lies in; position of its first tile
 };
-__device__ __forceinline__ int work_tiles(int n_used) { return (n_used + kWorkTileKeys - 1) / kWorkTileKeys; }
+template <int kKeys = kWorkTileKeys> __device__ __forceinline__ int work_tiles(int n_used) { return (n_used + kKeys - 1) / kKeys; }
 __device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clusters) {     // n_tiles * cluster / n_clusters in 32 bits
     const uint32_t n = n_tiles, c = cluster, m = n_clusters;
     return static_cast<int>(n / m * c + n % m * c / m);
@@ -307,11 +307,11 @@ __device__ __forceinline__ int range_start(int n_tiles, int cluster, int n_clust
 // the slot counts itself (a few per thread: 8192 queries are 32 KB out of L2, all in flight at once), so that the ranges need
 // no prefix sum made by a kernel before and no counter that would have to survive from launch to launch.
 // scratch: one word of shared memory per warp.  Returns, in the one thread that wrote *out, the launch's tiles; -1 in the others.
-template <int kThreads>
+template <int kThreads, int kKeys = kWorkTileKeys>
 __device__ __forceinline__ int find_range(const KParams& p, int cluster, int n_clusters, int* scratch, WorkRange* out) {
     if (p.every_slot) {
         if (threadIdx.x != 0) return -1;
-        const int tiles = work_tiles(p.every_slot), total = p.nq * tiles, begin = range_start(total, cluster, n_clusters);
+        const int tiles = work_tiles<kKeys>(p.every_slot), total = p.nq * tiles, begin = range_start(total, cluster, n_clusters);
         *out = WorkRange{begin, range_start(total, cluster + 1, n_clusters), p.q0 + begin / tiles, begin / tiles * tiles};
         return total;
     }
@@ -320,13 +320,13 @@ __device__ __forceinline__ int find_range(const KParams& p, int cluster, int n_c
     const int i0 = min(static_cast<int>(threadIdx.x) * per, p.nq), i1 = min(i0 + per, p.nq);
     int sum = 0, total;
 #pragma unroll 8
-    for (int i = i0; i < i1; ++i) sum += work_tiles(__ldcg(used + i));
+    for (int i = i0; i < i1; ++i) sum += work_tiles<kKeys>(__ldcg(used + i));
     int lo = block_exclusive_sum(sum, scratch, &total);
     const int begin = range_start(total, cluster, n_clusters);
     if (total == 0 ? threadIdx.x != 0 : begin < lo || begin >= lo + sum) return -1;
     int q = i0;
     if (total > 0) {
-        for (int n; begin >= lo + (n = work_tiles(__ldcg(used + q))); ++q) lo += n;
+        for (int n; begin >= lo + (n = work_tiles<kKeys>(__ldcg(used + q))); ++q) lo += n;
     }
     *out = WorkRange{begin, range_start(total, cluster + 1, n_clusters), p.q0 + q, lo};
     return total;
@@ -336,7 +336,7 @@ __device__ __forceinline__ WorkRange uniform_range(const WorkRange& w) {
     return WorkRange{__shfl_sync(0xffffffffu, w.begin, 0), __shfl_sync(0xffffffffu, w.end, 0), __shfl_sync(0xffffffffu, w.q, 0),
                      __shfl_sync(0xffffffffu, w.lo, 0)};
 }
-template <int kMul> struct TileIter {
+template <int kMul, int kKeys = kWorkTileKeys> struct TileIter {
     const int* used;
     int every_slot;               // KParams::every_slot
     int q, q_last, lo, hi, pos, end;
@@ -350,8 +350,8 @@ template <int kMul> struct TileIter {
     __device__ __forceinline__ int slots(int query) const { return every_slot ? every_slot : __ldcg(used + query); }
     __device__ __forceinline__ void open_query() {
         n_cur = n_next;
-        hi = lo + work_tiles(n_cur) * kMul;
-        stop = kMul > 1 ? lo + (n_cur + kWorkTileKeys / kMul - 1) / (kWorkTileKeys / kMul) : hi;
+        hi = lo + work_tiles<kKeys>(n_cur) * kMul;
+        stop = kMul > 1 ? lo + work_tiles<kKeys / kMul>(n_cur) : hi;
         n_next = slots(min(q + 1, q_last - 1));
     }
     __device__ __forceinline__ bool more() const { return pos < end; }
@@ -1559,7 +1559,11 @@ template <int HP> struct Cfg {
 // kStaged: instead of adding a slot's [576] contribution into dKV with fp32 reductions (whose order, and therefore
 // rounding, changes from run to run), write it to the slot's own row of a staging buffer; smla_dkv_segment_sum_kernel
 // then adds the rows that belong to one kv row in a fixed order.
-template <int HP, bool kStaged = false>
+// kFine: ranges of 128-key tiles, what a cluster takes its time for, instead of 256-key ones, of which a query's last may be half empty: in
+// six documents of 99 - 357 tokens some clusters took 157000 cycles and some 300000 (the kernel 203 -> 160 us; not so the call, whose dQ
+// CTAs had filled the SMs that became free), and few queries go to twice as many clusters: one query x 128 heads x top-k 2048 36.5 -> 34.1
+// us a call, 3 x 64 x 1000 27.3 -> 25.7.  Queries of one 128-key tile at most keep the other form: 64 queries x 16 heads x 64 19.4, 19.6 so.
+template <int HP, bool kStaged = false, bool kFine = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(dp::kThreads, 1)
 smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                      const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_ds, const KParams p) {
@@ -1612,14 +1616,15 @@ smla_dkv_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // are in place.  S, dS and a cleared dKV are not, before that kernel has ended: the first S / dS load waits for that, and no
     // reduction can be issued before UMMAs on what it has loaded.
     if (!p.early_start) pdl_wait();
-    find_range<kThreads>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + C::kOffIdx), range_s);    // (index buffers: not in use yet)
+    constexpr int kRangeKeys = kFine ? kTileKeys : kWorkTileKeys;
+    find_range<kThreads, kRangeKeys>(p, blockIdx.x >> 1, gridDim.x >> 1, reinterpret_cast<int*>(smem + C::kOffIdx), range_s);    // (index buffers: not in use yet)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();          // barriers of both CTAs are initialised before anyone signals across
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const WorkRange range = uniform_range(*range_s);
-    using Iter = TileIter<kWorkTileKeys / kTileKeys>;    // up to two tiles per work tile
+    using Iter = TileIter<kRangeKeys / kTileKeys, kRangeKeys>;
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
