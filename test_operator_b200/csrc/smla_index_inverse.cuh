@@ -71,8 +71,8 @@ struct Plan {
 // 26.4 / 24.3*, 257 x 999 on 44000 26.9* / 28.0, 512 x 2048 39.5 / 28.2*, 8192 x 128 on 4096 35.8* / 40.1, 1024 x 2048 41.7 / 37.3*, on
 // 52000 42.7* / 45.2, 2000 x 1000 on 40000 42.2* / 43.3, 4096 x 512 41.7* / 42.8, on 8192 39.1 / 35.0*, 8192 x 256 on 8192 39.1* / 46.2, 2048 x
 // 2048 72.5 / 55.0*, 4096 x 2048 134.8 / 87.9*, on 52000 135.1 / 103.8*, on 8192 129.4 / 78.8*, 8192 x 2048 on 16384 254 / 195*.
-// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 152, on 8192
-// 129 / 177; every slot the same row 138 / 275.  The slots a top-k selects are distinct, and nothing known before the launch tells.
+// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 153, on 8192
+// 129 / 178; every slot the same row 138 / 257.  The slots a top-k selects are distinct, and nothing known before the launch tells.
 inline bool direct_form(int32_t s_q, int32_t topk, int32_t s_kv) {
     const int64_t n = static_cast<int64_t>(s_q) * topk;
     if (n <= kSmallInput || s_kv >= kPlaceRows - 4 || n >= int64_t{1} << (32 - kPosShift)) return false;
@@ -686,11 +686,12 @@ place_kernel(const Source src, const uint32_t* __restrict__ counts, const uint32
             if (lane == 0) sh.none[k * kPlaceWarps + warp] = __popc(none);
             // neighbours with one row set its bit once: a row that fills a query's slots would have them all wait for one word
             const bool again = __shfl_up_sync(0xffffffffu, row[k], 1) == row[k] && lane > 0;
+            const bool third = (__ballot_sync(0xffffffffu, again) << 1 >> lane) & again;      // the one before it is such a one too
             if (valid) {
                 uint32_t old = 1u << ql;
                 if (!again) old &= atomicOr(&word[next[k]], old);
                 if (old) {
-                    atomicOr(&word[next[k]], kRepeated);
+                    if (!third) atomicOr(&word[next[k]], kRepeated);
                     repeated = true;
                 }
             }

@@ -1527,10 +1527,11 @@ __global__ void __maxnreg__(112) smla_fwd_combine_kernel(const KParams p, int n_
 //   read once (half a tile per CTA) instead of once per d-part.
 //
 //   blocks of d   0: [0,256)   1: [256,512)   2: [512,576) (Q^T . dS only: V has 512 columns)
-//   CTA r holds rows [128 r, 128 r + 128) of blocks 0 and 1 as resident Q^T / dO^T chunk pairs.  Block 2 is issued
-//   from the slot pair (3, 4) in both CTAs: slot 4 holds chunk 8 in both, so both compute the same 64 real rows in
-//   lanes 64-127 (lanes 0-63 repeat chunk 3's rows and are dropped); CTA (tile & 1) drains them, which keeps the
-//   reductions of the two CTAs equal over two tiles.
+//   CTA r holds rows [128 r, 128 r + 128) of blocks 0 and 1 as resident Q^T / dO^T chunk pairs.  Block 2 is M = 128 (slot 4 holds
+//   chunk 8 in both CTAs, so both compute the same 64 rows): lanes 0-63 end up with the first 64 keys of the tile, lanes 64-127 with the
+//   others, and each CTA drains one half, in turn.  As one half of an M = 256 UMMA, drained by the CTAs in turn and always from lanes 64-127,
+//   it took twice the tensor work and left two of the four sub-partitions a quarter more reductions than the others: 4096 queries x
+//   top-k 2048 back to back, at the power cap, 4578 -> 4507 us (128 heads), 3720 -> 3677 (64).
 //   warp 0      producer: resident chunks per query; per 128-key tile this CTA's 64 keys of S and dS, two or four stages
 //   warp 1      even CTA: UMMA issuer for the pair; odd CTA: relays "my half landed" to the even CTA's barriers
 //   warps 2-17  drain, two groups of eight on alternate accumulator units (ring of four 128-column units per CTA):
