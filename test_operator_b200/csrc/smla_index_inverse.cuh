@@ -67,12 +67,12 @@ struct Plan {
 
 // Whether the direct form is taken.  What it costs beyond its slots is the counters, three passes over [groups][rows], 0.36 us per 1024
 // rows, and 2 us per batch that a group goes through; the sort costs more per slot from 2 M slots on.  Sort / direct, us, distinct rows
-// (* what the rule takes), 32768 rows unless given: 16 x 2048 slots on 8192 rows 26.7 / 17.8*, 128 x 2048 26.3 / 22.7*, 256 x 2048
-// 26.4 / 24.3*, 257 x 999 on 44000 26.9* / 28.0, 512 x 2048 39.5 / 28.2*, 8192 x 128 on 4096 35.8* / 40.1, 1024 x 2048 41.7 / 37.3*, on
-// 52000 42.7* / 45.2, 2000 x 1000 on 40000 42.2* / 43.3, 4096 x 512 41.7* / 42.8, on 8192 39.1 / 35.0*, 8192 x 256 on 8192 39.1* / 46.2, 2048 x
-// 2048 72.5 / 55.0*, 4096 x 2048 134.8 / 87.9*, on 52000 135.1 / 103.8*, on 8192 129.4 / 78.8*, 8192 x 2048 on 16384 254 / 195*.
-// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 153, on 8192
-// 129 / 178; every slot the same row 138 / 257.  The slots a top-k selects are distinct, and nothing known before the launch tells.
+// (* what the rule takes), 32768 rows unless given: 16 x 2048 slots on 8192 rows 26.7 / 17.4*, 128 x 2048 26.3 / 22.7*, 256 x 2048
+// 26.4 / 24.3*, 257 x 999 on 44000 26.9* / 28.0, 512 x 2048 39.5 / 27.1*, 8192 x 128 on 4096 35.8* / 40.1, 1024 x 2048 41.7 / 36.3*, on
+// 52000 42.7* / 45.2, 2000 x 1000 on 40000 42.2* / 43.3, 4096 x 512 41.7* / 42.8, on 8192 39.1 / 34.8*, 8192 x 256 on 8192 39.1* / 46.2, 2048 x
+// 2048 72.5 / 53.6*, 4096 x 2048 134.8 / 85.9*, on 52000 135.1 / 97.9*, on 8192 129.4 / 77.4*, 8192 x 2048 on 16384 254 / 195*.
+// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 149, on 8192
+// 129 / 175; every slot the same row 138 / 257.  The slots a top-k selects are distinct, and nothing known before the launch tells.
 inline bool direct_form(int32_t s_q, int32_t topk, int32_t s_kv) {
     const int64_t n = static_cast<int64_t>(s_q) * topk;
     if (n <= kSmallInput || s_kv >= kPlaceRows - 4 || n >= int64_t{1} << (32 - kPosShift)) return false;
@@ -466,13 +466,13 @@ row_ptr_kernel(const int32_t* __restrict__ heads, const int32_t* __restrict__ fi
 // query name different rows.  Rows that a query names twice get a flag in their word, and their slots are placed one after the other
 // (place_repeated).  The words start at the rows' positions: group_count_kernel counts every group's slots per row, group_scan_kernel
 // turns these [group][row] counts into positions.
-// What bounds it: place_kernel (61 of 88 us with 8.4 M slots and 32768 rows; the sort: 135) stores four bytes at a time all over `entries`, a
+// What bounds it: place_kernel (61 of 86 us with 8.4 M slots and 32768 rows; the sort: 135) stores four bytes at a time all over `entries`, a
 // sector a cycle and SM (56000 cycles), and its phases between barriers take turns with that.  With 512 threads of sixteen slots 147 us, with one
 // query a batch 91; counting 10, positions 8.
 constexpr int kPlaceWarps = kPlaceThreads / 32;
 constexpr uint32_t kQueryMask = (1u << kQueryBits) - 1u, kRepeated = 1u << kQueryBits;
 constexpr uint32_t kNoRow = 0xffffffffu;
-constexpr int kScanRows = 128, kScanSegs = kPlaceThreads / kScanRows;       // a block of group_scan_kernel: rows x pieces of the groups
+constexpr int kScanThreads = 512, kScanRows = 64, kScanSegs = kScanThreads / kScanRows;      // a block of group_scan_kernel: rows x pieces of the groups
 constexpr int kHeads = 1024;
 constexpr uint32_t kNoNode = 2047;
 static_assert(kPlaceThreads <= kNoNode, "eleven bits");
@@ -490,7 +490,8 @@ struct PlaceShared {
 
 // counts[group][row] of the group's slots; row s_kv: its unused ones.  `entries` is cleared, so that its lines are in the L2, whole, when
 // place_kernel stores four bytes at a time into them: on lines that are not there these stores fetch their sectors (buffers that were
-// not in the L2, 8.4 M slots: 112.8 us without the clearing, 92.4 with it).
+// not in the L2, 8.4 M slots: 112.8 us without the clearing, 92.4 with it; done by group_scan_kernel, whose blocks are few with few rows:
+// on 32768 rows 90.9 against 89.9 us, on 8192 87.9 against 79.9).  Four slots a load: 92.4 -> 89.9, with smaller blocks of group_scan_kernel.
 __global__ void __launch_bounds__(kPlaceThreads, 1)
 group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __restrict__ entries, int s_q, int per_group, int rows_pad) {
     extern __shared__ __align__(16) uint32_t cnt[];
@@ -499,26 +500,52 @@ group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __r
     smla::pdl_trigger();
     __syncthreads();
     const uint32_t q0 = blockIdx.x * per_group, q1 = min(q0 + per_group, static_cast<uint32_t>(s_q));
-    const uint32_t end = q1 * src.topk;
+    const uint32_t begin = q0 * src.topk, end = q1 * src.topk;
     uint32_t none = 0;
-    int next[kPlaceItems];
-    auto load = [&](uint32_t i0) {
-#pragma unroll
-        for (int k = 0; k < kPlaceItems; ++k) next[k] = i0 + k * kPlaceThreads < end ? __ldg(src.indices + i0 + k * kPlaceThreads) : -1;
+    auto count = [&](uint32_t i, int idx) {
+        const uint32_t key = src.key(i, idx);
+        if (key != static_cast<uint32_t>(src.s_kv)) atomicAdd(&cnt[key], 1u);
+        else ++none;
     };
-    load(q0 * src.topk + threadIdx.x);
-    for (uint32_t i0 = q0 * src.topk + threadIdx.x; i0 < end; i0 += kBatch) {
-        int idx[kPlaceItems];
+    // four slots a load from the first 16-byte boundary on; what lies before and behind, one by one
+    const uint32_t head = min(end - begin, static_cast<uint32_t>((16 - (reinterpret_cast<uintptr_t>(src.indices + begin) & 15)) & 15) / 4);
+    const uint32_t body = begin + head, vectors = (end - body) / 4, tail = body + 4 * vectors;
+    const int4* in = reinterpret_cast<const int4*>(src.indices + body);
+    const bool wide = (reinterpret_cast<uintptr_t>(entries + body) & 15) == 0;
+    constexpr int kLoads = kPlaceItems / 2;
+    int4 next[kLoads];
+    auto load = [&](uint32_t v0) {
 #pragma unroll
-        for (int k = 0; k < kPlaceItems; ++k) idx[k] = next[k];
-        load(i0 + kBatch);
+        for (int k = 0; k < kLoads; ++k) next[k] = v0 + k * kPlaceThreads < vectors ? __ldg(in + v0 + k * kPlaceThreads) : make_int4(-1, -1, -1, -1);
+    };
+    load(threadIdx.x);
+    if (threadIdx.x < head) {
+        entries[begin + threadIdx.x] = 0;
+        count(begin + threadIdx.x, __ldg(src.indices + begin + threadIdx.x));
+    }
+    if (tail + threadIdx.x < end) {
+        entries[tail + threadIdx.x] = 0;
+        count(tail + threadIdx.x, __ldg(src.indices + tail + threadIdx.x));
+    }
+    for (uint32_t v0 = threadIdx.x; v0 < vectors; v0 += kLoads * kPlaceThreads) {
+        int4 idx[kLoads];
 #pragma unroll
-        for (int k = 0; k < kPlaceItems; ++k) {
-            const uint32_t i = i0 + k * kPlaceThreads;
-            if (i < end) entries[i] = 0;
-            const uint32_t key = i < end ? src.key(i, idx[k]) : 0u;
-            if (i < end && key != static_cast<uint32_t>(src.s_kv)) atomicAdd(&cnt[key], 1u);
-            else none += i < end;
+        for (int k = 0; k < kLoads; ++k) idx[k] = next[k];
+        load(v0 + kLoads * kPlaceThreads);
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) {
+            const uint32_t v = v0 + k * kPlaceThreads, i = body + 4 * v;
+            if (v >= vectors) continue;
+            if (wide) {
+                *reinterpret_cast<int4*>(entries + i) = make_int4(0, 0, 0, 0);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) entries[i + e] = 0;
+            }
+            count(i, idx[k].x);
+            count(i + 1, idx[k].y);
+            count(i + 2, idx[k].z);
+            count(i + 3, idx[k].w);
         }
     }
     none = __reduce_add_sync(0xffffffffu, none);
@@ -530,7 +557,7 @@ group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __r
 
 // counts[group][row] -> position of the group's first entry of the row, counted from the first entry of the block's rows; totals[block]:
 // entries of the block's rows.  "Row" s_kv, the unused slots, is the last one and so lands behind all others.
-__global__ void __launch_bounds__(kPlaceThreads)
+__global__ void __launch_bounds__(kScanThreads, 2)
 group_scan_kernel(uint32_t* __restrict__ counts, uint32_t* __restrict__ totals, int n_groups, int rows_pad) {
     constexpr int kPer = (kMaxGroups + kScanSegs - 1) / kScanSegs;
     __shared__ uint32_t seg_sum[kScanSegs][kScanRows];

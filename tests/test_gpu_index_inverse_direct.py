@@ -72,3 +72,22 @@ def test_a_workspace_for_the_sort_only_is_enough():
         assert rc == 0
         ref_ptr, ref_entries = index_inverse_ref(idx.cpu().numpy(), s_kv, None)
         assert np.array_equal(row_ptr.cpu().numpy(), ref_ptr) and np.array_equal(entries.cpu().numpy(), ref_entries)
+
+
+@pytest.mark.parametrize("at_in,at_out", [(0, 1), (1, 0), (2, 3), (3, 3)])
+@pytest.mark.parametrize("topk", [1500, 1501])
+def test_buffers_off_a_16_byte_boundary(at_in, at_out, topk):
+    from test_operator_b200 import op
+    lib = op.load_library()
+    s_q, s_kv = 300, 4000
+    flat = torch.randint(-1, s_kv, (s_q * topk + 8,), dtype=torch.int32, device="cuda")
+    idx = flat[at_in:at_in + s_q * topk].view(s_q, topk)
+    out = torch.full((s_q * topk + 8,), -7, dtype=torch.int32, device="cuda")
+    row_ptr = torch.empty(s_kv + 1, dtype=torch.int32, device="cuda")
+    ws = torch.empty(lib.smla_index_inverse_workspace_size(s_q, topk, s_kv), dtype=torch.uint8, device="cuda")
+    assert lib.smla_index_inverse(idx.data_ptr(), s_q, topk, s_kv, op.NO_CAUSAL, row_ptr.data_ptr(), out.data_ptr() + 4 * at_out, ws.data_ptr(),
+                                  ws.numel(), torch.cuda.current_stream().cuda_stream) == 0
+    ref_ptr, ref_entries = index_inverse_ref(idx.cpu().numpy(), s_kv, None)
+    got = out.cpu().numpy()
+    assert np.array_equal(row_ptr.cpu().numpy(), ref_ptr) and np.array_equal(got[at_out:at_out + s_q * topk], ref_entries)
+    assert (got[:at_out] == -7).all() and (got[at_out + s_q * topk:] == -7).all()
