@@ -472,12 +472,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 // The same under a predicate inside one asm block (`row` >= 0), so that a run of them compiles to predicated
 // instructions and not to a chain of branches around each one.
-__device__ __forceinline__ void red_add_f32_if_row(float* addr, float v, int row) {
+__device__ __forceinline__ void red_add_f32_if_row(float* addr, float v, int row, uint64_t policy) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ge.s32 p, %2, 0;\n\t"
-        "@p red.global.add.f32 [%0], %1;\n\t}"
-        ::"l"(addr), "f"(v), "r"(row)
+        "@p red.global.add.L2::cache_hint.f32 [%0], %1, %3;\n\t}"
+        ::"l"(addr), "f"(v), "r"(row), "l"(policy)
         : "memory");
 }
 
