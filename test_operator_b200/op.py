@@ -896,6 +896,7 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
         job = None
         if n_chunks > 1 and torch.get_num_threads() >= _HOST_DELTA_THREADS:
             delta = torch.empty(lse[:s_q].shape, dtype=torch.float32, pin_memory=True)
+            s_comp.synchronize()        # threads follow no stream: what the caller has queued may still be writing O and dO
             job = _host().delta_start(host[3], host[1], delta, _HOST_DELTA_THREADS)
         if job is not None:
             delta_d = torch.empty(delta.shape, dtype=torch.float32, device=dev)
