@@ -843,9 +843,34 @@ def last_launch_count() -> int:
 
 
 _HOST_BLOCK_BYTES = 4 << 20
-# Threads that find Delta on the host, where torch may use that many: 1024 queries x 128 heads on pinned buffers 11.0 ms with O copied, 12.0 with
-# three threads, 10.0 with four, 9.05 with five or six, 9.15 with eight, 9.45 with twelve (they take the host's memory from the copies).
+# Delta on the host: threads, as many as have to be idle, and the bytes of inputs from which on it is tried.  It takes as long as copying O and
+# slows the copies beside it, so it pays in long calls alone.  O copied / Delta found by six threads, ms, three sets of buffers in turn, 16
+# cores: 128 heads x 2048 slots 40 queries 0.74 / 1.37, 305 5.02 / 5.45, 458 6.42 / 6.60, 611 (256 MB) 7.67 / 7.65, 764 9.06 / 8.58, 1027 11.2 /
+# 9.91, 1434 15.2 / 13.2; 64 x 2048 1200 (256 MB) 7.80 / 7.11; 16 x 512 4801 (256 MB) 10.24 / 9.77.  With every core taken by others
+# 1024 queries x 128 heads 11.0 / 17.3.  Threads, the same buffers again: three 12.0, four 10.0, five or six 9.05, eight 9.15, twelve 9.45.
 _HOST_DELTA_THREADS = 6
+_HOST_DELTA_BYTES = 256 << 20
+
+
+def _idle_cores() -> int:
+    """Cores of this machine that no other process runs on at the moment, among those that this one may use; 0 where the system does not
+    say.  This process' own threads are not counted: torch's go on polling for some 10 ms after every operation on the CPU."""
+    try:
+        with open("/proc/loadavg") as f:
+            idle = os.cpu_count() - int(f.read().split()[3].split("/")[0])
+        if idle < _HOST_DELTA_THREADS:
+            idle += sum(_is_running(f"/proc/self/task/{t}/stat") for t in os.listdir("/proc/self/task"))
+        return max(0, min(len(os.sched_getaffinity(0)), idle))
+    except (OSError, AttributeError, IndexError, TypeError, ValueError):
+        return 0
+
+
+def _is_running(stat: str) -> bool:
+    try:
+        with open(stat) as f:
+            return f.read().rpartition(")")[2].split()[0] == "R"
+    except (OSError, IndexError):       # a thread that has ended
+        return False
 
 
 def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] = None,
@@ -856,9 +881,10 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
 
     The query dimension is cut into at most `n_chunks` blocks (of a few MB of inputs at least) and pipelined over three
     streams: block i+1 is copied to `device` while block i runs and the dQ of block i-1 travels back; every block adds into
-    one fp32 dKV on the device, which returns last.  With several blocks Delta is found on the host, by threads that end with the call, and
-    O does not cross PCIe (contiguous inputs, and a torch that may use six threads: `torch.set_num_threads`).  Returns (dQ, dKV) as host tensors (written into
-    `out_dq` / `out_dkv` when given) and synchronises before returning.
+    one fp32 dKV on the device, which returns last.  Inputs that the current stream is still writing are waited for.  In long calls (256 MB
+    of contiguous inputs) Delta is found on the host, by threads that end with the call, and O does not cross PCIe, where six cores are idle
+    and torch may use that many threads (`torch.set_num_threads`).  Returns (dQ, dKV) as host tensors (written into `out_dq` / `out_dkv` when
+    given) and synchronises before returning.
     """
     dev = torch.device(device)
     s_q = q.shape[0]
@@ -880,6 +906,9 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
     with torch.cuda.device(dev):
         s_comp = torch.cuda.current_stream()
         s_in, s_out = torch.cuda.Stream(), torch.cuda.Stream()
+        # O is needed for Delta alone: where idle cores find that faster than O crosses PCIe, O stays where it is.
+        find = (n_chunks > 1 and n_bytes >= _HOST_DELTA_BYTES and torch.get_num_threads() >= _HOST_DELTA_THREADS
+                and host[3].shape == host[1].shape and host[3].is_contiguous() and _idle_cores() >= _HOST_DELTA_THREADS)
         # (as `.to` would make them: a strided input arrives contiguous)
         dev_in = [torch.empty_like(t, device=dev) for t in host]
         kv_d = torch.empty_like(kv, device=dev)
@@ -892,9 +921,8 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
             t.record_stream(s_in)
         for t in (dkv_d, dq_d):
             t.record_stream(s_out)
-        # O is needed for Delta alone: where the host finds that fast enough, O stays where it is.
         job = None
-        if n_chunks > 1 and torch.get_num_threads() >= _HOST_DELTA_THREADS:
+        if find:
             delta = torch.empty(lse[:s_q].shape, dtype=torch.float32, pin_memory=True)
             s_comp.synchronize()        # threads follow no stream: what the caller has queued may still be writing O and dO
             job = _host().delta_start(host[3], host[1], delta, _HOST_DELTA_THREADS)

@@ -30,6 +30,8 @@ def test_host_entry_without_threads_copies_o(monkeypatch):
     given = []
     real = op.mla_bwd
     monkeypatch.setattr(op, "mla_bwd", lambda *a, **k: (given.append("delta" in k), real(*a, **k))[1])
+    monkeypatch.setattr(op, "_HOST_DELTA_BYTES", 0)          # calls of this size copy O, whatever the threads
+    monkeypatch.setattr(op, "_idle_cores", lambda: 64)
     results = []
     for threads in (1, 64):
         monkeypatch.setattr(torch, "get_num_threads", lambda: threads)

@@ -32,19 +32,27 @@ class _Stream:
 
 @pytest.fixture
 def caller(monkeypatch):
-    """The caller's stream; `mla_bwd` only keeps the Delta that it is given."""
+    """The caller's stream of calls that are long enough for Delta on the host; `mla_bwd` only keeps the Delta that it is given."""
     stream = _Stream()
     empty = torch.empty
     monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, **{n: v for n, v in k.items() if n != "pin_memory"}))
     monkeypatch.setattr(torch, "get_num_threads", lambda: 64)
+    monkeypatch.setattr(op, "_HOST_DELTA_BYTES", 0)
+    monkeypatch.setattr(op, "_idle_cores", lambda: 64)
     monkeypatch.setattr(torch.Tensor, "record_stream", lambda *_: None)
     for name, value in (("device", lambda _: contextlib.nullcontext()), ("stream", lambda _: contextlib.nullcontext()),
                         ("Stream", _Stream), ("current_stream", lambda *_: stream)):
         monkeypatch.setattr(torch.cuda, name, value)
     monkeypatch.setattr(op, "_validate", lambda *_: None)
     stream.given = []
-    monkeypatch.setattr(op, "mla_bwd", lambda *a, **k: stream.given.append(k["delta"].clone()))
+    monkeypatch.setattr(op, "mla_bwd", lambda *a, delta=None, **k: stream.given.append(delta if delta is None else delta.clone()))
     return stream
+
+
+def _call(O, dO):
+    rows, heads = O.shape[:2]
+    q, kv = torch.zeros(rows, heads, 576).bfloat16(), torch.zeros(300, 576).bfloat16()
+    op.mla_bwd_host(q, kv, dO, torch.zeros(rows, heads), O, torch.zeros(rows, 100, dtype=torch.int32), device="cpu")
 
 
 def test_delta_is_of_what_the_stream_has_written(caller):
@@ -52,7 +60,25 @@ def test_delta_is_of_what_the_stream_has_written(caller):
     old, new = (torch.full((rows, heads, 512), v).bfloat16() for v in (1.0, 2.0))
     O, dO = old.clone(), old.clone()
     caller.pending += [lambda: O.copy_(new), lambda: dO.copy_(new)]
-    q, kv = torch.zeros(rows, heads, 576).bfloat16(), torch.zeros(300, 576).bfloat16()
-    op.mla_bwd_host(q, kv, dO, torch.zeros(rows, heads), O, torch.zeros(rows, 100, dtype=torch.int32), device="cpu")
+    _call(O, dO)
     got = torch.cat(caller.given)
     assert got.shape == (rows, heads) and bool((got == 4 * 512).all())
+
+
+@pytest.mark.parametrize("what", ["short", "busy", "one thread", "neither"])
+def test_who_finds_delta(caller, monkeypatch, what):
+    """The host where the call is long and cores are idle; O is copied otherwise, as these calls take longer with threads beside them."""
+    O = torch.ones(130, 64, 512).bfloat16()
+    if what == "short":
+        monkeypatch.setattr(op, "_HOST_DELTA_BYTES", 28 << 20)
+    elif what == "busy":
+        monkeypatch.setattr(op, "_idle_cores", lambda: 5)
+    elif what == "one thread":
+        monkeypatch.setattr(torch, "get_num_threads", lambda: 1)
+    _call(O, O)
+    assert [d is None for d in caller.given] == [what != "neither"] * len(caller.given) and len(caller.given) > 1
+
+
+def test_the_limit_and_the_idle_cores():
+    assert op._HOST_DELTA_BYTES >= 256 << 20
+    assert 0 <= op._idle_cores() <= len(op.os.sched_getaffinity(0))
