@@ -703,10 +703,11 @@ int launch_index_inverse_direct(const inv::Source& src, const inv::Plan& pl, con
         return SMLA_ERR_LAUNCH;
     uint32_t* counts = reinterpret_cast<uint32_t*>(ws + l.counts);
     uint32_t* totals = reinterpret_cast<uint32_t*>(ws + l.totals);
-    const int smem = pl.rows_pad * 4, scan_blocks = (pl.rows_pad + inv::kScanRows - 1) / inv::kScanRows;
-    launch(inv::group_count_kernel, pl.groups, inv::kPlaceThreads, smem, st, true, 1, src, counts, entries, s_q, pl.per_group, pl.rows_pad);
+    // place_kernel: so much that an SM takes one block (two on some SMs and none on others, with few rows: 4096 x 2048 on 8192 102 us, 68 so)
+    const int smem = pl.rows_pad * 4, place_smem = std::max(smem, 116 << 10), scan_blocks = (pl.rows_pad + inv::kScanRows - 1) / inv::kScanRows;
+    launch(inv::group_count_kernel, pl.groups, inv::kCountThreads, smem, st, true, 1, src, counts, entries, s_q, pl.per_group, pl.rows_pad);
     launch(inv::group_scan_kernel, scan_blocks, inv::kScanThreads, 0, st, true, 1, counts, totals, pl.groups, pl.rows_pad);
-    launch(inv::place_kernel, pl.groups, inv::kPlaceThreads, smem, st, true, 1, src, counts, totals, row_ptr, entries, s_q, pl.per_group, pl.rows_pad,
+    launch(inv::place_kernel, pl.groups, inv::kPlaceThreads, place_smem, st, true, 1, src, counts, totals, row_ptr, entries, s_q, pl.per_group, pl.rows_pad,
            scan_blocks);
     return cudaGetLastError() == cudaSuccess ? SMLA_OK : SMLA_ERR_LAUNCH;
 }

@@ -46,12 +46,13 @@ constexpr int kRowTile = 1024;                   // rows per block of the row_pt
 constexpr int kMaxLook = 64;
 constexpr int kResidentBlocks = 2 * 148;         // scatter blocks that a B200 runs at once
 
-// Direct form (see there): one block per SM, the counters that fit into its shared memory, slots and queries of a batch at most, and
-// where the position begins in a counter.
+// Direct form (see there): one block per SM, the counters that fit into its shared memory, threads of the counting, threads and slots
+// a thread of the placing.
 constexpr int kMaxGroups = 148;
+constexpr int64_t kMaxDirect = 20 << 20;         // slots
 constexpr int kPlaceRows = 53248;
-constexpr int kPlaceThreads = 1024, kPlaceItems = 8, kBatch = kPlaceThreads * kPlaceItems;
-constexpr int kQueryBits = 6, kPosShift = kQueryBits + 1;
+constexpr int kCountThreads = 1024;
+constexpr int kPlaceThreads = 512, kPlaceItems = 10, kBatch = kPlaceThreads * kPlaceItems;
 
 struct Plan {
     int passes;      // 1..4
@@ -65,21 +66,23 @@ struct Plan {
     int rows_pad;    // s_kv + 1, padded
 };
 
-// Whether the direct form is taken.  What it costs beyond its slots is the counters, three passes over [groups][rows], 0.36 us per 1024
-// rows, and 2 us per batch that a group goes through; the sort costs more per slot from 2 M slots on.  Sort / direct, us, distinct rows
-// (* what the rule takes), 32768 rows unless given: 16 x 2048 slots on 8192 rows 26.7 / 17.4*, 128 x 2048 26.3 / 22.7*, 256 x 2048
-// 26.4 / 24.3*, 257 x 999 on 44000 26.9* / 28.0, 512 x 2048 39.5 / 27.1*, 8192 x 128 on 4096 35.8* / 40.1, 1024 x 2048 41.7 / 36.3*, on
-// 52000 42.7* / 45.2, 2000 x 1000 on 40000 42.2* / 43.3, 4096 x 512 41.7* / 42.8, on 8192 39.1 / 34.8*, 8192 x 256 on 8192 39.1* / 46.2, 2048 x
-// 2048 72.5 / 53.6*, 4096 x 2048 134.8 / 85.9*, on 52000 135.1 / 97.9*, on 8192 129.4 / 77.4*, 8192 x 2048 on 16384 254 / 195*.
-// Where queries name rows more than once it is the slower one: random rows with repetitions, 4096 x 2048 on 32768 134.6 / 149, on 8192
-// 129 / 175; every slot the same row 138 / 257.  The slots a top-k selects are distinct, and nothing known before the launch tells.
+// Whether the direct form is taken: where its time, by the slots of its largest group and the rows, is not above the sort's, by the slots
+// and the rounds of its blocks (units of 0.05 us, without 13.8 us that both have).  So long as `entries` stays in the L2: past that its
+// stores, four bytes at a time, go to memory.  Sort / direct, us, distinct rows (* what the rule takes): 16 x 2048 slots on 8192 rows 23.8 /
+// 16.7*, on 52000 24.1* / 25.6, 256 x 2048 on 16384 24.1 / 17.6*, on 36000 24.8 / 24.5*, on 44000 24.9* / 28.0, 1 x 20000 on 8192 23.7* /
+// 29.5, 300 x 2048 on 32768 29.8 / 25.1*, 512 x 2048 on 52000 41.0 / 35.2*, 8192 x 128 on 4096 36.6 / 19.1*, 1024 x 2048 on 32768 42.4 / 33.8*,
+// on 52000 43.4* / 42.0, 4096 x 512 on 8192 39.1 / 26.4*, 20 x 100000 on 50000 44.5* / 115, 2048 x 2048 on 32768 73.5 / 47.2*, 4096 x 2048
+// 135 / 75.8*, 8192 x 2048 on 16384 255 / 143*, 10000 x 2048 on 32768 314 / 249*, 12000 x 2048 374* / 385, 16000 x 2048 488* / 818.  However
+// often the queries name a row the direct form is the faster one there, too: 4096 x 2048 slots, random rows with repetitions 135 / 75.8, random
+// among 64 rows 139 / 104, all the same 135 / 61.5; 1024 x 2048 on 8192 39.2 / 26.2, 44.7 / 33.7 and 49.5 / 21.2.
 inline bool direct_form(int32_t s_q, int32_t topk, int32_t s_kv) {
     const int64_t n = static_cast<int64_t>(s_q) * topk;
-    if (n <= kSmallInput || s_kv >= kPlaceRows - 4 || n >= int64_t{1} << (32 - kPosShift)) return false;
-    const int64_t per_group = (s_q + kMaxGroups - 1) / kMaxGroups;
-    const int64_t batches = topk > kBatch ? per_group * ((topk + kBatch - 1) / kBatch)
-                                          : (per_group + std::min(kQueryBits, kBatch / topk) - 1) / std::min(kQueryBits, kBatch / topk);
-    return s_kv / 1024 * 9 + 50 * batches <= 412 + 175 * std::max<int64_t>(0, (n >> 20) - 2);      // units of 0.04 us
+    if (n <= kSmallInput || s_kv >= kPlaceRows - 4 || n > kMaxDirect) return false;
+    const int64_t slots = static_cast<int64_t>((s_q + kMaxGroups - 1) / kMaxGroups) * topk;
+    const int64_t sort = n <= kResidentBlocks * kThreads * kItemsMid ? 230
+                         : n < kLargeInput                           ? 300
+                                                                     : 480 + 300 * std::max<int64_t>(0, n - 2 * kLargeInput) / kLargeInput;
+    return slots * 19 / 1024 + 8 * std::max(0, s_kv / 1024 - 16) <= sort;
 }
 
 inline Plan make_plan(int32_t s_q, int32_t topk, int32_t s_kv, bool may_be_direct = true) {
@@ -459,43 +462,33 @@ row_ptr_kernel(const int32_t* __restrict__ heads, const int32_t* __restrict__ fi
 }
 
 // ---- direct form: a counter per kv row in shared memory, no sort ----------------------------------------------------------
-// The queries are cut into groups of consecutive ones, one block each.  place_kernel goes through its group in batches of up to six
-// queries.  A row's word in shared memory holds the position in `entries` of the row's next slot and one bit per query of the
-// batch: every slot sets its query's bit in its row's word, in any order, and behind a barrier finds its position as the word's
-// position plus the bits of the queries before its own.  So what order the atomics take does not matter, as long as the slots of one
-// query name different rows.  Rows that a query names twice get a flag in their word, and their slots are placed one after the other
-// (place_repeated).  The words start at the rows' positions: group_count_kernel counts every group's slots per row, group_scan_kernel
-// turns these [group][row] counts into positions.
-// What bounds it: place_kernel (61 of 86 us with 8.4 M slots and 32768 rows; the sort: 135) stores four bytes at a time all over `entries`, a
-// sector a cycle and SM (56000 cycles), and its phases between barriers take turns with that.  With 512 threads of sixteen slots 147 us, with one
-// query a batch 91; counting 10, positions 8.
-constexpr int kPlaceWarps = kPlaceThreads / 32;
-constexpr uint32_t kQueryMask = (1u << kQueryBits) - 1u, kRepeated = 1u << kQueryBits;
-constexpr uint32_t kNoRow = 0xffffffffu;
+// The queries are cut into groups of consecutive ones, one block each.  A row's word in shared memory holds the position in `entries` of
+// the row's next slot in the group; slots without a valid row have a word of their own, behind the rows'.  place_kernel goes through its
+// group's slots in batches, each warp through its piece of a batch.  The lanes of a warp that name the same row find each other by
+// marks in shared memory, the first of them takes positions for all of them by adding their number to the row's word, and the warps do
+// this one after the other, in the order of their pieces (a named barrier hands the turn on).  So the order holds whichever rows the
+// slots name and however often, and nothing but these additions is in turn: loads, marks and stores of other warps go on meanwhile.  The
+// words start at the rows' positions: group_count_kernel counts every group's slots per row, group_scan_kernel turns these [group][row]
+// counts into positions.
+// What bounds it: place_kernel (three quarters of 75.8 us with 8.4 M slots and 32768 rows; the sort: 135), its turns, and its stores of four bytes
+// all over `entries`, a sector each: where all slots name one row and the stores are whole lines 61.5.  Pieces of 512 slots 77.1, of 384
+// 74.5, of 256 76.8; where a group has 4096 slots 24.3, 23.5, 22.7 (these of 320: 75.7 and 23.2).  A bit per query in the row's word, a barrier
+// between phases, and slots that repeat a row placed one after the other: 87, with random rows 151, with two rows 475.  Lanes of a row found
+// by sixteen ballots 98, by match.any 98; additions under a predicate, not sent nowhere, 122: the warp waits for each.
+constexpr int kPlaceWarps = kPlaceThreads / 32, kPiece = kBatch / kPlaceWarps;
+static_assert(kPlaceWarps <= 16, "as many warps as named barriers");
+constexpr int kMarks = 512;
 constexpr int kScanThreads = 512, kScanRows = 64, kScanSegs = kScanThreads / kScanRows;      // a block of group_scan_kernel: rows x pieces of the groups
-constexpr int kHeads = 1024;
-constexpr uint32_t kNoNode = 2047;
-static_assert(kPlaceThreads <= kNoNode, "eleven bits");
-
-struct PlaceShared {
-    uint32_t none[kPlaceItems * kPlaceWarps];  // per step of 32 slots: unused ones, then the position of the first of them
-    uint32_t none_at;                          // position of the group's next unused slot
-    uint32_t items;                            // place_repeated: which items have a slot of a repeated row
-    // place_repeated: lists, by row modulo kHeads, of nodes; a node stands for the lanes of a warp that name the same row
-    uint32_t head[kHeads];
-    uint32_t node[kPlaceThreads];              // row, next node (kNoNode: none), slots less one: 16, 11, 5 bits
-    uint32_t warp_sums[32];
-    uint32_t total;
-};
 
 // counts[group][row] of the group's slots; row s_kv: its unused ones.  `entries` is cleared, so that its lines are in the L2, whole, when
-// place_kernel stores four bytes at a time into them: on lines that are not there these stores fetch their sectors (buffers that were
-// not in the L2, 8.4 M slots: 112.8 us without the clearing, 92.4 with it; done by group_scan_kernel, whose blocks are few with few rows:
-// on 32768 rows 90.9 against 89.9 us, on 8192 87.9 against 79.9).  Four slots a load: 92.4 -> 89.9, with smaller blocks of group_scan_kernel.
-__global__ void __launch_bounds__(kPlaceThreads, 1)
+// place_kernel stores four bytes at a time into them: on lines that are not there these stores fetch their sectors (8.4 M slots, buffers that
+// change from call to call: 81.2 us without the clearing, 79.3 with it; with an L2 full of other data 109.6 and 87.0; done by
+// group_scan_kernel, whose blocks are few with few rows, 1 us more on 32768 rows and 8 on 8192).  Four slots a load: 2.5 us less, with smaller
+// blocks of group_scan_kernel.
+__global__ void __launch_bounds__(kCountThreads, 1)
 group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __restrict__ entries, int s_q, int per_group, int rows_pad) {
     extern __shared__ __align__(16) uint32_t cnt[];
-    for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < rows_pad / 4; i += kCountThreads) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
     smla::pdl_wait();
     smla::pdl_trigger();
     __syncthreads();
@@ -512,11 +505,11 @@ group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __r
     const uint32_t body = begin + head, vectors = (end - body) / 4, tail = body + 4 * vectors;
     const int4* in = reinterpret_cast<const int4*>(src.indices + body);
     const bool wide = (reinterpret_cast<uintptr_t>(entries + body) & 15) == 0;
-    constexpr int kLoads = kPlaceItems / 2;
+    constexpr int kLoads = 4;
     int4 next[kLoads];
     auto load = [&](uint32_t v0) {
 #pragma unroll
-        for (int k = 0; k < kLoads; ++k) next[k] = v0 + k * kPlaceThreads < vectors ? __ldg(in + v0 + k * kPlaceThreads) : make_int4(-1, -1, -1, -1);
+        for (int k = 0; k < kLoads; ++k) next[k] = v0 + k * kCountThreads < vectors ? __ldg(in + v0 + k * kCountThreads) : make_int4(-1, -1, -1, -1);
     };
     load(threadIdx.x);
     if (threadIdx.x < head) {
@@ -527,14 +520,14 @@ group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __r
         entries[tail + threadIdx.x] = 0;
         count(tail + threadIdx.x, __ldg(src.indices + tail + threadIdx.x));
     }
-    for (uint32_t v0 = threadIdx.x; v0 < vectors; v0 += kLoads * kPlaceThreads) {
+    for (uint32_t v0 = threadIdx.x; v0 < vectors; v0 += kLoads * kCountThreads) {
         int4 idx[kLoads];
 #pragma unroll
         for (int k = 0; k < kLoads; ++k) idx[k] = next[k];
-        load(v0 + kLoads * kPlaceThreads);
+        load(v0 + kLoads * kCountThreads);
 #pragma unroll
         for (int k = 0; k < kLoads; ++k) {
-            const uint32_t v = v0 + k * kPlaceThreads, i = body + 4 * v;
+            const uint32_t v = v0 + k * kCountThreads, i = body + 4 * v;
             if (v >= vectors) continue;
             if (wide) {
                 *reinterpret_cast<int4*>(entries + i) = make_int4(0, 0, 0, 0);
@@ -552,7 +545,7 @@ group_count_kernel(const Source src, uint32_t* __restrict__ counts, int32_t* __r
     if ((threadIdx.x & 31) == 0 && none) atomicAdd(&cnt[src.s_kv], none);
     __syncthreads();
     uint4* out = reinterpret_cast<uint4*>(counts + static_cast<size_t>(blockIdx.x) * rows_pad);
-    for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) out[i] = reinterpret_cast<uint4*>(cnt)[i];
+    for (int i = threadIdx.x; i < rows_pad / 4; i += kCountThreads) out[i] = reinterpret_cast<uint4*>(cnt)[i];
 }
 
 // counts[group][row] -> position of the group's first entry of the row, counted from the first entry of the block's rows; totals[block]:
@@ -595,185 +588,85 @@ group_scan_kernel(uint32_t* __restrict__ counts, uint32_t* __restrict__ totals, 
     if (threadIdx.x == 0) totals[blockIdx.x] = total;
 }
 
-// Slots of rows that some query of the batch names more than once: 1024 at a time (an item of every thread), in flat order.  A slot's
-// position is its row's, plus the slots of the row in the warps before and in the lanes before; a row has at most one node a warp, so
-// the walk is short however many slots repeat it.  row: as in place_kernel, kNoRow for all other slots.
-__device__ __noinline__ void place_repeated(const uint32_t (&row)[kPlaceItems], uint32_t begin, uint32_t* word, PlaceShared& sh,
-                                            int32_t* __restrict__ entries) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t below = (1u << lane) - 1u;
-    uint32_t mine = 0;
-#pragma unroll
-    for (int k = 0; k < kPlaceItems; ++k) mine |= static_cast<uint32_t>(row[k] != kNoRow) << k;
-    mine = __reduce_or_sync(0xffffffffu, mine);
-    if (lane == 0 && mine) atomicOr(&sh.items, mine);
-    __syncthreads();
-    const uint32_t items = sh.items;
-#pragma unroll
-    for (int k = 0; k < kPlaceItems; ++k) {
-        if (!((items >> k) & 1u)) continue;              // (the same in the whole block)
-        const bool member = row[k] != kNoRow;
-        const uint32_t r = row[k] & 0xffffu;
-        uint32_t peers = __ballot_sync(0xffffffffu, member);
-        for (uint32_t rest = peers; rest;) {             // a step per row (`match.any` takes a warp at a time, some 64 cycles each)
-            const uint32_t lead = __shfl_sync(0xffffffffu, r, __ffs(rest) - 1);
-            const uint32_t same = __ballot_sync(0xffffffffu, member && r == lead);
-            if ((same >> lane) & 1u) peers = same;
-            rest &= ~same;
-        }
-        const bool first = member && (peers & below) == 0;
-        if (first) {
-            sh.node[threadIdx.x] = r | atomicExch(&sh.head[r % kHeads], threadIdx.x) << 16 | (__popc(peers) - 1) << 27;
-        }
-        __syncthreads();
-        uint32_t before = 0, all = 0, pos = 0;
-        if (member) {
-            for (uint32_t at = sh.head[r % kHeads]; at != kNoNode;) {
-                const uint32_t node = sh.node[at], size = (node & 0xffffu) == r ? (node >> 27) + 1 : 0u;
-                all += size;
-                if (at / 32 < threadIdx.x / 32) before += size;
-                at = node >> 16 & 2047u;
-            }
-            pos = word[r] >> kPosShift;
-            entries[pos + before + __popc(peers & below)] = static_cast<int32_t>(begin + k * kPlaceThreads + threadIdx.x);
-        }
-        __syncthreads();
-        if (first) {
-            sh.head[r % kHeads] = kNoNode;
-            if (before == 0) word[r] = (pos + all) << kPosShift;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) sh.items = 0;
-    __syncthreads();
-}
+// The turn: a barrier for the warp that gives it and the one that takes it, with the taker's number.  What the giver has done in shared
+// memory is there for the taker.
+__device__ __forceinline__ void take_turn(int warp) { asm volatile("bar.sync %0, 64;" ::"r"(warp) : "memory"); }
+__device__ __forceinline__ void give_turn(int warp) { asm volatile("bar.arrive %0, 64;" ::"r"(warp) : "memory"); }
 
 __global__ void __launch_bounds__(kPlaceThreads, 1)
 place_kernel(const Source src, const uint32_t* __restrict__ counts, const uint32_t* __restrict__ totals, int32_t* __restrict__ row_ptr,
              int32_t* __restrict__ entries, int s_q, int per_group, int rows_pad, int n_scan_blocks) {
     extern __shared__ __align__(16) uint32_t word[];
-    __shared__ PlaceShared sh;
-    __shared__ uint32_t base[kPlaceRows / kScanRows + 1];
+    static_assert(kPlaceRows / kScanRows + 1 <= 2 * kPlaceThreads, "two a thread");
+    __shared__ uint32_t base[2 * kPlaceThreads], warp_sums[32], total, nowhere[32];
+    __shared__ uint8_t marks[kPlaceWarps][kMarks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
-    static_assert(kPlaceRows / kScanRows + 1 <= kPlaceThreads && kHeads <= kPlaceThreads, "one a thread");
-    sh.head[threadIdx.x] = kNoNode;
-    if (threadIdx.x == 0) sh.items = 0;
-    // batches: as many whole queries as there are bits and slots, or a piece of one query
     const uint32_t q0 = blockIdx.x * per_group, q1 = min(q0 + per_group, static_cast<uint32_t>(s_q));
-    const uint32_t end = q1 * src.topk;
-    const uint32_t pieces = (src.topk + kBatch - 1) / kBatch;                // of a query
-    const uint32_t n_q = pieces > 1 ? 1u : min(static_cast<uint32_t>(kQueryBits), kBatch / src.topk);
-    const float inv_topk = 1.f / static_cast<float>(src.topk);
-    struct Batch { uint32_t q, begin, end; };
-    auto batch_at = [&](uint32_t b) {
-        const uint32_t q = q0 + b / pieces * n_q, begin = q * src.topk + b % pieces * kBatch;
-        return Batch{q, begin, min(min(begin + kBatch, (q + n_q) * src.topk), end)};
-    };
+    const uint32_t begin = q0 * src.topk, end = q1 * src.topk;
     smla::pdl_wait();
     smla::pdl_trigger();
-    int next[kPlaceItems];
-    auto load = [&](const Batch& t) {
+    int next[kPlaceItems];                       // the next piece's slots
+    auto load = [&](uint32_t first) {
 #pragma unroll
-        for (int k = 0; k < kPlaceItems; ++k) {
-            const uint32_t i = t.begin + k * kPlaceThreads + threadIdx.x;
-            next[k] = i < t.end ? __ldg(src.indices + i) : -1;
-        }
+        for (int k = 0; k < kPlaceItems; ++k) next[k] = first + 32 * k < end ? __ldg(src.indices + first + 32 * k) : -1;
     };
-    const uint32_t n_batches = (q1 - q0 + n_q - 1) / n_q * pieces;
-    Batch t = batch_at(0);
-    load(t);
-    const uint32_t at = block_exclusive_scan(static_cast<int>(threadIdx.x) < n_scan_blocks ? totals[threadIdx.x] : 0u, sh.warp_sums, &sh.total);
-    if (static_cast<int>(threadIdx.x) < n_scan_blocks) base[threadIdx.x] = at;
+    uint32_t first = begin + warp * kPiece + lane;
+    load(first);
+    const int i0 = 2 * threadIdx.x, i1 = i0 + 1;
+    const uint32_t t0 = i0 < n_scan_blocks ? totals[i0] : 0u, t1 = i1 < n_scan_blocks ? totals[i1] : 0u;
+    base[i0] = block_exclusive_scan(t0 + t1, warp_sums, &total);
+    base[i1] = base[i0] + t0;
     __syncthreads();
     const uint4* in = reinterpret_cast<const uint4*>(counts + static_cast<size_t>(blockIdx.x) * rows_pad);
-#pragma unroll 4
+#pragma unroll 8
     for (int i = threadIdx.x; i < rows_pad / 4; i += kPlaceThreads) {
         const uint4 v = __ldcg(in + i);
         const uint32_t b = base[i / (kScanRows / 4)];
-        reinterpret_cast<uint4*>(word)[i] = make_uint4((v.x + b) << kPosShift, (v.y + b) << kPosShift, (v.z + b) << kPosShift, (v.w + b) << kPosShift);
+        reinterpret_cast<uint4*>(word)[i] = make_uint4(v.x + b, v.y + b, v.z + b, v.w + b);
     }
     // row_ptr: where group 0's entries of the row begin; every block writes its share
     for (int r = blockIdx.x * kPlaceThreads + threadIdx.x; r <= src.s_kv; r += gridDim.x * kPlaceThreads)
         row_ptr[r] = static_cast<int32_t>(__ldcg(counts + r) + base[r / kScanRows]);
-    if (threadIdx.x == 0) sh.none_at = __ldcg(counts + static_cast<size_t>(blockIdx.x) * rows_pad + src.s_kv) + base[src.s_kv / kScanRows];
     __syncthreads();
-    for (uint32_t b = 0; b < n_batches; ++b) {
-        const Batch cur = t;
-        uint32_t row[kPlaceItems];                               // with the query's number in the batch above it; kNoRow: no valid slot
-        bool repeated = false;
+    // (a warp's piece has the number of its turn)
+    const uint32_t n_turns = (end - begin + kPiece - 1) / kPiece;
+    for (uint32_t turn = warp; turn < n_turns; turn += kPlaceWarps, first += kBatch) {
+        uint32_t who[kPlaceItems];               // its first lane, the lanes of the row before this one, all of them: 8 bits each; 0: no slot
+        uint32_t* at[kPlaceItems];
 #pragma unroll
         for (int k = 0; k < kPlaceItems; ++k) {
-            const uint32_t j = k * kPlaceThreads + threadIdx.x;
-            // (j + 1/2) / topk is at least 1 / (2 topk) away from every whole number, 6e-5 for a batch of more than one query
-            const uint32_t ql = pieces > 1 ? 0u : static_cast<uint32_t>((static_cast<float>(j) + 0.5f) * inv_topk);
-            const bool valid = next[k] >= 0 && next[k] < src.s_kv && (!src.causal || next[k] <= src.q_start + static_cast<int>(cur.q + ql));
-            row[k] = valid ? static_cast<uint32_t>(next[k]) | ql << 16 : kNoRow;
-            const uint32_t none = __ballot_sync(0xffffffffu, !valid && cur.begin + j < cur.end);
-            if (lane == 0) sh.none[k * kPlaceWarps + warp] = __popc(none);
-            // neighbours with one row set its bit once: a row that fills a query's slots would have them all wait for one word
-            const bool again = __shfl_up_sync(0xffffffffu, row[k], 1) == row[k] && lane > 0;
-            const bool third = (__ballot_sync(0xffffffffu, again) << 1 >> lane) & again;      // the one before it is such a one too
-            if (valid) {
-                uint32_t old = 1u << ql;
-                if (!again) old &= atomicOr(&word[next[k]], old);
-                if (old) {
-                    if (!third) atomicOr(&word[next[k]], kRepeated);
-                    repeated = true;
-                }
-            }
-        }
-        if (b + 1 < n_batches) {
-            t = batch_at(b + 1);
-            load(t);
-        }
-        const bool any_repeated = __syncthreads_or(repeated);
-        if (warp == 0) {                                         // positions of the unused slots: exclusive sum over the steps
-            constexpr int kPer = kPlaceItems * kPlaceWarps / 32;
-            uint32_t c[kPer], sum = 0;
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) sum += c[i] = sh.none[lane * kPer + i];
-            uint32_t incl = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += up;
-            }
-            uint32_t a = sh.none_at + incl - sum;
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                sh.none[lane * kPer + i] = a;
-                a += c[i];
-            }
+            const uint32_t i = first + 32 * k;
+            const bool active = i < end;
+            const uint32_t row = src.key(i, next[k]);
+            // Every lane leaves its number at its row's mark.  Where it finds another's, that lane has the same row, or one of the same mark.
+            uint8_t* mark = &marks[warp][row % kMarks];
+            if (active) *mark = static_cast<uint8_t>(lane);
             __syncwarp();
-            if (lane == 31) sh.none_at = a;
+            uint32_t peers = 1u << lane;
+            for (uint32_t rest = __ballot_sync(0xffffffffu, active && *mark != lane); rest;) {
+                const uint32_t lead = __shfl_sync(0xffffffffu, row, __ffs(rest) - 1);
+                const uint32_t same = __ballot_sync(0xffffffffu, active && row == lead);
+                if (row == lead) peers = same;
+                rest &= ~same;
+            }
+            who[k] = !active ? 0u : (__ffs(peers) - 1) | __popc(peers & below) << 8 | __popc(peers) << 16;
+            at[k] = active && (peers & below) == 0 ? &word[row] : &nowhere[lane];
+            __syncwarp();
         }
-        uint32_t w[kPlaceItems];
-#pragma unroll
-        for (int k = 0; k < kPlaceItems; ++k) w[k] = row[k] != kNoRow ? word[row[k] & 0xffffu] : kRepeated;
+        if (turn + kPlaceWarps < n_turns) load(first + kBatch);
+        uint32_t pos[kPlaceItems];
+        if (turn) take_turn(warp);
 #pragma unroll
         for (int k = 0; k < kPlaceItems; ++k) {
-            if (w[k] & kRepeated) continue;
-            const uint32_t before = w[k] & ((1u << (row[k] >> 16)) - 1u);
-            entries[(w[k] >> kPosShift) + __popc(before)] = static_cast<int32_t>(cur.begin + k * kPlaceThreads + threadIdx.x);
+            pos[k] = atomicAdd(at[k], who[k] >> 16);
+            __syncwarp();                            // (in this order, too)
         }
-        __syncthreads();
+        if (turn + 1 < n_turns) give_turn((warp + 1) % kPlaceWarps);
 #pragma unroll
         for (int k = 0; k < kPlaceItems; ++k) {
-            const uint32_t i = cur.begin + k * kPlaceThreads + threadIdx.x;
-            const bool unused = row[k] == kNoRow && i < cur.end;
-            const uint32_t none = __ballot_sync(0xffffffffu, unused);
-            if (unused) entries[sh.none[k * kPlaceWarps + warp] + __popc(none & below)] = static_cast<int32_t>(i);
-            // the row's last query of the batch moves its position on and clears the bits
-            if (!(w[k] & kRepeated) && (w[k] & kQueryMask) >> (row[k] >> 16) == 1u)
-                word[row[k] & 0xffffu] = ((w[k] >> kPosShift) + __popc(w[k] & kQueryMask)) << kPosShift;
-        }
-        __syncthreads();
-        if (any_repeated) {
-#pragma unroll
-            for (int k = 0; k < kPlaceItems; ++k)
-                if (!(w[k] & kRepeated)) row[k] = kNoRow;
-            place_repeated(row, cur.begin, word, sh, entries);
+            const uint32_t p = __shfl_sync(0xffffffffu, pos[k], who[k] & 31u) + (who[k] >> 8 & 31u);
+            if (who[k]) entries[p] = static_cast<int32_t>(first + 32 * k);
         }
     }
 }

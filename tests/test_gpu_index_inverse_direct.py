@@ -1,5 +1,5 @@
-"""The index inverse without a sort, bit for bit against the oracle: groups of one and of several queries, batches of whole queries, of the
-largest number of them, and of pieces of a query, the largest number of rows, and queries that name rows more than once."""
+"""The index inverse without a sort, bit for bit against the oracle: groups of one and of several queries, queries shorter and longer than a
+batch, the largest number of rows, and queries that name rows more than once."""
 import numpy as np
 import pytest
 import torch
@@ -13,9 +13,9 @@ CASES = [
     (5, 2048, 8192, None),        # a query a group, one unfinished batch
     (148, 1500, 3001, 2000),      # as many groups as there may be
     (149, 1501, 3001, 2000),      # two queries a group, an odd top-k, the last group with one
-    (1040, 1365, 5000, None),     # batches of six queries and a rest
-    (450, 8192, 9000, None),      # a query fills a batch
-    (300, 8193, 9000, 8800),      # two pieces a query
+    (1040, 1365, 5000, None),     # eight queries a group
+    (450, 8192, 9000, None),      # queries of more than a batch
+    (300, 8193, 9000, 8800),      # one slot more
     (700, 2047, 30000, None),
     (4096, 2048, 53243, None),    # the most rows
     (600, 1024, 7, None),         # every query names every row many times
