@@ -20,6 +20,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libsmla_bwd.so")
 
 HOST_SOURCE = os.path.join(CSRC, "smla_host.cpp")
 HOST_HEADER = os.path.join(ROOT, "include", "smla_bwd.h")
+HOST_DELTA = os.path.join(CSRC, "smla_host_delta.h")
 
 SOURCES = ["smla_api.cu"]
 HEADERS = ["sm100_ptx.cuh", "smla_kernels.cuh", "smla_index_inverse.cuh"]
@@ -52,7 +53,7 @@ def host_path() -> str:
     C++ interface and by the structs of the C header, so one that was built for others must not be loaded."""
     import torch
     tag = hashlib.sha256(torch.__version__.encode())
-    for path in (HOST_SOURCE, HOST_HEADER):
+    for path in (HOST_SOURCE, HOST_HEADER, HOST_DELTA):
         with open(path, "rb") as f:
             tag.update(f.read())
     return os.path.join(LIB_DIR, "_smla_host." + tag.hexdigest()[:16] + sysconfig.get_config_var("EXT_SUFFIX"))

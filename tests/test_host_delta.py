@@ -1,4 +1,8 @@
 """Delta = rowsum(O * dO) found on the host: the order of the device's sums, whatever the number of threads and rows."""
+import ctypes
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -44,3 +48,30 @@ def test_other_inputs_are_left_to_the_device(case):
              "negated": torch._neg_view(o)}[case]
     host, job, _ = _job(o, other, 2)
     assert job is None
+
+
+@pytest.mark.parametrize("flags", [[], ["-DSMLA_PLAIN_DELTA"]])
+def test_every_way_the_sum_is_compiled(flags, tmp_path):
+    """With vectors, and as the plain loop that other compilers and processors get."""
+    from test_operator_b200 import build
+    compiler = shutil.which("g++")
+    if compiler is None:
+        pytest.skip("no g++")
+    source, lib = tmp_path / "sum.cpp", tmp_path / "sum.so"
+    source.write_text(f'#include "{build.HOST_DELTA}"\nextern "C" void sums(const uint16_t* o, const uint16_t* g, float* out, int64_t n) '
+                      "{ delta_rows_host(o, g, out, n); }\n")
+    subprocess.run([compiler, "-O2", "-std=c++17", "-shared", "-fPIC", *flags, str(source), "-o", str(lib)], check=True)
+    o, g = (torch.randn(16, 8, 512, generator=torch.Generator().manual_seed(n)).bfloat16() for n in (1, 2))
+    got = torch.empty(16, 8)
+    ctypes.CDLL(str(lib)).sums(*(ctypes.c_void_p(t.data_ptr()) for t in (o, g, got)), ctypes.c_int64(128))
+    host, job, want = _job(o, g, 1)
+    assert host.delta_wait(job, want.numel(), True) and torch.equal(got, want)
+
+
+def test_the_module_is_named_by_the_sum_too(monkeypatch, tmp_path):
+    from test_operator_b200 import build
+    here, other = build.host_path(), tmp_path / "smla_host_delta.h"
+    with open(build.HOST_DELTA) as f:
+        other.write_text(f.read() + "// another one\n")
+    monkeypatch.setattr(build, "HOST_DELTA", str(other))
+    assert build.host_path() != here
