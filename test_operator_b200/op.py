@@ -908,9 +908,12 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
         s_in, s_out = torch.cuda.Stream(), torch.cuda.Stream()
         # O is needed for Delta alone: where idle cores find that faster than O crosses PCIe, O stays where it is.
         find = (n_chunks > 1 and n_bytes >= _HOST_DELTA_BYTES and torch.get_num_threads() >= _HOST_DELTA_THREADS
-                and host[3].shape == host[1].shape and host[3].is_contiguous() and _idle_cores() >= _HOST_DELTA_THREADS)
+                and host[3].dtype == host[1].dtype and host[3].shape == host[1].shape and host[3].is_contiguous()
+                and _idle_cores() >= _HOST_DELTA_THREADS)
         # (as `.to` would make them: a strided input arrives contiguous)
-        dev_in = [torch.empty_like(t, device=dev) for t in host]
+        dev_in = [None if find and k == 3 else torch.empty_like(t, device=dev) for k, t in enumerate(host)]
+        if find:
+            dev_in[3] = dev_in[1]       # stands for O, of its shape: what O holds is not read where Delta is given
         kv_d = torch.empty_like(kv, device=dev)
         if s_q:
             _validate(dev_in[0], kv_d, *dev_in[1:])
@@ -929,6 +932,9 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
         if job is not None:
             delta_d = torch.empty(delta.shape, dtype=torch.float32, device=dev)
             delta_d.record_stream(s_in)
+        elif find:
+            dev_in[3] = torch.empty_like(host[3], device=dev)
+            dev_in[3].record_stream(s_in)
         s_in.wait_stream(s_comp)
         with torch.cuda.stream(s_in):
             kv_d.copy_(kv, non_blocking=True)

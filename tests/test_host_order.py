@@ -44,8 +44,12 @@ def caller(monkeypatch):
                         ("Stream", _Stream), ("current_stream", lambda *_: stream)):
         monkeypatch.setattr(torch.cuda, name, value)
     monkeypatch.setattr(op, "_validate", lambda *_: None)
-    stream.given = []
-    monkeypatch.setattr(op, "mla_bwd", lambda *a, delta=None, **k: stream.given.append(delta if delta is None else delta.clone()))
+    stream.given, stream.args = [], []
+
+    def mla_bwd(*args, delta=None, **_):
+        stream.given.append(delta if delta is None else delta.clone())
+        stream.args.append(args)
+    monkeypatch.setattr(op, "mla_bwd", mla_bwd)
     return stream
 
 
@@ -77,6 +81,20 @@ def test_who_finds_delta(caller, monkeypatch, what):
         monkeypatch.setattr(torch, "get_num_threads", lambda: 1)
     _call(O, O)
     assert [d is None for d in caller.given] == [what != "neither"] * len(caller.given) and len(caller.given) > 1
+
+
+@pytest.mark.parametrize("by", ["host", "device"])
+def test_o_is_on_the_device_only_where_it_is_read(caller, monkeypatch, by):
+    O, dO = (torch.randn(130, 64, 512, generator=torch.Generator().manual_seed(n)).bfloat16() for n in (1, 2))
+    if by == "device":              # no compiled host module
+        monkeypatch.setattr(op, "_host", lambda: op._NoNativeHost)
+    _call(O, dO)
+    given, o, g = caller.given, [a[4] for a in caller.args], [a[2] for a in caller.args]
+    assert torch.equal(torch.cat(g), dO) and [d is None for d in given] == [by == "device"] * len(given)
+    if by == "device":
+        assert torch.equal(torch.cat(o), O)
+    else:
+        assert [t.data_ptr() for t in o] == [t.data_ptr() for t in g]
 
 
 def test_the_limit_and_the_idle_cores():
