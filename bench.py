@@ -593,23 +593,21 @@ def run_ours(args):
     # ---- end to end from pinned host buffers --------------------------------------------------------------
     e2e = None
     if seqs and not query_sharded and stages == op.STAGE_ALL and not args.no_e2e:
-        host = []
-        h2d = d2h = 0
-        for s in seqs:
-            hs = {k: (v.cpu().pin_memory() if torch.is_tensor(v) else v) for k, v in s.items()}
-            host.append(hs)
-            h2d += sum(v.numel() * v.element_size() for v in hs.values() if torch.is_tensor(v))
-            d2h += s["q"].numel() * 2 + s["kv"].numel() * 4
+        host = [{k: (v.cpu().pin_memory() if torch.is_tensor(v) else v) for k, v in s.items()} for s in seqs]
         out_pinned = [(torch.empty(s["q"].shape, dtype=torch.bfloat16).pin_memory(),
                        torch.empty(s["kv"].shape, dtype=torch.float32).pin_memory()) for s in seqs]
         n_e2e = max(1, min(args.steps, 3))
+
+        copied = []                   # bytes (to the device, from it) of every call: O goes over where the host does not find Delta
 
         def e2e_step():
             for hs, (hq, hkv) in zip(host, out_pinned):
                 op.mla_bwd_host(hs["q"], hs["kv"], hs["dO"], hs["lse"], hs["O"], hs["indices"], device=dev,
                                 q_start_index_s=hs["q_start_index_s"], workspace=ws, out_dq=hq, out_dkv=hkv)
+                copied.append(op.last_host_copy_bytes())
 
         e2e_step()
+        copied.clear()
         barrier()
         t0 = time.perf_counter()
         for _ in range(n_e2e):
@@ -617,7 +615,7 @@ def run_ours(args):
         barrier()
         e_ms = 1e3 * (time.perf_counter() - t0) / n_e2e
         te = torch.tensor([e_ms], dtype=torch.float64, device=dev)
-        hb = torch.tensor([h2d, d2h], dtype=torch.int64, device=dev)
+        hb = torch.tensor([sum(c) // n_e2e for c in zip(*copied)], dtype=torch.int64, device=dev)
         if world > 1:
             dist.all_reduce(te, op=dist.ReduceOp.MAX)
             dist.all_reduce(hb)

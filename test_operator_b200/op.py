@@ -843,6 +843,14 @@ def last_launch_count() -> int:
 
 
 _HOST_BLOCK_BYTES = 4 << 20
+_host_copies = threading.local()
+
+
+def last_host_copy_bytes() -> Tuple[int, int]:
+    """Bytes that the last `mla_bwd_host` of this thread copied to the device, and back from it."""
+    return getattr(_host_copies, "of_last_call", (0, 0))
+
+
 # Delta on the host: threads, as many as have to be idle, and the bytes of inputs from which on it is tried.  It takes as long as copying O and
 # slows the copies beside it, so it pays in long calls alone.  O copied / Delta found by six threads, ms, three sets of buffers in turn, 16
 # cores: 128 heads x 2048 slots 40 queries 0.74 / 1.37, 305 5.02 / 5.45, 458 6.42 / 6.60, 611 (256 MB) 7.67 / 7.65, 764 9.06 / 8.58, 1027 11.2 /
@@ -981,4 +989,6 @@ def mla_bwd_host(q, kv, dO, lse, O, indices, device, sm_scale: Optional[float] =
             out_dkv.copy_(dkv_d, non_blocking=True)
         s_out.synchronize()
         s_comp.synchronize()
+    size = lambda *tensors: sum(t.numel() * t.element_size() for t in tensors)  # noqa: E731
+    _host_copies.of_last_call = (size(kv, *host[:3], delta if job is not None else host[3], host[4]), size(out_dq, out_dkv))
     return out_dq, out_dkv

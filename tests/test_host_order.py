@@ -95,6 +95,9 @@ def test_o_is_on_the_device_only_where_it_is_read(caller, monkeypatch, by):
         assert torch.equal(torch.cat(o), O)
     else:
         assert [t.data_ptr() for t in o] == [t.data_ptr() for t in g]
+    rows = 130 * 64
+    of_o = rows * (1024 if by == "device" else 4)       # O, or Delta
+    assert op.last_host_copy_bytes() == (300 * 1152 + rows * (1152 + 1024 + 4) + of_o + 130 * 400, rows * 1152 + 300 * 2304)
 
 
 def test_the_limit_and_the_idle_cores():
