@@ -41,7 +41,7 @@ KERNEL_NAMES = {"recompute": "smla_recompute_pair_kernel", "dkv": "smla_dkv_pair
 # traffic grows in proportion to the number of queries).  They describe the kernels as captured there: a kernel
 # change needs a new capture, and `roofline.traffic_source` names the summary the figure came from.  (recompute: without the
 # 75 MB of dKV that it clears whatever the number of queries.)
-DRAM_BYTES_PER_QUERY_H128_TOPK2048 = {"recompute": 1.408e6, "dkv": 2.251e6, "dq": 0.721e6}
+DRAM_BYTES_PER_QUERY_H128_TOPK2048 = {"recompute": 1.409e6, "dkv": 1.781e6, "dq": 0.742e6}
 TRAFFIC_SOURCE = {"recompute": "profiles/smla_recompute_pair_kernel_head128_296q.txt",
                   "dkv": "profiles/smla_dkv_pair_kernel_head128_296q.txt", "dq": "profiles/smla_dq_kernel_head128_296q.txt"}
 # share of the 5504 FLOPs per slot each kernel carries: recompute = P + dP, dkv = dV + dK, dq = dQ

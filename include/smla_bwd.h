@@ -179,7 +179,9 @@ int smla_bwd_get_workspace_layout(const smla_bwd_params* p, size_t workspace_byt
  *   entries [s_q * topk] i32: flat slot ids q * topk + slot, ascending inside a row (a fixed order: the result is
  *     reproducible bit for bit); behind row_ptr[s_kv] follow the unused slots in ascending flat order.
  * s_q * topk must fit in 31 bits.  q_start_index_s has the meaning it has in the backward's parameter block; SMLA_NO_CAUSAL: no causal bound.
- * `workspace`: device memory, 256-byte aligned, at least smla_index_inverse_workspace_size() bytes (0 = bad shape). */
+ * `workspace`: device memory, 256-byte aligned, smla_index_inverse_workspace_size() bytes (0 = bad shape): the larger of about twelve bytes
+ * a slot (sixteen from 65536 rows on) and four a row, and, below 53244 rows, of four bytes a row for each of up to 148 groups of queries
+ * (31.5 MB at most).  With less, down to the first of the two, the call takes a slower form. */
 size_t smla_index_inverse_workspace_size(int32_t s_q, int32_t topk, int32_t s_kv);
 int smla_index_inverse(const int32_t* indices, int32_t s_q, int32_t topk, int32_t s_kv, int32_t q_start_index_s,
                        int32_t* row_ptr, int32_t* entries, void* workspace, size_t workspace_bytes, void* stream);

@@ -309,7 +309,7 @@ int resident_pairs(K kernel, int threads, int smem_bytes) {
     return n;
 }
 
-// No cluster has more than one tile, whatever the indices are (KParams::every_slot).
+// No cluster has more than one tile of 256 keys, whatever the indices are (KParams::every_slot).
 bool at_most_a_tile_each(int queries, int tiles_per_query, int clusters) {
     return static_cast<long long>(queries) * tiles_per_query <= clusters;
 }
@@ -418,7 +418,8 @@ int launch_chain(const smla_bwd_params* p, const Plan& pl, uint8_t* ws, cudaStre
             // of this pass in CSR order
             launch(smla_dkv_pair_kernel<HP, true>, grid_of(pairs, q_tiles), dp::kThreads, dp::Cfg<HP>::kSmemBytes, s_, pdl, 1, tm_qhp, tm_dohp, tm_s,
                    tm_ds, kp);
-            launch(smla_dkv_segment_sum_kernel, std::min((p->s_kv + kSegThreads / 32 - 1) / (kSegThreads / 32), 2 * kSmCount), kSegThreads, 0, s_, true, 1, det->row_ptr, det->entries, det->staging, p->dKV,
+            const int sum_blocks = std::min((p->s_kv + kSegThreads / 32 - 1) / (kSegThreads / 32), 2 * kSmCount);
+            launch(smla_dkv_segment_sum_kernel, sum_blocks, kSegThreads, 0, s_, true, 1, det->row_ptr, det->entries, det->staging, p->dKV,
                    p->s_kv, p->topk, pl.topk_pad, kp.q0, kp.q0 + kp.nq);
             return;
         }
@@ -923,7 +924,7 @@ int smla_selftest_wait_timeout(void* workspace, int which, long long limit_cycle
 size_t smla_index_inverse_workspace_size(int32_t s_q, int32_t topk, int32_t s_kv) {
     if (!inv_shape_ok(s_q, topk, s_kv)) return 0;
     const int64_t n = static_cast<int64_t>(s_q) * topk;
-    // (never less than twelve bytes a slot, what the documentation promises to be about the size)
+    // the larger of what the two forms take; never less than twelve bytes a slot, about what the sort takes
     size_t total = static_cast<size_t>(n) * 12;
     for (bool direct : {false, true}) total = std::max(total, inv_layout(n, s_kv, inv::make_plan(s_q, topk, s_kv, direct)).total);
     return total + 256;

@@ -283,8 +283,9 @@ __global__ void __launch_bounds__(256) smla_query_meta_kernel(int4* __restrict__
 // tiles over 74 clusters as whole queries would be 56 queries for some and 55 for the others), a few long queries
 // spread over the whole chip, and tiles without a valid slot do not exist.  kMul: tiles of 256 / kMul keys.
 //
-// In a call whose queries have no more tiles than there are clusters no cluster has more than one tile, and the kernels that go by
-// these ranges take as long as one tile takes, whether or not some of the tiles are empty.  There the ranges are cut as if every slot
+// In a call whose queries have no more tiles than there are clusters no cluster has more than one tile (the dKV kernel, which cuts
+// ranges of 128 keys, up to two of its own), and the kernels that go by these ranges take as long as one tile takes, whether or not
+// some of the tiles are empty.  There the ranges are cut as if every slot
 // were in use (every_slot): nothing has to look at the indices first, which saves both directions their prep kernel (own_prep in the
 // backward).  From the next tile on some cluster has two, and an empty tile would cost as much as a full one.
 // The dQ kernel, where a CTA goes through a query's tiles, does work on empty ones.  128 heads, with a prep kernel / so, us:
@@ -1946,7 +1947,7 @@ __global__ void __launch_bounds__(kSegThreads) smla_dkv_segment_sum_kernel(const
 //               the contraction and runs along shared-memory rows).  Heads are the M side so that N can be the 192
 //               columns of the part.  64 heads use M = 64: as fast in cycles as M = 128 with 64 rows to spare, but these
 //               cost power, and long calls run at the power cap: 4096 queries x 64 heads x top-k 2048 back to back 1207 ->
-//               1048 us for the kernel, 6073 -> 5885 for the call; 777 x 64 x 600 402 -> 388.
+//               1048 us for the kernel, 6064 -> 5917 for the call; 777 x 64 x 600 402 -> 388.
 // With few queries a cluster of up to eight CTAs splits the keys of one (query, d-part) and adds up in rank order.
 // =============================================================================================
 namespace dq {

@@ -853,7 +853,7 @@ def last_host_copy_bytes() -> Tuple[int, int]:
 
 # Delta on the host: threads, as many as have to be idle, and the bytes of inputs from which on it is tried.  It takes as long as copying O and
 # slows the copies beside it, so it pays in long calls alone.  O copied / Delta found by six threads, ms, three sets of buffers in turn, 16
-# cores: 128 heads x 2048 slots 40 queries 0.74 / 1.37, 305 5.02 / 5.45, 458 6.42 / 6.60, 611 (256 MB) 7.67 / 7.65, 764 9.06 / 8.58, 1027 11.2 /
+# cores: 40 queries x 128 heads x 512 slots 0.74 / 1.37, 128 x 2048 305 queries 5.02 / 5.45, 458 6.42 / 6.60, 611 (256 MB) 7.67 / 7.65, 764 9.06 / 8.58, 1027 11.2 /
 # 9.91, 1434 15.2 / 13.2; 64 x 2048 1200 (256 MB) 7.80 / 7.11; 16 x 512 4801 (256 MB) 10.24 / 9.77.  With every core taken by others
 # 1024 queries x 128 heads 11.0 / 17.3.  Threads, the same buffers again: three 12.0, four 10.0, five or six 9.05, eight 9.15, twelve 9.45.
 _HOST_DELTA_THREADS = 6

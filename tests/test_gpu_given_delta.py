@@ -2,7 +2,9 @@
 import pytest
 import torch
 
+from oracle.sparse_mla_ref import sparse_mla_bwd_ref
 from test_operator_b200.inputs import Workload, make_sequence
+from tests.metrics import assert_backward_close
 
 pytestmark = pytest.mark.gpu
 
@@ -17,10 +19,12 @@ def test_given_delta(s_q, h_q, topk):
     job = op._host().delta_start(s["O"].cpu(), s["dO"].cpu(), delta, 2)
     assert op._host().delta_wait(job, delta.numel(), True)
     want = op.mla_bwd(*args, q_start_index_s=None)
+    oracle = sparse_mla_bwd_ref(*args, q_start_index_s=None)
     args[4] = torch.full_like(s["O"], float("nan"))          # not read
     got = op.mla_bwd(*args, q_start_index_s=None, delta=delta.cuda(), check_device_status=True)
     assert torch.equal(got[0].view(torch.int16), want[0].view(torch.int16))
     assert (got[1] - want[1]).abs().max().item() <= 1e-5 * want[1].abs().max().item()
+    assert_backward_close(*got, *oracle)
 
 
 def test_host_entry_without_threads_copies_o(monkeypatch):
@@ -38,3 +42,4 @@ def test_host_entry_without_threads_copies_o(monkeypatch):
         results.append(op.mla_bwd_host(*args, device="cuda:0", q_start_index_s=None, n_chunks=4))
     assert given == [False] * 4 + [True] * 4
     assert torch.equal(results[0][0].view(torch.int16), results[1][0].view(torch.int16))
+    assert (results[0][1] - results[1][1]).abs().max().item() <= 1e-5 * results[0][1].abs().max().item()

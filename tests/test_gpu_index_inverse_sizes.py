@@ -1,6 +1,6 @@
 """The index inverse at the edges of its kernels' size ranges, bit for bit against the oracle: the one-block sort, four and
 sixteen entries per thread, 16- and 32-bit keys, rows without slots over more than one block of the row_ptr kernel, all slots
-on one row."""
+on one row.  Which form a shape takes goes by a rule on its slots and rows: `tests/test_gpu_index_inverse_forms.py` checks that with each."""
 import numpy as np
 import pytest
 import torch
